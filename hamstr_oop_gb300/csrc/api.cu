@@ -669,11 +669,10 @@ int hamstr::create_gpu(const hamstr_gpu_params* p, int nCell, int nFace, const i
       d.mx_block = 64;
       d.mx_chunk_chains = mx_solve_chunk_capacity(d.mx_block);
       d.sp_on = 1;   // long periodic chains of the FP32 form by segments (2: long open ones too)
-      // FP32 assembly inside the factorisation pays off on long chains, as
-      // do the hardware pivot divisions (their latency is shorter per row)
+      // FP32 assembly inside the factorisation pays off on long chains
       d.mx_fused = (P.nChain > 0 && P.nRow >= 16 * P.nChain) ? 1 : 0;
       d.face_soft = 1;
-      d.piv_soft = d.mx_fused ? 0 : 1;
+      d.piv_soft = 1;   // sd::rcp: shorter latency than the hardware sequence, and off the FP64 pipe
       g->nsm = nsm;
       // the shortest open chains one per lane where chains are short (the
       // autotuner checks the alternatives)

@@ -113,7 +113,7 @@ template <bool SD>
 __device__ __forceinline__ double lu_wavefront(double w, int base, int e)
 {
    const int k = e >> 2, j = e & 3;
-   const double piv0 = SD ? sd::div(1., __shfl_sync(kLaneMask, w, base)) : 1. / __shfl_sync(kLaneMask, w, base);
+   const double piv0 = SD ? sd::rcp(__shfl_sync(kLaneMask, w, base)) : 1. / __shfl_sync(kLaneMask, w, base);
    {
       const double m = w * piv0;
       if (k == 0 && j >= 1) w = m;
@@ -123,7 +123,7 @@ __device__ __forceinline__ double lu_wavefront(double w, int base, int e)
       const double t = w - L * U;
       if (k >= 1 && j >= 1) w = t;
    }
-   const double piv1 = SD ? sd::div(1., __shfl_sync(kLaneMask, w, base + 5)) : 1. / __shfl_sync(kLaneMask, w, base + 5);
+   const double piv1 = SD ? sd::rcp(__shfl_sync(kLaneMask, w, base + 5)) : 1. / __shfl_sync(kLaneMask, w, base + 5);
    {
       const double m = w * piv1;
       if (k == 1 && j >= 2) w = m;
@@ -133,7 +133,7 @@ __device__ __forceinline__ double lu_wavefront(double w, int base, int e)
       const double t = w - L * U;
       if (k >= 2 && j >= 2) w = t;
    }
-   const double piv2 = SD ? sd::div(1., __shfl_sync(kLaneMask, w, base + 10)) : 1. / __shfl_sync(kLaneMask, w, base + 10);
+   const double piv2 = SD ? sd::rcp(__shfl_sync(kLaneMask, w, base + 10)) : 1. / __shfl_sync(kLaneMask, w, base + 10);
    {
       const double m = w * piv2;
       if (k == 2 && j == 3) w = m;
@@ -143,7 +143,7 @@ __device__ __forceinline__ double lu_wavefront(double w, int base, int e)
       const double t = w - L * U;
       if (k == 3 && j == 3) w = t;
    }
-   const double piv3 = SD ? sd::div(1., __shfl_sync(kLaneMask, w, base + 15)) : 1. / __shfl_sync(kLaneMask, w, base + 15);
+   const double piv3 = SD ? sd::rcp(__shfl_sync(kLaneMask, w, base + 15)) : 1. / __shfl_sync(kLaneMask, w, base + 15);
    if (k == j) w = (k == 0) ? piv0 : (k == 1) ? piv1 : (k == 2) ? piv2 : piv3;
    return w;
 }
@@ -164,7 +164,7 @@ __device__ __forceinline__ double lu_wavefront_rhs(double w, double xc, double x
                                                    double (&df)[4], double (&U)[6])
 {
    const int k = e >> 2, j = e & 3;
-   const double piv0 = SD ? sd::div(1., __shfl_sync(kLaneMask, w, base)) : 1. / __shfl_sync(kLaneMask, w, base);
+   const double piv0 = SD ? sd::rcp(__shfl_sync(kLaneMask, w, base)) : 1. / __shfl_sync(kLaneMask, w, base);
    {
       const double m = w * piv0;
       if (k == 0 && j >= 1) w = m;
@@ -182,7 +182,7 @@ __device__ __forceinline__ double lu_wavefront_rhs(double w, double xc, double x
       U[2] = __shfl_sync(kLaneMask, w, base + 3);
       if (k >= 1 && j >= 1) w = t;
    }
-   const double piv1 = SD ? sd::div(1., __shfl_sync(kLaneMask, w, base + 5)) : 1. / __shfl_sync(kLaneMask, w, base + 5);
+   const double piv1 = SD ? sd::rcp(__shfl_sync(kLaneMask, w, base + 5)) : 1. / __shfl_sync(kLaneMask, w, base + 5);
    {
       const double m = w * piv1;
       if (k == 1 && j >= 2) w = m;
@@ -199,7 +199,7 @@ __device__ __forceinline__ double lu_wavefront_rhs(double w, double xc, double x
       U[4] = __shfl_sync(kLaneMask, w, base + 7);
       if (k >= 2 && j >= 2) w = t;
    }
-   const double piv2 = SD ? sd::div(1., __shfl_sync(kLaneMask, w, base + 10)) : 1. / __shfl_sync(kLaneMask, w, base + 10);
+   const double piv2 = SD ? sd::rcp(__shfl_sync(kLaneMask, w, base + 10)) : 1. / __shfl_sync(kLaneMask, w, base + 10);
    {
       const double m = w * piv2;
       if (k == 2 && j == 3) w = m;
@@ -215,7 +215,7 @@ __device__ __forceinline__ double lu_wavefront_rhs(double w, double xc, double x
       U[5] = Uj;
       if (k == 3 && j == 3) w = t;
    }
-   const double piv3 = SD ? sd::div(1., __shfl_sync(kLaneMask, w, base + 15)) : 1. / __shfl_sync(kLaneMask, w, base + 15);
+   const double piv3 = SD ? sd::rcp(__shfl_sync(kLaneMask, w, base + 15)) : 1. / __shfl_sync(kLaneMask, w, base + 15);
    {
       const double tc = xc * piv3, tf = F ? xf * piv3 : 0.0;
       dc[3] = __shfl_sync(kLaneMask, tc, base + 12 + j);
@@ -530,7 +530,7 @@ __device__ __forceinline__ void solve_line_pair(const double* __restrict__ fac, 
 template <bool SD>
 __device__ __forceinline__ void lu_rows_quad(double (&w)[4], int r, int base)
 {
-   const double piv0 = SD ? sd::div(1., __shfl_sync(kLaneMask, w[0], base)) : 1. / __shfl_sync(kLaneMask, w[0], base);
+   const double piv0 = SD ? sd::rcp(__shfl_sync(kLaneMask, w[0], base)) : 1. / __shfl_sync(kLaneMask, w[0], base);
 #pragma unroll
    for (int j = 1; j < 4; j++) {
       const double m = w[j] * piv0;
@@ -542,7 +542,7 @@ __device__ __forceinline__ void lu_rows_quad(double (&w)[4], int r, int base)
       const double t = w[j] - w[0] * U;
       if (r >= 1) w[j] = t;
    }
-   const double piv1 = SD ? sd::div(1., __shfl_sync(kLaneMask, w[1], base + 1))
+   const double piv1 = SD ? sd::rcp(__shfl_sync(kLaneMask, w[1], base + 1))
                           : 1. / __shfl_sync(kLaneMask, w[1], base + 1);
 #pragma unroll
    for (int j = 2; j < 4; j++) {
@@ -555,7 +555,7 @@ __device__ __forceinline__ void lu_rows_quad(double (&w)[4], int r, int base)
       const double t = w[j] - w[1] * U;
       if (r >= 2) w[j] = t;
    }
-   const double piv2 = SD ? sd::div(1., __shfl_sync(kLaneMask, w[2], base + 2))
+   const double piv2 = SD ? sd::rcp(__shfl_sync(kLaneMask, w[2], base + 2))
                           : 1. / __shfl_sync(kLaneMask, w[2], base + 2);
    {
       const double m = w[3] * piv2;
@@ -566,7 +566,7 @@ __device__ __forceinline__ void lu_rows_quad(double (&w)[4], int r, int base)
       const double t = w[3] - w[2] * U;
       if (r == 3) w[3] = t;
    }
-   const double piv3 = SD ? sd::div(1., __shfl_sync(kLaneMask, w[3], base + 3))
+   const double piv3 = SD ? sd::rcp(__shfl_sync(kLaneMask, w[3], base + 3))
                           : 1. / __shfl_sync(kLaneMask, w[3], base + 3);
    const double pv = (r == 0) ? piv0 : (r == 1) ? piv1 : (r == 2) ? piv2 : piv3;
 #pragma unroll
@@ -727,24 +727,24 @@ __device__ __forceinline__ void solve_line_quad(const double* __restrict__ fac, 
 template <bool SD>
 __device__ __forceinline__ void lu4_thread(double (&w)[16])
 {
-   const double piv0 = SD ? sd::div(1., w[0]) : 1. / w[0];
+   const double piv0 = SD ? sd::rcp(w[0]) : 1. / w[0];
 #pragma unroll
    for (int j = 1; j < 4; j++) w[j] = w[j] * piv0;
 #pragma unroll
    for (int k = 1; k < 4; k++)
 #pragma unroll
       for (int j = 1; j < 4; j++) w[4 * k + j] = w[4 * k + j] - w[4 * k] * w[j];
-   const double piv1 = SD ? sd::div(1., w[5]) : 1. / w[5];
+   const double piv1 = SD ? sd::rcp(w[5]) : 1. / w[5];
 #pragma unroll
    for (int j = 2; j < 4; j++) w[4 + j] = w[4 + j] * piv1;
 #pragma unroll
    for (int k = 2; k < 4; k++)
 #pragma unroll
       for (int j = 2; j < 4; j++) w[4 * k + j] = w[4 * k + j] - w[4 * k + 1] * w[4 + j];
-   const double piv2 = SD ? sd::div(1., w[10]) : 1. / w[10];
+   const double piv2 = SD ? sd::rcp(w[10]) : 1. / w[10];
    w[11] = w[11] * piv2;
    w[15] = w[15] - w[14] * w[11];
-   const double piv3 = SD ? sd::div(1., w[15]) : 1. / w[15];
+   const double piv3 = SD ? sd::rcp(w[15]) : 1. / w[15];
    w[0] = piv0;
    w[5] = piv1;
    w[10] = piv2;

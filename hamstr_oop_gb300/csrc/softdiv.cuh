@@ -11,14 +11,26 @@
 // else (zero, subnormal, infinite or NaN divisor; infinite or NaN
 // dividend; subnormal quotient) falls back to `/`.
 //
-// Method (Moller & Granlund, "Improved division by invariant integers",
-// IEEE Trans. Computers 60(2), 2011): the divisor's 53-bit significand,
-// shifted to a 64-bit word d, gets the reciprocal v = floor((2^128-1)/d)
-// - 2^64 (their Algorithm 2); a 128-by-64-bit division with that
-// reciprocal (their Algorithm 4) then yields the exact integer quotient
-// and remainder of the dividend's significand scaled by 2^54 or 2^55,
-// from which the rounded significand follows.  One reciprocal serves
-// every division by the same divisor.
+// Method: the divisor's 53-bit significand mb (value m = mb/2^52 in [1,2))
+// gets r ~ 2^64/m in one 64-bit word, a few units below the true value or at
+// most one above: an FP32 reciprocal estimate y of m's leading 24 bits, the
+// exact integer residual e = 1 - m y (it fits one signed word) and the first
+// terms of 1/m = y (1 + e + e^2 + ...), the Newton-Raphson series of the
+// reciprocal.  A quotient is then the high word of ma * r, with 10 or 11 bits
+// beyond the 53 kept.  The rounding follows from those bits except where they
+// lie within the error of r of the midpoint (about 1 in 200 quotients); there
+// the sign of the exact remainder at the midpoint decides, one 64-bit
+// product.  A quotient of two 53-bit numbers is never a midpoint itself
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34(1), 1990).
+//
+// What it replaced: a division by the exact word floor((2^128-1)/d) - 2^64 and
+// an exact quotient and remainder (Moller & Granlund, IEEE Trans. Computers
+// 60(2), 2011), about twice the integer instructions.  Measured on 512 x 128
+// half split, WENO, per launch: lin_recon5 189 -> 169 us, recon5 205 -> 183,
+// rhs_face 224 -> 196.  A dependent reciprocal takes 177 cycles (the hardware
+// sequence 354), so the line factorisations use it on every mesh: 128-row
+// loops 420 -> 377 us.
 // ##################################################################
 #ifndef HAMSTR_GPU_SOFTDIV_CUH
 #define HAMSTR_GPU_SOFTDIV_CUH
@@ -66,7 +78,8 @@ __host__ __device__ __forceinline__ double from_bits(uint64_t u)
 #endif
 }
 
-// v = floor((2^128 - 1) / d) - 2^64 for 2^63 <= d < 2^64 (Algorithm 2 of
+// The exact reciprocal word, kept as the check of 64-bit arithmetic that the
+// tests run on the host: v = floor((2^128 - 1) / d) - 2^64 for 2^63 <= d < 2^64 (Algorithm 2 of
 // Moller & Granlund; v0 = floor((2^19 - 3*2^8) / d9) from a correctly
 // rounded FP32 division: the true quotient is never within 1/d9 > 2^-13
 // below an integer, so the floor of the rounded quotient is exact)
@@ -92,32 +105,49 @@ __host__ __device__ __forceinline__ uint64_t reciprocal_word(uint64_t d)
    return v3 - hi2;
 }
 
-// exact floor((u1 * 2^64 + u0) / d) and remainder, u1 < d, v = reciprocal_word(d)
-// (Algorithm 4 of Moller & Granlund)
-__host__ __device__ __forceinline__ uint64_t div_2by1(uint64_t u1, uint64_t u0, uint64_t d, uint64_t v, uint64_t& r)
+// an estimate of 1/m from the leading 24 bits of the significand mb (2^52 <=
+// mb < 2^53, m = mb / 2^52), within 2^-22 of it
+__host__ __device__ __forceinline__ float recip_seed(uint64_t mb)
 {
-   uint64_t q0 = v * u1;
-   uint64_t q1 = mulhi(v, u1);
-   const uint64_t t = q0 + u0;
-   q1 = q1 + u1 + (t < q0 ? 1 : 0);
-   q0 = t;
-   q1 = q1 + 1;
-   r = u0 - q1 * d;
-   if (r > q0) {
-      q1 = q1 - 1;
-      r = r + d;
-   }
-   if (r >= d) {
-      q1 = q1 + 1;
-      r = r - d;
-   }
-   return q1;
+   const uint32_t u = 0x3F800000u | ((uint32_t)(mb >> 29) & 0x7FFFFFu);
+   float y;
+#ifdef __CUDA_ARCH__
+   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(u)));
+#else
+   float f;
+   std::memcpy(&f, &u, 4);
+   y = 1.0f / f;
+#endif
+   return y;
+}
+
+// 2^64 / m as a 64-bit word, from a seed y within 2^-21.6 of 1/m: the result is
+// less than 4 below the true value and less than 1 above it, and below 2^64
+// (for m = 1 every product here is exact up to the last floor).  With
+// Y = y 2^32, E = e 2^84 is exact in one word (|e| < 2^-21), the two terms of
+// the series are floored to 2^-64, and e^3 < 2^-64 is left out.
+__host__ __device__ __forceinline__ uint64_t recip64(uint64_t mb, float y)
+{
+   y = y < 0.5f ? 0.5f : y;
+   y = y > 0.99999994f ? 0.99999994f : y;   // 1 - 2^-24
+#ifdef __CUDA_ARCH__
+   const uint32_t u = __float_as_uint(y);
+#else
+   uint32_t u;
+   std::memcpy(&u, &y, 4);
+#endif
+   const uint32_t Y = (u << 8) | 0x80000000u;
+   const int64_t E = -(int64_t)(mb * (uint64_t)Y);
+   const int32_t Eh = (int32_t)(E >> 32);
+   const int64_t S = (E >> 20) + (((int64_t)Eh * Eh) >> 40);
+   return ((uint64_t)Y << 32) + (uint64_t)((int64_t)(S >> 32) * (int64_t)(uint64_t)Y) +
+          (((uint64_t)Y * (uint32_t)S) >> 32);
 }
 
 // a divisor prepared once for several divisions
 struct Divisor {
    double b;
-   uint64_t d, v;    // significand << 11, its reciprocal word
+   uint64_t mb, r;   // significand, recip64 of it
    int eb;           // biased exponent
    uint64_t sign;
    bool ok;          // normal and finite: the integer path applies
@@ -131,8 +161,8 @@ __host__ __device__ __forceinline__ Divisor divisor(double b)
    D.eb = (int)((B >> 52) & 0x7FF);
    D.sign = B & 0x8000000000000000ull;
    D.ok = D.eb != 0 && D.eb != 0x7FF;
-   D.d = ((B & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << 11;
-   D.v = D.ok ? reciprocal_word(D.d) : 0;
+   D.mb = (B & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+   D.r = recip64(D.mb, recip_seed(D.mb));
    return D;
 }
 
@@ -150,26 +180,45 @@ __host__ __device__ __forceinline__ double div(double a, const Divisor& D)
 {
    const uint64_t A = bits(a);
    const int ea = (int)((A >> 52) & 0x7FF);
-   if (!D.ok || ea == 0x7FF) return div_other(a, D.b);
-   const uint64_t sign = (A & 0x8000000000000000ull) ^ D.sign;
-   if ((A & 0x7FFFFFFFFFFFFFFFull) == 0) return from_bits(sign);   // +-0 / normal
-   if (ea == 0) return div_other(a, D.b);                           // subnormal dividend
    const uint64_t ma = (A & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
-   const uint64_t mb = D.d >> 11;
-   // quotient significand in [1, 2): scale by 2^54 (ma >= mb) or 2^55
-   const int s = ma < mb ? 1 : 0;
+   // quotient significand in [1, 2): s = 1 where ma < mb
+   const int s = ma < D.mb ? 1 : 0;
    const int e = ea - D.eb + 1023 - s;
-   if (e <= 0) return div_other(a, D.b);                            // subnormal or zero quotient
-   uint64_t r;
-   // floor(ma * 2^(54+s) / mb) = floor(ma * 2^(65+s) / d), numerator (ma << (1+s)) * 2^64
-   const uint64_t q = div_2by1(ma << (1 + s), 0, D.d, D.v, r);    // in [2^54, 2^55)
-   uint64_t m = q >> 2;
-   const uint64_t g = (q >> 1) & 1, low = (q & 1) | (r != 0 ? 1 : 0);
-   if (g && (low || (m & 1))) m = m + 1;                            // round to nearest even
-   // m in [2^52, 2^53]; 2^53 carries into the exponent (and to infinity past 2046)
-   const uint64_t out = ((uint64_t)e << 52) + m - 0x10000000000000ull;
-   if (e >= 0x7FF || (out >> 52) >= 0x7FF) return from_bits(sign | 0x7FF0000000000000ull);
-   return from_bits(sign | out);
+   if (!D.ok || ea == 0 || ea == 0x7FF || e <= 0 || e >= 0x7FE) {
+      // zero dividends are exact; subnormal, infinite and NaN operands and
+      // quotients near or past the normal range go to the operator
+      if (D.ok && (A << 1) == 0) return from_bits((A ^ D.sign) & 0x8000000000000000ull);
+      return div_other(a, D.b);
+   }
+   // floor of (ma/mb) 2^63 less an error in (-1, 5); 10 + (1 - s) bits are
+   // beyond the significand
+   const uint64_t H = mulhi(ma << 11, D.r);
+   const int sh = 11 - s;
+   uint64_t q = H >> sh;
+   const uint32_t half = 0x400u >> s, f = (uint32_t)H & (2 * half - 1);
+   bool up = f >= half;
+   if (f - (half - 6) <= 7u) up = (int64_t)((ma << (53 + s)) - D.mb * (2 * q + 1)) > 0;
+   q += up ? 1 : 0;
+   // q in [2^52, 2^53]; 2^53 carries into the exponent
+   return from_bits(((A ^ D.sign) & 0x8000000000000000ull) | (((uint64_t)e << 52) + q - 0x10000000000000ull));
+}
+
+// 1 / b rounded to nearest even, equal to the `/` operator.  One branch: the
+// line solvers wait for each pivot's reciprocal, so the operands that the
+// integer path does not take (zero, subnormal, inf, NaN, a subnormal result)
+// and the words too close to a midpoint (1 in 256) share the operator.
+__host__ __device__ __forceinline__ double rcp(double b)
+{
+   const uint64_t B = bits(b);
+   const int eb = (int)((B >> 52) & 0x7FF);
+   const uint64_t mb = (B & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+   const uint64_t r = recip64(mb, recip_seed(mb));
+   const uint64_t q = (r >> 11) + ((r >> 10) & 1);
+   const uint32_t f = (uint32_t)r & 0x7FFu;
+   const bool rare = (unsigned)(eb - 1) >= 2044u || f - 0x3FAu <= 7u;
+   double y = from_bits((B & 0x8000000000000000ull) | (((uint64_t)(2045 - eb) << 52) + q - 0x10000000000000ull));
+   if (rare) y = div_other(1., b);
+   return y;
 }
 
 __host__ __device__ __forceinline__ double div(double a, double b) { return div(a, divisor(b)); }
