@@ -92,15 +92,14 @@ __global__ void __launch_bounds__(256) adi_assemble_kernel(DeviceState d)
 }
 
 // block-Thomas factorisation of chain ich (its assembled rows in blk)
-// (prog: rows published for a following solve, line_solve.cuh publish_rows)
 template <bool SD>
-__device__ __forceinline__ bool factor_chain(const DeviceState& d, int ich, int lane, int* prog = nullptr)
+__device__ __forceinline__ bool factor_chain(const DeviceState& d, int ich, int lane)
 {
    const int N = d.chain_nrows[ich], row0 = d.chain_row0[ich];
    const bool per = d.chain_periodic[ich] != 0;
    const double* blk = d.blk + 48 * (size_t)row0;
    return factor_line<SD>(blk, blk + 16, blk + 32, 48, N, per, d.fac + (size_t)kFacRec * row0,
-               per ? d.facN + 16 * d.chain_facN[ich] : nullptr, lane, prog);
+               per ? d.facN + 16 * d.chain_facN[ich] : nullptr, lane);
 }
 
 // rows of chain ich for this half-warp's work: 0 once its instance is frozen
@@ -153,15 +152,10 @@ __device__ __forceinline__ int first_job(int* ctr, int ncrit, int off, int lane)
    return take_job(ctr, off, lane);
 }
 
-// one sweep's solve of chain ich: F = r[fcell] (ADI.cpp:116,187), the
-// replay, and the write-back r[scell] = F (ADI.cpp:232-244); FOLLOW: behind
-// its factorisation by another warp of the block (line_solve.cuh)
-template <bool FOLLOW = false>
-__device__ __forceinline__ void solve_chain(const DeviceState& d, int ich, int lane, const int* prog = nullptr,
-                                            bool* ok = nullptr)
+// a chain's right-hand side F = r[fcell] (ADI.cpp:116,187) into its rows of
+// fsc, and the write-back r[scell] = F (ADI.cpp:232-244)
+__device__ __forceinline__ void gather_rhs(const DeviceState& d, int row0, int N, int lane)
 {
-   const int N = d.chain_nrows[ich], row0 = d.chain_row0[ich];
-   const bool per = d.chain_periodic[ich] != 0;
    double* fs = d.fsc + 4 * (size_t)row0;
    for (int r = lane; r < N; r += 32) {
       const int fc = d.row_fcell[row0 + r];
@@ -171,8 +165,10 @@ __device__ __forceinline__ void solve_chain(const DeviceState& d, int ich, int l
       *reinterpret_cast<double2*>(fs + 4 * r + 2) = make_double2(v[2], v[3]);
    }
    __syncwarp();
-   solve_line<FOLLOW>(d.fac + (size_t)kFacRec * row0, per ? d.facN + 16 * d.chain_facN[ich] : nullptr, N, per, fs,
-                      lane, prog, ok);
+}
+__device__ __forceinline__ void scatter_solution(const DeviceState& d, int row0, int N, int lane)
+{
+   const double* fs = d.fsc + 4 * (size_t)row0;
    __syncwarp();
    for (int r = lane; r < N; r += 32) {
       const int sc = d.row_scell[row0 + r];
@@ -181,6 +177,38 @@ __device__ __forceinline__ void solve_chain(const DeviceState& d, int ich, int l
       *reinterpret_cast<double2*>(d.r + 4 * (size_t)sc) = make_double2(v[0], v[1]);
       *reinterpret_cast<double2*>(d.r + 4 * (size_t)sc + 2) = make_double2(v[2], v[3]);
    }
+}
+
+// one sweep's solve of chain ich
+__device__ __forceinline__ void solve_chain(const DeviceState& d, int ich, int lane)
+{
+   const int N = d.chain_nrows[ich], row0 = d.chain_row0[ich];
+   const bool per = d.chain_periodic[ich] != 0;
+   gather_rhs(d, row0, N, lane);
+   solve_line(d.fac + (size_t)kFacRec * row0, per ? d.facN + 16 * d.chain_facN[ich] : nullptr, N, per,
+              d.fsc + 4 * (size_t)row0, lane);
+   scatter_solution(d, row0, N, lane);
+}
+
+// chain ich by two warps of a block (line_solve.cuh): its factorisation, and
+// its fill column with its first sweep's solve behind it
+__device__ __forceinline__ bool factor_chain_team(const DeviceState& d, int ich, int lane, TeamShared* ts, bool* ok)
+{
+   const int N = d.chain_nrows[ich], row0 = d.chain_row0[ich];
+   const bool per = d.chain_periodic[ich] != 0;
+   const double* blk = d.blk + 48 * (size_t)row0;
+   return factor_line_team(blk, blk + 16, blk + 32, 48, N, per, d.fac + (size_t)kFacRec * row0,
+                           per ? d.facN + 16 * d.chain_facN[ich] : nullptr, lane, ts, ok);
+}
+__device__ __forceinline__ void follow_chain_team(const DeviceState& d, int ich, int lane, TeamShared* ts, bool* ok)
+{
+   const int N = d.chain_nrows[ich], row0 = d.chain_row0[ich];
+   const bool per = d.chain_periodic[ich] != 0;
+   gather_rhs(d, row0, N, lane);
+   follow_line_team<true>(d.blk + 48 * (size_t)row0, 48, d.fac + (size_t)kFacRec * row0,
+                          per ? d.facN + 16 * d.chain_facN[ich] : nullptr, N, per, d.fsc + 4 * (size_t)row0, lane, ts,
+                          ok);
+   scatter_solution(d, row0, N, lane);
 }
 
 // the same for two open chains, one per half-warp
@@ -317,16 +345,17 @@ __device__ __forceinline__ void solve_job(const DeviceState& d, int job, int ich
 //
 // A long first job of block b (ncrit != 0, b < |ncrit|) that carries its
 // first sweep's solve (kFusedJob, one chain or a pair) is solved by the
-// block's second warp behind the factorisation of the first (the rows are
-// published in shared memory as their records are stored), instead of by
-// the factoring warp after it: a row's factorisation takes about three
-// times its solve, so the solve adds only its last rows and the back
-// substitution to the job's time.  Beside an outlier (ncrit > 0) that
+// block's second warp behind the factorisation of the first, instead of by
+// the factoring warp after it, so the solve adds only its last rows and the
+// back substitution to the job's time.  One chain goes to the two warps as a
+// team (line_solve.cuh), which also takes the periodic fill column off the
+// factoring warp; of a pair the rows are published as their records are
+// stored.  Beside an outlier (ncrit > 0) that
 // second warp was idle; beside many long jobs it takes queued jobs after.
 template <bool SD>
 __global__ void __launch_bounds__(256, 1) adi_factor_kernel(DeviceState d, int nwarps)
 {
-   __shared__ int prog;   // rows of the block's followed job that are factored
+   __shared__ TeamShared team;   // the block's followed job
    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, b = blockIdx.x;
    const int nj = d.sched_njobs[0], j0 = d.sched_job0[0];
    const int ncrit = d.sched_ncrit[0], nlong = ncrit < 0 ? -ncrit : ncrit;
@@ -338,20 +367,19 @@ __global__ void __launch_bounds__(256, 1) adi_factor_kernel(DeviceState d, int n
          fich = head & ~kFusedJob;
       }
    }
-   if (threadIdx.x == 0) prog = 0;
+   if (fjob >= 0) team_init(&team);
    __syncthreads();
    if (halted(d)) return;
    const int w = b * (blockDim.x >> 5) + wib;
    if (w >= nwarps) return;
    int* ctr = d.sched_ctr;
-   bool bad = false;
+   bool bad = false, ok = true;
    const int off = ncrit ? (int)gridDim.x : 0;
    int k0;
    if (fjob >= 0 && wib == 1) {
-      bool ok = true;
-      if (fich & kPairJob) solve_pair<true>(d, fich & ~kPairJob, d.sched_jobs[fjob + 1], lane, &prog, &ok);
-      else if (!frozen_chain(d, fich)) solve_chain<true>(d, fich, lane, &prog, &ok);
-      if (!ok && lane == 0) atomicOr(d.status, DEV_ERR_WAIT);
+      if (fich & kPairJob) solve_pair<true>(d, fich & ~kPairJob, d.sched_jobs[fjob + 1], lane, &team.prog, &ok);
+      else if (!frozen_chain(d, fich)) follow_chain_team(d, fich, lane, &team, &ok);
+      if (!ok) atomicOr(d.status, DEV_ERR_WAIT);
       if (ncrit > 0) return;
       k0 = take_job(ctr, off, lane);
    } else {
@@ -368,8 +396,8 @@ __global__ void __launch_bounds__(256, 1) adi_factor_kernel(DeviceState d, int n
       const int head = d.sched_jobs[job], ich = head & ~kFusedJob;
       if (job == fjob) {
          // factorisation only, its solve follows in warp 1
-         if (ich & kPairJob) bad |= factor_pair<SD>(d, ich & ~kPairJob, d.sched_jobs[job + 1], lane, &prog);
-         else if (!frozen_chain(d, ich)) bad |= factor_chain<SD>(d, ich, lane, &prog);
+         if (ich & kPairJob) bad |= factor_pair<SD>(d, ich & ~kPairJob, d.sched_jobs[job + 1], lane, &team.prog);
+         else if (!frozen_chain(d, ich)) bad |= factor_chain_team(d, ich, lane, &team, &ok);
       } else if ((head & kFusedJob) && (ich & kPairJob)) {
          bad |= factor_solve_pair<SD>(d, ich & ~kPairJob, d.sched_jobs[job + 1], lane);
       } else {
@@ -383,6 +411,7 @@ __global__ void __launch_bounds__(256, 1) adi_factor_kernel(DeviceState d, int n
       k = __shfl_sync(kLaneMask, kn, 0);
    }
    if (__any_sync(kLaneMask, bad) && lane == 0) atomicOr(d.status, DEV_ERR_PIVOT);
+   if (!ok) atomicOr(d.status, DEV_ERR_WAIT);
 }
 
 

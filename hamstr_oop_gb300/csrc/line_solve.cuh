@@ -31,6 +31,11 @@
 namespace hamstr {
 
 constexpr int kFacRec = 80;
+// Rows of records loaded ahead in the back substitutions and the last-row
+// elimination.  A row there is 500 to 600 cycles of dependent operations and a
+// record load up to about 900 (L2): with one or two rows ahead, as before, the
+// loads set the pace (back substitution 1,000 cycles a row, elimination 890).
+constexpr int kBackAhead = 4;
 constexpr unsigned kLaneMask = 0xffffffffu;
 
 // A factorisation followed by a solving warp of the same block (adi.cu):
@@ -44,7 +49,7 @@ constexpr unsigned kLaneMask = 0xffffffffu;
 // elimination) only guards against a broken schedule: a wait that gives up
 // returns false, the follower waits no more and the caller raises an error
 // word.
-constexpr long kFollowSpin = 1L << 24;
+constexpr long kFollowSpin = 1L << 23;
 
 __device__ __forceinline__ void publish_rows(int* prog, int n, int lane)
 {
@@ -56,8 +61,10 @@ __device__ __forceinline__ void publish_rows(int* prog, int n, int lane)
 __device__ __forceinline__ bool wait_rows(const int* prog, int need)
 {
    long it = 0;
-   while (*(const volatile int*)prog < need)
+   while (*(const volatile int*)prog < need) {
       if (++it > kFollowSpin) return false;
+      __nanosleep(40);   // the factoring warp's shuffles share the pipe with these loads
+   }
    __threadfence_block();
    return true;
 }
@@ -236,19 +243,50 @@ __device__ __forceinline__ void lu_back4(const double (&d)[4], const double (&U)
    x[0] = ((d[0] - U[0] * x[1]) - U[1] * x[2]) - U[2] * x[3];
 }
 
+// Last-row elimination of a periodic line (triSolvers.cpp:967-999): cN is
+// element (k,j) of c_{N-1} at step 0 (both halves), the result element (k,j) of
+// the final last-row block in lanes 16-31; the steps' c_{N-1} go to the records.
+__device__ __forceinline__ double eliminate_last_row(double* __restrict__ fac, int N, double cN, int lane, int* prog)
+{
+   const int h = lane >> 4, e = lane & 15, k = e >> 2, j = e & 3;
+   double bN = (k == j) ? 1.0 : 0.0;
+   double Y[kBackAhead];   // c'(i) (lanes 0-15) and a'(i) (lanes 16-31) of the next rows
+#pragma unroll
+   for (int u = 0; u < kBackAhead; u++)
+      Y[u] = (u < N - 1) ? ldf<true>(&fac[(size_t)kFacRec * u + 32 + 16 * h + e]) : 0.0;
+   for (int i0 = 0; i0 < N - 1; i0 += kBackAhead) {
+#pragma unroll
+      for (int u = 0; u < kBackAhead; u++) {
+         const int i = i0 + u, in = i + kBackAhead;
+         if (i >= N - 1) break;
+         const double Yi = Y[u];
+         Y[u] = (in < N - 1) ? ldf<true>(&fac[(size_t)kFacRec * in + 32 + 16 * h + e]) : 0.0;
+         if (h == 0) fac[(size_t)kFacRec * i + 64 + e] = cN;
+         double acc = h ? bN : 0.0;
+#pragma unroll
+         for (int l = 0; l < 4; l++) {
+            const double c = __shfl_sync(kLaneMask, cN, 16 * h + 4 * k + l);
+            const double y = __shfl_sync(kLaneMask, Yi, 16 * h + 4 * l + j);
+            acc -= c * y;
+         }
+         if (h) bN = acc;
+         cN = __shfl_sync(kLaneMask, acc, e);
+         if (prog && ((i & 7) == 7 || i == N - 2)) publish_rows(prog, N + 1 + i, lane);
+      }
+   }
+   return bN;
+}
+
 // Block-Thomas factorisation of one line of N rows by one warp: blocks
 // A_i = Ab + i*stride, B_i = Bb + i*stride, C_i = Cb + i*stride (row-major
 // 4x4); writes the per-row records `fac` (kFacRec doubles per row) and,
 // periodic, the LU of the final last-row block into facN.  Returns, in the
 // lanes that hold a pivot, whether a stored reciprocal pivot is infinite or
 // NaN (a zero or non-finite pivot; the reference divides by it regardless).
-// With prog, the rows are published as they are stored (publish_rows),
-// and N + 1 once a periodic line's last-row records are.
 template <bool SD = true>
 __device__ __forceinline__ bool factor_line(const double* __restrict__ Ab, const double* __restrict__ Bb,
                                             const double* __restrict__ Cb, size_t stride, int N, bool per,
-                                            double* __restrict__ fac, double* __restrict__ facN, int lane,
-                                            int* prog = nullptr)
+                                            double* __restrict__ fac, double* __restrict__ facN, int lane)
 {
    const int h = lane >> 4, e = lane & 15, k = e >> 2, j = e & 3;
    double A = Ab[e], B = Bb[e], C = Cb[e];
@@ -301,34 +339,15 @@ __device__ __forceinline__ bool factor_line(const double* __restrict__ Ab, const
       }
       Yp = sel4(P, k);
       rec[32 + 16 * h + e] = Yp;
-      if (prog) publish_rows(prog, i + 1, lane);
       A = An;
       B = Bn;
       C = Cn;
    }
    if (!per) return bad;
-   // last-row elimination (triSolvers.cpp:967-999)
-   double cN = __shfl_sync(kLaneMask, Yp, e);
-   double bN = (k == j) ? 1.0 : 0.0;
-   double Y = (N > 1) ? fac[32 + 16 * h + e] : 0.0;
-   for (int i = 0; i < N - 1; i++) {
-      double* rec = fac + (size_t)kFacRec * i;
-      const double Yn = (i + 2 < N) ? rec[kFacRec + 32 + 16 * h + e] : 0.0;
-      if (h == 0) rec[64 + e] = cN;
-      double acc = h ? bN : 0.0;
-#pragma unroll
-      for (int l = 0; l < 4; l++) {
-         const double c = __shfl_sync(kLaneMask, cN, 16 * h + 4 * k + l);
-         const double y = __shfl_sync(kLaneMask, Y, 16 * h + 4 * l + j);
-         acc -= c * y;
-      }
-      if (h) bN = acc;
-      cN = __shfl_sync(kLaneMask, acc, e);
-      Y = Yn;
-   }
+   __syncwarp();
+   const double bN = eliminate_last_row(fac, N, __shfl_sync(kLaneMask, Yp, e), lane, nullptr);
    const double w = lu_wavefront<SD>(__shfl_sync(kLaneMask, bN, 16 + e), 16 * h, e);
    if (h == 0) facN[e] = w;
-   if (prog) publish_rows(prog, N + 1, lane);
    return bad || (h == 0 && k == j && nonfinite(w));
 }
 
@@ -434,35 +453,30 @@ __device__ __forceinline__ void back_line_pair(const double* __restrict__ fac, i
    double xnext[4];
 #pragma unroll
    for (int m = 0; m < 4; m++) xnext[m] = xlast[m];
-   // a row here is a few dependent operations, shorter than a load: rows
-   // ii-1 and ii-2 are in flight while row ii is solved
-   double mv = 0.0, xi = 0.0, mv1 = 0.0, xi1 = 0.0;
-   if (N >= 2) {
-      mv = ldf<FOLLOW>(&fac[(size_t)kFacRec * (N - 2) + 32 + e]);
-      xi = fs[4 * (N - 2) + r];
+   // a row here is a few dependent operations, shorter than a load: the next
+   // kBackAhead rows are in flight while row ii is solved
+   double mv[kBackAhead], xi[kBackAhead];
+#pragma unroll
+   for (int u = 0; u < kBackAhead; u++) {
+      const int ii = N - 2 - u;
+      mv[u] = ii >= 0 ? ldf<FOLLOW>(&fac[(size_t)kFacRec * ii + 32 + e]) : 0.0;
+      xi[u] = ii >= 0 ? fs[4 * ii + r] : 0.0;
    }
-   if (N >= 3) {
-      mv1 = ldf<FOLLOW>(&fac[(size_t)kFacRec * (N - 3) + 32 + e]);
-      xi1 = fs[4 * (N - 3) + r];
-   }
-   for (int t = 0; t <= Nmax - 2; t++) {
-      const int ii = N - 2 - t;
-      double mv2 = 0.0, xi2 = 0.0;
-      if (ii > 1) {
-         mv2 = ldf<FOLLOW>(&fac[(size_t)kFacRec * (ii - 2) + 32 + e]);
-         xi2 = fs[4 * (ii - 2) + r];
+   for (int t0 = 0; t0 <= Nmax - 2; t0 += kBackAhead) {
+#pragma unroll
+      for (int u = 0; u < kBackAhead; u++) {
+         if (t0 + u > Nmax - 2) break;
+         const int ii = N - 2 - t0 - u, in = ii - kBackAhead;
+         const double prod = mv[u] * sel4(xnext, pj);
+         double x = xi[u];
+         mv[u] = in >= 0 ? ldf<FOLLOW>(&fac[(size_t)kFacRec * in + 32 + e]) : 0.0;
+         xi[u] = in >= 0 ? fs[4 * in + r] : 0.0;
+#pragma unroll
+         for (int jj = 0; jj < 4; jj++) x = x - __shfl_sync(kLaneMask, prod, hb + 4 * r + jj);
+#pragma unroll
+         for (int m = 0; m < 4; m++) xnext[m] = __shfl_sync(kLaneMask, x, hb + m);
+         if (e < 4 && ii >= 0) fs[4 * ii + e] = x;
       }
-      const double prod = mv * sel4(xnext, pj);
-      double x = xi;
-#pragma unroll
-      for (int jj = 0; jj < 4; jj++) x = x - __shfl_sync(kLaneMask, prod, hb + 4 * r + jj);
-#pragma unroll
-      for (int m = 0; m < 4; m++) xnext[m] = __shfl_sync(kLaneMask, x, hb + m);
-      if (e < 4 && ii >= 0) fs[4 * ii + e] = x;
-      mv = mv1;
-      xi = xi1;
-      mv1 = mv2;
-      xi1 = xi2;
    }
 }
 
@@ -933,6 +947,98 @@ __device__ __forceinline__ void ld4(const double* __restrict__ p, double (&v)[4]
    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
 
+// The rest of a solve after its forward sweep: a periodic line's last row and
+// the back substitution.  fs holds the forward sweep's rows (written by this
+// warp, a __syncwarp before the call), xprev row N-1's on every lane.  FOLLOW:
+// behind the factorisation by another warp (factor_line_team); a periodic
+// line's last-row records are published as rows N+1 .. 2N-1 and its final LU as
+// row 2N.
+template <bool FOLLOW = false>
+__device__ __forceinline__ void solve_line_tail(const double* __restrict__ fac, const double* __restrict__ facN, int N,
+                                                bool per, double* __restrict__ fs, int lane,
+                                                const double (&xprev)[4], const int* prog = nullptr,
+                                                bool* ok = nullptr)
+{
+   const int e = lane & 15, pj = e & 3, hi = lane >> 4;
+   const int r = lane & 3;
+   if (per) {
+      // f(N-1) -= c_{N-1}^{(i)} f(i), i = 0..N-2 (triSolvers.cpp:991-999);
+      // the products of rows i and i+1 in one instruction (lanes 0-15, 16-31)
+      double fN = sel4(xprev, r);
+      int i = 0;
+      double c = 0.0, f = 0.0;
+      if (FOLLOW && *ok && !wait_rows(prog, N + min(2, N - 1))) *ok = false;
+      if (hi < N - 1) {
+         c = ldf<FOLLOW>(&fac[(size_t)kFacRec * hi + 64 + e]);
+         f = fs[4 * hi + pj];
+      }
+      for (; i < N - 1; i += 2) {
+         const int rn = i + 2 + hi;
+         double cn = 0.0, fn = 0.0;
+         if (FOLLOW && *ok && i + 2 < N - 1 && !wait_rows(prog, N + min(i + 4, N - 1))) *ok = false;
+         if (rn < N - 1) {
+            cn = ldf<FOLLOW>(&fac[(size_t)kFacRec * rn + 64 + e]);
+            fn = fs[4 * rn + pj];
+         }
+         const double p = c * f;
+#pragma unroll
+         for (int jj = 0; jj < 4; jj++) fN = fN - __shfl_sync(kLaneMask, p, 4 * r + jj);
+         if (i + 1 < N - 1) {
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++) fN = fN - __shfl_sync(kLaneMask, p, 16 + 4 * r + jj);
+         }
+         c = cn;
+         f = fn;
+      }
+      if (FOLLOW && *ok && !wait_rows(prog, 2 * N)) *ok = false;
+      double luN[4], xn[4];
+#pragma unroll
+      for (int cc = 0; cc < 4; cc++) luN[cc] = ldf<FOLLOW>(&facN[4 * r + cc]);
+      fN = lu_solve_lanes(luN, r, fN, 0, 1, xn);
+      __syncwarp();
+      if (lane < 4) fs[4 * (N - 1) + lane] = fN;
+      // back substitution (triSolvers.cpp:1032-1045):
+      // f(i) -= (c'(i) f(i+1) + a'(i) f(N-1)), c' products in lanes 0-15 and
+      // a' products in lanes 16-31 of one instruction
+      double fNall[4];
+#pragma unroll
+      for (int m = 0; m < 4; m++) fNall[m] = xn[m];
+      double xnext[4];
+#pragma unroll
+      for (int m = 0; m < 4; m++) xnext[m] = xn[m];
+      // the next kBackAhead rows are in flight while row ii is solved
+      double mv[kBackAhead], xi[kBackAhead];
+#pragma unroll
+      for (int u = 0; u < kBackAhead; u++) {
+         const int ii = N - 2 - u;
+         mv[u] = ii >= 0 ? ldf<FOLLOW>(&fac[(size_t)kFacRec * ii + 32 + 16 * hi + e]) : 0.0;
+         xi[u] = ii >= 0 ? fs[4 * ii + r] : 0.0;
+      }
+      for (int i0 = N - 2; i0 >= 0; i0 -= kBackAhead) {
+#pragma unroll
+         for (int u = 0; u < kBackAhead; u++) {
+            const int ii = i0 - u, in = ii - kBackAhead;
+            if (ii < 0) break;
+            const double prod = mv[u] * (hi ? sel4(fNall, pj) : sel4(xnext, pj));
+            double x = xi[u];
+            mv[u] = in >= 0 ? ldf<FOLLOW>(&fac[(size_t)kFacRec * in + 32 + 16 * hi + e]) : 0.0;
+            xi[u] = in >= 0 ? fs[4 * in + r] : 0.0;
+            const double other = __shfl_sync(kLaneMask, prod, e + 16);
+            const double sterm = (ii == N - 2) ? prod : prod + other;
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++) x = x - __shfl_sync(kLaneMask, sterm, 4 * r + jj);
+#pragma unroll
+            for (int m = 0; m < 4; m++) xnext[m] = __shfl_sync(kLaneMask, x, m);
+            if (lane < 4) fs[4 * ii + lane] = x;
+         }
+      }
+   } else {
+      // back substitution (triSolvers.cpp:839-846): f(i) -= c'(i) f(i+1); both
+      // halves of the warp on the same line
+      back_line_pair<FOLLOW>(fac, N, fs, lane, xprev);
+   }
+}
+
 // Right-hand-side replay of a factored line: fs (N rows of 4, in place)
 // <- solution, with the records of factor_line.  All 32 lanes take part.
 //
@@ -941,30 +1047,24 @@ __device__ __forceinline__ void ld4(const double* __restrict__ p, double (&v)[4]
 // lanes e = 4*pr + pj (e = lane & 15) and handed to their owner lanes with
 // shuffles, so each row costs about 35 FP64 instructions instead of 60.
 // The subtraction order of every component is the reference's.
-// FOLLOW: behind the factorisation of the same line by another warp of the
-// block (prog, publish_rows); ok turns false if a wait gave up.
-template <bool FOLLOW = false>
 __device__ __forceinline__ void solve_line(const double* __restrict__ fac, const double* __restrict__ facN, int N,
-                                           bool per, double* __restrict__ fs, int lane, const int* prog = nullptr,
-                                           bool* ok = nullptr)
+                                           bool per, double* __restrict__ fs, int lane)
 {
-   const int e = lane & 15, pr = e >> 2, pj = e & 3, hi = lane >> 4;
+   const int e = lane & 15, pj = e & 3;
    const int r = lane & 3;
    // ---- forward sweep (triSolvers.cpp:778-822 / 859-933); row i+1 prefetched
    double xprev[4] = {0.0, 0.0, 0.0, 0.0};
-   if (FOLLOW && *ok && !wait_rows(prog, 1)) *ok = false;
    double fv = fs[r], av = 0.0, lu[4];
 #pragma unroll
-   for (int c = 0; c < 4; c++) lu[c] = ldf<FOLLOW>(&fac[16 + 4 * r + c]);
+   for (int c = 0; c < 4; c++) lu[c] = fac[16 + 4 * r + c];
    for (int i = 0; i < N; i++) {
       double fvn = 0.0, avn = 0.0, lun[4] = {0.0, 0.0, 0.0, 0.0};
       if (i + 1 < N) {
-         if (FOLLOW && *ok && !wait_rows(prog, i + 2)) *ok = false;
          const double* nr = fac + (size_t)kFacRec * (i + 1);
          fvn = fs[4 * (i + 1) + r];
-         avn = ldf<FOLLOW>(&nr[e]);
+         avn = nr[e];
 #pragma unroll
-         for (int c = 0; c < 4; c++) lun[c] = ldf<FOLLOW>(&nr[16 + 4 * r + c]);
+         for (int c = 0; c < 4; c++) lun[c] = nr[16 + 4 * r + c];
       }
       double x = fv;
       if (i > 0) {
@@ -982,113 +1082,237 @@ __device__ __forceinline__ void solve_line(const double* __restrict__ fac, const
       av = avn;
    }
    __syncwarp();
-   if (FOLLOW && *ok && !wait_rows(prog, per ? N + 1 : N)) *ok = false;
-   if (per) {
-      // f(N-1) -= c_{N-1}^{(i)} f(i), i = 0..N-2 (triSolvers.cpp:991-999);
-      // the products of rows i and i+1 in one instruction (lanes 0-15, 16-31)
-      double fN = sel4(xprev, r);
-      int i = 0;
-      double c = 0.0, f = 0.0;
-      if (hi < N - 1) {
-         c = ldf<FOLLOW>(&fac[(size_t)kFacRec * hi + 64 + e]);
-         f = fs[4 * hi + pj];
-      }
-      for (; i < N - 1; i += 2) {
-         const int rn = i + 2 + hi;
-         double cn = 0.0, fn = 0.0;
-         if (rn < N - 1) {
-            cn = ldf<FOLLOW>(&fac[(size_t)kFacRec * rn + 64 + e]);
-            fn = fs[4 * rn + pj];
-         }
-         const double p = c * f;
-#pragma unroll
-         for (int jj = 0; jj < 4; jj++) fN = fN - __shfl_sync(kLaneMask, p, 4 * r + jj);
-         if (i + 1 < N - 1) {
-#pragma unroll
-            for (int jj = 0; jj < 4; jj++) fN = fN - __shfl_sync(kLaneMask, p, 16 + 4 * r + jj);
-         }
-         c = cn;
-         f = fn;
-      }
-      double luN[4], xn[4];
-#pragma unroll
-      for (int cc = 0; cc < 4; cc++) luN[cc] = ldf<FOLLOW>(&facN[4 * r + cc]);
-      fN = lu_solve_lanes(luN, r, fN, 0, 1, xn);
-      __syncwarp();
-      if (lane < 4) fs[4 * (N - 1) + lane] = fN;
-      // back substitution (triSolvers.cpp:1032-1045):
-      // f(i) -= (c'(i) f(i+1) + a'(i) f(N-1)), c' products in lanes 0-15 and
-      // a' products in lanes 16-31 of one instruction
-      double fNall[4];
-#pragma unroll
-      for (int m = 0; m < 4; m++) fNall[m] = xn[m];
-      double xnext[4];
-#pragma unroll
-      for (int m = 0; m < 4; m++) xnext[m] = xn[m];
-      // rows ii-1 and ii-2 are in flight while row ii is solved
-      double mv = 0.0, xi = 0.0, mv1 = 0.0, xi1 = 0.0;
-      if (N >= 2) {
-         mv = ldf<FOLLOW>(&fac[(size_t)kFacRec * (N - 2) + 32 + 16 * hi + e]);
-         xi = fs[4 * (N - 2) + r];
-      }
-      if (N >= 3) {
-         mv1 = ldf<FOLLOW>(&fac[(size_t)kFacRec * (N - 3) + 32 + 16 * hi + e]);
-         xi1 = fs[4 * (N - 3) + r];
-      }
-      for (int ii = N - 2; ii >= 0; ii--) {
-         double mv2 = 0.0, xi2 = 0.0;
-         if (ii > 1) {
-            mv2 = ldf<FOLLOW>(&fac[(size_t)kFacRec * (ii - 2) + 32 + 16 * hi + e]);
-            xi2 = fs[4 * (ii - 2) + r];
-         }
-         const double prod = mv * (hi ? sel4(fNall, pj) : sel4(xnext, pj));
-         const double other = __shfl_sync(kLaneMask, prod, e + 16);
-         const double sterm = (ii == N - 2) ? prod : prod + other;
-         double x = xi;
-#pragma unroll
-         for (int jj = 0; jj < 4; jj++) x = x - __shfl_sync(kLaneMask, sterm, 4 * r + jj);
-#pragma unroll
-         for (int m = 0; m < 4; m++) xnext[m] = __shfl_sync(kLaneMask, x, m);
-         if (lane < 4) fs[4 * ii + lane] = x;
-         mv = mv1;
-         xi = xi1;
-         mv1 = mv2;
-         xi1 = xi2;
-      }
-   } else {
-      // back substitution (triSolvers.cpp:839-846): f(i) -= c'(i) f(i+1)
-      double xnext[4];
-#pragma unroll
-      for (int m = 0; m < 4; m++) xnext[m] = xprev[m];
-      // rows ii-1 and ii-2 are in flight while row ii is solved
-      double mv = 0.0, xi = 0.0, mv1 = 0.0, xi1 = 0.0;
-      if (N >= 2) {
-         mv = ldf<FOLLOW>(&fac[(size_t)kFacRec * (N - 2) + 32 + e]);
-         xi = fs[4 * (N - 2) + r];
-      }
-      if (N >= 3) {
-         mv1 = ldf<FOLLOW>(&fac[(size_t)kFacRec * (N - 3) + 32 + e]);
-         xi1 = fs[4 * (N - 3) + r];
-      }
-      for (int ii = N - 2; ii >= 0; ii--) {
-         double mv2 = 0.0, xi2 = 0.0;
-         if (ii > 1) {
-            mv2 = ldf<FOLLOW>(&fac[(size_t)kFacRec * (ii - 2) + 32 + e]);
-            xi2 = fs[4 * (ii - 2) + r];
-         }
-         const double prod = mv * sel4(xnext, pj);
-         double x = xi;
-#pragma unroll
-         for (int jj = 0; jj < 4; jj++) x = x - __shfl_sync(kLaneMask, prod, 4 * r + jj);
-#pragma unroll
-         for (int m = 0; m < 4; m++) xnext[m] = __shfl_sync(kLaneMask, x, m);
-         if (lane < 4) fs[4 * ii + lane] = x;
-         mv = mv1;
-         xi = xi1;
-         mv1 = mv2;
-         xi1 = xi2;
-      }
+   solve_line_tail(fac, facN, N, per, fs, lane, xprev);
+}
+
+// ---- one line by two warps ---------------------------------------------
+// The factorisation's recurrence is a chain of dependent FP64 operations of
+// one warp (64 cycles each, whatever the lanes do), so its length is what a
+// long line costs.  Two warps of a block (two SM sub-partitions) share a line:
+//   * factor_line_team runs the recurrence through c' alone, with lanes 0-15
+//     on B' and lanes 16-31 on the columns of c(i): an elimination step and
+//     the forward substitution of the columns are one instruction each, and
+//     the products of b(i) -= a(i) c'(i-1) are formed two to a half.  25 FP64
+//     instructions and four pivot reciprocals a row, against 39 and four in
+//     factor_line.
+//   * follow_line_team solves behind it: lanes 0-15 the fill-in column a'
+//     (periodic), lanes 16-31 the line's first right-hand side, which take
+//     the same instructions with the stored LU; then the last row and the
+//     back substitution.
+// Row N-2 of a periodic line adds a(N-2) = -a a'(N-3) to c(N-2), so there the
+// factoring warp waits for the follower's fill column; everywhere else only
+// the follower waits.  Records as factor_line's, bit for bit, except that row
+// N-1's fill column, which nothing reads, is not stored.
+// Measured (384 x 96 block_tridag4, both directions): see trisolve.cu.
+// The LU rows travel through a ring in shared memory whose words are their own
+// flags: a word is kTeamEmpty until the factoring warp has stored it, and again
+// once the follower has read it.  So the recurrence neither waits for its record
+// stores to be performed, as publish_rows would make it, nor spends a barrier on
+// a row (both measured about 490 cycles a row).  kTeamEmpty is a NaN no
+// arithmetic gives; an input block that holds it would make a wait give up.
+// A row whose pivots' integer reciprocals are undecided (sd::rcp_try) is done
+// again with the operator, so that a row has one such branch instead of four.
+// Cycles per row of a line (one warp each on its sub-partition): factorisation
+// 3,760 in factor_line, see trisolve.cu for whole solves.
+constexpr int kTeamRing = 16;
+constexpr unsigned long long kTeamEmpty = 0xFFF4C3A59B7D6E21ull;
+struct TeamShared {
+   unsigned long long lu[kTeamRing][16];
+   unsigned long long fill[16];   // a(N-2) for the factoring warp; the fill column is then stored up to row N-3
+   int prog;                      // rows published by the factoring warp, from N + 1 on (factor_line)
+};
+
+// by the whole block, a __syncthreads before the team starts
+__device__ __forceinline__ void team_init(TeamShared* ts)
+{
+   for (int t = threadIdx.x; t < kTeamRing * 16; t += blockDim.x) (&ts->lu[0][0])[t] = kTeamEmpty;
+   for (int t = threadIdx.x; t < 16; t += blockDim.x) ts->fill[t] = kTeamEmpty;
+   if (threadIdx.x == 0) ts->prog = 0;
+}
+
+// the word at p once it is (not) kTeamEmpty; ok turns false if the wait gives
+// up, bounded as wait_rows is
+template <bool EMPTY>
+__device__ __forceinline__ unsigned long long team_word(const unsigned long long* p, bool* ok)
+{
+   unsigned long long v = *(const volatile unsigned long long*)p;
+   for (long it = 0; (v == kTeamEmpty) != EMPTY && *ok; it++) {
+      if (it >= kFollowSpin) *ok = false;
+      __nanosleep(40);   // shuffles share the pipe with these loads
+      v = *(const volatile unsigned long long*)p;
    }
+   return v;
+}
+
+// one elimination step of factor_line_team: pivot S of the LU of B' (lanes
+// 0-15) with the columns of c (lanes 16-31) substituted along it
+template <int S, bool SOFT>
+__device__ __forceinline__ void team_step(double& w, int h, int k, int j, bool& rare)
+{
+   const double b = __shfl_sync(kLaneMask, w, 5 * S);
+   const double L = __shfl_sync(kLaneMask, w, 4 * k + S);
+   const double piv = SOFT ? sd::rcp_try(b, rare) : 1. / b;
+   const double m = w * piv;
+   if (k == S && (h || j > S)) w = m;
+   if (S < 3) {
+      const double U = __shfl_sync(kLaneMask, w, 16 * h + 4 * S + j);
+      const double t = w - L * U;
+      if (k > S && (h || j > S)) w = t;
+   }
+   if (h == 0 && k == S && j == S) w = piv;
+}
+
+// Ab, Bb, Cb, stride, N, per, fac, facN and the result as factor_line's
+__device__ __forceinline__ bool factor_line_team(const double* __restrict__ Ab, const double* __restrict__ Bb,
+                                                 const double* __restrict__ Cb, size_t stride, int N, bool per,
+                                                 double* __restrict__ fac, double* __restrict__ facN, int lane,
+                                                 TeamShared* __restrict__ ts, bool* ok)
+{
+   const int h = lane >> 4, e = lane & 15, k = e >> 2, j = e & 3;
+   const double* Wb = h ? Cb : Bb;   // lanes 0-15 hold B', lanes 16-31 the columns of c(i)
+   double2 A = *reinterpret_cast<const double2*>(Ab + 4 * k + 2 * h);   // a(k, 2h) and a(k, 2h+1)
+   double W = Wb[e];
+   double P0 = 0.0, P1 = 0.0;        // c'(i-1) entries (2h, j) and (2h+1, j)
+   bool bad = false;
+   for (int i = 0; i < N; i++) {
+      double2 An = make_double2(0.0, 0.0);
+      double Wn = 0.0;
+      if (i + 1 < N) {
+         const size_t o = stride * (size_t)(i + 1);
+         An = *reinterpret_cast<const double2*>(Ab + o + 4 * k + 2 * h);
+         Wn = Wb[o + e];
+      }
+      double* rec = fac + (size_t)kFacRec * i;
+      if (j == 0) *reinterpret_cast<double2*>(rec + 4 * k + 2 * h) = A;
+      double w = W;
+      if (i > 0) {
+         // b(i) -= a(i) c'(i-1), the four products subtracted in order
+         const double p0 = A.x * P0, p1 = A.y * P1;
+         const double p2 = __shfl_sync(kLaneMask, p0, 16 + e), p3 = __shfl_sync(kLaneMask, p1, 16 + e);
+         const double t = (((w - p0) - p1) - p2) - p3;
+         if (h == 0) w = t;
+      }
+      if (per && i == N - 2) {
+         const double v = w + __longlong_as_double((long long)team_word<false>(&ts->fill[e], ok));
+         if (h) w = v;
+      }
+      const double w0 = w;
+      bool rare = false;
+      team_step<0, true>(w, h, k, j, rare);
+      team_step<1, true>(w, h, k, j, rare);
+      team_step<2, true>(w, h, k, j, rare);
+      team_step<3, true>(w, h, k, j, rare);
+      if (__any_sync(kLaneMask, rare)) {
+         w = w0;
+         team_step<0, false>(w, h, k, j, rare);
+         team_step<1, false>(w, h, k, j, rare);
+         team_step<2, false>(w, h, k, j, rare);
+         team_step<3, false>(w, h, k, j, rare);
+      }
+      // back substitution of the columns (lanes 16-31; the others compute
+      // values nobody reads), every product as the reference's
+      const double x3 = __shfl_sync(kLaneMask, w, 28 + j);
+      const double u3 = __shfl_sync(kLaneMask, w, 4 * k + 3);
+      const double q3 = u3 * x3;
+      const double u1 = __shfl_sync(kLaneMask, w, 4 * k + 1), u2 = __shfl_sync(kLaneMask, w, 4 * k + 2);
+      if (h == 0) {
+         unsigned long long* s = &ts->lu[i % kTeamRing][e];
+         team_word<true>(s, ok);
+         *(volatile unsigned long long*)s = (unsigned long long)__double_as_longlong(w);
+         rec[16 + e] = w;
+         bad |= k == j && nonfinite(w);
+      }
+      __syncwarp();
+      const double y2 = w - q3;
+      const double x2 = __shfl_sync(kLaneMask, y2, 24 + j);
+      const double q2 = u2 * x2;
+      const double y1 = (w - q2) - q3;
+      const double x1 = __shfl_sync(kLaneMask, y1, 20 + j);
+      const double q1 = u1 * x1;
+      const double y0 = ((w - q1) - q2) - q3;
+      const double x0 = __shfl_sync(kLaneMask, y0, 16 + j);
+      P0 = h ? x2 : x0;
+      P1 = h ? x3 : x1;
+      if (h) {
+         const double x = (k == 0) ? x0 : (k == 1) ? x1 : (k == 2) ? x2 : x3;
+         rec[32 + e] = x;
+         if (per && i == N - 2) rec[48 + e] = x;   // a'(N-2) = c'(N-2)
+      }
+      A = An;
+      W = Wn;
+   }
+   if (!per) {
+      publish_rows(&ts->prog, N + 1, lane);   // every row's c' for the back substitution
+      return bad;
+   }
+   __threadfence_block();   // c' of the other lanes, a' of the follower (its fill was read above)
+   __syncwarp();
+   const double bN =
+      eliminate_last_row(fac, N, ldf<true>(&fac[(size_t)kFacRec * (N - 1) + 32 + e]), lane, &ts->prog);
+   const double w = lu_wavefront<true>(__shfl_sync(kLaneMask, bN, 16 + e), 16 * h, e);
+   if (h == 0) facN[e] = w;
+   publish_rows(&ts->prog, 2 * N, lane);
+   return bad || (h == 0 && k == j && nonfinite(w));
+}
+
+// The second warp of the team: the fill column (periodic) and, with F, the
+// solve of fs (N rows of 4, in place).  A row's a(i) comes from the input
+// blocks, so the fill of row N-2, which the factoring warp waits for, needs
+// nothing of that row's factorisation.
+template <bool F>
+__device__ __forceinline__ void follow_line_team(const double* __restrict__ Ab, size_t stride,
+                                                 double* __restrict__ fac, const double* __restrict__ facN, int N,
+                                                 bool per, double* __restrict__ fs, int lane,
+                                                 TeamShared* __restrict__ ts, bool* ok)
+{
+   const int h = lane >> 4, e = lane & 15, k = e >> 2, j = e & 3;
+   double X[4] = {0.0, 0.0, 0.0, 0.0};   // the previous row's column j of a' (lanes 0-15) or solution
+   const int rows = F ? N : N - 1;       // the fill column ends with a(N-2)
+   double f = F ? fs[k] : 0.0;
+   double2 A0 = *reinterpret_cast<const double2*>(Ab + 4 * k), A1 = *reinterpret_cast<const double2*>(Ab + 4 * k + 2);
+   for (int i = 0; i < rows; i++) {
+      const double a[4] = {A0.x, A0.y, A1.x, A1.y};
+      double fn = 0.0;
+      if (i + 1 < rows) {
+         const double* an = Ab + stride * (size_t)(i + 1) + 4 * k;
+         A0 = *reinterpret_cast<const double2*>(an);
+         A1 = *reinterpret_cast<const double2*>(an + 2);
+         if (F) fn = fs[4 * (i + 1) + k];
+      }
+      // a(i) = -a(i) a'(i-1), f(i) -= a(i) f(i-1)
+      double x;
+      if (i == 0) {
+         x = h ? f : sel4(a, j);
+      } else {
+         x = h ? f : 0.0;
+#pragma unroll
+         for (int l = 0; l < 4; l++) x = x - a[l] * X[l];
+      }
+      if (per && i == N - 2) {
+         __threadfence_block();   // the fill column's records, before the word the factoring warp waits for
+         __syncwarp();
+         if (h == 0) *(volatile unsigned long long*)&ts->fill[e] = (unsigned long long)__double_as_longlong(x);
+         if (!F) return;
+      }
+      double* rec = fac + (size_t)kFacRec * i;
+      unsigned long long* slot = ts->lu[i % kTeamRing];
+      double lu[4];
+#pragma unroll
+      for (int l = 0; l < 4; l++) lu[l] = __longlong_as_double((long long)team_word<false>(&slot[4 * k + l], ok));
+      __syncwarp();   // every lane has read the row
+      if (h == 0) *(volatile unsigned long long*)&slot[e] = kTeamEmpty;
+      x = lu_solve_lanes(lu, k, x, 16 * h + j, 4, X);
+      if (per && h == 0 && i < N - 2) rec[48 + e] = x;
+      if (F && h && j == 0) fs[4 * i + k] = x;
+      f = fn;
+   }
+   if (!F) return;
+   double xl[4];
+#pragma unroll
+   for (int m = 0; m < 4; m++) xl[m] = __shfl_sync(kLaneMask, X[m], 16);
+   __syncwarp();
+   if (*ok && !wait_rows(&ts->prog, N + 1)) *ok = false;
+   solve_line_tail<true>(fac, facN, N, per, fs, lane, xl, &ts->prog, ok);
 }
 
 }  // namespace hamstr

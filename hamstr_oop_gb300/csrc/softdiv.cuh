@@ -12,13 +12,13 @@
 // dividend; subnormal quotient) falls back to `/`.
 //
 // Method: the divisor's 53-bit significand mb (value m = mb/2^52 in [1,2))
-// gets r ~ 2^64/m in one 64-bit word, a few units below the true value or at
-// most one above: an FP32 reciprocal estimate y of m's leading 24 bits, the
-// exact integer residual e = 1 - m y (it fits one signed word) and the first
+// gets r ~ 2^64/m in one 64-bit word, a few units below the true value: an
+// FP32 reciprocal estimate y of m's leading 24 bits, kept below 1/m, the
+// exact integer residual e = 1 - m y (it fits one word) and the first
 // terms of 1/m = y (1 + e + e^2 + ...), the Newton-Raphson series of the
 // reciprocal.  A quotient is then the high word of ma * r, with 10 or 11 bits
 // beyond the 53 kept.  The rounding follows from those bits except where they
-// lie within the error of r of the midpoint (about 1 in 200 quotients); there
+// lie within the error of r of the midpoint (about 1 in 150 quotients); there
 // the sign of the exact remainder at the midpoint decides, one 64-bit
 // product.  A quotient of two 53-bit numbers is never a midpoint itself
 // (Markstein, "Computation of elementary functions on the IBM RISC System/6000
@@ -105,11 +105,11 @@ __host__ __device__ __forceinline__ uint64_t reciprocal_word(uint64_t d)
    return v3 - hi2;
 }
 
-// an estimate of 1/m from the leading 24 bits of the significand mb (2^52 <=
-// mb < 2^53, m = mb / 2^52), within 2^-22 of it
+// an FP32 estimate of 1/m, m = mb / 2^52 in [1, 2): of the reciprocal of m
+// rounded to 24 bits, within 1.5 * 2^-23 of 1/m relative
 __host__ __device__ __forceinline__ float recip_seed(uint64_t mb)
 {
-   const uint32_t u = 0x3F800000u | ((uint32_t)(mb >> 29) & 0x7FFFFFu);
+   const uint32_t u = 0x3F800000u + (uint32_t)((mb - 0x10000000000000ull + (1u << 28)) >> 29);
    float y;
 #ifdef __CUDA_ARCH__
    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(u)));
@@ -121,27 +121,25 @@ __host__ __device__ __forceinline__ float recip_seed(uint64_t mb)
    return y;
 }
 
-// 2^64 / m as a 64-bit word, from a seed y within 2^-21.6 of 1/m: the result is
-// less than 4 below the true value and less than 1 above it, and below 2^64
-// (for m = 1 every product here is exact up to the last floor).  With
-// Y = y 2^32, E = e 2^84 is exact in one word (|e| < 2^-21), the two terms of
-// the series are floored to 2^-64, and e^3 < 2^-64 is left out.
+// 2^64 / m as a 64-bit word from such an estimate: less than 8 below the true
+// value and never above it.  The estimate is lowered by 3 * 2^-24 so that
+// Y = y 2^32 stays below 2^32/m: then e = 1 - m y is in [0, 2^-20.8) and
+// E = e 2^84 is exact in one word, (e + e^2) 2^64 is formed with both terms
+// floored, and e^3 and what follows (less than 3 units) is left out.
 __host__ __device__ __forceinline__ uint64_t recip64(uint64_t mb, float y)
 {
-   y = y < 0.5f ? 0.5f : y;
-   y = y > 0.99999994f ? 0.99999994f : y;   // 1 - 2^-24
 #ifdef __CUDA_ARCH__
-   const uint32_t u = __float_as_uint(y);
+   uint32_t u = __float_as_uint(y);
 #else
    uint32_t u;
    std::memcpy(&u, &y, 4);
 #endif
-   const uint32_t Y = (u << 8) | 0x80000000u;
-   const int64_t E = -(int64_t)(mb * (uint64_t)Y);
-   const int32_t Eh = (int32_t)(E >> 32);
-   const int64_t S = (E >> 20) + (((int64_t)Eh * Eh) >> 40);
-   return ((uint64_t)Y << 32) + (uint64_t)((int64_t)(S >> 32) * (int64_t)(uint64_t)Y) +
-          (((uint64_t)Y * (uint32_t)S) >> 32);
+   u = u < 0x3F000000u ? 0x3F000000u : u > 0x3F7FFFFFu ? 0x3F7FFFFFu : u;   // [1/2, 1)
+   const uint32_t Y = ((u << 8) | 0x80000000u) - 0x300u;
+   const uint64_t E = 0 - mb * (uint64_t)Y;
+   const uint32_t Eh = (uint32_t)(E >> 32);
+   const uint64_t S = (E >> 20) + (((uint64_t)Eh * Eh) >> 40);
+   return ((uint64_t)Y << 32) + (uint64_t)(uint32_t)(S >> 32) * Y + (((uint64_t)(uint32_t)S * Y) >> 32);
 }
 
 // a divisor prepared once for several divisions
@@ -190,33 +188,39 @@ __host__ __device__ __forceinline__ double div(double a, const Divisor& D)
       if (D.ok && (A << 1) == 0) return from_bits((A ^ D.sign) & 0x8000000000000000ull);
       return div_other(a, D.b);
    }
-   // floor of (ma/mb) 2^63 less an error in (-1, 5); 10 + (1 - s) bits are
+   // floor of (ma/mb) 2^63 less an error in [0, 9); 10 + (1 - s) bits are
    // beyond the significand
    const uint64_t H = mulhi(ma << 11, D.r);
    const int sh = 11 - s;
    uint64_t q = H >> sh;
    const uint32_t half = 0x400u >> s, f = (uint32_t)H & (2 * half - 1);
    bool up = f >= half;
-   if (f - (half - 6) <= 7u) up = (int64_t)((ma << (53 + s)) - D.mb * (2 * q + 1)) > 0;
+   if (f - (half - 9) <= 8u) up = (int64_t)((ma << (53 + s)) - D.mb * (2 * q + 1)) > 0;
    q += up ? 1 : 0;
    // q in [2^52, 2^53]; 2^53 carries into the exponent
    return from_bits(((A ^ D.sign) & 0x8000000000000000ull) | (((uint64_t)e << 52) + q - 0x10000000000000ull));
 }
 
-// 1 / b rounded to nearest even, equal to the `/` operator.  One branch: the
-// line solvers wait for each pivot's reciprocal, so the operands that the
-// integer path does not take (zero, subnormal, inf, NaN, a subnormal result)
-// and the words too close to a midpoint (1 in 256) share the operator.
-__host__ __device__ __forceinline__ double rcp(double b)
+// 1 / b rounded to nearest even, equal to the `/` operator unless `rare` is
+// raised: for the operands the integer path does not take (zero, subnormal,
+// inf, NaN, a subnormal result) and the words too close to a midpoint (1 in
+// 228), which the caller leaves to the operator
+__host__ __device__ __forceinline__ double rcp_try(double b, bool& rare)
 {
    const uint64_t B = bits(b);
-   const int eb = (int)((B >> 52) & 0x7FF);
+   const uint32_t eb = (uint32_t)(B >> 52) & 0x7FFu;
    const uint64_t mb = (B & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
    const uint64_t r = recip64(mb, recip_seed(mb));
    const uint64_t q = (r >> 11) + ((r >> 10) & 1);
-   const uint32_t f = (uint32_t)r & 0x7FFu;
-   const bool rare = (unsigned)(eb - 1) >= 2044u || f - 0x3FAu <= 7u;
-   double y = from_bits((B & 0x8000000000000000ull) | (((uint64_t)(2045 - eb) << 52) + q - 0x10000000000000ull));
+   rare |= eb - 1u >= 2044u || ((uint32_t)r & 0x7FFu) - 0x3F7u <= 8u;
+   return from_bits((B & 0x8000000000000000ull) | (((uint64_t)(2044u - eb) << 52) + q));
+}
+
+// 1 / b rounded to nearest even, equal to the `/` operator
+__host__ __device__ __forceinline__ double rcp(double b)
+{
+   bool rare = false;
+   double y = rcp_try(b, rare);
    if (rare) y = div_other(1., b);
    return y;
 }

@@ -4,8 +4,12 @@
 //
 // The reference's TRISOLVER::blockTridag4 (triSolvers.cpp:769-847) and
 // blockTridagPeriodic4 (triSolvers.cpp:850-1046) as a batched entry point:
-// one warp per line, factor_line + solve_line of line_solve.cuh, so each
-// line's solution is bit-identical to one reference call.
+// two warps per line, factor_line_team and follow_line_team of
+// line_solve.cuh, so each line's solution is bit-identical to one reference
+// call.  A line is a recurrence over its rows; with the solve (and the periodic
+// fill column) behind the factorisation in a second warp a row takes 4,480
+// cycles open and 5,460 periodic, against 7,150 and 8,000 in one warp, and 52
+// FP64 instructions against 66, so it is the better split at any number of lines.
 // ##################################################################
 #include <cuda_runtime.h>
 
@@ -23,18 +27,27 @@ namespace {
 
 using namespace hamstr;
 
-__global__ void __launch_bounds__(32) block_tridag_kernel(int N, int periodic, const double* __restrict__ A,
+__global__ void __launch_bounds__(64) block_tridag_kernel(int N, int periodic, const double* __restrict__ A,
                                                           const double* __restrict__ B, const double* __restrict__ C,
                                                           double* __restrict__ F, double* __restrict__ scratch)
 {
+   __shared__ TeamShared ts;
    const size_t line = blockIdx.x;
    const size_t nb = (size_t)N * 16;
    double* fac = scratch + line * ((size_t)kFacRec * N + 16);
    double* facN = fac + (size_t)kFacRec * N;
    const bool per = periodic != 0;
-   factor_line(A + line * nb, B + line * nb, C + line * nb, 16, N, per, fac, facN, threadIdx.x);
-   __syncwarp();
-   solve_line(fac, facN, N, per, F + line * (size_t)N * 4, threadIdx.x);
+   const int lane = threadIdx.x & 31;
+   team_init(&ts);
+   __syncthreads();
+   bool ok = true;
+   if (threadIdx.x < 32)
+      factor_line_team(A + line * nb, B + line * nb, C + line * nb, 16, N, per, fac, facN, lane, &ts, &ok);
+   else
+      follow_line_team<true>(A + line * nb, 16, fac, facN, N, per, F + line * (size_t)N * 4, lane, &ts, &ok);
+   // a wait that gave up (never expected, line_solve.cuh) leaves no plausible solution behind
+   if (__syncthreads_or(!ok))
+      for (int i = threadIdx.x; i < 4 * N; i += 64) F[line * (size_t)N * 4 + i] = __longlong_as_double(-1);
 }
 
 }  // namespace
@@ -60,7 +73,7 @@ int block_tridag_launch(int nlines, int N, int periodic, const double* A, const 
                         double* F, double* scratch, cudaStream_t st)
 {
    if (nlines == 0) return HAMSTR_GPU_OK;
-   block_tridag_kernel<<<nlines, 32, 0, st>>>(N, periodic, A, B, C, F, scratch);
+   block_tridag_kernel<<<nlines, 64, 0, st>>>(N, periodic, A, B, C, F, scratch);
    const cudaError_t e = cudaGetLastError();
    if (e != cudaSuccess) {
       set_last_error(std::string("block_tridag4 launch: ") + cudaGetErrorString(e));
@@ -71,6 +84,49 @@ int block_tridag_launch(int nlines, int N, int periodic, const double* A, const 
 
 }  // namespace hamstr
 
+namespace {
+
+// The allocating entry point's scratch: a stream-ordered pool of its own per
+// device, so that a call neither maps fresh memory nor waits for the whole
+// device as cudaMalloc and cudaFree do (384 x 96, both directions: about 80 us
+// of two calls).  It keeps at most kPoolKept bytes between calls; more goes
+// back to the device when the call's stream is synchronised.  The allocator
+// orders reuse between streams and threads.
+constexpr unsigned long long kPoolKept = 64ull << 20;
+constexpr int kMaxDevices = 64;
+std::mutex g_pool_mutex;
+cudaMemPool_t g_pool[kMaxDevices] = {};
+
+cudaError_t scratch_pool(cudaMemPool_t* out)
+{
+   int dev = 0;
+   cudaError_t e = cudaGetDevice(&dev);
+   if (e != cudaSuccess) return e;
+   if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+   std::lock_guard<std::mutex> lock(g_pool_mutex);
+   if (!g_pool[dev]) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.handleTypes = cudaMemHandleTypeNone;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      cudaMemPool_t p = nullptr;
+      e = cudaMemPoolCreate(&p, &props);
+      if (e != cudaSuccess) return e;
+      unsigned long long kept = kPoolKept;
+      e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &kept);
+      if (e != cudaSuccess) {
+         cudaMemPoolDestroy(p);
+         return e;
+      }
+      g_pool[dev] = p;
+   }
+   *out = g_pool[dev];
+   return cudaSuccess;
+}
+
+}  // namespace
+
 extern "C" int hamstr_gpu_block_tridag4(int nlines, int N, int periodic, const double* A, const double* B,
                                         const double* C, double* F, void* stream)
 {
@@ -79,14 +135,17 @@ extern "C" int hamstr_gpu_block_tridag4(int nlines, int N, int periodic, const d
    const cudaStream_t s = (cudaStream_t)stream;
    double* scratch = nullptr;
    const size_t bytes = (size_t)nlines * ((size_t)kFacRec * N + 16) * sizeof(double);
-   cudaError_t e = cudaMalloc((void**)&scratch, bytes);
+   cudaMemPool_t pool = nullptr;
+   cudaError_t e = scratch_pool(&pool);
+   if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void**)&scratch, bytes, pool, s);
    if (e != cudaSuccess) {
+      cudaGetLastError();
       set_last_error(std::string("block_tridag4 scratch: ") + cudaGetErrorString(e));
       return e == cudaErrorMemoryAllocation ? HAMSTR_GPU_ERR_NOMEM : HAMSTR_GPU_ERR_CUDA;
    }
    st = block_tridag_launch(nlines, N, periodic, A, B, C, F, scratch, s);
+   cudaFreeAsync(scratch, s);
    e = cudaStreamSynchronize(s);
-   cudaFree(scratch);
    if (st) return st;
    if (e != cudaSuccess) {
       set_last_error(std::string("block_tridag4: ") + cudaGetErrorString(e));
@@ -112,7 +171,6 @@ namespace {
 constexpr size_t kNoAllocScratchDoubles = size_t(1) << 20;   // 8 MiB
 static __device__ __align__(256) double g_tridag_scratch[kNoAllocScratchDoubles];
 
-constexpr int kMaxDevices = 64;
 std::mutex g_scratch_mutex;
 double* g_scratch_addr[kMaxDevices] = {};
 

@@ -3,7 +3,7 @@ integers and IEEE division.
 
 recip64 gives 2^64/m from an FP32 estimate of 1/m; the rounding of every
 quotient rests on its error bounds, which must hold for any estimate within
-2^-21.6 (the device's approximate reciprocal differs from the host's in the
+1.5 * 2^-23 of the reciprocal, relative (the device's approximate reciprocal differs from the host's in the
 last place).  The header is compiled with the host compiler."""
 import os
 import subprocess
@@ -37,7 +37,7 @@ int main(int, char** argv) {
       const uint64_t r = recip64(mb, y);
       const unsigned __int128 one = (unsigned __int128)1 << 116;             // 2^64 / m = 2^116 / mb
       const __int128 below = (__int128)(one / mb) - (__int128)r;             // floor(true) - r
-      if (below < -1 || below > 3) bad++;
+      if (below < 0 || below > 7) bad++;
       n++;
       int e = 1 + (int)(rng() % 2046);
       if (i % 3) e = 1000 + (int)(rng() % 46);
@@ -57,7 +57,7 @@ int main(int, char** argv) {
 """
 
 
-@pytest.mark.parametrize("ulps", [-2, 0, 2])
+@pytest.mark.parametrize("ulps", [-1, 0, 1])
 def test_reciprocal_bounds_and_rounding_on_the_host(tmp_path, ulps):
     src = tmp_path / "r.cpp"
     src.write_text(PROGRAM)
