@@ -8,7 +8,7 @@
 // (jacobianRoe.cpp:92-620, frozen eigenvalues, IMODE 1) and the 5x5
 // block-tridiagonal solvers TRISOLVER::blockTridag / blockTridagPeriodic
 // (triSolvers.cpp:443-766).  They are given here batched on device arrays:
-// one thread per face or per line, every expression with the reference's
+// one thread per face or six lanes per line, every expression with the reference's
 // operands and association (-fmad=false, IEEE division and square root),
 // so each output equals one reference call's bit for bit.
 // ##################################################################
@@ -17,6 +17,7 @@
 #include <string>
 
 #include "../../include/hamstr_gpu.h"
+#include "softdiv.cuh"
 
 namespace hamstr {
 void set_last_error(const std::string& m);
@@ -206,148 +207,258 @@ __global__ void __launch_bounds__(kThreads) jacobian_roe3d_kernel(int n, const d
    }
 }
 
-// ---------------- 5x5 block-tridiagonal solvers (triSolvers.cpp:443-766) -
-// unpivoted LU with reciprocal pivots (triSolvers.cpp:481-506)
-struct LU5 {
-   double b11, b21, b22, b31, b32, b33, b41, b42, b43, b44, b51, b52, b53, b54, b55;
-   double u12, u13, u14, u15, u23, u24, u25, u34, u35, u45;
-};
+// ---------------- 5x5 block-tridiagonal lines (triSolvers.cpp:443-766) ----
+// Six lanes a line, five lines a warp: lane c < 5 of a line holds column c of
+// B', of c(i) and, periodic, of a(i) as it is eliminated, lane 5 the right-hand
+// side.  A row's work is the same instruction on every column, so the block
+// product, the LU and the substitutions of a row are 120 FP64 instructions a
+// warp (215 periodic) for five lines.  One thread a line, as before, spent 587
+// a row for 32 lines: fewer in all, but 4,099 lines were 129 warps on 608 SM
+// sub-partitions, each with 587 instructions of 64 cycles to a row (a
+// sub-partition issues one FP64 instruction per 64 cycles whatever its lanes
+// do), every load on 32 cache lines.  Measured, before -> now: 4,099 lines of 33
+// rows 1,092 -> 313 us open, 2,713 -> 709 periodic; one line 828 -> 233; 60,000
+// lines of 17 rows 2,640 -> 1,750.
+//
+// The LU is unpivoted with reciprocal pivots, each entry's products subtracted
+// in the order of triSolvers.cpp:486-505; the reciprocals are the integer
+// pipes' (softdiv.cuh), equal to 1./x.
+constexpr int kLaneCols = 6, kLinesPerWarp = 5;
 
-__device__ __forceinline__ LU5 lu5_factor(const double* b)
+__device__ __forceinline__ double from_lane(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+
+// x[k] -= sum over l, in order, of m[5k+l] * p[l]
+__device__ __forceinline__ void sub_product5(double (&x)[5], const double (&m)[25], const double (&p)[5])
 {
-   LU5 u;
-   u.b11 = 1. / b[0];
-   u.u12 = b[1] * u.b11;
-   u.u13 = b[2] * u.b11;
-   u.u14 = b[3] * u.b11;
-   u.u15 = b[4] * u.b11;
-   u.b21 = b[5];
-   u.b22 = 1. / (b[6] - u.b21 * u.u12);
-   u.u23 = (b[7] - u.b21 * u.u13) * u.b22;
-   u.u24 = (b[8] - u.b21 * u.u14) * u.b22;
-   u.u25 = (b[9] - u.b21 * u.u15) * u.b22;
-   u.b31 = b[10];
-   u.b32 = b[11] - u.b31 * u.u12;
-   u.b33 = 1. / (b[12] - u.b31 * u.u13 - u.b32 * u.u23);
-   u.u34 = (b[13] - u.b31 * u.u14 - u.b32 * u.u24) * u.b33;
-   u.u35 = (b[14] - u.b31 * u.u15 - u.b32 * u.u25) * u.b33;
-   u.b41 = b[15];
-   u.b42 = b[16] - u.b41 * u.u12;
-   u.b43 = b[17] - u.b41 * u.u13 - u.b42 * u.u23;
-   u.b44 = 1. / (b[18] - u.b41 * u.u14 - u.b42 * u.u24 - u.b43 * u.u34);
-   u.u45 = (b[19] - u.b41 * u.u15 - u.b42 * u.u25 - u.b43 * u.u35) * u.b44;
-   u.b51 = b[20];
-   u.b52 = b[21] - u.b51 * u.u12;
-   u.b53 = b[22] - u.b51 * u.u13 - u.b52 * u.u23;
-   u.b54 = b[23] - u.b51 * u.u14 - u.b52 * u.u24 - u.b53 * u.u34;
-   u.b55 = 1. / (b[24] - u.b51 * u.u15 - u.b52 * u.u25 - u.b53 * u.u35 - u.b54 * u.u45);
-   return u;
+#pragma unroll
+   for (int k = 0; k < 5; k++)
+#pragma unroll
+      for (int l = 0; l < 5; l++) x[k] -= m[5 * k + l] * p[l];
 }
 
-// x[0], x[s], ..., x[4s] <- LU^{-1} x (triSolvers.cpp:508-518)
-__device__ __forceinline__ void lu5_solve(const LU5& u, double* x, int s)
+// LU of the line's block, its columns in x of lanes base .. base+4, with the
+// columns of NX further right-hand sides per lane (and x of lane base+5)
+// substituted along it; U receives the multipliers u(s, j), j > s
+template <int NX>
+__device__ __forceinline__ void lu5_columns(double (&x)[5], double (&y)[NX][5], int base, int c, double (&U)[10])
 {
-   const double d1 = x[0] * u.b11;
-   const double d2 = (x[s] - u.b21 * d1) * u.b22;
-   const double d3 = (x[2 * s] - u.b31 * d1 - u.b32 * d2) * u.b33;
-   const double d4 = (x[3 * s] - u.b41 * d1 - u.b42 * d2 - u.b43 * d3) * u.b44;
-   const double d5 = (x[4 * s] - u.b51 * d1 - u.b52 * d2 - u.b53 * d3 - u.b54 * d4) * u.b55;
-   const double x3 = d4 - u.u45 * d5;
-   const double x2 = d3 - u.u34 * x3 - u.u35 * d5;
-   const double x1 = d2 - u.u23 * x2 - u.u24 * x3 - u.u25 * d5;
-   x[4 * s] = d5;
-   x[3 * s] = x3;
-   x[2 * s] = x2;
-   x[s] = x1;
-   x[0] = d1 - u.u12 * x1 - u.u13 * x2 - u.u14 * x3 - u.u15 * d5;
+   int n = 0;
+#pragma unroll
+   for (int s = 0; s < 5; s++) {
+      const double piv = hamstr::sd::rcp(from_lane(x[s], base + s));
+      double L[5];
+#pragma unroll
+      for (int k = s + 1; k < 5; k++) L[k] = from_lane(x[k], base + s);
+      const double m = x[s] * piv;
+      if (c > s) x[s] = m;
+#pragma unroll
+      for (int k = s + 1; k < 5; k++) {
+         const double t = x[k] - L[k] * m;
+         if (c > s) x[k] = t;
+      }
+#pragma unroll
+      for (int v = 0; v < NX; v++) {
+         y[v][s] = y[v][s] * piv;
+#pragma unroll
+         for (int k = s + 1; k < 5; k++) y[v][k] = y[v][k] - L[k] * y[v][s];
+      }
+#pragma unroll
+      for (int j = s + 1; j < 5; j++) U[n++] = from_lane(x[s], base + j);
+   }
 }
 
-// one line per thread, in place: a, b, c [N][5][5] are the reference's
-// scratch, f [N][5] becomes the solution
-__global__ void __launch_bounds__(kThreads) block_tridag5_kernel(int nlines, int N, int periodic,
-                                                                 double* __restrict__ av, double* __restrict__ bv,
-                                                                 double* __restrict__ cv, double* __restrict__ fv)
+// back substitution of one column with those multipliers (triSolvers.cpp:513-518)
+__device__ __forceinline__ void lu5_back(double (&y)[5], const double (&U)[10])
 {
-   const int line = blockIdx.x * blockDim.x + threadIdx.x;
-   if (line >= nlines) return;
-   const size_t nb = 25 * (size_t)N;
-   double* a = av + line * nb;
-   double* b = bv + line * nb;
-   double* c = cv + line * nb;
-   double* f = fv + line * 5 * (size_t)N;
-   auto A = [&](int i, int k, int j) -> double& { return a[25 * (size_t)i + 5 * k + j]; };
-   auto Bm = [&](int i, int k, int j) -> double& { return b[25 * (size_t)i + 5 * k + j]; };
-   auto C = [&](int i, int k, int j) -> double& { return c[25 * (size_t)i + 5 * k + j]; };
-   auto F = [&](int i, int k) -> double& { return f[5 * (size_t)i + k]; };
-   double t[5][5];
+   y[3] = y[3] - U[9] * y[4];
+   y[2] = (y[2] - U[7] * y[3]) - U[8] * y[4];
+   y[1] = ((y[1] - U[4] * y[2]) - U[5] * y[3]) - U[6] * y[4];
+   y[0] = (((y[0] - U[0] * y[1]) - U[1] * y[2]) - U[2] * y[3]) - U[3] * y[4];
+}
+
+// in place: a, b, c [N][5][5] become the reference's scratch, f [N][5] the
+// solution
+template <bool PER>
+__global__ void __launch_bounds__(32) block_tridag5_kernel(int nlines, int N, double* __restrict__ av,
+                                                           double* __restrict__ bv, double* __restrict__ cv,
+                                                           double* __restrict__ fv)
+{
+   const int lane = threadIdx.x, g = lane / kLaneCols, c = lane - kLaneCols * g, base = kLaneCols * g;
+   const long long line = (long long)blockIdx.x * kLinesPerWarp + g;
+   const bool live = g < kLinesPerWarp && line < nlines;
+   const bool col = live && c < 5, rhs = live && c == 5;
+   const size_t nb = 25 * (size_t)N, l0 = live ? (size_t)line : 0;
+   double* a = av + l0 * nb;
+   double* b = bv + l0 * nb;
+   double* cc = cv + l0 * nb;
+   double* f = fv + l0 * 5 * (size_t)N;
+   double A[25], x[5], y[PER ? 2 : 1][5];   // a(i) whole; column of B' or f; columns of c and a
+#pragma unroll
+   for (int m = 0; m < 25; m++) A[m] = live ? a[m] : 0.0;
+#pragma unroll
+   for (int k = 0; k < 5; k++) {
+      x[k] = col ? b[5 * k + c] : rhs ? f[k] : 0.0;
+      y[0][k] = col ? cc[5 * k + c] : 0.0;
+      if (PER) y[1][k] = 0.0;
+   }
+   double P[5] = {0.0, 0.0, 0.0, 0.0, 0.0};   // previous row: column of c' (lanes 0-4) or f (lane 5)
+   double Q[5] = {0.0, 0.0, 0.0, 0.0, 0.0};   // PER: column of a'
    for (int i = 0; i < N; i++) {
-      if (i != 0) {
-         for (int k = 0; k < 5; k++)
-            for (int j = 0; j < 5; j++)
-               for (int l = 0; l < 5; l++) Bm(i, k, j) -= A(i, k, l) * C(i - 1, l, j);
-         for (int k = 0; k < 5; k++)
-            for (int j = 0; j < 5; j++) F(i, k) -= A(i, k, j) * F(i - 1, j);
-         if (periodic) {
-            for (int k = 0; k < 5; k++)
-               for (int j = 0; j < 5; j++) t[k][j] = 0;
-            for (int k = 0; k < 5; k++)
-               for (int j = 0; j < 5; j++)
-                  for (int l = 0; l < 5; l++) t[k][j] -= A(i, k, l) * A(i - 1, l, j);
-            for (int k = 0; k < 5; k++)
-               for (int j = 0; j < 5; j++) A(i, k, j) = t[k][j];
-         }
-      }
-      const LU5 u = lu5_factor(&Bm(i, 0, 0));
-      lu5_solve(u, &F(i, 0), 1);
-      if (!periodic) {
-         if (i != N - 1)
-            for (int j = 0; j < 5; j++) lu5_solve(u, &C(i, 0, j), 5);
-      } else if (i != N - 2) {
-         for (int j = 0; j < 5; j++) {
-            lu5_solve(u, &C(i, 0, j), 5);
-            lu5_solve(u, &A(i, 0, j), 5);
-         }
-      } else {
-         for (int k = 0; k < 5; k++)
-            for (int j = 0; j < 5; j++) C(i, j, k) += A(i, j, k);
-         for (int j = 0; j < 5; j++) lu5_solve(u, &C(i, 0, j), 5);
-         for (int k = 0; k < 5; k++)
-            for (int j = 0; j < 5; j++) A(i, k, j) = C(i, k, j);
-      }
-   }
-   if (!periodic) {
-      for (int i = N - 2; i >= 0; i--)
-         for (int k = 0; k < 5; k++)
-            for (int j = 0; j < 5; j++) F(i, k) -= C(i, k, j) * F(i + 1, j);
-      return;
-   }
-   // last-row elimination and solve (triSolvers.cpp:671-749)
-   for (int k = 0; k < 5; k++)
-      for (int j = 0; j < 5; j++) Bm(N - 1, j, k) = (j == k) ? 1.0 : 0.0;
-   for (int i = 0; i < N - 1; i++) {
-      for (int k = 0; k < 5; k++)
-         for (int j = 0; j < 5; j++) t[k][j] = 0;
-      for (int k = 0; k < 5; k++)
-         for (int j = 0; j < 5; j++)
-            for (int l = 0; l < 5; l++) {
-               t[k][j] -= C(N - 1, k, l) * C(i, l, j);
-               Bm(N - 1, k, j) -= C(N - 1, k, l) * A(i, l, j);
+      const size_t o = 25 * (size_t)i;
+      if (i != 0) sub_product5(x, A, P);
+      if (PER) {
+         // a(i) = 0 - a(i) a'(i-1), its column c
+         if (i != 0) {
+#pragma unroll
+            for (int k = 0; k < 5; k++) y[PER ? 1 : 0][k] = 0.0;
+            sub_product5(y[PER ? 1 : 0], A, Q);
+         } else {
+#pragma unroll
+            for (int k = 0; k < 5; k++) {
+               double v = A[5 * k];
+#pragma unroll
+               for (int j = 1; j < 5; j++) v = (c == j) ? A[5 * k + j] : v;
+               y[PER ? 1 : 0][k] = v;
             }
-      for (int k = 0; k < 5; k++)
-         for (int j = 0; j < 5; j++) F(N - 1, k) -= C(N - 1, k, j) * F(i, j);
-      for (int k = 0; k < 5; k++)
-         for (int j = 0; j < 5; j++) C(N - 1, k, j) = t[k][j];
+         }
+      }
+      if (col && i != 0) {
+#pragma unroll
+         for (int k = 0; k < 5; k++) b[o + 5 * k + c] = x[k];
+      }
+      // the next row, while this one is eliminated
+      double xn[5], yn[5];
+      const bool more = i + 1 < N;
+#pragma unroll
+      for (int m = 0; m < 25; m++) A[m] = (live && more) ? a[o + 25 + m] : 0.0;
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+         xn[k] = (col && more) ? b[o + 25 + 5 * k + c] : (rhs && more) ? f[5 * (i + 1) + k] : 0.0;
+         yn[k] = (col && more) ? cc[o + 25 + 5 * k + c] : 0.0;
+      }
+      const bool last2 = PER && i == N - 2;
+      if (last2) {
+#pragma unroll
+         for (int k = 0; k < 5; k++) y[0][k] = y[0][k] + y[PER ? 1 : 0][k];
+      }
+      double U[10];
+      lu5_columns<PER ? 2 : 1>(x, y, base, c, U);
+      // f's forward substitution ran beside B's columns; its back substitution
+      // runs beside c's
+      if (c == 5) {
+#pragma unroll
+         for (int k = 0; k < 5; k++) y[0][k] = x[k];
+      }
+      lu5_back(y[0], U);
+      if (PER) {
+         lu5_back(y[PER ? 1 : 0], U);
+         if (last2) {
+#pragma unroll
+            for (int k = 0; k < 5; k++) y[PER ? 1 : 0][k] = y[0][k];
+         }
+      }
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+         if (rhs) f[5 * i + k] = y[0][k];
+         if (col && (PER || i != N - 1)) cc[o + 5 * k + c] = y[0][k];
+         if (PER && col) a[o + 5 * k + c] = y[PER ? 1 : 0][k];
+         P[k] = y[0][k];
+         if (PER) Q[k] = y[PER ? 1 : 0][k];
+         x[k] = xn[k];
+         y[0][k] = yn[k];
+      }
    }
-   {
-      const LU5 u = lu5_factor(&Bm(N - 1, 0, 0));
-      lu5_solve(u, &F(N - 1, 0), 1);
+   double z[5];   // the last row's solution, in every lane
+   if (PER) {
+      // last-row elimination and solve (triSolvers.cpp:671-749): lane c < 5
+      // carries column c of the row's c and b, lane 5 its f; row i's columns of
+      // c' and a' (lane 5: f) are loaded a row ahead
+      double t[5], Ci[5], Ai[5];
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+         t[k] = P[k];                                                // column c of c(N-1)
+         x[k] = c == 5 ? P[k] : (k == c) ? 1.0 : 0.0;                // f(N-1) | column c of the identity
+         Ci[k] = col ? cc[5 * k + c] : 0.0;
+         Ai[k] = col ? a[5 * k + c] : rhs ? f[k] : 0.0;
+      }
+      for (int i = 0; i < N - 1; i++) {
+         double M[25];
+#pragma unroll
+         for (int k = 0; k < 5; k++)
+#pragma unroll
+            for (int l = 0; l < 5; l++) M[5 * k + l] = from_lane(t[k], base + l);
+         double Cn[5], An[5];
+         const bool more = i + 1 < N - 1;
+         const size_t o = 25 * (size_t)(i + 1);
+#pragma unroll
+         for (int k = 0; k < 5; k++) {
+            Cn[k] = (col && more) ? cc[o + 5 * k + c] : 0.0;
+            An[k] = (col && more) ? a[o + 5 * k + c] : (rhs && more) ? f[5 * (i + 1) + k] : 0.0;
+            t[k] = 0.0;
+         }
+         sub_product5(t, M, Ci);
+         sub_product5(x, M, Ai);
+#pragma unroll
+         for (int k = 0; k < 5; k++) {
+            Ci[k] = Cn[k];
+            Ai[k] = An[k];
+         }
+      }
+      const size_t o = 25 * (size_t)(N - 1);
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+         if (col) cc[o + 5 * k + c] = t[k];
+         if (col) b[o + 5 * k + c] = x[k];
+      }
+      double U[10], none[1][5] = {{0.0, 0.0, 0.0, 0.0, 0.0}};
+      lu5_columns<1>(x, none, base, c, U);
+      lu5_back(x, U);   // lane 5: f(N-1)
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+         if (rhs) f[5 * (N - 1) + k] = x[k];
+         z[k] = from_lane(x[k], base + 5);
+      }
+   } else {
+#pragma unroll
+      for (int k = 0; k < 5; k++) z[k] = from_lane(P[k], base + 5);
    }
-   // back substitution (triSolvers.cpp:751-765)
-   for (int k = 0; k < 5; k++)
-      for (int j = 0; j < 5; j++) F(N - 2, k) -= (C(N - 2, k, j) * F(N - 1, j));
-   for (int i = N - 3; i >= 0; i--)
-      for (int k = 0; k < 5; k++)
-         for (int j = 0; j < 5; j++) F(i, k) -= (C(i, k, j) * F(i + 1, j) + A(i, k, j) * F(N - 1, j));
+   __syncwarp();
+   // back substitution (triSolvers.cpp:520-528, :751-765), lane c < 5 on row c
+   // of the blocks: f(i) -= c'(i) f(i+1), periodic f(i) -= (c'(i) f(i+1) + a'(i) f(N-1))
+   double zn[5], Cr[5], Ar[5], fi = 0.0;
+#pragma unroll
+   for (int j = 0; j < 5; j++) {
+      zn[j] = z[j];
+      Cr[j] = (col && N >= 2) ? cc[25 * (size_t)(N - 2) + 5 * c + j] : 0.0;
+      Ar[j] = 0.0;
+   }
+   if (col && N >= 2) fi = f[5 * (N - 2) + c];
+   for (int i = N - 2; i >= 0; i--) {
+      double Crn[5], Arn[5], fin = 0.0;
+      const bool more = col && i > 0;
+      const size_t o = 25 * (size_t)(i - (i > 0));
+#pragma unroll
+      for (int j = 0; j < 5; j++) {
+         Crn[j] = more ? cc[o + 5 * c + j] : 0.0;
+         Arn[j] = (PER && more) ? a[o + 5 * c + j] : 0.0;
+      }
+      if (more) fin = f[5 * (i - 1) + c];
+      double v = fi;
+#pragma unroll
+      for (int j = 0; j < 5; j++) {
+         const double p = Cr[j] * zn[j];
+         v -= (PER && i != N - 2) ? p + Ar[j] * z[j] : p;
+      }
+      if (col) f[5 * i + c] = v;
+#pragma unroll
+      for (int j = 0; j < 5; j++) {
+         zn[j] = from_lane(v, base + j);
+         Cr[j] = Crn[j];
+         Ar[j] = Arn[j];
+      }
+      fi = fin;
+   }
 }
 
 }  // namespace
@@ -390,7 +501,9 @@ int hamstr_gpu_block_tridag5(int nlines, int N, int periodic, double* A, double*
       return HAMSTR_GPU_ERR_ARG;
    }
    if (nlines == 0) return HAMSTR_GPU_OK;
-   block_tridag5_kernel<<<blocks(nlines), kThreads, 0, (cudaStream_t)stream>>>(nlines, N, periodic, A, B, C, F);
+   const unsigned nb = (unsigned)((nlines - 1) / kLinesPerWarp + 1);
+   if (periodic) block_tridag5_kernel<true><<<nb, 32, 0, (cudaStream_t)stream>>>(nlines, N, A, B, C, F);
+   else block_tridag5_kernel<false><<<nb, 32, 0, (cudaStream_t)stream>>>(nlines, N, A, B, C, F);
    return launched("block_tridag5");
 }
 
