@@ -16,7 +16,6 @@ extern "C" int hamstr_mlp_gemm(const void* A, const void* B, int M, int N, int K
    a.N = N;
    a.K = K;
    a.splits = splits;
-   a.mode = mlp::EPI_F32;
    a.C = C;
    a.err = err;
    return mlp::gemm(a, static_cast<cudaStream_t>(stream));

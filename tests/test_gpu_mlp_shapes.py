@@ -1,0 +1,56 @@
+"""The network's fused kernels at the edges of their tiles and variants.
+
+A row's output does not depend on the other rows or on which variant of the
+kernel carries its tile (one block to an SM up to one tile per SM, two
+beyond), so outputs of different calls are equal bit for bit; gradients are
+checked against the oracle as in test_gpu_mlp.py (2% in norm, BF16
+activations)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(n, seed):
+    import torch
+    rng = np.random.default_rng(seed)
+    f = rng.uniform(-1.5, 1.5, (n, 5)).astype(np.float32)
+    t = np.stack([np.sin(f[:, 0]), f[:, 1] * f[:, 3], np.cos(f[:, 4]), f[:, 2] ** 2], axis=1).astype(np.float32)
+    return f, t, torch.from_numpy(f).cuda(), torch.from_numpy(t).cuda()
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 1000, 19456, 19457, 45000])
+def test_forward_rows_do_not_depend_on_the_call(native_lib, n):
+    import torch
+    from hamstr_oop_gb300 import native
+    net = native.Mlp(batch_capacity=256, seed=3)
+    _, _, fd, _ = _rows(45000, 1)
+    y = net.forward(fd[:n].contiguous())
+    take = torch.unique(torch.cat([torch.arange(min(n, 200)), torch.arange(max(0, n - 200), n)]))
+    z = net.forward(fd[take.cuda()].contiguous())
+    assert torch.equal(y[take.cuda()], z)
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 300])
+def test_gradient_of_ragged_batches_matches_the_oracle(native_lib, oracle_lib, n):
+    from hamstr_oop_gb300 import native
+    net = native.Mlp(batch_capacity=384, seed=5)
+    f, t, fd, td = _rows(n, 7)
+    loss_o, g_o, _ = oracle_lib.mlp_loss_grad(net.get_params().astype(np.float64), f, t, bf16=True)
+    assert abs(net.grad(fd, td) - loss_o) <= 2e-3 * loss_o
+    g = net.get_grads().astype(np.float64)
+    bounds = np.cumsum([0, 1280, 256, 65536, 256, 65536, 256, 1024, 4])
+    for a, b in zip(bounds[:-1], bounds[1:]):
+        assert np.linalg.norm(g[a:b] - g_o[a:b]) <= 2e-2 * np.linalg.norm(g_o[a:b]), (a, b)
+
+
+def test_a_batch_below_capacity_trains_the_same(native_lib):
+    """4,864 rows use more splits of the weight gradients than 16,384 do."""
+    from hamstr_oop_gb300 import native
+    _, _, fd, td = _rows(9000, 9)
+    got = []
+    for capacity in (4864, 16384):
+        net = native.Mlp(batch_capacity=capacity, seed=2)
+        loss = [net.train_step(fd, td, batch=4864, seed=11, step=k, lr=1e-3) for k in range(2)]
+        got.append((loss, net.get_params()))
+    assert got[0][0] == got[1][0] and np.array_equal(got[0][1], got[1][1])
