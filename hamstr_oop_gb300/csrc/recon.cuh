@@ -273,34 +273,67 @@ __device__ __forceinline__ void muscl_deriv2(T fm1, T f0, T fp1, T fp2, T dm1, T
    }
 }
 
+// Below, 6 x is taken as twice 3 x and the factor 2 moved into the addition that
+// follows, so that it costs nothing.  That is exact where nothing in between is
+// subnormal.  In FP32 the weights' derivatives do reach that range (smoothness
+// sums of 1e-10 to the fourth power), and in FP64 they may where a caller's eps is
+// tiny (EXACT), so there the factors stay as written.
+template <typename T, bool EXACT>
+constexpr bool kAsWritten = EXACT || sizeof(T) == 4;
+
+// the differences d_k, e_k and the candidate stencils of five values
+// (reconstruction.cpp:84-104).  Every factor 2 or 4 goes into the addition it
+// feeds (add2); SC: the multiples 3, 5, 7, 11 on the integer pipes
+template <typename T>
+struct Weno5Diff {
+   T djm1, ejm1, dj, ej, djp1, ejp1, q30, q31, q32;
+};
+template <bool SC, typename T>
+__device__ __forceinline__ Weno5Diff<T> weno5_diff(T a, T b, T c, T d, T e)
+{
+   Weno5Diff<T> w;
+   const T c3 = pc<3, SC>(c);
+   w.djm1 = add2<1, -1>(b, a) + c;
+   w.ejm1 = add2<2, -1>(b, a) + c3;
+   w.dj = add2<1, -1>(c, b) + d;
+   w.ej = b - d;
+   w.djp1 = add2<1, -1>(d, c) + e;
+   w.ejp1 = add2<2, -1>(d, c3) + e;
+   w.q30 = add2<1>(a, -pc<7, SC>(b)) + pc<11, SC>(c);
+   w.q31 = add2<1>(d, -b + pc<5, SC>(c));
+   w.q32 = add2<1>(c, pc<5, SC>(d)) - e;
+   return w;
+}
+
+// a smoothness sum without its eps: b1 d d + 0.25 e e.  0.25 e e is formed as
+// 0.25 (e e): they differ only where e e is subnormal, which the eps (1e-15 or
+// 1e-10) added next absorbs
+template <bool SD, bool EXACT = false, typename T>
+__device__ __forceinline__ T weno5_smooth(T d, T e)
+{
+   const T s = pm<SD>(pm<SD>(T(13. / 12.), d), d);
+   if (kAsWritten<T, EXACT>) return s + pm<SD>(p2<-2, SD>(e), e);
+   return add2<-2>(pm<SD>(e, e), s);
+}
+
 // WENO5 (reconstruction.cpp:193-239); pow(x, 1) is x.  With SD the
-// multiplies run on the integer pipes (p2, pm: identical results)
+// multiplies run on the integer pipes (pc, pm: identical results)
 template <bool SD>
 __device__ __forceinline__ double weno5(double a, double b, double c, double d, double e)
 {
-   const double epsw = 1e-15;
-   const double b1 = 13. / 12., b2 = 1. / 6.;
-   const double c3 = pm<SD>(3., c);
-   const double djm1 = a - p2<1, SD>(b) + c;
-   const double ejm1 = a - p2<2, SD>(b) + c3;
-   const double dj = b - p2<1, SD>(c) + d;
-   const double ej = b - d;
-   const double djp1 = c - p2<1, SD>(d) + e;
-   const double ejp1 = c3 - p2<2, SD>(d) + e;
-   const double dis0 = pm<SD>(pm<SD>(b1, djm1), djm1) + pm<SD>(p2<-2, SD>(ejm1), ejm1) + epsw;
-   const double dis1 = pm<SD>(pm<SD>(b1, dj), dj) + pm<SD>(p2<-2, SD>(ej), ej) + epsw;
-   const double dis2 = pm<SD>(pm<SD>(b1, djp1), djp1) + pm<SD>(p2<-2, SD>(ejp1), ejp1) + epsw;
-   const double q30 = p2<1, SD>(a) - pm<SD>(7., b) + pm<SD>(11., c);
-   const double q31 = -b + pm<SD>(5., c) + p2<1, SD>(d);
-   const double q32 = p2<1, SD>(c) + pm<SD>(5., d) - e;
+   const double epsw = 1e-15, b2 = 1. / 6.;
+   const Weno5Diff<double> w = weno5_diff<SD>(a, b, c, d, e);
+   const double dis0 = weno5_smooth<SD>(w.djm1, w.ejm1) + epsw;
+   const double dis1 = weno5_smooth<SD>(w.dj, w.ej) + epsw;
+   const double dis2 = weno5_smooth<SD>(w.djp1, w.ejp1) + epsw;
    const double d01 = Dv<double, SD>(dis1).div(dis0);
    const double d02 = Dv<double, SD>(dis2).div(dis0);
-   const double a1ba0 = pm<SD>(6., d01);
-   const double a2ba0 = pm<SD>(3., d02);
-   const double w0 = Dv<double, SD>(1.0 + a1ba0 + a2ba0).div(1.0);
-   const double w1 = pm<SD>(a1ba0, w0);
-   const double w2 = 1. - w0 - w1;
-   return pm<SD>(b2, pm<SD>(w0, q30) + pm<SD>(w1, q31) + pm<SD>(w2, q32));
+   const double ha1 = pc<3, SD>(d01);   // half of a1ba0 = 6 d01: 6 x = 2 (3 x) exactly
+   const double a2ba0 = pc<3, SD>(d02);
+   const double w0 = Dv<double, SD>(add2<1>(ha1, 1.0) + a2ba0).div(1.0);
+   const double hw1 = pm<SD>(ha1, w0);  // half of w1
+   const double w2 = add2<1, -1>(hw1, 1. - w0);
+   return pm<SD>(b2, add2<1>(pm<SD>(hw1, w.q31), pm<SD>(w0, w.q30)) + pm<SD>(w2, w.q32));
 }
 
 // WENO_5 linearisation (reconstruction.cpp:358-462); the linear residual
@@ -348,14 +381,19 @@ __device__ __forceinline__ Weno5Lin<T> weno5_lin_get(const T* __restrict__ in, s
 // (eps added) and the candidate stencils; shared by weno5_lin_pre and
 // weno5_with_lin.  Each is an intermediate value of the reference's
 // expressions, formed the same way (b1 * 2 is exact).
-// The linearisation's multiplies: its divisions already load the integer
-// pipes, so only the increment part's first multiplies (candidate
-// stencils, the weight and smoothness derivative terms) go there with SD,
-// about half of them, and the rest stay on the FP64 pipe (all of them
-// there, or none, measured slower)
+// Which multiplies of the linearisation run on the integer pipes with SD (the
+// divisions are there too; results are the same): the candidate stencils'
+// constants, the constant 3 of the weights' derivatives, the products with the
+// weights' common denominator, and in weno5_with_lin the smoothness sums and
+// the final weighting.  A multiply costs there about what it costs on the FP64
+// pipe, so the split that fills both wins; the rest (kLinSoftMul) stay on the
+// FP64 pipe.  Measured, 512 x 128 half split, the two lin_recon5 launches of a
+// step: these 315 us, none 366, the candidate and smoothness terms as well 317,
+// all 380; recon5 157 us, without the final weighting 164, without the
+// smoothness sums either 175, without the constants too 187.
 constexpr bool kLinSoftMul = false;
 
-template <typename T, bool SD>
+template <typename T, bool SD, bool EXACT = false>
 __device__ __forceinline__ void weno5_lin_fill(Weno5Lin<T>& p, T djm1, T ejm1, T dj, T ej, T djp1, T ejp1)
 {
    const T b1 = T(13. / 12.), b2 = T(1. / 6.);
@@ -369,79 +407,87 @@ __device__ __forceinline__ void weno5_lin_fill(Weno5Lin<T>& p, T djm1, T ejm1, T
    const Dv<T, SD> r1(p.beta1), r2(p.beta2);
    const T d01 = r1.div(p.beta0);
    const T d02 = r2.div(p.beta0);
-   const T a1ba0 = pm<kLinSoftMul>(T(6.), d01);
-   const T a2ba0 = pm<kLinSoftMul>(T(3.), d02);
-   const T w0 = Dv<T, SD>(T(1.0) + a1ba0 + a2ba0).div(T(1.0));
-   const T w1 = pm<kLinSoftMul>(a1ba0, w0);
-   const T w2 = T(1.) - w0 - w1;
+   if constexpr (kAsWritten<T, EXACT>) {
+      const T a1ba0 = T(6.) * d01, a2ba0 = T(3.) * d02;
+      const T w0 = Dv<T, SD>(T(1.0) + a1ba0 + a2ba0).div(T(1.0));
+      const T w1 = a1ba0 * w0;
+      const T w2 = T(1.) - w0 - w1;
+      p.b2w0 = b2 * w0;
+      p.b2w1 = b2 * w1;
+      p.b2w2 = b2 * w2;
+      p.bb12 = p.beta1 * p.beta2;
+      p.dwd = p.bb12 + T(6) * p.beta0 * p.beta2 + T(3) * p.beta0 * p.beta1;
+      p.dwd2 = p.dwd * p.dwd;
+      return;
+   }
+   const T ha1 = pc<3, SD>(d01);   // half of a1ba0 = 6 d01
+   const T a2ba0 = pc<3, SD>(d02);
+   const T w0 = Dv<T, SD>(add2<1>(ha1, T(1.0)) + a2ba0).div(T(1.0));
+   const T hw1 = pm<kLinSoftMul>(ha1, w0);   // half of w1
+   const T w2 = add2<1, -1>(hw1, T(1.) - w0);
    p.b2w0 = pm<kLinSoftMul>(b2, w0);
-   p.b2w1 = pm<kLinSoftMul>(b2, w1);
+   p.b2w1 = p2<1, SD>(pm<kLinSoftMul>(b2, hw1));
    p.b2w2 = pm<kLinSoftMul>(b2, w2);
    p.bb12 = pm<kLinSoftMul>(p.beta1, p.beta2);
-   p.dwd = p.bb12 + pm<kLinSoftMul>(pm<kLinSoftMul>(T(6), p.beta0), p.beta2) + pm<kLinSoftMul>(pm<kLinSoftMul>(T(3), p.beta0), p.beta1);
+   const T b03 = pc<3, SD>(p.beta0);   // 6 beta0 is twice it
+   p.dwd = add2<1>(pm<kLinSoftMul>(b03, p.beta2), p.bb12) + pm<kLinSoftMul>(b03, p.beta1);
    p.dwd2 = pm<kLinSoftMul>(p.dwd, p.dwd);
 }
 
-template <typename T, bool SD>
-__device__ __forceinline__ Weno5Lin<T> weno5_lin_pre(T a, T b, T c, T d, T e)
+template <typename T, bool SD, bool EXACT = false>
+__device__ __forceinline__ Weno5Lin<T> weno5_lin_pre(T a, T b, T c, T d, T e, T epsw = T(1e-10))
 {
-   const T epsw = T(1e-10);
-   const T b1 = T(13. / 12.);
    Weno5Lin<T> p;
-   const T c3 = pm<kLinSoftMul>(T(3.), c);
-   const T djm1 = a - p2<1, SD>(b) + c;
-   const T ejm1 = a - p2<2, SD>(b) + c3;
-   const T dj = b - p2<1, SD>(c) + d;
-   const T ej = b - d;
-   const T djp1 = c - p2<1, SD>(d) + e;
-   const T ejp1 = c3 - p2<2, SD>(d) + e;
-   p.beta0 = pm<kLinSoftMul>(pm<kLinSoftMul>(b1, djm1), djm1) + pm<kLinSoftMul>(p2<-2, SD>(ejm1), ejm1) + epsw;
-   p.beta1 = pm<kLinSoftMul>(pm<kLinSoftMul>(b1, dj), dj) + pm<kLinSoftMul>(p2<-2, SD>(ej), ej) + epsw;
-   p.beta2 = pm<kLinSoftMul>(pm<kLinSoftMul>(b1, djp1), djp1) + pm<kLinSoftMul>(p2<-2, SD>(ejp1), ejp1) + epsw;
-   p.q30 = p2<1, SD>(a) - pm<kLinSoftMul>(T(7.), b) + pm<kLinSoftMul>(T(11.), c);
-   p.q31 = -b + pm<kLinSoftMul>(T(5.), c) + p2<1, SD>(d);
-   p.q32 = p2<1, SD>(c) + pm<kLinSoftMul>(T(5.), d) - e;
-   weno5_lin_fill<T, SD>(p, djm1, ejm1, dj, ej, djp1, ejp1);
+   const Weno5Diff<T> w = weno5_diff<SD>(a, b, c, d, e);
+   p.beta0 = weno5_smooth<kLinSoftMul, EXACT>(w.djm1, w.ejm1) + epsw;
+   p.beta1 = weno5_smooth<kLinSoftMul, EXACT>(w.dj, w.ej) + epsw;
+   p.beta2 = weno5_smooth<kLinSoftMul, EXACT>(w.djp1, w.ejp1) + epsw;
+   p.q30 = w.q30;
+   p.q31 = w.q31;
+   p.q32 = w.q32;
+   weno5_lin_fill<T, SD, EXACT>(p, w.djm1, w.ejm1, w.dj, w.ej, w.djp1, w.ejp1);
    return p;
 }
 
-template <typename T, bool SD>
+template <typename T, bool SD, bool EXACT = false>
 __device__ __forceinline__ T weno5_lin_apply(const Weno5Lin<T>& p, T a_d, T b_d, T c_d, T d_d, T e_d)
 {
    const T b2 = T(1. / 6.);
-   const T c3 = pm<SD>(T(3.), c_d);
-   const T djm1_d = a_d - p2<1, SD>(b_d) + c_d;
-   const T ejm1_d = a_d - p2<2, SD>(b_d) + c3;
-   const T dj_d = b_d - p2<1, SD>(c_d) + d_d;
-   const T ej_d = b_d - d_d;
-   const T djp1_d = c_d - p2<1, SD>(d_d) + e_d;
-   const T ejp1_d = c3 - p2<2, SD>(d_d) + e_d;
-   const T q30_d = p2<1, SD>(a_d) - pm<SD>(T(7.), b_d) + pm<SD>(T(11.), c_d);
-   const T q31_d = -b_d + pm<SD>(T(5.), c_d) + p2<1, SD>(d_d);
-   const T q32_d = p2<1, SD>(c_d) + pm<SD>(T(5.), d_d) - e_d;
-   const T term1 = pm<SD>(p.b2w0, q30_d);
-   const T term2 = pm<SD>(p.b2w1, q31_d);
-   const T term3 = pm<SD>(p.b2w2, q32_d);
-   const T dbeta0 = pm<SD>(p.cdjm1, djm1_d) + pm<SD>(p.cejm1, ejm1_d);
-   const T dbeta1 = pm<SD>(p.cdj, dj_d) + pm<SD>(p.cej, ej_d);
-   const T dbeta2 = pm<SD>(p.cdjp1, djp1_d) + pm<SD>(p.cejp1, ejp1_d);
+   const Weno5Diff<T> w = weno5_diff<SD>(a_d, b_d, c_d, d_d, e_d);
+   const T term1 = pm<kLinSoftMul>(p.b2w0, w.q30);
+   const T term2 = pm<kLinSoftMul>(p.b2w1, w.q31);
+   const T term3 = pm<kLinSoftMul>(p.b2w2, w.q32);
+   const T dbeta0 = pm<kLinSoftMul>(p.cdjm1, w.djm1) + pm<kLinSoftMul>(p.cejm1, w.ejm1);
+   const T dbeta1 = pm<kLinSoftMul>(p.cdj, w.dj) + pm<kLinSoftMul>(p.cej, w.ej);
+   const T dbeta2 = pm<kLinSoftMul>(p.cdjp1, w.djp1) + pm<kLinSoftMul>(p.cejp1, w.ejp1);
    const T beta0 = p.beta0, beta1 = p.beta1, beta2 = p.beta2;
    const T dw0_down = p.dwd;
    const T s12 = pm<kLinSoftMul>(dbeta1, beta2) + pm<kLinSoftMul>(beta1, dbeta2);
-   const T s6 = pm<kLinSoftMul>(T(6), pm<kLinSoftMul>(dbeta0, beta2) + pm<kLinSoftMul>(beta0, dbeta2));
-   const T s3 = pm<kLinSoftMul>(T(3), pm<kLinSoftMul>(dbeta0, beta1) + pm<kLinSoftMul>(beta0, dbeta1));
+   if constexpr (kAsWritten<T, EXACT>) {
+      const T s6 = T(6) * (dbeta0 * beta2 + beta0 * dbeta2);
+      const T s3 = T(3) * (dbeta0 * beta1 + beta0 * dbeta1);
+      const T up = p.bb12 * (s12 + s6 + s3);
+      const Dv<T, SD> rd(p.dwd2);
+      const T dw0 = rd.div(s12 * dw0_down - up);
+      const T dw1 = rd.div(s6 * dw0_down - Dv<T, SD>(beta1).div(T(6) * up) * beta0);
+      const T dw2 = rd.div(s3 * dw0_down - Dv<T, SD>(beta2).div(T(3) * up) * beta0);
+      return term1 + term2 + term3 + b2 * dw0 * p.q30 + b2 * dw1 * p.q31 + b2 * dw2 * p.q32;
+   }
+   const T h6 = pc<3, SD>(pm<kLinSoftMul>(dbeta0, beta2) + pm<kLinSoftMul>(beta0, dbeta2));
+   const T s3 = pc<3, SD>(pm<kLinSoftMul>(dbeta0, beta1) + pm<kLinSoftMul>(beta0, dbeta1));
    const T dw0_up_1 = pm<SD>(s12, dw0_down);
-   const T dw0_up_2 = pm<kLinSoftMul>(p.bb12, s12 + s6 + s3);
+   const T dw0_up_2 = pm<kLinSoftMul>(p.bb12, add2<1>(h6, s12) + s3);
    const Dv<T, SD> rd(p.dwd2);
    const T dw0 = rd.div(dw0_up_1 - dw0_up_2);
-   const T dw1_up_1 = pm<SD>(s6, dw0_down);
-   const T dw1_up_2 = pm<kLinSoftMul>(Dv<T, SD>(beta1).div(pm<kLinSoftMul>(T(6), dw0_up_2)), beta0);
-   const T dw1 = rd.div(dw1_up_1 - dw1_up_2);
+   const T dw1_up_1 = pm<SD>(h6, dw0_down);   // half of it
+   const T u3 = pc<3, SD>(dw0_up_2);
+   const T dw1_up_2 = pm<kLinSoftMul>(Dv<T, SD>(beta1).div(u3), beta0);   // half of it
+   const T dw1 = rd.div(dw1_up_1 - dw1_up_2);   // half of it
    const T dw2_up_1 = pm<SD>(s3, dw0_down);
-   const T dw2_up_2 = pm<kLinSoftMul>(Dv<T, SD>(beta2).div(pm<kLinSoftMul>(T(3), dw0_up_2)), beta0);
+   const T dw2_up_2 = pm<kLinSoftMul>(Dv<T, SD>(beta2).div(u3), beta0);
    const T dw2 = rd.div(dw2_up_1 - dw2_up_2);
-   return term1 + term2 + term3 + pm<kLinSoftMul>(pm<kLinSoftMul>(b2, dw0), p.q30) + pm<kLinSoftMul>(pm<kLinSoftMul>(b2, dw1), p.q31) +
-          pm<kLinSoftMul>(pm<kLinSoftMul>(b2, dw2), p.q32);
+   const T sum = term1 + term2 + term3 + pm<kLinSoftMul>(pm<kLinSoftMul>(b2, dw0), p.q30);
+   return add2<1>(pm<kLinSoftMul>(pm<kLinSoftMul>(b2, dw1), p.q31), sum) + pm<kLinSoftMul>(pm<kLinSoftMul>(b2, dw2), p.q32);
 }
 
 template <typename T, bool SD>
@@ -457,33 +503,26 @@ template <bool SD>
 __device__ __forceinline__ double weno5_with_lin(double a, double b, double c, double d, double e,
                                                  Weno5Lin<double>& p)
 {
-   const double b1 = 13. / 12., b2 = 1. / 6.;
-   const double c3 = pm<SD>(3., c);
-   const double djm1 = a - p2<1, SD>(b) + c;
-   const double ejm1 = a - p2<2, SD>(b) + c3;
-   const double dj = b - p2<1, SD>(c) + d;
-   const double ej = b - d;
-   const double djp1 = c - p2<1, SD>(d) + e;
-   const double ejp1 = c3 - p2<2, SD>(d) + e;
-   const double s0 = pm<SD>(pm<SD>(b1, djm1), djm1) + pm<SD>(p2<-2, SD>(ejm1), ejm1);
-   const double s1 = pm<SD>(pm<SD>(b1, dj), dj) + pm<SD>(p2<-2, SD>(ej), ej);
-   const double s2 = pm<SD>(pm<SD>(b1, djp1), djp1) + pm<SD>(p2<-2, SD>(ejp1), ejp1);
+   const double b2 = 1. / 6.;
+   const Weno5Diff<double> w = weno5_diff<SD>(a, b, c, d, e);
+   const double s0 = weno5_smooth<SD>(w.djm1, w.ejm1), s1 = weno5_smooth<SD>(w.dj, w.ej),
+                s2 = weno5_smooth<SD>(w.djp1, w.ejp1);
    const double dis0 = s0 + 1e-15, dis1 = s1 + 1e-15, dis2 = s2 + 1e-15;
-   p.q30 = p2<1, SD>(a) - pm<SD>(7., b) + pm<SD>(11., c);
-   p.q31 = -b + pm<SD>(5., c) + p2<1, SD>(d);
-   p.q32 = p2<1, SD>(c) + pm<SD>(5., d) - e;
+   p.q30 = w.q30;
+   p.q31 = w.q31;
+   p.q32 = w.q32;
    const double d01 = Dv<double, SD>(dis1).div(dis0);
    const double d02 = Dv<double, SD>(dis2).div(dis0);
-   const double a1ba0 = pm<kLinSoftMul>(6., d01);
-   const double a2ba0 = pm<kLinSoftMul>(3., d02);
-   const double w0 = Dv<double, SD>(1.0 + a1ba0 + a2ba0).div(1.0);
-   const double w1 = pm<kLinSoftMul>(a1ba0, w0);
-   const double w2 = 1. - w0 - w1;
+   const double ha1 = pc<3, SD>(d01);   // half of a1ba0
+   const double a2ba0 = pc<3, SD>(d02);
+   const double w0 = Dv<double, SD>(add2<1>(ha1, 1.0) + a2ba0).div(1.0);
+   const double hw1 = ha1 * w0;         // half of w1
+   const double w2 = add2<1, -1>(hw1, 1. - w0);
    p.beta0 = s0 + 1e-10;
    p.beta1 = s1 + 1e-10;
    p.beta2 = s2 + 1e-10;
-   weno5_lin_fill<double, SD>(p, djm1, ejm1, dj, ej, djp1, ejp1);
-   return pm<kLinSoftMul>(b2, pm<kLinSoftMul>(w0, p.q30) + pm<kLinSoftMul>(w1, p.q31) + pm<kLinSoftMul>(w2, p.q32));
+   weno5_lin_fill<double, SD>(p, w.djm1, w.ejm1, w.dj, w.ej, w.djp1, w.ejp1);
+   return pm<SD>(b2, add2<1>(pm<SD>(hw1, p.q31), pm<SD>(w0, p.q30)) + pm<SD>(w2, p.q32));
 }
 
 // reconstructed states at the two sides of a face slot, FP64

@@ -44,6 +44,7 @@ __device__ __forceinline__ bool roe_face(double nxd, double nyd, const double (&
    const double gm1 = gam - 1.0;
    const double area = sqrt(nxd * nxd + nyd * nyd);
    const Dv<double, SD> by_area(area);
+   const double half = p2<-1, SD>(area);   // 0.5 x area = x (0.5 area)
    const double invArea = by_area.div(1.);
    const double nx = nxd * invArea;
    const double ny = nyd * invArea;
@@ -52,13 +53,13 @@ __device__ __forceinline__ bool roe_face(double nxd, double nyd, const double (&
    const Dv<double, SD> by_rol(rol);
    const double ul = by_rol.div(ql[1]);
    const double vl = by_rol.div(ql[2]);
-   const double pl = gm1 * (ql[3] - p2<-1, SD>(rol) * (ul * ul + vl * vl));
+   const double pl = gm1 * add2<-1, -1>(rol * (ul * ul + vl * vl), ql[3]);
    const double hl = by_rol.div(ql[3] + pl);
    const double ror = qr[0];
    const Dv<double, SD> by_ror(ror);
    const double ur = by_ror.div(qr[1]);
    const double vr = by_ror.div(qr[2]);
-   const double pr = gm1 * (qr[3] - p2<-1, SD>(ror) * (ur * ur + vr * vr));
+   const double pr = gm1 * add2<-1, -1>(ror * (ur * ur + vr * vr), qr[3]);
    const double hr = by_ror.div(qr[3] + pr);
    const double dp = pr - pl;
    const double uconr = ur * nx + vr * ny;
@@ -72,7 +73,7 @@ __device__ __forceinline__ bool roe_face(double nxd, double nyd, const double (&
    const double ubar = ul * A + ur * B;
    const double vbar = vl * A + vr * B;
    const double hbar = hl * A + hr * B;
-   double cbar = gm1 * (hbar - p2<-1, SD>(ubar * ubar + vbar * vbar));
+   double cbar = gm1 * add2<-1, -1>(ubar * ubar + vbar * vbar, hbar);
    cbar = sqrt(cbar);
    const Dv<double, SD> by_c(cbar);
    const double uconbar = ubar * nx + vbar * ny;
@@ -83,7 +84,7 @@ __device__ __forceinline__ bool roe_face(double nxd, double nyd, const double (&
       const double eig3 = fabs(uconbar - cbar);
       double spec = eig1 + cbar;
       if (spec != spec) return false;
-      const double term1 = -eig1 + p2<-1, SD>(eig2 + eig3);
+      const double term1 = add2<-1>(eig2 + eig3, -eig1);
       const double term2 = p2<-1, SD>(eig2 - eig3);
       const double del1 = by_c.div(by_c.div(term1 * dp)) + by_c.div(term2 * robar * (uconr - uconl));
       const double del2 = term1 * (uconr - uconl) * robar + by_c.div(term2 * dp);
@@ -99,14 +100,10 @@ __device__ __forceinline__ bool roe_face(double nxd, double nyd, const double (&
       const double fl1 = rol * uconl * ul + nx * pl, fr1 = ror * uconr * ur + nx * pr;
       const double fl2 = rol * uconl * vl + ny * pl, fr2 = ror * uconr * vr + ny * pr;
       const double fl3 = (ql[3] + pl) * uconl, fr3 = (qr[3] + pr) * uconr;
-      o.flux[0] = p2<-1, SD>(fl0 + fr0 - fm0);
-      o.flux[1] = p2<-1, SD>(fl1 + fr1 - fm1);
-      o.flux[2] = p2<-1, SD>(fl2 + fr2 - fm2);
-      o.flux[3] = p2<-1, SD>(fl3 + fr3 - fm3);
-      o.flux[0] *= area;
-      o.flux[1] *= area;
-      o.flux[2] *= area;
-      o.flux[3] *= area;
+      o.flux[0] = (fl0 + fr0 - fm0) * half;
+      o.flux[1] = (fl1 + fr1 - fm1) * half;
+      o.flux[2] = (fl2 + fr2 - fm2) * half;
+      o.flux[3] = (fl3 + fr3 - fm3) * half;
       spec *= area;
       o.spec = spec;
    }
@@ -121,7 +118,7 @@ __device__ __forceinline__ bool roe_face(double nxd, double nyd, const double (&
    const double e1 = fabs(uconbarj);
    const double e2 = fabs(uconbarj + cbar);
    const double e3 = fabs(uconbarj - cbar);
-   const double t1 = -e1 + p2<-1, SD>(e2 + e3);
+   const double t1 = add2<-1>(e2 + e3, -e1);
    const double t2 = p2<-1, SD>(e2 - e3);
    const double t2rb = t2 * robar;
 
@@ -130,7 +127,8 @@ __device__ __forceinline__ bool roe_face(double nxd, double nyd, const double (&
    const double du0l = by_rol.div(-ul);
    const double irl = by_rol.div(1.0);
    const double dv0l = by_rol.div(-vl);
-   const double dp0l = p2<-1, SD>(gm1) * (ul * ul + vl * vl);
+   const double hgm1 = p2<-1, SD>(gm1);
+   const double dp0l = hgm1 * (ul * ul + vl * vl);
    const double dp1l = -gm1 * ul;
    const double dp2l = -gm1 * vl;
    const double dc0l = by_rol.div(-uconlj);
@@ -140,7 +138,7 @@ __device__ __forceinline__ bool roe_face(double nxd, double nyd, const double (&
    const double du0r = by_ror.div(-ur);
    const double irr = by_ror.div(1.0);
    const double dv0r = by_ror.div(-vr);
-   const double dp0r = p2<-1, SD>(gm1) * (ur * ur + vr * vr);
+   const double dp0r = hgm1 * (ur * ur + vr * vr);
    const double dp1r = -gm1 * ur;
    const double dp2r = -gm1 * vr;
    const double dc0r = by_ror.div(-uconrj);
@@ -157,15 +155,15 @@ __device__ __forceinline__ bool roe_face(double nxd, double nyd, const double (&
    D2l[0] = mt1 * dc0l * robar - by_c.div(t2 * dp0l);
    D2l[1] = mt1 * dc1l * robar - by_c.div(t2 * dp1l);
    D2l[2] = mt1 * dc2l * robar - by_c.div(t2 * dp2l);
-   D2l[3] = -by_c.div(t2 * gm1);
    D1r[0] = by_c.div(by_c.div(t1 * dp0r)) + by_c.div(t2rb * dc0r);
    D1r[1] = by_c.div(by_c.div(t1 * dp1r)) + by_c.div(t2rb * dc1r);
    D1r[2] = by_c.div(by_c.div(t1 * dp2r)) + by_c.div(t2rb * dc2r);
-   D1r[3] = by_c.div(by_c.div(t1 * gm1));
+   D1r[3] = -D1l[3];   // the same products with the sign of t1
    D2r[0] = t1 * dc0r * robar + by_c.div(t2 * dp0r);
    D2r[1] = t1 * dc1r * robar + by_c.div(t2 * dp1r);
    D2r[2] = t1 * dc2r * robar + by_c.div(t2 * dp2r);
    D2r[3] = by_c.div(t2 * gm1);
+   D2l[3] = -D2r[3];
 
    // native flux Jacobians (jacobianRoe.cpp:573-605), kept rows/columns
    const double el = ql[3] + pl, er = qr[3] + pr;
@@ -225,8 +223,8 @@ __device__ __forceinline__ bool roe_face(double nxd, double nyd, const double (&
                mr = D1r[c] * rowc[rI] + D2r[c] * rown[rI];
             }
          }
-         lm[4 * rI + c] = p2<-1, SD>(L1[4 * rI + c] - ml) * area;
-         rm[4 * rI + c] = p2<-1, SD>(R1[4 * rI + c] - mr) * area;
+         lm[4 * rI + c] = (L1[4 * rI + c] - ml) * half;
+         rm[4 * rI + c] = (R1[4 * rI + c] - mr) * half;
       }
    }
    return true;

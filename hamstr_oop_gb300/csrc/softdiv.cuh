@@ -290,6 +290,33 @@ __host__ __device__ __forceinline__ double mul(double a, double b)
    return from_bits(sign | ((uint64_t)e << 52) | (m & kMant));
 }
 
+// x * C for a small odd C (3, 5, 7, 11) on the integer pipes, equal to the FP64
+// multiply: the product of the significand fits one word, so it costs about
+// half of mul
+#ifdef __CUDA_ARCH__
+__device__ __noinline__ double mulc_other(double x, double c) { return x * c; }
+#else
+inline double mulc_other(double x, double c) { return x * c; }
+#endif
+
+template <int C>
+__host__ __device__ __forceinline__ double mulc(double x)
+{
+   static_assert(C == 3 || C == 5 || C == 7 || C == 11, "small odd constants");
+   constexpr int kShift = C == 3 ? 1 : C == 11 ? 3 : 2;   // floor(log2 C)
+   const uint64_t u = bits(x);
+   const uint32_t e = (uint32_t)(u >> 52) & 0x7FFu;
+   if (e - 1u >= 0x7FAu) {   // zero, subnormal, inf, NaN, or a product that may overflow
+      if ((u << 1) == 0) return x;
+      return mulc_other(x, (double)C);
+   }
+   uint64_t p = ((u & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) * (uint64_t)C;
+   const int s = kShift + (int)(p >> (53 + kShift));
+   p += (1ull << (s - 1)) - 1 + ((p >> s) & 1);   // to nearest even
+   const uint64_t m = p >> s;                      // 2^53 carries into the exponent
+   return from_bits((u & 0x8000000000000000ull) | (((uint64_t)(e + s - 1) << 52) + m));
+}
+
 // 0.0 + v (sub false) or 0.0 - v (sub true) on the integer pipes, equal to
 // the FP64 add: +-v with the sign flipped for sub, except that a zero v
 // gives +0.0 either way
@@ -312,6 +339,39 @@ template <bool SOFT>
 __host__ __device__ __forceinline__ float pm(float a, float b)
 {
    return a * b;
+}
+
+// C * x for a small odd C, as pm
+template <int C, bool SOFT>
+__host__ __device__ __forceinline__ double pc(double x)
+{
+   return SOFT ? sd::mulc<C>(x) : (double)C * x;
+}
+template <int C, bool SOFT>
+__host__ __device__ __forceinline__ float pc(float x)
+{
+   return (float)C * x;
+}
+
+// 2^K x + y with one rounding of the sum: the product is exact wherever it
+// neither overflows nor turns subnormal, so this is the reference's multiply
+// and add, in one FP64 instruction instead of one and a scaling on the integer
+// pipes.  S = -1: y - 2^K x.
+template <int K, int S = 1>
+__host__ __device__ __forceinline__ double add2(double x, double y)
+{
+   constexpr double kScale = S * (K >= 0 ? double(1ull << (K >= 0 ? K : 0)) : 1.0 / double(1ull << (K < 0 ? -K : 0)));
+#ifdef __CUDA_ARCH__
+   return __fma_rn(kScale, x, y);
+#else
+   return kScale * x + y;
+#endif
+}
+template <int K, int S = 1>
+__host__ __device__ __forceinline__ float add2(float x, float y)
+{
+   constexpr float kScale = S * (K >= 0 ? float(1u << (K >= 0 ? K : 0)) : 1.0f / float(1u << (K < 0 ? -K : 0)));
+   return kScale * x + y;
 }
 
 // x * 2^K in the reconstructions: with SOFT (FP64 only) on the integer
