@@ -663,6 +663,7 @@ int hamstr::create_gpu(const hamstr_gpu_params* p, int nCell, int nFace, const i
       if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm <= 0) nsm = 1;
       if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) optin = 0;
       d.exclusive_smem = adi_configure(optin);
+      d.nsm = nsm;
       d.face_block = 256;
       d.adi_wpb = 4;
       d.adi_fwpb = 4;

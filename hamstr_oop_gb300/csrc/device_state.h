@@ -111,7 +111,8 @@ struct DeviceState {
    int exclusive_smem;     // dynamic shared memory that keeps ADI blocks one per SM
 
    // launch shapes chosen by hamstr_gpu_autotune (host-side only)
-   int face_block;         // threads per block of the face kernels (<= 256)
+   int nsm;                // SMs of the device
+   int face_block;         // threads per block of the face kernels on large meshes (face_threads)
    int adi_wpb;            // warps per block (= per SM) of the persistent FP64 solve kernel (4 or 8)
    int adi_fwpb;           // the same for the FP64 factorisation kernel
    int mx_block;           // threads per block of the FP32 thread-per-chain line kernels
@@ -195,6 +196,28 @@ __device__ __forceinline__ int norm_cell(const DeviceState& d)
    const int c = cb.x + (int)threadIdx.x;
    if (d.nInst > 1 && d.inst_done[d.block_inst[blockIdx.x]] != 0) return -1;
    return c < cb.y ? c : -1;
+}
+
+// Threads per block of a launch of one thread per face slot.  The face kernels
+// are bound by each SM's FP64 issue, so a launch lasts as long as its fullest
+// SM: of the tuned block and 64 and 32 threads, the one whose blocks, dealt out
+// evenly, load it least (the larger one where they tie).  164,399 slots: 256
+// threads put 5 blocks on the fullest SM for 4.2 on average, 64 put 17 for 16.9
+// (rhs_face 204 -> 183 us); 8,320 slots: 256 threads use 33 of 152 SMs, 32 all of
+// them (rhs_face 65 -> 38 us).
+inline int face_threads(const DeviceState& d)
+{
+   const int nsm = d.nsm > 0 ? d.nsm : 1;
+   int best = 0;
+   long long least = 0;
+   for (int t : {d.face_block, 64, 32}) {
+      const long long load = (((d.nSlot + t - 1) / t + nsm - 1) / nsm) * (long long)t;
+      if (best == 0 || 50 * load < 49 * least) {
+         best = t;
+         least = load;
+      }
+   }
+   return best;
 }
 
 // launchers (rhs.cu)

@@ -28,16 +28,17 @@ constexpr int kThreads = 256;
 static_assert(kThreads == kNormBlock, "cell kernels run one norm block per thread block");
 
 // ---------------- residual + FP32 Jacobian ----------------
+constexpr int kFaceSmem = 9 * 16 + 16;
 // PRE: the order-5 face states come from recon5_kernel
 template <int ORDER, bool SD, bool PRE = false>
 __global__ void __launch_bounds__(kThreads) mx_rhs_face_kernel(DeviceState d)
 {
    // the FP32 Jacobians leave through shared memory, so their stores are
    // whole lines (8 float4 per slot, consecutive slots; row stride 9)
-   __shared__ float4 sj[kThreads * 9];
-   __shared__ unsigned char live[kThreads];
-   if (halted(d)) return;
+   extern __shared__ float4 sj[];   // kFaceSmem bytes a thread
    const int nb = blockDim.x, s0 = blockIdx.x * nb, s = s0 + threadIdx.x;
+   unsigned char* live = reinterpret_cast<unsigned char*>(sj + 9 * nb);
+   if (halted(d)) return;
    const bool act = s < d.nSlot && !frozen_slot(d, s);
    live[threadIdx.x] = act ? 1 : 0;
    if (act) {
@@ -1558,21 +1559,21 @@ template <bool SD>
 void mx_rhs_face_go(const DeviceState& d, int b, int t, cudaStream_t st)
 {
    switch (d.recon) {
-      case 1: mx_rhs_face_kernel<1, SD><<<b, t, 0, st>>>(d); break;
-      case 3: mx_rhs_face_kernel<3, SD><<<b, t, 0, st>>>(d); break;
+      case 1: mx_rhs_face_kernel<1, SD><<<b, t, kFaceSmem * t, st>>>(d); break;
+      case 3: mx_rhs_face_kernel<3, SD><<<b, t, kFaceSmem * t, st>>>(d); break;
       case 5:
-         if (d.qface) mx_rhs_face_kernel<5, SD, true><<<b, t, 0, st>>>(d);
-         else mx_rhs_face_kernel<5, SD><<<b, t, 0, st>>>(d);
+         if (d.qface) mx_rhs_face_kernel<5, SD, true><<<b, t, kFaceSmem * t, st>>>(d);
+         else mx_rhs_face_kernel<5, SD><<<b, t, kFaceSmem * t, st>>>(d);
          break;
-      case 31: mx_rhs_face_kernel<31, SD><<<b, t, 0, st>>>(d); break;
-      default: mx_rhs_face_kernel<32, SD><<<b, t, 0, st>>>(d); break;
+      case 31: mx_rhs_face_kernel<31, SD><<<b, t, kFaceSmem * t, st>>>(d); break;
+      default: mx_rhs_face_kernel<32, SD><<<b, t, kFaceSmem * t, st>>>(d); break;
    }
 }
 }  // namespace
 
 void launch_mx_rhs_face(const DeviceState& d, cudaStream_t st)
 {
-   const int t = d.face_block;
+   const int t = face_threads(d);
    const int b = (d.nSlot + t - 1) / t;
    if (d.face_soft) mx_rhs_face_go<true>(d, b, t, st);
    else mx_rhs_face_go<false>(d, b, t, st);

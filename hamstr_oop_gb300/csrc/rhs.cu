@@ -354,7 +354,7 @@ void launch_recon5(const DeviceState& d, bool keep_lin, cudaStream_t st)
 
 void launch_rhs_face(const DeviceState& d, bool jac, cudaStream_t st)
 {
-   const int t = d.face_block;
+   const int t = face_threads(d);
    const int b = (d.nSlot + t - 1) / t;
    if (d.face_soft) rhs_face_go<true>(d, jac, b, t, st);
    else rhs_face_go<false>(d, jac, b, t, st);
@@ -382,7 +382,7 @@ void launch_lin_recon5(const DeviceState& d, bool kept, cudaStream_t st)
 
 void launch_lin_face(const DeviceState& d, cudaStream_t st)
 {
-   const int kThreads = d.face_block;
+   const int kThreads = face_threads(d);
    const int b = (d.nSlot + kThreads - 1) / kThreads;
    // only the WENO linearisation divides in FP64 here
    if (d.lin_order == 1) {
