@@ -111,7 +111,7 @@ struct hamstr_gpu {
    double* wall_scr = nullptr;          // device: 3 per wall face + 3 sums per instance
 
    int nsm = 1;                         // SMs of the device (persistent-warp schedules)
-   int adi_lanes = 4;                   // lanes per open chain in the FP64 line kernels: 32, 16 or 4
+   int adi_lanes = 16;                  // lanes per open chain in the FP64 line kernels: 32, 16 or 4
    int adi_bundle = 0;                  // open chains of up to this many rows one per lane (0: none)
    int adi_fuse = 1;                    // first wave's first-sweep solve inside the factorisation kernel
    // order 5, FP64: the WENO linearisation's f-only values kept from the
@@ -483,6 +483,38 @@ int hamstr_gpu_create(const hamstr_gpu_params* p, int nCell, int nFace, const in
 
 }  // extern "C"
 
+namespace {
+// How the FP64 line kernels pack open chains before any tuning.
+//   lanes    16 (two chains to a warp) is the shorter recurrence by far: a row
+//            takes some 3,700 cycles of a pair's factorisation and 16,800 of a
+//            group of eight's (4 lanes each).  Only where pairs would queue
+//            several deep on every SM sub-partition does the groups' solve pay:
+//            31 conditions in a batch (754 rows of open chains per pair slot,
+//            the longest 128) 4.0 against 5.7 ms, 8 conditions (202) 2.2 against
+//            2.3 the other way, with the factorisation 3.7 against 3.2.
+//   bundle   chains of up to 8 rows one per lane: the fewest FP64 instructions a
+//            row, but a bundle's rows run one after the other.  Factorisation
+//            and solves of a step, with / without: 33,327 chains 0.40 / 0.69 ms,
+//            20,046 0.73 / 0.80, 8,420 0.28 / 0.25, 551 0.22 / 0.16, so from 24
+//            chains to a sub-partition on.
+void default_line_packing(const Plan& P, int nsm, int* lanes, int* bundle)
+{
+   const long long slots = 4LL * nsm;   // SM sub-partitions
+   long long open = 0, rows = 0;
+   int longest = 0;
+   for (int c = 0; c < P.nChain; c++) {
+      if (P.chain_periodic[c]) continue;
+      open++;
+      longest = std::max(longest, P.chain_nrows[c]);
+   }
+   *bundle = open >= 24 * slots && P.nRow < 16 * (long long)P.nChain ? 8 : 0;
+   for (int c = 0; c < P.nChain; c++)
+      if (!P.chain_periodic[c] && P.chain_nrows[c] > *bundle) rows += P.chain_nrows[c];
+   *lanes = rows > 3 * 2 * slots * longest ? 4 : 16;
+}
+
+}  // namespace
+
 int hamstr::create_gpu(const hamstr_gpu_params* p, int nCell, int nFace, const int* faces, const double* normVec,
                        const double* refMtx, int nChain, const int* faceStartPerChain, const int* chainConn,
                        const InstanceInfo* inst, hamstr_gpu** out)
@@ -675,9 +707,7 @@ int hamstr::create_gpu(const hamstr_gpu_params* p, int nCell, int nFace, const i
       d.face_soft = 1;
       d.piv_soft = 1;   // sd::rcp: shorter latency than the hardware sequence, and off the FP64 pipe
       g->nsm = nsm;
-      // the shortest open chains one per lane where chains are short (the
-      // autotuner checks the alternatives)
-      g->adi_bundle = (P.nChain > 0 && P.nRow < 16 * P.nChain) ? 8 : 0;
+      default_line_packing(P, nsm, &g->adi_lanes, &g->adi_bundle);
       g->sched = build_schedule(P, d.adi_wpb * nsm, g->adi_lanes, g->adi_bundle, g->adi_fuse != 0, d.adi_fwpb * nsm,
                                 nsm);
    }
