@@ -118,7 +118,7 @@ struct hamstr_gpu {
    // implicit computeRHS for the sweeps (d.wlin points here when on)
    double* wlin_buf = nullptr;
    int weno_keep = 1;
-   int mx_chunk = 1;                    // FP32 solve: rows loaded in chunks where a wave's chains all fit
+   int mx_chunk = 1;                    // FP32 last-row elimination: rows loaded in chunks where all chains fit
    std::vector<int> sp_wave_ptr;        // segmented FP32 solve: spike chains of each wave (host copy)
    bool wlin_valid = false;             // kept values match the current q (standalone entry points)
 
@@ -484,6 +484,23 @@ int hamstr_gpu_create(const hamstr_gpu_params* p, int nCell, int nFace, const in
 }  // extern "C"
 
 namespace {
+// FP32 assembly inside the factorisation (1), or by a kernel of its own (0).  Of
+// its own it costs a pass over the blocks, some 0.2 ns a row; inside, a row of a
+// chain takes 1.8 us instead of 0.6 us, as its terms are behind two lookups, and
+// the longest chain that one thread walks sets the time (long periodic chains go
+// by segments).  Assembly and factorisation, own / inside: 512 x 128 0.11 / 0.23
+// ms, the same mesh 30% split 0.11 / 0.21 ms, 32 meshes of 983,040 cells in all
+// 0.44 / 0.27 ms.  Short chains fill the GPU either way and save the terms' lookups;
+// above 2^22 rows of longer chains the blocks (192 bytes a row) are not kept.
+int default_mx_fused(const Plan& P)
+{
+   long long longest = 0;
+   for (int c = 0; c < P.nChain; c++)
+      if (!P.chain_periodic[c]) longest = std::max(longest, (long long)P.chain_nrows[c]);
+   const long long rows = P.nRow;
+   return P.nChain > 0 && rows >= 16ll * P.nChain && rows > std::min(5000 * longest, 1ll << 22) ? 1 : 0;
+}
+
 // How the FP64 line kernels pack open chains before any tuning.
 //   lanes    16 (two chains to a warp) is the shorter recurrence by far: a row
 //            takes some 3,700 cycles of a pair's factorisation and 16,800 of a
@@ -699,11 +716,13 @@ int hamstr::create_gpu(const hamstr_gpu_params* p, int nCell, int nFace, const i
       d.face_block = 256;
       d.adi_wpb = 4;
       d.adi_fwpb = 4;
-      d.mx_block = 64;
+      d.mx_fused = default_mx_fused(P);
+      // one warp a block reaches the most SMs (a 512 x 128 march 4.14 ms, 4.18 and
+      // 4.29 with two and four); with the assembly inside, two leave the chains by
+      // segments beside it more room (32 meshes: 8.76 ms, 10.0 with one, 8.77 with four)
+      d.mx_block = d.mx_fused ? 64 : 32;
       d.mx_chunk_chains = mx_solve_chunk_capacity(d.mx_block);
       d.sp_on = 1;   // long periodic chains of the FP32 form by segments (2: long open ones too)
-      // FP32 assembly inside the factorisation pays off on long chains
-      d.mx_fused = (P.nChain > 0 && P.nRow >= 16 * P.nChain) ? 1 : 0;
       d.face_soft = 1;
       d.piv_soft = 1;   // sd::rcp: shorter latency than the hardware sequence, and off the FP64 pipe
       g->nsm = nsm;

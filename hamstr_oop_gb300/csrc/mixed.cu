@@ -83,51 +83,6 @@ __global__ void __launch_bounds__(kThreads) mx_init_kernel(DeviceState d)
    st4(d.dq32 + 4 * (size_t)c, z);
 }
 
-// FP32 blocks in the reference's term order (ADI.cpp:62-217), one thread
-// per block entry (coalesced); the unfused alternative to mx_row below,
-// faster where chains are short (the autotuner picks)
-__global__ void __launch_bounds__(kThreads) mx_assemble_kernel(DeviceState d)
-{
-   // one thread per tiled entry (DeviceState: blk32), in memory order, so
-   // stores are whole lines: t = tix(srow, 48, e48, lane)
-   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-   if (t >= 48 * 32 * (size_t)d.tile_rows || halted(d)) return;
-   const int lane = (int)((t >> 2) & 31);
-   const size_t g = t >> 7;
-   const int e48 = (int)(g % 12) * 4 + (int)(t & 3), srow = (int)(g / 12), b = e48 >> 4, e = e48 & 15;
-   const int row = d.tile_row[32 * (size_t)srow + lane];
-   if (row < 0 || frozen_cell(d, d.row_scell[row])) return;
-   const int* ops = d.row_ops + 3 * kOpsPerBlock * row + kOpsPerBlock * b;
-   float acc = 0.f;
-#pragma unroll
-   for (int o = 0; o < kOpsPerBlock; o++) {
-      const int op = ops[o];
-      if (op < 0) break;
-      const int slot = op >> 3, sel = (op >> 1) & 3, col = e & 3;
-      const float* m = d.ff32 + 32 * (size_t)slot;
-      float v;
-      if (sel == OP_SEL_RREFL && (col == 1 || col == 2)) {
-         const double4 rf = d.refl[d.slot_face[slot]];
-         const float r01 = m[16 + (e & ~3) + 1], r02 = m[16 + (e & ~3) + 2];
-         v = (col == 1) ? (float(rf.x) * r01 + float(rf.y) * r02) : (float(rf.z) * r01 + float(rf.w) * r02);
-      } else {
-         v = m[(sel == OP_SEL_L ? 0 : 16) + e];
-      }
-      if (op & 1) acc -= v;
-      else acc += v;
-   }
-   acc *= float(d.dtfac[d.row_scell[row]]);
-   if (b == 1 && (e >> 2) == (e & 3)) acc += 1.f;
-   d.blk32[t] = acc;
-}
-
-// whether chain ich takes the segmented solve: sp_on 1 takes the long
-// periodic chains, 2 the long open ones as well
-__device__ __forceinline__ bool spike_active(const DeviceState& d, int ich)
-{
-   return d.sp_on && d.chain_spike[ich] >= 0 && (d.sp_on == 2 || d.chain_periodic[ich]);
-}
-
 // the tiled index of element e of tile row s in lane `lane` of a W-wide
 // array (W a multiple of 4): each lane's elements 4k .. 4k+3 are one float4,
 // and the 32 lanes' float4 of one group lie together, so a warp's access of
@@ -135,6 +90,64 @@ __device__ __forceinline__ bool spike_active(const DeviceState& d, int ich)
 __device__ __forceinline__ size_t tix(int s, int W, int e, int lane)
 {
    return (((size_t)s * W + (e & ~3)) << 5) + 4 * lane + (e & 3);
+}
+
+// FP32 blocks in the reference's term order (ADI.cpp:62-217), one thread per
+// row of a block (a float4 of every term, the term list and the scale once for
+// the four entries); the unfused alternative to mx_row below (the autotuner
+// picks).  Bound by the latency of the term lists' gathers.  512 x 128, 30%
+// split: 70 us with a thread per entry, 29 us so (31 us with a warp on one row k
+// of 32 lanes; 32 meshes of 983,040 cells 425 us that way, 349 us so).
+__global__ void __launch_bounds__(kThreads) mx_assemble_kernel(DeviceState d)
+{
+   // a warp: eight lanes of a tile row times the four rows k of one block, so
+   // that a term's block is 64 contiguous bytes of four neighbouring lanes and
+   // a store fills four whole lines of 128 bytes
+   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+   if (t >= 12 * 32 * (size_t)d.tile_rows || halted(d)) return;
+   const int k = (int)(t & 3);
+   const size_t g = t >> 7;
+   const int lane = (int)((t >> 2) & 31), b = (int)(g % 3), srow = (int)(g / 3);
+   const int row = d.tile_row[32 * (size_t)srow + lane];
+   if (row < 0) return;
+   const int sc = d.row_scell[row];
+   if (frozen_cell(d, sc)) return;
+   const int4 list = *reinterpret_cast<const int4*>(d.row_ops + 3 * kOpsPerBlock * (size_t)row + kOpsPerBlock * b);
+   const int ops[kOpsPerBlock] = {list.x, list.y, list.z, list.w};
+   float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+   for (int o = 0; o < kOpsPerBlock; o++) {
+      const int op = ops[o];
+      if (op < 0) break;
+      const int slot = op >> 3, sel = (op >> 1) & 3;
+      float v[4];
+      ld4(d.ff32 + 32 * (size_t)slot + (sel == OP_SEL_L ? 0 : 16) + 4 * k, v);
+      if (sel == OP_SEL_RREFL) {
+         const double4 rf = d.refl[d.slot_face[slot]];
+         const float r01 = v[1], r02 = v[2];
+         v[1] = float(rf.x) * r01 + float(rf.y) * r02;
+         v[2] = float(rf.z) * r01 + float(rf.w) * r02;
+      }
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+         if (op & 1) acc[m] -= v[m];
+         else acc[m] += v[m];
+      }
+   }
+   const float s = float(d.dtfac[sc]);
+#pragma unroll
+   for (int m = 0; m < 4; m++) {
+      acc[m] *= s;
+      if (b == 1 && m == k) acc[m] += 1.f;
+   }
+   st4(d.blk32 + tix(srow, 48, 16 * b + 4 * k, lane), acc);
+}
+
+// whether chain ich takes the segmented solve: sp_on 1 takes the long
+// periodic chains, 2 the long open ones as well
+__device__ __forceinline__ bool spike_active(const DeviceState& d, int ich)
+{
+   return d.sp_on && d.chain_spike[ich] >= 0 && (d.sp_on == 2 || d.chain_periodic[ich]);
 }
 
 // 16 consecutive elements of a tiled record (4 float4, 128 floats apart: each load of
@@ -216,6 +229,14 @@ __device__ __forceinline__ LUf luf_load(const float* p)
       const float4 a = *reinterpret_cast<const float4*>(p + m);
       v[m] = a.x; v[m + 1] = a.y; v[m + 2] = a.z; v[m + 3] = a.w;
    }
+   LUf u;
+   u.p0 = v[0]; u.u01 = v[1]; u.u02 = v[2]; u.u03 = v[3]; u.l10 = v[4]; u.p1 = v[5]; u.u12 = v[6]; u.u13 = v[7];
+   u.l20 = v[8]; u.l21 = v[9]; u.p2 = v[10]; u.u23 = v[11]; u.l30 = v[12]; u.l31 = v[13]; u.l32 = v[14]; u.p3 = v[15];
+   return u;
+}
+
+__device__ __forceinline__ LUf luf_of(const float (&v)[16])
+{
    LUf u;
    u.p0 = v[0]; u.u01 = v[1]; u.u02 = v[2]; u.u03 = v[3]; u.l10 = v[4]; u.p1 = v[5]; u.u12 = v[6]; u.u13 = v[7];
    u.l20 = v[8]; u.l21 = v[9]; u.p2 = v[10]; u.u23 = v[11]; u.l30 = v[12]; u.l31 = v[13]; u.l32 = v[14]; u.p3 = v[15];
@@ -351,23 +372,6 @@ __device__ __forceinline__ void mx_row_ref(const DeviceState& d, const RowRef& r
    for (int k = 0; k < 4; k++) B[5 * k] += 1.f;
 }
 
-// FUSED: each thread builds its chain's blocks straight from the FP32 face
-// Jacobians (no block array round trip; best for long chains) from the
-// references r of the row; otherwise it reads the blocks mx_assemble_kernel
-// wrote (tile row s, its lane)
-template <bool FUSED>
-__device__ __forceinline__ void mx_rows(const DeviceState& d, const RowRef& r, int s, int lane, float (&A)[16],
-                                        float (&B)[16], float (&C)[16])
-{
-   if (FUSED) {
-      mx_row_ref(d, r, A, B, C);
-   } else {
-      ld16t(d.blk32 + tix(s, 48, 0, lane), A);
-      ld16t(d.blk32 + tix(s, 48, 16, lane), B);
-      ld16t(d.blk32 + tix(s, 48, 32, lane), C);
-   }
-}
-
 // ---- fused assembly with the next row's terms staged in shared memory ----
 // Each of a row's up to 3 x kOpsPerBlock face-Jacobian terms is a 64-byte
 // block of ff32.  Summing them as they arrive makes the row wait on one
@@ -387,6 +391,50 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
+// all but the newest N groups of this thread's copies have arrived
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// copies through L2 only: the rows are read once
+__device__ __forceinline__ void cp_async16_cg(void* smem, const void* gmem)
+{
+   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+
+// A thread's rows on their way: a ring of DEPTH rows of V float4 in shared
+// memory, each filled by the thread's own asynchronous copies, one group to a
+// row, DEPTH - 1 rows ahead.  A row of a chain is a few dozen dependent FP32
+// operations in the solve, some thousand cycles in the factorisation; a load is
+// 600 to 1,000 cycles, and there are not registers for that many rows.  Slot
+// (row, v) of thread `tid` at ((row % DEPTH) * V + v) * blockDim + tid: a
+// warp's access of one float4 is 512 contiguous bytes.
+template <int V, int DEPTH>
+struct RowRing {
+   float4* buf;
+   __device__ __forceinline__ explicit RowRing(float4* stage) : buf(stage + threadIdx.x) {}
+   __device__ __forceinline__ float4* at(int row, int v) const
+   {
+      return buf + (size_t)((row % DEPTH) * V + v) * blockDim.x;
+   }
+   // N float4 of a tiled record (128 floats apart) into v, v + 1, ..
+   template <int N>
+   __device__ __forceinline__ void copy(int row, int v, const float* src) const
+   {
+#pragma unroll
+      for (int q = 0; q < N; q++) cp_async16_cg(at(row, v + q), src + 128 * q);
+   }
+   template <int N>
+   __device__ __forceinline__ void read(int row, int v, float (&x)[N]) const
+   {
+#pragma unroll
+      for (int q = 0; q < N / 4; q++) {
+         const float4 y = *at(row, v + q);
+         x[4 * q] = y.x; x[4 * q + 1] = y.y; x[4 * q + 2] = y.z; x[4 * q + 3] = y.w;
+      }
+   }
+};
 
 __device__ __forceinline__ float4* stage_at(float4* stage, int term, int q)
 {
@@ -470,7 +518,13 @@ __device__ __forceinline__ void mx_row_staged(const DeviceState& d, const RowRef
 constexpr int kElimChunk = 2;
 
 // all chains, thread p on the chain at position p of line_chains; ED rows of
-// the last-row elimination per chunk
+// the last-row elimination per chunk.  FUSED: each thread builds its chain's
+// blocks straight from the FP32 face Jacobians; otherwise it reads those that
+// mx_assemble_kernel wrote, through its ring (512 x 128, 30% split: 124 us with
+// the next row's blocks in registers, 76 us so; 32 meshes of 983,040 cells: 89 us).
+constexpr int kFactorDepth = 4, kFactorVec = 12;
+static_assert(kFactorDepth * kFactorVec == kStageTerms * 4, "either form takes the same shared memory");
+
 template <bool FUSED, int ED>
 __global__ void __launch_bounds__(256) mx_factor_kernel(DeviceState d, int count)
 {
@@ -485,26 +539,36 @@ __global__ void __launch_bounds__(256) mx_factor_kernel(DeviceState d, int count
    RowRef rnext{};   // fused: references of row i + 1, looked up a row ahead
    RowRef rstaged{};  // fused: references of the row whose terms are staged
    float snext = 0.f;  // fused: its CFL/sigma factor
-   extern __shared__ float4 stage[];   // fused: kStageTerms x 4 float4 per thread
+   extern __shared__ float4 stage[];   // fused: kStageTerms x 4 float4 per thread; otherwise the ring
+   const RowRing<kFactorVec, kFactorDepth> ring(stage);
+   constexpr int AHEAD = kFactorDepth - 1;
+   auto fetch = [&](int i) {   // unfused: row i's blocks, as mx_assemble_kernel left them
+      if (i < N) ring.copy<12>(i, 0, d.blk32 + tix(s0 + i, 48, 0, lane));
+      cp_async_commit();
+   };
    if (FUSED) {
       const RowRef r0 = mx_rowref(d, row0);
       if (N > 1) rnext = mx_rowref(d, row0 + 1);
-      mx_rows<FUSED>(d, r0, s0, lane, A, B, C);
+      mx_row_ref(d, r0, A, B, C);
    } else {
-      mx_rows<FUSED>(d, rnext, s0, lane, A, B, C);
+#pragma unroll
+      for (int i = 0; i < AHEAD; i++) fetch(i);
    }
    for (int i = 0; i < N; i++) {
-      float An[16], Bn[16], Cn[16];
-      if (i + 1 < N) {
-         if (FUSED) {
+      if (FUSED) {
+         if (i + 1 < N) {
             // row i+1's terms are copied while row i is factored
             mx_stage_row(d, rnext, stage);
             rstaged = rnext;
             snext = float(d.dtfac[rnext.scell]);
             if (i + 2 < N) rnext = mx_rowref(d, row0 + i + 2);
-         } else {
-            mx_rows<FUSED>(d, rnext, s0 + i + 1, lane, An, Bn, Cn);
          }
+      } else {
+         cp_async_wait<AHEAD - 1>();
+         ring.read(i, 0, A);
+         ring.read(i, 4, B);
+         ring.read(i, 8, C);
+         fetch(i + AHEAD);
       }
       float* rec = d.fac32 + tix(s0 + i, kRec, 0, lane);
       st16t(rec, A);
@@ -535,16 +599,12 @@ __global__ void __launch_bounds__(256) mx_factor_kernel(DeviceState d, int count
       if (per) st16t(rec + 32 * 48, fill);
 #pragma unroll
       for (int m = 0; m < 16; m++) { cp[m] = C[m]; ap[m] = fill[m]; }
-      if (i + 1 < N) {
-         if (FUSED) {
-            cp_async_wait_all();
-            mx_row_staged(d, rstaged, stage, snext, A, B, C);
-         } else {
-#pragma unroll
-            for (int m = 0; m < 16; m++) { A[m] = An[m]; B[m] = Bn[m]; C[m] = Cn[m]; }
-         }
+      if (FUSED && i + 1 < N) {
+         cp_async_wait_all();
+         mx_row_staged(d, rstaged, stage, snext, A, B, C);
       }
    }
+   if (!FUSED) cp_async_wait_all();
    if (!per) {
       if (bad) atomicOr(d.status, DEV_ERR_PIVOT);
       return;
@@ -586,11 +646,17 @@ __global__ void __launch_bounds__(256) mx_factor_kernel(DeviceState d, int count
 
 // One sweep's solve of one chain per thread (the chain at position first +
 // t of line_chains).  The recurrence only carries the 4-vector x in
-// registers; everything a row needs (its factor record, its right-hand
-// side, the cell it writes) is loaded one row ahead, so the loads overlap
-// the previous row's arithmetic.  Solutions go straight to r32 (each cell
-// is written once per chain; chains of a wave share no cell).
-__global__ void __launch_bounds__(256) mx_solve_kernel(DeviceState d, int first, int count)
+// registers; what a row needs comes through the thread's ring (its factor
+// record, its right-hand side through the cell looked up kSolveLook rows before
+// that, later the forward sweep's row).  Solutions go straight to r32 (each
+// cell is written once per chain; chains of a wave share no cell).
+// Bound by the chain: with the loads of four rows issued together a row of the
+// longest chain took 480 cycles forward or back, through the ring 330 (512 x 128,
+// 30% split: the four solves of a step 207 -> 141 us; unsplit 170 -> 116 us; 32
+// meshes of 983,040 cells 270 -> 142 us).
+constexpr int kSolveDepth = 8, kSolveVec = 9, kSolveLook = 4;
+
+__global__ void __launch_bounds__(128) mx_solve_kernel(DeviceState d, int first, int count)
 {
    const int t = blockIdx.x * blockDim.x + threadIdx.x;
    if (t >= count || halted(d)) return;
@@ -601,288 +667,139 @@ __global__ void __launch_bounds__(256) mx_solve_kernel(DeviceState d, int first,
    const bool per = d.chain_periodic[ich] != 0;
    const int* fcell = d.row_fcell + row0;
    const int* scell = d.row_scell + row0;
-   // forward: f(i) = LU^{-1}(F(i) - A(i) f(i-1)), F(i) = r[fcell]
-   float xp[4] = {0.f, 0.f, 0.f, 0.f};
-   float a[16], xr[4] = {0.f, 0.f, 0.f, 0.f};
-   LUf u;
-   int fcn = -1;   // the next row's right-hand-side cell, looked up a row ahead
-   {
-      const int fc = fcell[0];
-      if (fc >= 0) ld4(d.r32 + 4 * (size_t)fc, xr);
-      if (N > 1) fcn = fcell[1];
-      u = luf_load_t(d.fac32 + tix(s0, kRec, 16, lane));
+   extern __shared__ float4 stage[];
+   const RowRing<kSolveVec, kSolveDepth> ring(stage);
+   constexpr int AHEAD = kSolveDepth - 1;
+   const float* fac = d.fac32 + tix(s0, kRec, 0, lane);      // row i at + 32 * kRec * i
+   float* fsr = d.fsc32 + tix(s0, 4, 0, lane);               // row i at + 128 * i
+   constexpr size_t kFacRow = 32 * kRec, kFsRow = 128;
+   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+
+   // forward: f(i) = LU^{-1}(F(i) - A(i) f(i-1)), F(i) = r[fcell] (0 without one)
+   float x[4], xp[4] = {0.f, 0.f, 0.f, 0.f};
+   auto fetch = [&](int i, int cell) {
+      if (i < N) {
+         ring.copy<8>(i, 0, fac + kFacRow * i);
+         if (cell >= 0) cp_async16_cg(ring.at(i, 8), d.r32 + 4 * (size_t)cell);
+         else *ring.at(i, 8) = zero4;
+      }
+      cp_async_commit();
+   };
+   auto look = [&](const int* cells, int i) { return i >= 0 && i < N ? cells[i] : -1; };
 #pragma unroll
-      for (int m = 0; m < 16; m++) a[m] = 0.f;
+   for (int i = 0; i < AHEAD; i++) fetch(i, look(fcell, i));
+   int fc[kSolveLook];
+#pragma unroll
+   for (int u = 0; u < kSolveLook; u++) fc[u] = look(fcell, AHEAD + u);
+   for (int i0 = 0; i0 < N; i0 += kSolveLook) {
+      int fcn[kSolveLook];
+#pragma unroll
+      for (int u = 0; u < kSolveLook; u++) fcn[u] = look(fcell, i0 + AHEAD + kSolveLook + u);
+#pragma unroll
+      for (int u = 0; u < kSolveLook; u++) {
+         const int i = i0 + u;
+         if (i >= N) break;
+         cp_async_wait<AHEAD - 1>();
+         float a[16], lu[16];
+         ring.read(i, 0, a);
+         ring.read(i, 4, lu);
+         ring.read(i, 8, x);
+         fetch(i + AHEAD, fc[u]);
+         if (i > 0) {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+#pragma unroll
+               for (int j = 0; j < 4; j++) x[k] = __fmaf_rn(-a[4 * k + j], xp[j], x[k]);
+         }
+         luf_solve(luf_of(lu), x[0], x[1], x[2], x[3]);
+         *reinterpret_cast<float4*>(fsr + kFsRow * i) = make_float4(x[0], x[1], x[2], x[3]);
+#pragma unroll
+         for (int k = 0; k < 4; k++) xp[k] = x[k];
+      }
+#pragma unroll
+      for (int u = 0; u < kSolveLook; u++) fc[u] = fcn[u];
    }
-   for (int i = 0; i < N; i++) {
-      // next row's record and right-hand side, in flight during this row
-      float an[16], xrn[4] = {0.f, 0.f, 0.f, 0.f};
-      LUf un;
-      if (i + 1 < N) {
-         const float* rn = d.fac32 + tix(s0 + i + 1, kRec, 0, lane);
-         if (fcn >= 0) ld4(d.r32 + 4 * (size_t)fcn, xrn);
-         fcn = (i + 2 < N) ? fcell[i + 2] : -1;
-         ld16t(rn, an);
-         un = luf_load_t(rn + 32 * 16);
-      }
-      float x[4] = {xr[0], xr[1], xr[2], xr[3]};
-      if (i > 0) {
-#pragma unroll
-         for (int k = 0; k < 4; k++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) x[k] = __fmaf_rn(-a[4 * k + j], xp[j], x[k]);
-      }
-      luf_solve(u, x[0], x[1], x[2], x[3]);
-      float* fs = d.fsc32 + tix(s0 + i, 4, 0, lane);
-      *reinterpret_cast<float4*>(fs) = make_float4(x[0], x[1], x[2], x[3]);
-#pragma unroll
-      for (int k = 0; k < 4; k++) xp[k] = x[k];
-      if (i + 1 < N) {
-#pragma unroll
-         for (int m = 0; m < 16; m++) a[m] = an[m];
-#pragma unroll
-         for (int k = 0; k < 4; k++) xr[k] = xrn[k];
-         u = un;
-      }
-   }
-   float xn[4];
+   cp_async_wait_all();
+   __threadfence_block();   // the forward rows, before the copies below read them
+   float xn[4], fN[4] = {xp[0], xp[1], xp[2], xp[3]};
    if (per) {
-      float fN[4] = {xp[0], xp[1], xp[2], xp[3]};
+      // last row: f(N-1) - sum over i < N-1 of cN(i) f(i), in row order
+      auto fetch_last = [&](int i) {
+         if (i < N - 1) {
+            ring.copy<4>(i, 0, fac + kFacRow * i + 32 * 64);
+            cp_async16_cg(ring.at(i, 8), fsr + kFsRow * i);
+         }
+         cp_async_commit();
+      };
+#pragma unroll
+      for (int i = 0; i < AHEAD; i++) fetch_last(i);
       for (int i = 0; i < N - 1; i++) {
+         cp_async_wait<AHEAD - 1>();
          float c[16], f[4];
-         ld16t(d.fac32 + tix(s0 + i, kRec, 64, lane), c);
-         const float* fs = d.fsc32 + tix(s0 + i, 4, 0, lane);
-         { const float4 y = *reinterpret_cast<const float4*>(fs); f[0] = y.x; f[1] = y.y; f[2] = y.z; f[3] = y.w; }
+         ring.read(i, 0, c);
+         ring.read(i, 8, f);
+         fetch_last(i + AHEAD);
 #pragma unroll
          for (int k = 0; k < 4; k++)
 #pragma unroll
             for (int j = 0; j < 4; j++) fN[k] = __fmaf_rn(-c[4 * k + j], f[j], fN[k]);
       }
+      cp_async_wait_all();
       const LUf uN = luf_load(d.facN32 + 16 * d.chain_facN[ich]);
       luf_solve(uN, fN[0], fN[1], fN[2], fN[3]);
-      st4(d.r32 + 4 * (size_t)scell[N - 1], fN);
+   }
 #pragma unroll
-      for (int k = 0; k < 4; k++) xn[k] = fN[k];
-      for (int i = N - 2; i >= 0; i--) {
-         const float* rec = d.fac32 + tix(s0 + i, kRec, 0, lane);
-         float c[16], aa[16], x[4];
-         ld16t(rec + 32 * 32, c);
-         ld16t(rec + 32 * 48, aa);
-         const float* fs = d.fsc32 + tix(s0 + i, 4, 0, lane);
-         { const float4 y = *reinterpret_cast<const float4*>(fs); x[0] = y.x; x[1] = y.y; x[2] = y.z; x[3] = y.w; }
+   for (int k = 0; k < 4; k++) xn[k] = fN[k];
+   st4(d.r32 + 4 * (size_t)scell[N - 1], xn);
+   // back substitution, rows N-2 down to 0 (step s = N-2-i), periodic with the
+   // fill-in column
+   auto fetch_back = [&](int s) {
+      const int i = N - 2 - s;
+      if (i >= 0) {
+         ring.copy<4>(s, 0, fac + kFacRow * i + 32 * 32);
+         if (per) ring.copy<4>(s, 4, fac + kFacRow * i + 32 * 48);
+         cp_async16_cg(ring.at(s, 8), fsr + kFsRow * i);
+      }
+      cp_async_commit();
+   };
+#pragma unroll
+   for (int s = 0; s < AHEAD; s++) fetch_back(s);
+   int sc[kSolveLook];
+#pragma unroll
+   for (int u = 0; u < kSolveLook; u++) sc[u] = look(scell, N - 2 - u);
+   for (int q0 = 0; q0 <= N - 2; q0 += kSolveLook) {
+      int scn[kSolveLook];
+#pragma unroll
+      for (int u = 0; u < kSolveLook; u++) scn[u] = look(scell, N - 2 - q0 - kSolveLook - u);
+#pragma unroll
+      for (int u = 0; u < kSolveLook; u++) {
+         const int s = q0 + u;
+         if (s > N - 2) break;
+         cp_async_wait<AHEAD - 1>();
+         float c[16], aa[16];
+         ring.read(s, 0, c);
+         if (per) ring.read(s, 4, aa);
+         ring.read(s, 8, x);
+         fetch_back(s + AHEAD);
 #pragma unroll
          for (int k = 0; k < 4; k++)
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-               const float sv = (i == N - 2) ? c[4 * k + j] * xn[j] : __fmaf_rn(aa[4 * k + j], fN[j], c[4 * k + j] * xn[j]);
-               x[k] -= sv;
+               if (per) {
+                  const float v = c[4 * k + j] * xn[j];
+                  x[k] -= (s == 0) ? v : __fmaf_rn(aa[4 * k + j], fN[j], v);
+               } else {
+                  x[k] = __fmaf_rn(-c[4 * k + j], xn[j], x[k]);
+               }
             }
-         st4(d.r32 + 4 * (size_t)scell[i], x);
+         st4(d.r32 + 4 * (size_t)sc[u], x);
 #pragma unroll
          for (int k = 0; k < 4; k++) xn[k] = x[k];
       }
-   } else {
 #pragma unroll
-      for (int k = 0; k < 4; k++) xn[k] = xp[k];
-      st4(d.r32 + 4 * (size_t)scell[N - 1], xn);
-      // back substitution, row i-1's factor and f prefetched
-      float c[16], x[4];
-      int sc = 0;
-      if (N >= 2) {
-         ld16t(d.fac32 + tix(s0 + N - 2, kRec, 32, lane), c);
-         const float* fs = d.fsc32 + tix(s0 + N - 2, 4, 0, lane);
-         { const float4 y = *reinterpret_cast<const float4*>(fs); x[0] = y.x; x[1] = y.y; x[2] = y.z; x[3] = y.w; }
-         sc = scell[N - 2];
-      }
-      for (int i = N - 2; i >= 0; i--) {
-         float cn[16], xnx[4];
-         int scn = 0;
-         if (i >= 1) {
-            ld16t(d.fac32 + tix(s0 + i - 1, kRec, 32, lane), cn);
-            const float* fs = d.fsc32 + tix(s0 + i - 1, 4, 0, lane);
-            { const float4 y = *reinterpret_cast<const float4*>(fs); xnx[0] = y.x; xnx[1] = y.y; xnx[2] = y.z; xnx[3] = y.w; }
-            scn = scell[i - 1];
-         }
-#pragma unroll
-         for (int k = 0; k < 4; k++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) x[k] = __fmaf_rn(-c[4 * k + j], xn[j], x[k]);
-         st4(d.r32 + 4 * (size_t)sc, x);
-#pragma unroll
-         for (int k = 0; k < 4; k++) xn[k] = x[k];
-         if (i >= 1) {
-#pragma unroll
-            for (int m = 0; m < 16; m++) c[m] = cn[m];
-#pragma unroll
-            for (int k = 0; k < 4; k++) x[k] = xnx[k];
-            sc = scn;
-         }
-      }
+      for (int u = 0; u < kSolveLook; u++) sc[u] = scn[u];
    }
-}
-
-// rows whose loads mx_solve_chunk_kernel issues together
-constexpr int kSolveChunk = 4;
-
-// The same solve with the loads of kSolveChunk rows issued together before
-// their arithmetic, in each of the row loops.  A row's own arithmetic is a
-// few dozen dependent FP32 operations, far shorter than one memory round
-// trip, so a chain of N rows waits about N / kSolveChunk round trips instead
-// of N.  The operations and their order are those of mx_solve_kernel, so
-// the results are identical.  It takes more registers; the host launches it
-// for waves whose chains are all resident at once.
-__global__ void __launch_bounds__(256) mx_solve_chunk_kernel(DeviceState d, int first, int count)
-{
-   constexpr int D = kSolveChunk;
-   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-   if (t >= count || halted(d)) return;
-   const int p = first + t;
-   const int ich = d.line_chains[p];
-   if (frozen_chain(d, ich) || spike_active(d, ich)) return;
-   const int N = d.chain_nrows[ich], row0 = d.chain_row0[ich], lane = p & 31, s0 = d.grp_row0[p >> 5];
-   const bool per = d.chain_periodic[ich] != 0;
-   const int* fcell = d.row_fcell + row0;
-   const int* scell = d.row_scell + row0;
-   // forward: f(i) = LU^{-1}(F(i) - A(i) f(i-1)), F(i) = r[fcell]; the
-   // right-hand-side cells of a chunk are looked up during the chunk before
-   float xp[4] = {0.f, 0.f, 0.f, 0.f};
-   int fcb[D];
-#pragma unroll
-   for (int u = 0; u < D; u++) fcb[u] = (u < N) ? fcell[u] : -1;
-   for (int i0 = 0; i0 < N; i0 += D) {
-      float ab[D][16], xb[D][4];
-      LUf ub[D];
-#pragma unroll
-      for (int u = 0; u < D; u++) {
-         const int i = i0 + u;
-#pragma unroll
-         for (int k = 0; k < 4; k++) xb[u][k] = 0.f;
-         if (i < N) {
-            const float* rec = d.fac32 + tix(s0 + i, kRec, 0, lane);
-            if (fcb[u] >= 0) ld4(d.r32 + 4 * (size_t)fcb[u], xb[u]);
-            if (i > 0) ld16t(rec, ab[u]);
-            ub[u] = luf_load_t(rec + 32 * 16);
-         }
-      }
-#pragma unroll
-      for (int u = 0; u < D; u++) fcb[u] = (i0 + D + u < N) ? fcell[i0 + D + u] : -1;
-#pragma unroll
-      for (int u = 0; u < D; u++) {
-         const int i = i0 + u;
-         if (i < N) {
-            float x[4] = {xb[u][0], xb[u][1], xb[u][2], xb[u][3]};
-            if (i > 0) {
-#pragma unroll
-               for (int k = 0; k < 4; k++)
-#pragma unroll
-                  for (int j = 0; j < 4; j++) x[k] = __fmaf_rn(-ab[u][4 * k + j], xp[j], x[k]);
-            }
-            luf_solve(ub[u], x[0], x[1], x[2], x[3]);
-            float* fs = d.fsc32 + tix(s0 + i, 4, 0, lane);
-            *reinterpret_cast<float4*>(fs) = make_float4(x[0], x[1], x[2], x[3]);
-#pragma unroll
-            for (int k = 0; k < 4; k++) xp[k] = x[k];
-         }
-      }
-   }
-   float xn[4];
-   if (per) {
-      // last row: f(N-1) - sum over i < N-1 of cN(i) f(i), in row order
-      float fN[4] = {xp[0], xp[1], xp[2], xp[3]};
-      for (int i0 = 0; i0 < N - 1; i0 += D) {
-         float cb[D][16], fb[D][4];
-#pragma unroll
-         for (int u = 0; u < D; u++) {
-            const int i = i0 + u;
-            if (i < N - 1) {
-               ld16t(d.fac32 + tix(s0 + i, kRec, 64, lane), cb[u]);
-               const float* fs = d.fsc32 + tix(s0 + i, 4, 0, lane);
-               { const float4 y = *reinterpret_cast<const float4*>(fs); fb[u][0] = y.x; fb[u][1] = y.y; fb[u][2] = y.z; fb[u][3] = y.w; }
-            }
-         }
-#pragma unroll
-         for (int u = 0; u < D; u++) {
-            if (i0 + u < N - 1) {
-#pragma unroll
-               for (int k = 0; k < 4; k++)
-#pragma unroll
-                  for (int j = 0; j < 4; j++) fN[k] = __fmaf_rn(-cb[u][4 * k + j], fb[u][j], fN[k]);
-            }
-         }
-      }
-      const LUf uN = luf_load(d.facN32 + 16 * d.chain_facN[ich]);
-      luf_solve(uN, fN[0], fN[1], fN[2], fN[3]);
-      st4(d.r32 + 4 * (size_t)scell[N - 1], fN);
-#pragma unroll
-      for (int k = 0; k < 4; k++) xn[k] = fN[k];
-      // back substitution with the fill-in column, rows N-2 down to 0
-      for (int i0 = N - 2; i0 >= 0; i0 -= D) {
-         float cb[D][16], ab[D][16], fb[D][4];
-         int sb[D];
-#pragma unroll
-         for (int u = 0; u < D; u++) {
-            const int i = i0 - u;
-            if (i >= 0) {
-               const float* rec = d.fac32 + tix(s0 + i, kRec, 0, lane);
-               ld16t(rec + 32 * 32, cb[u]);
-               ld16t(rec + 32 * 48, ab[u]);
-               const float* fs = d.fsc32 + tix(s0 + i, 4, 0, lane);
-               { const float4 y = *reinterpret_cast<const float4*>(fs); fb[u][0] = y.x; fb[u][1] = y.y; fb[u][2] = y.z; fb[u][3] = y.w; }
-               sb[u] = scell[i];
-            }
-         }
-#pragma unroll
-         for (int u = 0; u < D; u++) {
-            const int i = i0 - u;
-            if (i >= 0) {
-               float x[4] = {fb[u][0], fb[u][1], fb[u][2], fb[u][3]};
-#pragma unroll
-               for (int k = 0; k < 4; k++)
-#pragma unroll
-                  for (int j = 0; j < 4; j++) {
-                     const float sv = (i == N - 2) ? cb[u][4 * k + j] * xn[j]
-                                                   : __fmaf_rn(ab[u][4 * k + j], fN[j], cb[u][4 * k + j] * xn[j]);
-                     x[k] -= sv;
-                  }
-               st4(d.r32 + 4 * (size_t)sb[u], x);
-#pragma unroll
-               for (int k = 0; k < 4; k++) xn[k] = x[k];
-            }
-         }
-      }
-   } else {
-#pragma unroll
-      for (int k = 0; k < 4; k++) xn[k] = xp[k];
-      st4(d.r32 + 4 * (size_t)scell[N - 1], xn);
-      // back substitution, rows N-2 down to 0
-      for (int i0 = N - 2; i0 >= 0; i0 -= D) {
-         float cb[D][16], fb[D][4];
-         int sb[D];
-#pragma unroll
-         for (int u = 0; u < D; u++) {
-            const int i = i0 - u;
-            if (i >= 0) {
-               ld16t(d.fac32 + tix(s0 + i, kRec, 32, lane), cb[u]);
-               const float* fs = d.fsc32 + tix(s0 + i, 4, 0, lane);
-               { const float4 y = *reinterpret_cast<const float4*>(fs); fb[u][0] = y.x; fb[u][1] = y.y; fb[u][2] = y.z; fb[u][3] = y.w; }
-               sb[u] = scell[i];
-            }
-         }
-#pragma unroll
-         for (int u = 0; u < D; u++) {
-            if (i0 - u >= 0) {
-               float x[4] = {fb[u][0], fb[u][1], fb[u][2], fb[u][3]};
-#pragma unroll
-               for (int k = 0; k < 4; k++)
-#pragma unroll
-                  for (int j = 0; j < 4; j++) x[k] = __fmaf_rn(-cb[u][4 * k + j], xn[j], x[k]);
-               st4(d.r32 + 4 * (size_t)sb[u], x);
-#pragma unroll
-               for (int k = 0; k < 4; k++) xn[k] = x[k];
-            }
-         }
-      }
-   }
+   cp_async_wait_all();
 }
 
 // ---------------- long chains by segments -------------------------------
@@ -1581,23 +1498,24 @@ void launch_mx_rhs_face(const DeviceState& d, cudaStream_t st)
 
 void launch_mx_assemble(const DeviceState& d, cudaStream_t st)
 {
-   const size_t n = 48 * 32 * (size_t)d.tile_rows;
+   const size_t n = 12 * 32 * (size_t)d.tile_rows;
    if (!d.mx_fused && n > 0) mx_assemble_kernel<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, st>>>(d);
 }
 
 void launch_mx_init(const DeviceState& d, cudaStream_t st) { mx_init_kernel<<<blocks_for(d.nCell), kThreads, 0, st>>>(d); }
 
-// dynamic shared memory of the fused factorisation: the staged terms
+// dynamic shared memory of the factorisation (staged terms or ring) and of the solve (ring)
 size_t mx_factor_stage_bytes(int block) { return (size_t)kStageTerms * 4 * sizeof(float4) * block; }
+size_t mx_solve_ring_bytes(int block) { return (size_t)kSolveDepth * kSolveVec * sizeof(float4) * block; }
 
 int mx_configure()
 {
-   const int want = (int)mx_factor_stage_bytes(128);
-   if (cudaFuncSetAttribute(mx_factor_kernel<true, kElimChunk>, cudaFuncAttributeMaxDynamicSharedMemorySize, want) !=
-           cudaSuccess ||
-       cudaFuncSetAttribute(mx_factor_kernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, want) !=
-           cudaSuccess)
-      return 1;
+   const int want = (int)mx_factor_stage_bytes(128), ring = (int)mx_solve_ring_bytes(128);
+   const void* factor[] = {(const void*)mx_factor_kernel<true, kElimChunk>, (const void*)mx_factor_kernel<true, 1>,
+                           (const void*)mx_factor_kernel<false, kElimChunk>, (const void*)mx_factor_kernel<false, 1>};
+   for (const void* f : factor)
+      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, want) != cudaSuccess) return 1;
+   if (cudaFuncSetAttribute(mx_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ring) != cudaSuccess) return 1;
    return 0;
 }
 
@@ -1606,13 +1524,13 @@ void launch_mx_factor(const DeviceState& d, cudaStream_t st)
    const int tb = d.mx_block;
    const unsigned nb = (d.nChain + tb - 1) / tb;
    const bool chunk = d.nChain <= d.mx_chunk_chains;
+   const size_t sm = mx_factor_stage_bytes(tb);
    if (d.mx_fused) {
-      const size_t sm = mx_factor_stage_bytes(tb);
       if (chunk) mx_factor_kernel<true, kElimChunk><<<nb, tb, sm, st>>>(d, d.nChain);
       else mx_factor_kernel<true, 1><<<nb, tb, sm, st>>>(d, d.nChain);
    } else {
-      if (chunk) mx_factor_kernel<false, kElimChunk><<<nb, tb, 0, st>>>(d, d.nChain);
-      else mx_factor_kernel<false, 1><<<nb, tb, 0, st>>>(d, d.nChain);
+      if (chunk) mx_factor_kernel<false, kElimChunk><<<nb, tb, sm, st>>>(d, d.nChain);
+      else mx_factor_kernel<false, 1><<<nb, tb, sm, st>>>(d, d.nChain);
    }
 }
 
@@ -1620,8 +1538,7 @@ void launch_mx_solve(const DeviceState& d, int first, int count, cudaStream_t st
 {
    const int tb = d.mx_block;
    if (count <= 0) return;
-   if (count <= d.mx_chunk_chains) mx_solve_chunk_kernel<<<(count + tb - 1) / tb, tb, 0, st>>>(d, first, count);
-   else mx_solve_kernel<<<(count + tb - 1) / tb, tb, 0, st>>>(d, first, count);
+   mx_solve_kernel<<<(count + tb - 1) / tb, tb, mx_solve_ring_bytes(tb), st>>>(d, first, count);
 }
 
 int mx_solve_chunk_capacity(int block)
@@ -1629,7 +1546,7 @@ int mx_solve_chunk_capacity(int block)
    int dev = 0, sms = 0, per_sm = 0;
    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mx_solve_chunk_kernel, block, 0) != cudaSuccess)
+   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mx_solve_kernel, block, mx_solve_ring_bytes(block)) != cudaSuccess)
       return 0;
    return sms * per_sm * block;
 }
