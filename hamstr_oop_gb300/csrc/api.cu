@@ -154,6 +154,7 @@ struct hamstr_gpu {
       L("rhs_cell", n, [&] { launch_rhs_cell(d, true, stream); });
       L("norm_final", n, [&] { launch_norm_final(d, 0, check_tol, stream); });
       L("mx_init", n, [&] { launch_mx_init(d, stream); });
+      if (!d.mx_fused) L("mx_assemble", n, [&] { launch_mx_assemble(d, stream); });
       // the segmented chains' kernels touch no chain of the others and no
       // cell of another chain of their wave, so they run beside them on the
       // side stream (a parallel branch of the captured graph); per-kernel
@@ -165,7 +166,6 @@ struct hamstr_gpu {
          CK(cudaStreamWaitEvent(stream2, ev_fork, 0));
       }
       if (d.sp_on && d.nSpike > 0) L("mx_spike_factor", n, [&] { launch_mx_spike_factor(d, sst); });
-      if (!d.mx_fused) L("mx_assemble", n, [&] { launch_mx_assemble(d, stream); });
       L("mx_factor", n, [&] { launch_mx_factor(d, stream); });
       for (int s = 0; s < msweep; s++) {
          for (int w = 0; w < plan.nWave; w++) {
@@ -228,7 +228,6 @@ struct hamstr_gpu {
       if ((st = upload(&d.grp_row0, grp_row0, owned))) return st;
       if ((st = upload(&d.tile_row, tile_row, owned))) return st;
       const size_t tiles = 32 * (size_t)std::max(d.tile_rows, 1);
-      if (!d.mx_fused && (st = ensure_blk32())) return st;
       if ((st = dalloc(&d.fsc32, 4 * tiles, owned))) return st;
       if ((st = dalloc(&d.fac32, 80 * tiles, owned))) return st;
       int nper = 0;
@@ -242,7 +241,8 @@ struct hamstr_gpu {
       // kSpikeRows rows each (at most kSpikeMaxSeg), grouped by wave; their
       // rows are tiled across the segments (sp_rec0 in tile rows)
       {
-         std::vector<int> chain_spike(std::max(plan.nChain, 1), -1), sp_chain, sp_seg, sp_nseg, sp_rec0;
+         std::vector<int> chain_spike(std::max(plan.nChain, 1), -1), sp_chain, sp_pos, sp_seg, sp_nseg, sp_rec0, pos(plan.nChain);
+         for (int p = 0; p < plan.nChain; p++) pos[lc[p]] = p;
          sp_wave_ptr.assign(plan.nWave + 1, 0);
          int rows = 0;
          for (int w = 0; w < plan.nWave; w++) {
@@ -253,6 +253,7 @@ struct hamstr_gpu {
                const int P = std::min(kSpikeMaxSeg, n / kSpikeRows);
                chain_spike[c] = (int)sp_chain.size();
                sp_chain.push_back(c);
+               sp_pos.push_back(pos[c]);
                sp_nseg.push_back(P);
                sp_rec0.push_back(rows);
                int longest = 0;
@@ -267,18 +268,26 @@ struct hamstr_gpu {
          d.nSpike = (int)sp_chain.size();
          if (sp_chain.empty()) {
             sp_chain.push_back(0);
+            sp_pos.push_back(0);
             sp_nseg.push_back(0);
             sp_rec0.push_back(0);
             sp_seg.assign(kSpikeMaxSeg + 1, 0);
          }
          if ((st = upload(&d.chain_spike, chain_spike, owned))) return st;
          if ((st = upload(&d.sp_chain, sp_chain, owned))) return st;
+         if ((st = upload(&d.sp_pos, sp_pos, owned))) return st;
          if ((st = upload(&d.sp_seg, sp_seg, owned))) return st;
          if ((st = upload(&d.sp_nseg, sp_nseg, owned))) return st;
          if ((st = upload(&d.sp_rec0, sp_rec0, owned))) return st;
          if ((st = dalloc(&d.sp_fac, 80 * 32 * (size_t)std::max(rows, 1), owned))) return st;
          if ((st = dalloc(&d.sp_y, 4 * 32 * (size_t)std::max(rows, 1), owned))) return st;
          if ((st = dalloc(&d.sp_red, (size_t)kSpikeRedStride * std::max(d.nSpike, 1), owned))) return st;
+      }
+      // last, and without it the assembly goes inside
+      if (!d.mx_fused && (st = ensure_blk32())) {
+         if (st != HAMSTR_GPU_ERR_NOMEM) return st;
+         cudaGetLastError();
+         d.mx_fused = 1;
       }
       CK(cudaMemsetAsync(d.ff32, 0, 32 * (size_t)d.nSlot * sizeof(float), stream));
       CK(cudaMemsetAsync(d.dq32, 0, 4 * nc * sizeof(float), stream));
@@ -485,20 +494,14 @@ int hamstr_gpu_create(const hamstr_gpu_params* p, int nCell, int nFace, const in
 
 namespace {
 // FP32 assembly inside the factorisation (1), or by a kernel of its own (0).  Of
-// its own it costs a pass over the blocks, some 0.2 ns a row; inside, a row of a
-// chain takes 1.8 us instead of 0.6 us, as its terms are behind two lookups, and
-// the longest chain that one thread walks sets the time (long periodic chains go
-// by segments).  Assembly and factorisation, own / inside: 512 x 128 0.11 / 0.23
-// ms, the same mesh 30% split 0.11 / 0.21 ms, 32 meshes of 983,040 cells in all
-// 0.44 / 0.27 ms.  Short chains fill the GPU either way and save the terms' lookups;
-// above 2^22 rows of longer chains the blocks (192 bytes a row) are not kept.
+// its own it costs a pass over the blocks; inside, a row of a chain takes 1.8 us
+// instead of 0.65 us, as its terms are behind two lookups.  A step, own / inside:
+// 512 x 128 0.51 / 0.63 ms, the same mesh 30% split 0.50 / 0.61 ms, 32 meshes of
+// 983,040 cells in all 2.05 / 2.25 ms.  Above 2^24 rows of longer chains the blocks (192
+// bytes a row) are not kept.
 int default_mx_fused(const Plan& P)
 {
-   long long longest = 0;
-   for (int c = 0; c < P.nChain; c++)
-      if (!P.chain_periodic[c]) longest = std::max(longest, (long long)P.chain_nrows[c]);
-   const long long rows = P.nRow;
-   return P.nChain > 0 && rows >= 16ll * P.nChain && rows > std::min(5000 * longest, 1ll << 22) ? 1 : 0;
+   return P.nChain > 0 && P.nRow >= 16ll * P.nChain && P.nRow > (1 << 24) ? 1 : 0;
 }
 
 // How the FP64 line kernels pack open chains before any tuning.
@@ -717,9 +720,8 @@ int hamstr::create_gpu(const hamstr_gpu_params* p, int nCell, int nFace, const i
       d.adi_wpb = 4;
       d.adi_fwpb = 4;
       d.mx_fused = default_mx_fused(P);
-      // one warp a block reaches the most SMs (a 512 x 128 march 4.14 ms, 4.18 and
-      // 4.29 with two and four); with the assembly inside, two leave the chains by
-      // segments beside it more room (32 meshes: 8.76 ms, 10.0 with one, 8.77 with four)
+      // one warp a block reaches the most SMs (eight steps of 512 x 128 4.14 ms, 4.18
+      // and 4.29 with two and four; with the assembly inside 1% the other way)
       d.mx_block = d.mx_fused ? 64 : 32;
       d.mx_chunk_chains = mx_solve_chunk_capacity(d.mx_block);
       d.sp_on = 1;   // long periodic chains of the FP32 form by segments (2: long open ones too)

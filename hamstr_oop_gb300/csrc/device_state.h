@@ -152,6 +152,7 @@ struct DeviceState {
    int nSpike;             // chains solved by segments
    int* chain_spike;       // [nChain] index into the sp_* arrays, or -1
    int* sp_chain;          // [nSpike] chain id
+   int* sp_pos;            // [nSpike] its position in line_chains
    int* sp_wave_ptr;       // [nWave+1] spike chains of each wave: sp indices sp_wave_ptr[w] .. [w+1]-1
    int* sp_seg;            // [nSpike][kSpikeMaxSeg+1] first row (in the chain) of each segment, then N
    int* sp_nseg;           // [nSpike] P

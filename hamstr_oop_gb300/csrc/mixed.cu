@@ -15,6 +15,7 @@
 // chain running the block Thomas elimination in registers, with chains of
 // similar length sharing a warp.
 // ##################################################################
+#include <algorithm>
 #include "device_state.h"
 #include "plan.h"
 #include "recon.cuh"
@@ -93,54 +94,57 @@ __device__ __forceinline__ size_t tix(int s, int W, int e, int lane)
 }
 
 // FP32 blocks in the reference's term order (ADI.cpp:62-217), one thread per
-// row of a block (a float4 of every term, the term list and the scale once for
-// the four entries); the unfused alternative to mx_row below (the autotuner
-// picks).  Bound by the latency of the term lists' gathers.  512 x 128, 30%
-// split: 70 us with a thread per entry, 29 us so (31 us with a warp on one row k
-// of 32 lanes; 32 meshes of 983,040 cells 425 us that way, 349 us so).
+// row k of a mesh row's three blocks (a float4 of every term; the row's lists
+// and scale once for the twelve entries); the alternative to mx_row below.
+// Bound by the latency of the lookups, tile row to term list to face.  512 x 128,
+// 30% split: 70 us with a thread per entry, 29 us with one per block row, 27 us
+// so; 32 meshes of 983,040 cells 349 us with one per block row, 253 us so.
 __global__ void __launch_bounds__(kThreads) mx_assemble_kernel(DeviceState d)
 {
-   // a warp: eight lanes of a tile row times the four rows k of one block, so
+   // a warp: eight lanes of a tile row times the four rows k of its blocks, so
    // that a term's block is 64 contiguous bytes of four neighbouring lanes and
    // a store fills four whole lines of 128 bytes
    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-   if (t >= 12 * 32 * (size_t)d.tile_rows || halted(d)) return;
-   const int k = (int)(t & 3);
-   const size_t g = t >> 7;
-   const int lane = (int)((t >> 2) & 31), b = (int)(g % 3), srow = (int)(g / 3);
+   if (t >= 128 * (size_t)d.tile_rows || halted(d)) return;
+   const int k = (int)(t & 3), lane = (int)((t >> 2) & 31), srow = (int)(t >> 7);
    const int row = d.tile_row[32 * (size_t)srow + lane];
    if (row < 0) return;
    const int sc = d.row_scell[row];
    if (frozen_cell(d, sc)) return;
-   const int4 list = *reinterpret_cast<const int4*>(d.row_ops + 3 * kOpsPerBlock * (size_t)row + kOpsPerBlock * b);
-   const int ops[kOpsPerBlock] = {list.x, list.y, list.z, list.w};
-   float acc[4] = {0.f, 0.f, 0.f, 0.f};
+   int4 list[3];
 #pragma unroll
-   for (int o = 0; o < kOpsPerBlock; o++) {
-      const int op = ops[o];
-      if (op < 0) break;
-      const int slot = op >> 3, sel = (op >> 1) & 3;
-      float v[4];
-      ld4(d.ff32 + 32 * (size_t)slot + (sel == OP_SEL_L ? 0 : 16) + 4 * k, v);
-      if (sel == OP_SEL_RREFL) {
-         const double4 rf = d.refl[d.slot_face[slot]];
-         const float r01 = v[1], r02 = v[2];
-         v[1] = float(rf.x) * r01 + float(rf.y) * r02;
-         v[2] = float(rf.z) * r01 + float(rf.w) * r02;
+   for (int b = 0; b < 3; b++) list[b] = reinterpret_cast<const int4*>(d.row_ops + 3 * kOpsPerBlock * (size_t)row)[b];
+   const float s = float(d.dtfac[sc]);
+#pragma unroll
+   for (int b = 0; b < 3; b++) {
+      const int ops[kOpsPerBlock] = {list[b].x, list[b].y, list[b].z, list[b].w};
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int o = 0; o < kOpsPerBlock; o++) {
+         const int op = ops[o];
+         if (op < 0) break;
+         const int slot = op >> 3, sel = (op >> 1) & 3;
+         float v[4];
+         ld4(d.ff32 + 32 * (size_t)slot + (sel == OP_SEL_L ? 0 : 16) + 4 * k, v);
+         if (sel == OP_SEL_RREFL) {
+            const double4 rf = d.refl[d.slot_face[slot]];
+            const float r01 = v[1], r02 = v[2];
+            v[1] = float(rf.x) * r01 + float(rf.y) * r02;
+            v[2] = float(rf.z) * r01 + float(rf.w) * r02;
+         }
+#pragma unroll
+         for (int m = 0; m < 4; m++) {
+            if (op & 1) acc[m] -= v[m];
+            else acc[m] += v[m];
+         }
       }
 #pragma unroll
       for (int m = 0; m < 4; m++) {
-         if (op & 1) acc[m] -= v[m];
-         else acc[m] += v[m];
+         acc[m] *= s;
+         if (b == 1 && m == k) acc[m] += 1.f;
       }
+      st4(d.blk32 + tix(srow, 48, 16 * b + 4 * k, lane), acc);
    }
-   const float s = float(d.dtfac[sc]);
-#pragma unroll
-   for (int m = 0; m < 4; m++) {
-      acc[m] *= s;
-      if (b == 1 && m == k) acc[m] += 1.f;
-   }
-   st4(d.blk32 + tix(srow, 48, 16 * b + 4 * k, lane), acc);
 }
 
 // whether chain ich takes the segmented solve: sp_on 1 takes the long
@@ -523,7 +527,6 @@ constexpr int kElimChunk = 2;
 // mx_assemble_kernel wrote, through its ring (512 x 128, 30% split: 124 us with
 // the next row's blocks in registers, 76 us so; 32 meshes of 983,040 cells: 89 us).
 constexpr int kFactorDepth = 4, kFactorVec = 12;
-static_assert(kFactorDepth * kFactorVec == kStageTerms * 4, "either form takes the same shared memory");
 
 template <bool FUSED, int ED>
 __global__ void __launch_bounds__(256) mx_factor_kernel(DeviceState d, int count)
@@ -644,6 +647,84 @@ __global__ void __launch_bounds__(256) mx_factor_kernel(DeviceState d, int count
    if (bad) atomicOr(d.status, DEV_ERR_PIVOT);
 }
 
+// y -= M x (4x4, 4-vector)
+__device__ __forceinline__ void mv_sub(const float (&M)[16], const float (&x)[4], float (&y)[4])
+{
+#pragma unroll
+   for (int k = 0; k < 4; k++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) y[k] = __fmaf_rn(-M[4 * k + j], x[j], y[k]);
+}
+
+__device__ __forceinline__ void mv_add(const float (&M)[16], const float (&x)[4], float (&y)[4])
+{
+#pragma unroll
+   for (int k = 0; k < 4; k++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) y[k] = __fmaf_rn(M[4 * k + j], x[j], y[k]);
+}
+
+// The rings of the solves: a row's record by halves (A and LU, or two of C', V,
+// W), and a 4-vector; cells are looked up kSolveLook rows before their copies.
+constexpr int kSolveVec = 9, kSolveLook = 4;
+constexpr size_t kFacRow = 32 * kRec, kFsRow = 128;   // floats from a tile row to the next
+
+// f(i) = LU^{-1}(F(i) - A(i) f(i-1)) for a thread's n tiled rows, F(i) =
+// r32[fcell[i]] (0 without a cell); f into fs, the last f in xp
+template <int DEPTH>
+__device__ __forceinline__ void forward_rows(const RowRing<kSolveVec, DEPTH>& ring, int n, const float* fac, float* fs, const int* fcell,
+                                             const float* r32, float (&xp)[4])
+{
+   constexpr int AHEAD = DEPTH - 1;
+   auto fetch = [&](int i, int cell) {
+      if (i < n) {
+         ring.template copy<8>(i, 0, fac + kFacRow * i);
+         if (cell >= 0) cp_async16_cg(ring.at(i, 8), r32 + 4 * (size_t)cell);
+         else *ring.at(i, 8) = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      cp_async_commit();
+   };
+   auto look = [&](int i) { return i < n ? fcell[i] : -1; };
+#pragma unroll
+   for (int i = 0; i < AHEAD; i++) fetch(i, look(i));
+   int fc[kSolveLook];
+#pragma unroll
+   for (int u = 0; u < kSolveLook; u++) fc[u] = look(AHEAD + u);
+   // a row leaves the ring while the one before it is solved
+   float a[16], lu[16], x[4];
+   cp_async_wait<AHEAD - 1>();
+   ring.read(0, 0, a);
+   ring.read(0, 4, lu);
+   ring.read(0, 8, x);
+   for (int i0 = 0; i0 < n; i0 += kSolveLook) {
+      int fcn[kSolveLook];
+#pragma unroll
+      for (int u = 0; u < kSolveLook; u++) fcn[u] = look(i0 + AHEAD + kSolveLook + u);
+#pragma unroll
+      for (int u = 0; u < kSolveLook; u++) {
+         const int i = i0 + u;
+         if (i >= n) break;
+         float an[16], ln[16], y[4];
+         cp_async_wait<AHEAD - 2>();
+         ring.read(i + 1, 0, an);   // (past the last row: what the slot holds, unused)
+         ring.read(i + 1, 4, ln);
+         ring.read(i + 1, 8, y);
+         fetch(i + AHEAD, fc[u]);
+         if (i > 0) mv_sub(a, xp, x);
+         luf_solve(luf_of(lu), x[0], x[1], x[2], x[3]);
+         *reinterpret_cast<float4*>(fs + kFsRow * i) = make_float4(x[0], x[1], x[2], x[3]);
+#pragma unroll
+         for (int k = 0; k < 4; k++) { xp[k] = x[k]; x[k] = y[k]; }
+#pragma unroll
+         for (int m = 0; m < 16; m++) { a[m] = an[m]; lu[m] = ln[m]; }
+      }
+#pragma unroll
+      for (int u = 0; u < kSolveLook; u++) fc[u] = fcn[u];
+   }
+   cp_async_wait_all();
+   __threadfence_block();   // f, before copies of it into the ring
+}
+
 // One sweep's solve of one chain per thread (the chain at position first +
 // t of line_chains).  The recurrence only carries the 4-vector x in
 // registers; what a row needs comes through the thread's ring (its factor
@@ -651,10 +732,10 @@ __global__ void __launch_bounds__(256) mx_factor_kernel(DeviceState d, int count
 // that, later the forward sweep's row).  Solutions go straight to r32 (each
 // cell is written once per chain; chains of a wave share no cell).
 // Bound by the chain: with the loads of four rows issued together a row of the
-// longest chain took 480 cycles forward or back, through the ring 330 (512 x 128,
-// 30% split: the four solves of a step 207 -> 141 us; unsplit 170 -> 116 us; 32
-// meshes of 983,040 cells 270 -> 142 us).
-constexpr int kSolveDepth = 8, kSolveVec = 9, kSolveLook = 4;
+// longest chain took 480 cycles forward or back, through the ring 310 (512 x 128,
+// 30% split: the four solves of a step 207 -> 136 us; unsplit 170 -> 108 us; 32
+// meshes of 983,040 cells 270 -> 143 us).
+constexpr int kSolveDepth = 8;
 
 __global__ void __launch_bounds__(128) mx_solve_kernel(DeviceState d, int first, int count)
 {
@@ -670,57 +751,11 @@ __global__ void __launch_bounds__(128) mx_solve_kernel(DeviceState d, int first,
    extern __shared__ float4 stage[];
    const RowRing<kSolveVec, kSolveDepth> ring(stage);
    constexpr int AHEAD = kSolveDepth - 1;
-   const float* fac = d.fac32 + tix(s0, kRec, 0, lane);      // row i at + 32 * kRec * i
-   float* fsr = d.fsc32 + tix(s0, 4, 0, lane);               // row i at + 128 * i
-   constexpr size_t kFacRow = 32 * kRec, kFsRow = 128;
-   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-
-   // forward: f(i) = LU^{-1}(F(i) - A(i) f(i-1)), F(i) = r[fcell] (0 without one)
-   float x[4], xp[4] = {0.f, 0.f, 0.f, 0.f};
-   auto fetch = [&](int i, int cell) {
-      if (i < N) {
-         ring.copy<8>(i, 0, fac + kFacRow * i);
-         if (cell >= 0) cp_async16_cg(ring.at(i, 8), d.r32 + 4 * (size_t)cell);
-         else *ring.at(i, 8) = zero4;
-      }
-      cp_async_commit();
-   };
-   auto look = [&](const int* cells, int i) { return i >= 0 && i < N ? cells[i] : -1; };
-#pragma unroll
-   for (int i = 0; i < AHEAD; i++) fetch(i, look(fcell, i));
-   int fc[kSolveLook];
-#pragma unroll
-   for (int u = 0; u < kSolveLook; u++) fc[u] = look(fcell, AHEAD + u);
-   for (int i0 = 0; i0 < N; i0 += kSolveLook) {
-      int fcn[kSolveLook];
-#pragma unroll
-      for (int u = 0; u < kSolveLook; u++) fcn[u] = look(fcell, i0 + AHEAD + kSolveLook + u);
-#pragma unroll
-      for (int u = 0; u < kSolveLook; u++) {
-         const int i = i0 + u;
-         if (i >= N) break;
-         cp_async_wait<AHEAD - 1>();
-         float a[16], lu[16];
-         ring.read(i, 0, a);
-         ring.read(i, 4, lu);
-         ring.read(i, 8, x);
-         fetch(i + AHEAD, fc[u]);
-         if (i > 0) {
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-#pragma unroll
-               for (int j = 0; j < 4; j++) x[k] = __fmaf_rn(-a[4 * k + j], xp[j], x[k]);
-         }
-         luf_solve(luf_of(lu), x[0], x[1], x[2], x[3]);
-         *reinterpret_cast<float4*>(fsr + kFsRow * i) = make_float4(x[0], x[1], x[2], x[3]);
-#pragma unroll
-         for (int k = 0; k < 4; k++) xp[k] = x[k];
-      }
-#pragma unroll
-      for (int u = 0; u < kSolveLook; u++) fc[u] = fcn[u];
-   }
-   cp_async_wait_all();
-   __threadfence_block();   // the forward rows, before the copies below read them
+   const float* fac = d.fac32 + tix(s0, kRec, 0, lane);
+   float* fsr = d.fsc32 + tix(s0, 4, 0, lane);
+   float x[4], xp[4];
+   forward_rows(ring, N, fac, fsr, fcell, d.r32, xp);
+   auto look = [&](const int* cells, int i) { return i >= 0 ? cells[i] : -1; };
    float xn[4], fN[4] = {xp[0], xp[1], xp[2], xp[3]};
    if (per) {
       // last row: f(N-1) - sum over i < N-1 of cN(i) f(i), in row order
@@ -739,10 +774,7 @@ __global__ void __launch_bounds__(128) mx_solve_kernel(DeviceState d, int first,
          ring.read(i, 0, c);
          ring.read(i, 8, f);
          fetch_last(i + AHEAD);
-#pragma unroll
-         for (int k = 0; k < 4; k++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) fN[k] = __fmaf_rn(-c[4 * k + j], f[j], fN[k]);
+         mv_sub(c, f, fN);
       }
       cp_async_wait_all();
       const LUf uN = luf_load(d.facN32 + 16 * d.chain_facN[ich]);
@@ -767,6 +799,11 @@ __global__ void __launch_bounds__(128) mx_solve_kernel(DeviceState d, int first,
    int sc[kSolveLook];
 #pragma unroll
    for (int u = 0; u < kSolveLook; u++) sc[u] = look(scell, N - 2 - u);
+   float c[16], aa[16];
+   cp_async_wait<AHEAD - 1>();
+   ring.read(0, 0, c);
+   if (per) ring.read(0, 4, aa);
+   ring.read(0, 8, x);
    for (int q0 = 0; q0 <= N - 2; q0 += kSolveLook) {
       int scn[kSolveLook];
 #pragma unroll
@@ -775,11 +812,11 @@ __global__ void __launch_bounds__(128) mx_solve_kernel(DeviceState d, int first,
       for (int u = 0; u < kSolveLook; u++) {
          const int s = q0 + u;
          if (s > N - 2) break;
-         cp_async_wait<AHEAD - 1>();
-         float c[16], aa[16];
-         ring.read(s, 0, c);
-         if (per) ring.read(s, 4, aa);
-         ring.read(s, 8, x);
+         float cn[16], an[16], y[4];
+         cp_async_wait<AHEAD - 2>();
+         ring.read(s + 1, 0, cn);
+         if (per) ring.read(s + 1, 4, an);
+         ring.read(s + 1, 8, y);
          fetch_back(s + AHEAD);
 #pragma unroll
          for (int k = 0; k < 4; k++)
@@ -794,7 +831,12 @@ __global__ void __launch_bounds__(128) mx_solve_kernel(DeviceState d, int first,
             }
          st4(d.r32 + 4 * (size_t)sc[u], x);
 #pragma unroll
-         for (int k = 0; k < 4; k++) xn[k] = x[k];
+         for (int k = 0; k < 4; k++) { xn[k] = x[k]; x[k] = y[k]; }
+#pragma unroll
+         for (int m = 0; m < 16; m++) {
+            c[m] = cn[m];
+            if (per) aa[m] = an[m];
+         }
       }
 #pragma unroll
       for (int u = 0; u < kSolveLook; u++) sc[u] = scn[u];
@@ -849,23 +891,6 @@ constexpr int kRedLast = kRedRow * (kSpikeMaxSeg - 1);
 static_assert(kRedLast + 64 + 32 <= kSpikeRedStride, "boundary-system factors fit their stride");
 enum { RX = 0, RS = 16, RGT = 32, RGB = 48, RHT = 64, RHB = 80, RWE = 96, RWS = 112 };
 
-// y -= M x (4x4, 4-vector)
-__device__ __forceinline__ void mv_sub(const float (&M)[16], const float (&x)[4], float (&y)[4])
-{
-#pragma unroll
-   for (int k = 0; k < 4; k++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) y[k] = __fmaf_rn(-M[4 * k + j], x[j], y[k]);
-}
-
-__device__ __forceinline__ void mv_add(const float (&M)[16], const float (&x)[4], float (&y)[4])
-{
-#pragma unroll
-   for (int k = 0; k < 4; k++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) y[k] = __fmaf_rn(M[4 * k + j], x[j], y[k]);
-}
-
 // out = M X (4x4)
 __device__ __forceinline__ void mm_mul(const float (&M)[16], const float (&X)[16], float (&out)[16])
 {
@@ -891,14 +916,18 @@ __device__ __forceinline__ void st16s(float* p, const float (&v)[16])
 // 8x8 row-major LU with reciprocal pivots (K, once per chain and step):
 // M = L U, U unit upper; L below and on the diagonal (the diagonal holding
 // 1/L_kk)
-__device__ void m8_lu(float* M)
+__device__ __forceinline__ void m8_lu(float (&M)[64])
 {
+#pragma unroll   // M stays in registers
    for (int k = 0; k < 8; k++) {
       const float piv = 1.f / M[9 * k];
       M[9 * k] = piv;
+#pragma unroll
       for (int j = k + 1; j < 8; j++) M[8 * k + j] *= piv;
+#pragma unroll
       for (int i = k + 1; i < 8; i++) {
          const float l = M[8 * i + k];
+#pragma unroll
          for (int j = k + 1; j < 8; j++) M[8 * i + j] = __fmaf_rn(-l, M[8 * k + j], M[8 * i + j]);
       }
    }
@@ -937,8 +966,14 @@ __device__ __forceinline__ void schur_cols(const float (&X)[16], const LUf& s, c
    mm_sub(X, Vv, U);
 }
 
+// One warp per chain.  Bound by the chain of its rows, then of the boundary
+// system's.  FUSED: as in mx_factor_kernel; otherwise the blocks that
+// mx_assemble_kernel wrote, through the lane's ring (512 x 128: 82 us
+// inside, 59 us so; 32 meshes of 983,040 cells 304 and 221 us).
+template <bool FUSED>
 __global__ void __launch_bounds__(32) mx_spike_factor_kernel(DeviceState d)
 {
+   extern __shared__ float4 stage[];
    __shared__ __align__(16) float tips[kSpikeMaxSeg * 64];   // per segment: V_s, W_s, V_e, W_e
    const int sp = blockIdx.x, lane = threadIdx.x;
    const int ich = d.sp_chain[sp];
@@ -954,18 +989,40 @@ __global__ void __launch_bounds__(32) mx_spike_factor_kernel(DeviceState d)
       // at the last row the right spike B'^{-1}(-C_e).  The next row's blocks
       // are assembled from references looked up a row earlier.
       float A[16], B[16], C[16], cp[16], gw[16];
-      RowRef rnext = mx_rowref(d, row0 + s + 1);
-      mx_row_ref(d, mx_rowref(d, row0 + s), A, B, C);
-      // an open chain: no coupling from its first row back to its last
-      if (!per && lane == 0) {
+      RowRef rnext{};
+      const RowRing<kFactorVec, kFactorDepth> ring(stage);
+      constexpr int AHEAD = kFactorDepth - 1;
+      const int pos = d.sp_pos[sp];
+      const float* blk = FUSED ? nullptr : d.blk32 + tix(d.grp_row0[pos >> 5] + s, 48, 0, pos & 31);
+      auto fetch = [&](int k) {
+         if (k < n) ring.copy<12>(k, 0, blk + 32 * 48 * (size_t)k);
+         cp_async_commit();
+      };
+      if (FUSED) {
+         rnext = mx_rowref(d, row0 + s + 1);
+         mx_row_ref(d, mx_rowref(d, row0 + s), A, B, C);
+      } else {
 #pragma unroll
-         for (int m = 0; m < 16; m++) A[m] = 0.f;
+         for (int k = 0; k < AHEAD; k++) fetch(k);
       }
       for (int k = 0; k < n; k++) {
          float An[16], Bn[16], Cn[16];
-         if (k + 1 < n) {
-            mx_row_ref(d, rnext, An, Bn, Cn);
-            if (k + 2 < n) rnext = mx_rowref(d, row0 + s + k + 2);
+         if (FUSED) {
+            if (k + 1 < n) {
+               mx_row_ref(d, rnext, An, Bn, Cn);
+               if (k + 2 < n) rnext = mx_rowref(d, row0 + s + k + 2);
+            }
+         } else {
+            cp_async_wait<AHEAD - 1>();
+            ring.read(k, 0, A);
+            ring.read(k, 4, B);
+            ring.read(k, 8, C);
+            fetch(k + AHEAD);
+         }
+         // an open chain: no coupling from its first row back to its last
+         if (k == 0 && !per && lane == 0) {
+#pragma unroll
+            for (int m = 0; m < 16; m++) A[m] = 0.f;
          }
          float* rec = d.sp_fac + tix(R0 + k, kSpRec, 0, lane);
          st16t(rec, A);
@@ -990,7 +1047,11 @@ __global__ void __launch_bounds__(32) mx_spike_factor_kernel(DeviceState d)
             luf_cols(u, C);
             st16t(rec + 32 * 32, C);
 #pragma unroll
-            for (int m = 0; m < 16; m++) { cp[m] = C[m]; A[m] = An[m]; B[m] = Bn[m]; C[m] = Cn[m]; }
+            for (int m = 0; m < 16; m++) cp[m] = C[m];
+            if (FUSED) {
+#pragma unroll
+               for (int m = 0; m < 16; m++) { A[m] = An[m]; B[m] = Bn[m]; C[m] = Cn[m]; }
+            }
          } else {
             // (an open chain's last row has no coupling forward to its first)
             const bool wrap = per || lane + 1 < P;
@@ -1001,37 +1062,45 @@ __global__ void __launch_bounds__(32) mx_spike_factor_kernel(DeviceState d)
          }
       }
       // back substitution of both spikes: V_k = -C'_k V_{k+1},
-      // W_k = g_k - C'_k W_{k+1}; row k-1's C' and g are loaded while row k
-      // is formed
-      float vn[16], wn[16], c[16], g[16];
-      ld16t(d.sp_fac + tix(R0 + n - 1, kSpRec, 48, lane), vn);
-      ld16t(d.sp_fac + tix(R0 + n - 1, kSpRec, 64, lane), wn);
+      // W_k = g_k - C'_k W_{k+1}, C' and g through the ring (step j: row n-2-j)
+      cp_async_wait_all();
+      __threadfence_block();   // the rows above, before copies of them
+      float* rec = d.sp_fac + tix(R0, kSpRec, 0, lane);
+      constexpr int BD = FUSED ? 2 : kFactorDepth, BA = BD - 1;
+      const RowRing<8, BD> back(stage);
+      auto fetch_back = [&](int j) {
+         const int k = n - 2 - j;
+         if (k >= 0) {
+            back.template copy<4>(j, 0, rec + kFacRow * k + 32 * 32);
+            back.template copy<4>(j, 4, rec + kFacRow * k + 32 * 64);
+         }
+         cp_async_commit();
+      };
+#pragma unroll
+      for (int j = 0; j < BA; j++) fetch_back(j);
+      float vn[16], wn[16];
+#pragma unroll
+      for (int m = 0; m < 16; m++) { vn[m] = C[m]; wn[m] = gw[m]; }
       float* tip = tips + 64 * lane;
       st16s(tip + 32, vn);   // V_e
       st16s(tip + 48, wn);   // W_e
-      ld16t(d.sp_fac + tix(R0 + n - 2, kSpRec, 32, lane), c);
-      ld16t(d.sp_fac + tix(R0 + n - 2, kSpRec, 64, lane), g);
       for (int k = n - 2; k >= 0; k--) {
-         float cn[16], gn[16];
-         if (k > 0) {
-            ld16t(d.sp_fac + tix(R0 + k - 1, kSpRec, 32, lane), cn);
-            ld16t(d.sp_fac + tix(R0 + k - 1, kSpRec, 64, lane), gn);
-         }
-         float v[16];
+         const int j = n - 2 - k;
+         cp_async_wait<BA - 1>();
+         float c[16], g[16], v[16];
+         back.read(j, 0, c);
+         back.read(j, 4, g);
+         fetch_back(j + BA);
 #pragma unroll
          for (int m = 0; m < 16; m++) v[m] = 0.f;
          mm_sub(c, vn, v);
          mm_sub(c, wn, g);
-         float* rec = d.sp_fac + tix(R0 + k, kSpRec, 0, lane);
-         st16t(rec + 32 * 48, v);
-         st16t(rec + 32 * 64, g);
+         st16t(rec + kFacRow * k + 32 * 48, v);
+         st16t(rec + kFacRow * k + 32 * 64, g);
 #pragma unroll
          for (int m = 0; m < 16; m++) { vn[m] = v[m]; wn[m] = g[m]; }
-         if (k > 0) {
-#pragma unroll
-            for (int m = 0; m < 16; m++) { c[m] = cn[m]; g[m] = gn[m]; }
-         }
       }
+      cp_async_wait_all();
       st16s(tip, vn);        // V_s
       st16s(tip + 16, wn);   // W_s
    }
@@ -1137,8 +1206,10 @@ __global__ void __launch_bounds__(32) mx_spike_factor_kernel(DeviceState d)
 #pragma unroll
       for (int j = 0; j < 4; j++) K[8 * (4 + k) + 4 + j] = ((k == j) ? 1.f : 0.f) - M4[4 * k + j];
    m8_lu(K);
+#pragma unroll
    for (int k = 0; k < 8; k++) kbad |= nonfinite(K[9 * k]);
    float* last = red + kRedLast;
+#pragma unroll
    for (int m = 0; m < 64; m++) last[m] = K[m];
    st16s(last + 64, We);
    st16s(last + 80, Vs0);
@@ -1146,7 +1217,13 @@ __global__ void __launch_bounds__(32) mx_spike_factor_kernel(DeviceState d)
 }
 
 // one sweep's solve of the spike chains sp = first .. first+count-1 of a
-// wave: right-hand sides r32[fcell], solutions into r32[scell]
+// wave: right-hand sides r32[fcell], solutions into r32[scell].  Every pass over
+// a segment's rows goes through the lane's ring, the last one's first rows and
+// the boundary system's factors while other work runs.  The two solves of a step
+// (512 x 128): 90 us with each row's loads a row ahead, 58 us so; 32 meshes of
+// 983,040 cells 330 and 259 us.
+constexpr int kSpikeSolveDepth = 4;   // 36 KB a block with the boundary system's factors: six to an SM
+
 __global__ void __launch_bounds__(32) mx_spike_solve_kernel(DeviceState d, int first)
 {
    // (red_s is read with float4 loads: 16-byte aligned)
@@ -1163,78 +1240,62 @@ __global__ void __launch_bounds__(32) mx_spike_solve_kernel(DeviceState d, int f
       // one step after another below)
       const float* red = d.sp_red + (size_t)kSpikeRedStride * sp;
       const int nrow = kRedRow * (P - 1);
-      for (int m = lane; m < nrow; m += 32) red_s[m] = red[m];
-      for (int m = lane; m < 96; m += 32) red_s[kRedLast + m] = red[kRedLast + m];
+      for (int m = 4 * lane; m < nrow; m += 128) cp_async16_cg(red_s + m, red + m);
+      if (lane < 24) cp_async16_cg(red_s + kRedLast + 4 * lane, red + kRedLast + 4 * lane);
    }
+   extern __shared__ float4 stage[];
+   const RowRing<kSolveVec, kSpikeSolveDepth> ring(stage);
+   constexpr int AHEAD = kSpikeSolveDepth - 1;
+   const float* fac = d.sp_fac + tix(R0, kSpRec, 0, lane);
+   float* ys = d.sp_y + tix(R0, 4, 0, lane);
+   auto fetch_rows = [&](int k, int n) {   // V, W and y of row k
+      if (k < n) {
+         ring.copy<8>(k, 0, fac + kFacRow * k + 32 * 48);
+         cp_async16_cg(ring.at(k, 8), ys + kFsRow * k);
+      }
+      cp_async_commit();
+   };
    int s = 0, n = 0;
    if (lane < P) {
       s = seg[lane];
       n = seg[lane + 1] - s;
-      const int* fcell = d.row_fcell + row0 + s;
-      // forward: y'_k = B'^{-1}(f_k - A_k y'_{k-1}); row k+1's record and
-      // right-hand side are loaded while row k is solved
-      float a[16], yp[4] = {0.f, 0.f, 0.f, 0.f}, x[4] = {0.f, 0.f, 0.f, 0.f};
-      LUf u = luf_load_t(d.sp_fac + tix(R0, kSpRec, 16, lane));
-      {
-         const int fc = fcell[0];
-         if (fc >= 0) ld4(d.r32 + 4 * (size_t)fc, x);
-      }
-#pragma unroll
-      for (int m = 0; m < 16; m++) a[m] = 0.f;
-      for (int k = 0; k < n; k++) {
-         float an[16], xn[4] = {0.f, 0.f, 0.f, 0.f};
-         LUf un;
-         if (k + 1 < n) {
-            const float* rn = d.sp_fac + tix(R0 + k + 1, kSpRec, 0, lane);
-            ld16t(rn, an);
-            un = luf_load_t(rn + 32 * 16);
-            const int fc = fcell[k + 1];
-            if (fc >= 0) ld4(d.r32 + 4 * (size_t)fc, xn);
-         }
-         if (k > 0) mv_sub(a, yp, x);
-         luf_solve(u, x[0], x[1], x[2], x[3]);
-#pragma unroll
-         for (int c = 0; c < 4; c++) {
-            d.sp_y[tix(R0 + k, 4, c, lane)] = x[c];
-            yp[c] = x[c];
-         }
-         if (k + 1 < n) {
-#pragma unroll
-            for (int m = 0; m < 16; m++) a[m] = an[m];
-            u = un;
-#pragma unroll
-            for (int c = 0; c < 4; c++) x[c] = xn[c];
-         }
-      }
-      // back: y_k = y'_k - C'_k y_{k+1}
+      // forward: y'_k = B'^{-1}(f_k - A_k y'_{k-1})
+      float yp[4];
+      forward_rows(ring, n, fac, ys, d.row_fcell + row0 + s, d.r32, yp);
+      // back: y_k = y'_k - C'_k y_{k+1} (step j: row n-2-j)
 #pragma unroll
       for (int c = 0; c < 4; c++) ry[8 * lane + 4 + c] = yp[c];
-      float cm[16], yk[4];
-      ld16t(d.sp_fac + tix(R0 + n - 2, kSpRec, 32, lane), cm);
+      auto fetch_back = [&](int j) {
+         const int k = n - 2 - j;
+         if (k >= 0) {
+            ring.copy<4>(j, 0, fac + kFacRow * k + 32 * 32);
+            cp_async16_cg(ring.at(j, 8), ys + kFsRow * k);
+         }
+         cp_async_commit();
+      };
 #pragma unroll
-      for (int c = 0; c < 4; c++) yk[c] = d.sp_y[tix(R0 + n - 2, 4, c, lane)];
+      for (int j = 0; j < AHEAD; j++) fetch_back(j);
       for (int k = n - 2; k >= 0; k--) {
-         float cn[16], ykn[4];
-         if (k > 0) {
-            ld16t(d.sp_fac + tix(R0 + k - 1, kSpRec, 32, lane), cn);
-#pragma unroll
-            for (int c = 0; c < 4; c++) ykn[c] = d.sp_y[tix(R0 + k - 1, 4, c, lane)];
-         }
+         const int j = n - 2 - k;
+         cp_async_wait<AHEAD - 1>();
+         float cm[16], yk[4];
+         ring.read(j, 0, cm);
+         ring.read(j, 8, yk);
+         fetch_back(j + AHEAD);
          mv_sub(cm, yp, yk);
+         *reinterpret_cast<float4*>(ys + kFsRow * k) = make_float4(yk[0], yk[1], yk[2], yk[3]);
 #pragma unroll
-         for (int c = 0; c < 4; c++) {
-            d.sp_y[tix(R0 + k, 4, c, lane)] = yk[c];
-            yp[c] = yk[c];
-         }
-         if (k > 0) {
-#pragma unroll
-            for (int m = 0; m < 16; m++) cm[m] = cn[m];
-#pragma unroll
-            for (int c = 0; c < 4; c++) yk[c] = ykn[c];
-         }
+         for (int c = 0; c < 4; c++) yp[c] = yk[c];
       }
+      cp_async_wait_all();
+      __threadfence_block();   // y, before copies of it
 #pragma unroll
       for (int c = 0; c < 4; c++) ry[8 * lane + c] = yp[c];
+      // on their way while lane 0 solves the boundary system
+#pragma unroll
+      for (int k = 0; k < AHEAD; k++) fetch_rows(k, n);
+   } else {
+      cp_async_wait_all();
    }
    __syncwarp();
    if (lane == 0) {
@@ -1320,8 +1381,7 @@ __global__ void __launch_bounds__(32) mx_spike_solve_kernel(DeviceState d, int f
    }
    __syncwarp();
    if (lane < P) {
-      // x_k = y_k + V_k t_{p+1} + W_k b_{p-1}; row k+1's data loaded while
-      // row k is formed
+      // x_k = y_k + V_k t_{p+1} + W_k b_{p-1}
       float tn[4], bp[4];
       const int pm = (lane == 0) ? P - 1 : lane - 1;
 #pragma unroll
@@ -1330,33 +1390,31 @@ __global__ void __launch_bounds__(32) mx_spike_solve_kernel(DeviceState d, int f
          bp[c] = zs[8 * pm + c];
       }
       const int* scell = d.row_scell + row0 + s;
-      float v[16], w[16], x[4];
-      ld16t(d.sp_fac + tix(R0, kSpRec, 48, lane), v);
-      ld16t(d.sp_fac + tix(R0, kSpRec, 64, lane), w);
+      int sc[kSolveLook];
 #pragma unroll
-      for (int c = 0; c < 4; c++) x[c] = d.sp_y[tix(R0, 4, c, lane)];
-      int sc = scell[0];
-      for (int k = 0; k < n; k++) {
-         float vn[16], wn[16], xn[4];
-         int scn = 0;
-         if (k + 1 < n) {
-            ld16t(d.sp_fac + tix(R0 + k + 1, kSpRec, 48, lane), vn);
-            ld16t(d.sp_fac + tix(R0 + k + 1, kSpRec, 64, lane), wn);
+      for (int u = 0; u < kSolveLook; u++) sc[u] = u < n ? scell[u] : 0;
+      for (int k0 = 0; k0 < n; k0 += kSolveLook) {
+         int scn[kSolveLook];
 #pragma unroll
-            for (int c = 0; c < 4; c++) xn[c] = d.sp_y[tix(R0 + k + 1, 4, c, lane)];
-            scn = scell[k + 1];
+         for (int u = 0; u < kSolveLook; u++) scn[u] = k0 + kSolveLook + u < n ? scell[k0 + kSolveLook + u] : 0;
+#pragma unroll
+         for (int u = 0; u < kSolveLook; u++) {
+            const int k = k0 + u;
+            if (k >= n) break;
+            cp_async_wait<AHEAD - 1>();
+            float v[16], w[16], x[4];
+            ring.read(k, 0, v);
+            ring.read(k, 4, w);
+            ring.read(k, 8, x);
+            fetch_rows(k + AHEAD, n);
+            mv_add(w, bp, x);
+            mv_add(v, tn, x);
+            st4(d.r32 + 4 * (size_t)sc[u], x);
          }
-         mv_add(w, bp, x);
-         mv_add(v, tn, x);
-         st4(d.r32 + 4 * (size_t)sc, x);
-         if (k + 1 < n) {
 #pragma unroll
-            for (int m = 0; m < 16; m++) { v[m] = vn[m]; w[m] = wn[m]; }
-#pragma unroll
-            for (int c = 0; c < 4; c++) x[c] = xn[c];
-            sc = scn;
-         }
+         for (int u = 0; u < kSolveLook; u++) sc[u] = scn[u];
       }
+      cp_async_wait_all();
    }
 }
 
@@ -1498,15 +1556,16 @@ void launch_mx_rhs_face(const DeviceState& d, cudaStream_t st)
 
 void launch_mx_assemble(const DeviceState& d, cudaStream_t st)
 {
-   const size_t n = 12 * 32 * (size_t)d.tile_rows;
+   const size_t n = 128 * (size_t)d.tile_rows;
    if (!d.mx_fused && n > 0) mx_assemble_kernel<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, st>>>(d);
 }
 
 void launch_mx_init(const DeviceState& d, cudaStream_t st) { mx_init_kernel<<<blocks_for(d.nCell), kThreads, 0, st>>>(d); }
 
 // dynamic shared memory of the factorisation (staged terms or ring) and of the solve (ring)
-size_t mx_factor_stage_bytes(int block) { return (size_t)kStageTerms * 4 * sizeof(float4) * block; }
+size_t mx_factor_stage_bytes(int block) { return (size_t)std::max(kStageTerms * 4, kFactorDepth * kFactorVec) * sizeof(float4) * block; }
 size_t mx_solve_ring_bytes(int block) { return (size_t)kSolveDepth * kSolveVec * sizeof(float4) * block; }
+constexpr size_t kSpikeRingBytes = (size_t)kSpikeSolveDepth * kSolveVec * sizeof(float4) * 32;
 
 int mx_configure()
 {
@@ -1516,6 +1575,16 @@ int mx_configure()
    for (const void* f : factor)
       if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, want) != cudaSuccess) return 1;
    if (cudaFuncSetAttribute(mx_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ring) != cudaSuccess) return 1;
+   // these run beside each other: an SM takes blocks of two kernels at a time
+   // only where both ask for the same split of its L1 (eight steps of 512 x 128
+   // with the assembly inside 6.6 -> 5.1 ms)
+   const void* beside[] = {factor[0], factor[1], factor[2], factor[3], (const void*)mx_solve_kernel,
+                           (const void*)mx_spike_factor_kernel<true>, (const void*)mx_spike_factor_kernel<false>,
+                           (const void*)mx_spike_solve_kernel};
+   for (const void* f : beside)
+      if (cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) !=
+          cudaSuccess)
+         return 1;
    return 0;
 }
 
@@ -1553,12 +1622,14 @@ int mx_solve_chunk_capacity(int block)
 
 void launch_mx_spike_factor(const DeviceState& d, cudaStream_t st)
 {
-   if (d.sp_on && d.nSpike > 0) mx_spike_factor_kernel<<<d.nSpike, 32, 0, st>>>(d);
+   if (!d.sp_on || d.nSpike <= 0) return;
+   if (d.mx_fused) mx_spike_factor_kernel<true><<<d.nSpike, 32, 2 * 8 * 32 * sizeof(float4), st>>>(d);
+   else mx_spike_factor_kernel<false><<<d.nSpike, 32, mx_factor_stage_bytes(32), st>>>(d);
 }
 
 void launch_mx_spike_solve(const DeviceState& d, int first, int count, cudaStream_t st)
 {
-   if (d.sp_on && count > 0) mx_spike_solve_kernel<<<count, 32, 0, st>>>(d, first);
+   if (d.sp_on && count > 0) mx_spike_solve_kernel<<<count, 32, kSpikeRingBytes, st>>>(d, first);
 }
 
 void launch_mx_dq_update(const DeviceState& d, cudaStream_t st)
