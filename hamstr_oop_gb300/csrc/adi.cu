@@ -41,54 +41,72 @@ namespace hamstr {
 namespace {
 
 
-// one block entry (row-major element e) in the reference's term order
-// (ADI.cpp:103-188): 0.0, then += / -= the listed face-matrix entries.
+// two entries of a block's row k (columns 2 c2 and 2 c2 + 1) in the reference's
+// term order (ADI.cpp:103-188): 0.0, then += / -= the listed face-matrix entries.
 // The first term needs no FP64 add: 0.0 + v is v and 0.0 - v is -v, except
 // that both are +0.0 when v is a zero, so it is formed on the integer pipes
-// with the same result (this kernel is FP64-issue bound).
-__device__ __forceinline__ double assemble(const DeviceState& d, const int* __restrict__ ops, int e)
+// with the same result.
+__device__ __forceinline__ double2 assemble(const DeviceState& d, const int4& list, int k, int c2)
 {
-   double acc = 0.0;
+   const int ops[kOpsPerBlock] = {list.x, list.y, list.z, list.w};
+   double2 acc = make_double2(0.0, 0.0);
 #pragma unroll
    for (int o = 0; o < kOpsPerBlock; o++) {
       const int op = ops[o];
       if (op < 0) break;
       const int slot = op >> 3, sel = (op >> 1) & 3;
-      const double* m = d.ff + 32 * (size_t)slot;
-      double v;
-      const int col = e & 3;
-      if (sel == OP_SEL_RREFL && (col == 1 || col == 2)) {
+      const double* m = d.ff + 32 * (size_t)slot + (sel == OP_SEL_L ? 0 : 16) + 4 * k;
+      double2 v = *reinterpret_cast<const double2*>(m + 2 * c2);
+      if (sel == OP_SEL_RREFL) {
          // rmat with reflected momentum columns (ADI.cpp:151-163)
          const double4 rf = d.refl[d.slot_face[slot]];
-         const double r01 = m[16 + (e & ~3) + 1], r02 = m[16 + (e & ~3) + 2];
-         v = (col == 1) ? (rf.x * r01 + rf.y * r02) : (rf.z * r01 + rf.w * r02);
-      } else {
-         v = m[(sel == OP_SEL_L ? 0 : 16) + e];
+         const double r01 = m[1], r02 = m[2];
+         if (c2) v.x = rf.z * r01 + rf.w * r02;
+         else v.y = rf.x * r01 + rf.y * r02;
       }
+      const bool sub = (op & 1) != 0;
       if (o == 0) {
-         acc = sd::zero_plus(v, (op & 1) != 0);
-      } else if (op & 1) {
-         acc -= v;
+         acc.x = sd::zero_plus(v.x, sub);
+         acc.y = sd::zero_plus(v.y, sub);
+      } else if (sub) {
+         acc.x -= v.x;
+         acc.y -= v.y;
       } else {
-         acc += v;
+         acc.x += v.x;
+         acc.y += v.y;
       }
    }
    return acc;
 }
 
 // blocks A, B, C of every row, scaled by CFL/sigma with B += I
-// (ADI.cpp:197-217); one thread per entry, all rows at once
+// (ADI.cpp:197-217); eight threads to a row, each two entries of every block, so
+// that a row's lists and scale are read once for six entries.  Bound by the
+// latency of those lookups, then by FP64 and integer issue.  512 x 128, half
+// split: 64 us with a thread per entry, 47 us so.
 __global__ void __launch_bounds__(256) adi_assemble_kernel(DeviceState d)
 {
    const int t = blockIdx.x * blockDim.x + threadIdx.x;
    if (t < d.sched_nctr) d.sched_ctr[t] = 0;   // the line kernels' job counters, for this step
-   if (t >= 48 * d.nRow || halted(d)) return;
-   const int row = t / 48, e48 = t - 48 * row, b = e48 >> 4, e = e48 & 15;
-   if (frozen_cell(d, d.row_scell[row])) return;
-   double v = assemble(d, d.row_ops + 3 * kOpsPerBlock * row + kOpsPerBlock * b, e);
-   v = sd::mul(v, d.dtfac[d.row_scell[row]]);   // v * CFL/sigma on the integer pipes, identical
-   if (b == 1 && (e >> 2) == (e & 3)) v += 1.0;
-   d.blk[t] = v;
+   if (t >= 8 * d.nRow || halted(d)) return;
+   const int row = t >> 3, k = (t >> 1) & 3, c2 = t & 1;
+   const int sc = d.row_scell[row];
+   if (frozen_cell(d, sc)) return;
+   int4 list[3];
+#pragma unroll
+   for (int b = 0; b < 3; b++) list[b] = reinterpret_cast<const int4*>(d.row_ops + 3 * kOpsPerBlock * (size_t)row)[b];
+   const double s = d.dtfac[sc];
+#pragma unroll
+   for (int b = 0; b < 3; b++) {
+      double2 v = assemble(d, list[b], k, c2);
+      v.x = sd::mul(v.x, s);   // v * CFL/sigma on the integer pipes, identical
+      v.y = sd::mul(v.y, s);
+      if (b == 1 && k >> 1 == c2) {
+         if (k & 1) v.y += 1.0;
+         else v.x += 1.0;
+      }
+      *reinterpret_cast<double2*>(d.blk + 48 * (size_t)row + 16 * b + 4 * k + 2 * c2) = v;
+   }
 }
 
 // block-Thomas factorisation of chain ich (its assembled rows in blk)
@@ -462,7 +480,7 @@ int adi_configure(int max_dynamic_smem)
 
 void launch_adi_assemble(const DeviceState& d, cudaStream_t st)
 {
-   const int n = std::max(48 * d.nRow, d.sched_nctr);
+   const int n = std::max(8 * d.nRow, d.sched_nctr);
    adi_assemble_kernel<<<(n + 255) / 256, 256, 0, st>>>(d);
 }
 

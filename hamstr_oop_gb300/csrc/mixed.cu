@@ -16,6 +16,7 @@
 // similar length sharing a warp.
 // ##################################################################
 #include <algorithm>
+#include "cell_sum.cuh"
 #include "device_state.h"
 #include "plan.h"
 #include "recon.cuh"
@@ -1485,16 +1486,25 @@ __global__ void __launch_bounds__(kThreads) mx_lin_cell_kernel(DeviceState d)
       for (int k = 0; k < 4; k++) r[k] = r0[k] - dq[k];
       const float dt = float(d.dtfac[c]);
       const int e1 = d.cell_ptr[c + 1];
-      for (int e = d.cell_ptr[c]; e < e1; e++) {
-         const int ent = d.cell_ent[e];
-         float g[4];
-         ld4(d.g32 + 4 * (size_t)(ent >> 1), g);
-         if (ent & 1) {
+      for (int e = d.cell_ptr[c]; e < e1; e += kGather) {
+         int ent[kGather];
+         float g[kGather][4];
+         cell_entries(d, e, e1, ent);
 #pragma unroll
-            for (int k = 0; k < 4; k++) r[k] += g[k] * dt;
-         } else {
+         for (int u = 0; u < kGather; u++) {
+            if (e + u >= e1) break;
+            ld4(d.g32 + 4 * (size_t)(ent[u] >> 1), g[u]);
+         }
 #pragma unroll
-            for (int k = 0; k < 4; k++) r[k] -= g[k] * dt;
+         for (int u = 0; u < kGather; u++) {
+            if (e + u >= e1) break;
+            if (ent[u] & 1) {
+#pragma unroll
+               for (int k = 0; k < 4; k++) r[k] += g[u][k] * dt;
+            } else {
+#pragma unroll
+               for (int k = 0; k < 4; k++) r[k] -= g[u][k] * dt;
+            }
          }
       }
       st4(d.r32 + 4 * (size_t)c, r);
@@ -1508,21 +1518,7 @@ __global__ void __launch_bounds__(kThreads) mx_lin_cell_kernel(DeviceState d)
          st4(d.q + 4 * (size_t)c, q);
       }
    }
-   // deterministic block reduction into norm_part
-   __shared__ double s_sq[kThreads / 32], s_am[kThreads / 32];
-#pragma unroll
-   for (int o = 16; o > 0; o >>= 1) {
-      sq += __shfl_xor_sync(0xffffffffu, sq, o);
-      am = fmax(am, __shfl_xor_sync(0xffffffffu, am, o));
-   }
-   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-   if (l == 0) { s_sq[w] = sq; s_am[w] = am; }
-   __syncthreads();
-   if (threadIdx.x == 0) {
-      double a = 0.0, b = 0.0;
-      for (int i = 0; i < kThreads / 32; i++) { a += s_sq[i]; b = fmax(b, s_am[i]); }
-      d.norm_part[blockIdx.x] = make_double2(a, b);
-   }
+   block_norm(d, sq, am);
 }
 
 inline int blocks_for(int n) { return (n + kThreads - 1) / kThreads; }

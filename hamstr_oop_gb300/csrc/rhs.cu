@@ -22,6 +22,7 @@
 // The L2 norm is reduced as a fixed-shape tree (deterministic, within a
 // few ulp of the reference's serial sum); the L-infinity norm is exact.
 // ##################################################################
+#include "cell_sum.cuh"
 #include "device_state.h"
 #include "plan.h"
 #include "recon.cuh"
@@ -108,25 +109,8 @@ __global__ void __launch_bounds__(kThreads) lin_face_kernel(DeviceState d)
    st4(d.flux + 4 * (size_t)s, g);
 }
 
-// deterministic block reduction of {sum, max} into norm_part[blockIdx.x]
-__device__ __forceinline__ void block_norm(const DeviceState& d, double sq, double am)
-{
-   __shared__ double s_sq[kThreads / 32], s_am[kThreads / 32];
-#pragma unroll
-   for (int o = 16; o > 0; o >>= 1) {
-      sq += __shfl_xor_sync(0xffffffffu, sq, o);
-      am = fmax(am, __shfl_xor_sync(0xffffffffu, am, o));
-   }
-   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-   if (l == 0) { s_sq[w] = sq; s_am[w] = am; }
-   __syncthreads();
-   if (threadIdx.x == 0) {
-      double a = 0.0, b = 0.0;
-      for (int i = 0; i < kThreads / 32; i++) { a += s_sq[i]; b = fmax(b, s_am[i]); }
-      d.norm_part[blockIdx.x] = make_double2(a, b);
-   }
-}
-
+// The loads of a cell's faces go out together (kGather): 512 x 128, half split,
+// 23 us one face after another, 16 us so.
 template <bool ADI_INIT>
 __global__ void __launch_bounds__(kThreads) rhs_cell_kernel(DeviceState d)
 {
@@ -137,19 +121,28 @@ __global__ void __launch_bounds__(kThreads) rhs_cell_kernel(DeviceState d)
       double r[4] = {0.0, 0.0, 0.0, 0.0};
       double sg = 0.0;
       const int e1 = d.cell_ptr[c + 1];
-      for (int e = d.cell_ptr[c]; e < e1; e++) {
-         const int ent = d.cell_ent[e];
-         const int s = ent >> 1;
-         double f[4];
-         ld4(d.flux + 4 * (size_t)s, f);
-         if (ent & 1) {
+      for (int e = d.cell_ptr[c]; e < e1; e += kGather) {
+         int ent[kGather];
+         double f[kGather][4], sp[kGather];
+         cell_entries(d, e, e1, ent);
 #pragma unroll
-            for (int k = 0; k < 4; k++) r[k] += f[k];
-         } else {
-#pragma unroll
-            for (int k = 0; k < 4; k++) r[k] -= f[k];
+         for (int u = 0; u < kGather; u++) {
+            if (e + u >= e1) break;
+            ld4(d.flux + 4 * (size_t)(ent[u] >> 1), f[u]);
+            sp[u] = d.spec[ent[u] >> 1];
          }
-         sg += d.spec[s];
+#pragma unroll
+         for (int u = 0; u < kGather; u++) {
+            if (e + u >= e1) break;
+            if (ent[u] & 1) {
+#pragma unroll
+               for (int k = 0; k < 4; k++) r[k] += f[u][k];
+            } else {
+#pragma unroll
+               for (int k = 0; k < 4; k++) r[k] -= f[u][k];
+            }
+            sg += sp[u];
+         }
       }
       sq = r[0] * r[0];
       am = fabs(r[0]);
@@ -170,7 +163,12 @@ __global__ void __launch_bounds__(kThreads) rhs_cell_kernel(DeviceState d)
    block_norm(d, sq, am);
 }
 
-template <bool UPDATE_Q>
+// The faces' loads go out together, as in rhs_cell_kernel.  SOFT: the products with
+// CFL/sigma on the integer pipes, identical; that pays where a sub-partition has
+// several warps to fill both.  512 x 128, half split: 28 us with a face's loads
+// after the face before, 20 us without SOFT, 16 us with; 256 x 64 (two warps on
+// fewer than half of the sub-partitions) 10 us without, 12 us with.
+template <bool UPDATE_Q, bool SOFT>
 __global__ void __launch_bounds__(kThreads) lin_cell_kernel(DeviceState d)
 {
    if (halted(d)) return;
@@ -184,16 +182,25 @@ __global__ void __launch_bounds__(kThreads) lin_cell_kernel(DeviceState d)
       for (int k = 0; k < 4; k++) r[k] = (r0[k] - dq[k]);
       const double dt = d.dtfac[c];
       const int e1 = d.cell_ptr[c + 1];
-      for (int e = d.cell_ptr[c]; e < e1; e++) {
-         const int ent = d.cell_ent[e];
-         double g[4];
-         ld4(d.flux + 4 * (size_t)(ent >> 1), g);
-         if (ent & 1) {
+      for (int e = d.cell_ptr[c]; e < e1; e += kGather) {
+         int ent[kGather];
+         double g[kGather][4];
+         cell_entries(d, e, e1, ent);
 #pragma unroll
-            for (int k = 0; k < 4; k++) r[k] += (g[k] * dt);
-         } else {
+         for (int u = 0; u < kGather; u++) {
+            if (e + u >= e1) break;
+            ld4(d.flux + 4 * (size_t)(ent[u] >> 1), g[u]);
+         }
 #pragma unroll
-            for (int k = 0; k < 4; k++) r[k] -= (g[k] * dt);
+         for (int u = 0; u < kGather; u++) {
+            if (e + u >= e1) break;
+            if (ent[u] & 1) {
+#pragma unroll
+               for (int k = 0; k < 4; k++) r[k] += pm<SOFT>(g[u][k], dt);
+            } else {
+#pragma unroll
+               for (int k = 0; k < 4; k++) r[k] -= pm<SOFT>(g[u][k], dt);
+            }
          }
       }
       st4(d.r + 4 * (size_t)c, r);
@@ -404,8 +411,13 @@ void launch_lin_face(const DeviceState& d, cudaStream_t st)
 
 void launch_lin_cell(const DeviceState& d, bool update_q, cudaStream_t st)
 {
-   if (update_q) lin_cell_kernel<true><<<d.norm_blocks, kThreads, 0, st>>>(d);
-   else lin_cell_kernel<false><<<d.norm_blocks, kThreads, 0, st>>>(d);
+   if (d.norm_blocks >= d.nsm) {
+      if (update_q) lin_cell_kernel<true, true><<<d.norm_blocks, kThreads, 0, st>>>(d);
+      else lin_cell_kernel<false, true><<<d.norm_blocks, kThreads, 0, st>>>(d);
+   } else {
+      if (update_q) lin_cell_kernel<true, false><<<d.norm_blocks, kThreads, 0, st>>>(d);
+      else lin_cell_kernel<false, false><<<d.norm_blocks, kThreads, 0, st>>>(d);
+   }
 }
 
 void launch_norm_final(const DeviceState& d, int off, bool check_tol, cudaStream_t st)
