@@ -494,10 +494,10 @@ int hamstr_gpu_create(const hamstr_gpu_params* p, int nCell, int nFace, const in
 
 namespace {
 // FP32 assembly inside the factorisation (1), or by a kernel of its own (0).  Of
-// its own it costs a pass over the blocks; inside, a row of a chain takes 1.8 us
-// instead of 0.65 us, as its terms are behind two lookups.  A step, own / inside:
-// 512 x 128 0.51 / 0.63 ms, the same mesh 30% split 0.50 / 0.61 ms, 32 meshes of
-// 983,040 cells in all 2.05 / 2.25 ms.  Above 2^24 rows of longer chains the blocks (192
+// its own it costs a pass over the blocks; inside, a row of a chain takes 1.6 us
+// instead of 0.44 us, as its terms are behind two lookups.  A step, own / inside:
+// 512 x 128 0.45 / 0.57 ms, the same mesh 30% split 0.43 / 0.54 ms, 32 meshes of
+// 983,040 cells in all 2.01 / 2.21 ms.  Above 2^24 rows of longer chains the blocks (192
 // bytes a row) are not kept.
 int default_mx_fused(const Plan& P)
 {
@@ -720,8 +720,8 @@ int hamstr::create_gpu(const hamstr_gpu_params* p, int nCell, int nFace, const i
       d.adi_wpb = 4;
       d.adi_fwpb = 4;
       d.mx_fused = default_mx_fused(P);
-      // one warp a block reaches the most SMs (eight steps of 512 x 128 4.14 ms, 4.18
-      // and 4.29 with two and four; with the assembly inside 1% the other way)
+      // one warp a block reaches the most SMs (eight steps of 512 x 128 3.59 ms, 3.65
+      // with two; with the assembly inside batches are within 1% either way)
       d.mx_block = d.mx_fused ? 64 : 32;
       d.mx_chunk_chains = mx_solve_chunk_capacity(d.mx_block);
       d.sp_on = 1;   // long periodic chains of the FP32 form by segments (2: long open ones too)

@@ -16,6 +16,7 @@
 // similar length sharing a warp.
 // ##################################################################
 #include <algorithm>
+#include <type_traits>
 #include "cell_sum.cuh"
 #include "device_state.h"
 #include "plan.h"
@@ -412,30 +413,30 @@ __device__ __forceinline__ void cp_async16_cg(void* smem, const void* gmem)
 // memory, each filled by the thread's own asynchronous copies, one group to a
 // row, DEPTH - 1 rows ahead.  A row of a chain is a few dozen dependent FP32
 // operations in the solve, some thousand cycles in the factorisation; a load is
-// 600 to 1,000 cycles, and there are not registers for that many rows.  Slot
-// (row, v) of thread `tid` at ((row % DEPTH) * V + v) * blockDim + tid: a
-// warp's access of one float4 is 512 contiguous bytes.
+// 600 to 1,000 cycles, and there are not registers for that many rows.  A
+// row's slot is its number modulo DEPTH, known at compile time in loops unrolled
+// by DEPTH; a warp's access of one float4 is 512 contiguous bytes.
 template <int V, int DEPTH>
 struct RowRing {
    float4* buf;
-   __device__ __forceinline__ explicit RowRing(float4* stage) : buf(stage + threadIdx.x) {}
-   __device__ __forceinline__ float4* at(int row, int v) const
+   __device__ __forceinline__ explicit RowRing(float4* stage)
+       : buf(stage + (threadIdx.x >> 5) * (32 * V * DEPTH) + (threadIdx.x & 31))
    {
-      return buf + (size_t)((row % DEPTH) * V + v) * blockDim.x;
    }
+   __device__ __forceinline__ float4* at(int slot, int v) const { return buf + 32 * (slot * V + v); }
    // N float4 of a tiled record (128 floats apart) into v, v + 1, ..
    template <int N>
-   __device__ __forceinline__ void copy(int row, int v, const float* src) const
+   __device__ __forceinline__ void copy(int slot, int v, const float* src) const
    {
 #pragma unroll
-      for (int q = 0; q < N; q++) cp_async16_cg(at(row, v + q), src + 128 * q);
+      for (int q = 0; q < N; q++) cp_async16_cg(at(slot, v + q), src + 128 * q);
    }
    template <int N>
-   __device__ __forceinline__ void read(int row, int v, float (&x)[N]) const
+   __device__ __forceinline__ void read(int slot, int v, float (&x)[N]) const
    {
 #pragma unroll
       for (int q = 0; q < N / 4; q++) {
-         const float4 y = *at(row, v + q);
+         const float4 y = *at(slot, v + q);
          x[4 * q] = y.x; x[4 * q + 1] = y.y; x[4 * q + 2] = y.z; x[4 * q + 3] = y.w;
       }
    }
@@ -526,7 +527,7 @@ constexpr int kElimChunk = 2;
 // the last-row elimination per chunk.  FUSED: each thread builds its chain's
 // blocks straight from the FP32 face Jacobians; otherwise it reads those that
 // mx_assemble_kernel wrote, through its ring (512 x 128, 30% split: 124 us with
-// the next row's blocks in registers, 76 us so; 32 meshes of 983,040 cells: 89 us).
+// the next row's blocks in registers, 50 us so; 32 meshes of 983,040 cells 75 us).
 constexpr int kFactorDepth = 4, kFactorVec = 12;
 
 template <bool FUSED, int ED>
@@ -546,8 +547,8 @@ __global__ void __launch_bounds__(256) mx_factor_kernel(DeviceState d, int count
    extern __shared__ float4 stage[];   // fused: kStageTerms x 4 float4 per thread; otherwise the ring
    const RowRing<kFactorVec, kFactorDepth> ring(stage);
    constexpr int AHEAD = kFactorDepth - 1;
-   auto fetch = [&](int i) {   // unfused: row i's blocks, as mx_assemble_kernel left them
-      if (i < N) ring.copy<12>(i, 0, d.blk32 + tix(s0 + i, 48, 0, lane));
+   auto fetch = [&](int i, int slot) {   // unfused: row i's blocks, as mx_assemble_kernel left them
+      if (i < N) ring.copy<12>(slot, 0, d.blk32 + tix(s0 + i, 48, 0, lane));
       cp_async_commit();
    };
    if (FUSED) {
@@ -556,58 +557,77 @@ __global__ void __launch_bounds__(256) mx_factor_kernel(DeviceState d, int count
       mx_row_ref(d, r0, A, B, C);
    } else {
 #pragma unroll
-      for (int i = 0; i < AHEAD; i++) fetch(i);
+      for (int i = 0; i < AHEAD; i++) fetch(i, i);
    }
-   for (int i = 0; i < N; i++) {
-      if (FUSED) {
-         if (i + 1 < N) {
-            // row i+1's terms are copied while row i is factored
-            mx_stage_row(d, rnext, stage);
-            rstaged = rnext;
-            snext = float(d.dtfac[rnext.scell]);
-            if (i + 2 < N) rnext = mx_rowref(d, row0 + i + 2);
+   // the rows, with or without the fill-in column (periodic chains): the loop for
+   // both was 380 instructions an open row, 85 us for 512 x 128; apart 67 us, and
+   // 56 us with the ring's slots known at compile time
+   auto rows = [&](auto fill_in) {
+      constexpr bool PER = decltype(fill_in)::value;
+      auto one = [&](int i, int slot) {
+         if (FUSED) {
+            if (i + 1 < N) {
+               // row i+1's terms are copied while row i is factored
+               mx_stage_row(d, rnext, stage);
+               rstaged = rnext;
+               snext = float(d.dtfac[rnext.scell]);
+               if (i + 2 < N) rnext = mx_rowref(d, row0 + i + 2);
+            }
+         } else {
+            cp_async_wait<AHEAD - 1>();
+            ring.read(slot, 0, A);
+            ring.read(slot, 4, B);
+            ring.read(slot, 8, C);
+            fetch(i + AHEAD, (slot + AHEAD) % kFactorDepth);
          }
-      } else {
-         cp_async_wait<AHEAD - 1>();
-         ring.read(i, 0, A);
-         ring.read(i, 4, B);
-         ring.read(i, 8, C);
-         fetch(i + AHEAD);
+         float* rec = d.fac32 + tix(s0 + i, kRec, 0, lane);
+         st16t(rec, A);
+         float fill[16];
+         if (i > 0) {
+            mm_sub(A, cp, B);
+#pragma unroll
+            for (int m = 0; m < 16; m++) fill[m] = 0.f;
+            if (PER) mm_sub(A, ap, fill);
+         } else {
+#pragma unroll
+            for (int m = 0; m < 16; m++) fill[m] = A[m];
+         }
+         const LUf u = luf_factor(B);
+         luf_store_t(rec + 32 * 16, u);
+         bad |= nonfinite(u.p0) || nonfinite(u.p1) || nonfinite(u.p2) || nonfinite(u.p3);
+         if (PER && i == N - 2) {
+#pragma unroll
+            for (int m = 0; m < 16; m++) C[m] += fill[m];
+            luf_cols(u, C);
+#pragma unroll
+            for (int m = 0; m < 16; m++) fill[m] = C[m];
+         } else {
+            luf_cols(u, C);
+            if (PER) luf_cols(u, fill);
+         }
+         st16t(rec + 32 * 32, C);
+         if (PER) st16t(rec + 32 * 48, fill);
+#pragma unroll
+         for (int m = 0; m < 16; m++) {
+            cp[m] = C[m];
+            if (PER) ap[m] = fill[m];
+         }
+         if (FUSED && i + 1 < N) {
+            cp_async_wait_all();
+            mx_row_staged(d, rstaged, stage, snext, A, B, C);
+         }
+      };
+      constexpr int UNROLL = FUSED ? 1 : kFactorDepth;
+      for (int i0 = 0; i0 < N; i0 += UNROLL) {
+#pragma unroll
+         for (int u = 0; u < UNROLL; u++) {
+            if (i0 + u >= N) break;
+            one(i0 + u, u);
+         }
       }
-      float* rec = d.fac32 + tix(s0 + i, kRec, 0, lane);
-      st16t(rec, A);
-      float fill[16];
-      if (i > 0) {
-         mm_sub(A, cp, B);
-#pragma unroll
-         for (int m = 0; m < 16; m++) fill[m] = 0.f;
-         if (per) mm_sub(A, ap, fill);
-      } else {
-#pragma unroll
-         for (int m = 0; m < 16; m++) fill[m] = A[m];
-      }
-      const LUf u = luf_factor(B);
-      luf_store_t(rec + 32 * 16, u);
-      bad |= nonfinite(u.p0) || nonfinite(u.p1) || nonfinite(u.p2) || nonfinite(u.p3);
-      if (per && i == N - 2) {
-#pragma unroll
-         for (int m = 0; m < 16; m++) C[m] += fill[m];
-         luf_cols(u, C);
-#pragma unroll
-         for (int m = 0; m < 16; m++) fill[m] = C[m];
-      } else {
-         luf_cols(u, C);
-         if (per) luf_cols(u, fill);
-      }
-      st16t(rec + 32 * 32, C);
-      if (per) st16t(rec + 32 * 48, fill);
-#pragma unroll
-      for (int m = 0; m < 16; m++) { cp[m] = C[m]; ap[m] = fill[m]; }
-      if (FUSED && i + 1 < N) {
-         cp_async_wait_all();
-         mx_row_staged(d, rstaged, stage, snext, A, B, C);
-      }
-   }
+   };
+   if (per) rows(std::true_type{});
+   else rows(std::false_type{});
    if (!FUSED) cp_async_wait_all();
    if (!per) {
       if (bad) atomicOr(d.status, DEV_ERR_PIVOT);
@@ -666,8 +686,8 @@ __device__ __forceinline__ void mv_add(const float (&M)[16], const float (&x)[4]
 }
 
 // The rings of the solves: a row's record by halves (A and LU, or two of C', V,
-// W), and a 4-vector; cells are looked up kSolveLook rows before their copies.
-constexpr int kSolveVec = 9, kSolveLook = 4;
+// W), and a 4-vector; cells are looked up a ring's rows before their copies.
+constexpr int kSolveVec = 9;
 constexpr size_t kFacRow = 32 * kRec, kFsRow = 128;   // floats from a tile row to the next
 
 // f(i) = LU^{-1}(F(i) - A(i) f(i-1)) for a thread's n tiled rows, F(i) =
@@ -677,40 +697,40 @@ __device__ __forceinline__ void forward_rows(const RowRing<kSolveVec, DEPTH>& ri
                                              const float* r32, float (&xp)[4])
 {
    constexpr int AHEAD = DEPTH - 1;
-   auto fetch = [&](int i, int cell) {
+   auto fetch = [&](int i, int slot, int cell) {
       if (i < n) {
-         ring.template copy<8>(i, 0, fac + kFacRow * i);
-         if (cell >= 0) cp_async16_cg(ring.at(i, 8), r32 + 4 * (size_t)cell);
-         else *ring.at(i, 8) = make_float4(0.f, 0.f, 0.f, 0.f);
+         ring.template copy<8>(slot, 0, fac + kFacRow * i);
+         if (cell >= 0) cp_async16_cg(ring.at(slot, 8), r32 + 4 * (size_t)cell);
+         else *ring.at(slot, 8) = make_float4(0.f, 0.f, 0.f, 0.f);
       }
       cp_async_commit();
    };
    auto look = [&](int i) { return i < n ? fcell[i] : -1; };
 #pragma unroll
-   for (int i = 0; i < AHEAD; i++) fetch(i, look(i));
-   int fc[kSolveLook];
+   for (int i = 0; i < AHEAD; i++) fetch(i, i, look(i));
+   int fc[DEPTH];
 #pragma unroll
-   for (int u = 0; u < kSolveLook; u++) fc[u] = look(AHEAD + u);
+   for (int u = 0; u < DEPTH; u++) fc[u] = look(AHEAD + u);
    // a row leaves the ring while the one before it is solved
    float a[16], lu[16], x[4];
    cp_async_wait<AHEAD - 1>();
    ring.read(0, 0, a);
    ring.read(0, 4, lu);
    ring.read(0, 8, x);
-   for (int i0 = 0; i0 < n; i0 += kSolveLook) {
-      int fcn[kSolveLook];
+   for (int i0 = 0; i0 < n; i0 += DEPTH) {
+      int fcn[DEPTH];
 #pragma unroll
-      for (int u = 0; u < kSolveLook; u++) fcn[u] = look(i0 + AHEAD + kSolveLook + u);
+      for (int u = 0; u < DEPTH; u++) fcn[u] = look(i0 + AHEAD + DEPTH + u);
 #pragma unroll
-      for (int u = 0; u < kSolveLook; u++) {
+      for (int u = 0; u < DEPTH; u++) {
          const int i = i0 + u;
          if (i >= n) break;
          float an[16], ln[16], y[4];
          cp_async_wait<AHEAD - 2>();
-         ring.read(i + 1, 0, an);   // (past the last row: what the slot holds, unused)
-         ring.read(i + 1, 4, ln);
-         ring.read(i + 1, 8, y);
-         fetch(i + AHEAD, fc[u]);
+         ring.read((u + 1) % DEPTH, 0, an);   // (past the last row: what the slot holds, unused)
+         ring.read((u + 1) % DEPTH, 4, ln);
+         ring.read((u + 1) % DEPTH, 8, y);
+         fetch(i + AHEAD, (u + AHEAD) % DEPTH, fc[u]);
          if (i > 0) mv_sub(a, xp, x);
          luf_solve(luf_of(lu), x[0], x[1], x[2], x[3]);
          *reinterpret_cast<float4*>(fs + kFsRow * i) = make_float4(x[0], x[1], x[2], x[3]);
@@ -720,7 +740,7 @@ __device__ __forceinline__ void forward_rows(const RowRing<kSolveVec, DEPTH>& ri
          for (int m = 0; m < 16; m++) { a[m] = an[m]; lu[m] = ln[m]; }
       }
 #pragma unroll
-      for (int u = 0; u < kSolveLook; u++) fc[u] = fcn[u];
+      for (int u = 0; u < DEPTH; u++) fc[u] = fcn[u];
    }
    cp_async_wait_all();
    __threadfence_block();   // f, before copies of it into the ring
@@ -729,13 +749,14 @@ __device__ __forceinline__ void forward_rows(const RowRing<kSolveVec, DEPTH>& ri
 // One sweep's solve of one chain per thread (the chain at position first +
 // t of line_chains).  The recurrence only carries the 4-vector x in
 // registers; what a row needs comes through the thread's ring (its factor
-// record, its right-hand side through the cell looked up kSolveLook rows before
+// record, its right-hand side through the cell looked up a ring's rows before
 // that, later the forward sweep's row).  Solutions go straight to r32 (each
 // cell is written once per chain; chains of a wave share no cell).
 // Bound by the chain: with the loads of four rows issued together a row of the
-// longest chain took 480 cycles forward or back, through the ring 310 (512 x 128,
-// 30% split: the four solves of a step 207 -> 136 us; unsplit 170 -> 108 us; 32
-// meshes of 983,040 cells 270 -> 143 us).
+// longest chain took 480 cycles forward or back, through the ring 230 (512 x 128,
+// 30% split: the four solves of a step 207 -> 103 us; unsplit 170 -> 79 us; 32
+// meshes of 983,040 cells 270 -> 129 us).  Of these 230 about 100 are the chain of
+// operations; with the slots computed a row and not unrolled it was 310.
 constexpr int kSolveDepth = 8;
 
 __global__ void __launch_bounds__(128) mx_solve_kernel(DeviceState d, int first, int count)
@@ -756,14 +777,13 @@ __global__ void __launch_bounds__(128) mx_solve_kernel(DeviceState d, int first,
    float* fsr = d.fsc32 + tix(s0, 4, 0, lane);
    float x[4], xp[4];
    forward_rows(ring, N, fac, fsr, fcell, d.r32, xp);
-   auto look = [&](const int* cells, int i) { return i >= 0 ? cells[i] : -1; };
    float xn[4], fN[4] = {xp[0], xp[1], xp[2], xp[3]};
    if (per) {
       // last row: f(N-1) - sum over i < N-1 of cN(i) f(i), in row order
       auto fetch_last = [&](int i) {
          if (i < N - 1) {
-            ring.copy<4>(i, 0, fac + kFacRow * i + 32 * 64);
-            cp_async16_cg(ring.at(i, 8), fsr + kFsRow * i);
+            ring.copy<4>(i % kSolveDepth, 0, fac + kFacRow * i + 32 * 64);
+            cp_async16_cg(ring.at(i % kSolveDepth, 8), fsr + kFsRow * i);
          }
          cp_async_commit();
       };
@@ -772,8 +792,8 @@ __global__ void __launch_bounds__(128) mx_solve_kernel(DeviceState d, int first,
       for (int i = 0; i < N - 1; i++) {
          cp_async_wait<AHEAD - 1>();
          float c[16], f[4];
-         ring.read(i, 0, c);
-         ring.read(i, 8, f);
+         ring.read(i % kSolveDepth, 0, c);
+         ring.read(i % kSolveDepth, 8, f);
          fetch_last(i + AHEAD);
          mv_sub(c, f, fN);
       }
@@ -786,62 +806,68 @@ __global__ void __launch_bounds__(128) mx_solve_kernel(DeviceState d, int first,
    st4(d.r32 + 4 * (size_t)scell[N - 1], xn);
    // back substitution, rows N-2 down to 0 (step s = N-2-i), periodic with the
    // fill-in column
-   auto fetch_back = [&](int s) {
-      const int i = N - 2 - s;
-      if (i >= 0) {
-         ring.copy<4>(s, 0, fac + kFacRow * i + 32 * 32);
-         if (per) ring.copy<4>(s, 4, fac + kFacRow * i + 32 * 48);
-         cp_async16_cg(ring.at(s, 8), fsr + kFsRow * i);
-      }
-      cp_async_commit();
-   };
-#pragma unroll
-   for (int s = 0; s < AHEAD; s++) fetch_back(s);
-   int sc[kSolveLook];
-#pragma unroll
-   for (int u = 0; u < kSolveLook; u++) sc[u] = look(scell, N - 2 - u);
-   float c[16], aa[16];
-   cp_async_wait<AHEAD - 1>();
-   ring.read(0, 0, c);
-   if (per) ring.read(0, 4, aa);
-   ring.read(0, 8, x);
-   for (int q0 = 0; q0 <= N - 2; q0 += kSolveLook) {
-      int scn[kSolveLook];
-#pragma unroll
-      for (int u = 0; u < kSolveLook; u++) scn[u] = look(scell, N - 2 - q0 - kSolveLook - u);
-#pragma unroll
-      for (int u = 0; u < kSolveLook; u++) {
-         const int s = q0 + u;
-         if (s > N - 2) break;
-         float cn[16], an[16], y[4];
-         cp_async_wait<AHEAD - 2>();
-         ring.read(s + 1, 0, cn);
-         if (per) ring.read(s + 1, 4, an);
-         ring.read(s + 1, 8, y);
-         fetch_back(s + AHEAD);
-#pragma unroll
-         for (int k = 0; k < 4; k++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-               if (per) {
-                  const float v = c[4 * k + j] * xn[j];
-                  x[k] -= (s == 0) ? v : __fmaf_rn(aa[4 * k + j], fN[j], v);
-               } else {
-                  x[k] = __fmaf_rn(-c[4 * k + j], xn[j], x[k]);
-               }
-            }
-         st4(d.r32 + 4 * (size_t)sc[u], x);
-#pragma unroll
-         for (int k = 0; k < 4; k++) { xn[k] = x[k]; x[k] = y[k]; }
-#pragma unroll
-         for (int m = 0; m < 16; m++) {
-            c[m] = cn[m];
-            if (per) aa[m] = an[m];
+   auto back = [&](auto fill_in) {
+      constexpr bool PER = decltype(fill_in)::value;
+      auto fetch_back = [&](int s, int slot) {
+         const int i = N - 2 - s;
+         if (i >= 0) {
+            ring.copy<4>(slot, 0, fac + kFacRow * i + 32 * 32);
+            if (PER) ring.copy<4>(slot, 4, fac + kFacRow * i + 32 * 48);
+            cp_async16_cg(ring.at(slot, 8), fsr + kFsRow * i);
          }
-      }
+         cp_async_commit();
+      };
+      auto look = [&](int i) { return i >= 0 ? scell[i] : -1; };
 #pragma unroll
-      for (int u = 0; u < kSolveLook; u++) sc[u] = scn[u];
-   }
+      for (int s = 0; s < AHEAD; s++) fetch_back(s, s);
+      int sc[kSolveDepth];
+#pragma unroll
+      for (int u = 0; u < kSolveDepth; u++) sc[u] = look(N - 2 - u);
+      float c[16], aa[16];
+      cp_async_wait<AHEAD - 1>();
+      ring.read(0, 0, c);
+      if (PER) ring.read(0, 4, aa);
+      ring.read(0, 8, x);
+      for (int q0 = 0; q0 <= N - 2; q0 += kSolveDepth) {
+         int scn[kSolveDepth];
+#pragma unroll
+         for (int u = 0; u < kSolveDepth; u++) scn[u] = look(N - 2 - q0 - kSolveDepth - u);
+#pragma unroll
+         for (int u = 0; u < kSolveDepth; u++) {
+            const int s = q0 + u;
+            if (s > N - 2) break;
+            float cn[16], an[16], y[4];
+            cp_async_wait<AHEAD - 2>();
+            ring.read((u + 1) % kSolveDepth, 0, cn);
+            if (PER) ring.read((u + 1) % kSolveDepth, 4, an);
+            ring.read((u + 1) % kSolveDepth, 8, y);
+            fetch_back(s + AHEAD, (u + AHEAD) % kSolveDepth);
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+#pragma unroll
+               for (int j = 0; j < 4; j++) {
+                  if (PER) {
+                     const float v = c[4 * k + j] * xn[j];
+                     x[k] -= (s == 0) ? v : __fmaf_rn(aa[4 * k + j], fN[j], v);
+                  } else {
+                     x[k] = __fmaf_rn(-c[4 * k + j], xn[j], x[k]);
+                  }
+               }
+            st4(d.r32 + 4 * (size_t)sc[u], x);
+#pragma unroll
+            for (int k = 0; k < 4; k++) { xn[k] = x[k]; x[k] = y[k]; }
+#pragma unroll
+            for (int m = 0; m < 16; m++) {
+               c[m] = cn[m];
+               if (PER) aa[m] = an[m];
+            }
+         }
+#pragma unroll
+         for (int u = 0; u < kSolveDepth; u++) sc[u] = scn[u];
+      }
+   };
+   if (per) back(std::true_type{});
+   else back(std::false_type{});
    cp_async_wait_all();
 }
 
@@ -996,7 +1022,7 @@ __global__ void __launch_bounds__(32) mx_spike_factor_kernel(DeviceState d)
       const int pos = d.sp_pos[sp];
       const float* blk = FUSED ? nullptr : d.blk32 + tix(d.grp_row0[pos >> 5] + s, 48, 0, pos & 31);
       auto fetch = [&](int k) {
-         if (k < n) ring.copy<12>(k, 0, blk + 32 * 48 * (size_t)k);
+         if (k < n) ring.copy<12>(k % kFactorDepth, 0, blk + 32 * 48 * (size_t)k);
          cp_async_commit();
       };
       if (FUSED) {
@@ -1015,9 +1041,9 @@ __global__ void __launch_bounds__(32) mx_spike_factor_kernel(DeviceState d)
             }
          } else {
             cp_async_wait<AHEAD - 1>();
-            ring.read(k, 0, A);
-            ring.read(k, 4, B);
-            ring.read(k, 8, C);
+            ring.read(k % kFactorDepth, 0, A);
+            ring.read(k % kFactorDepth, 4, B);
+            ring.read(k % kFactorDepth, 8, C);
             fetch(k + AHEAD);
          }
          // an open chain: no coupling from its first row back to its last
@@ -1072,8 +1098,8 @@ __global__ void __launch_bounds__(32) mx_spike_factor_kernel(DeviceState d)
       auto fetch_back = [&](int j) {
          const int k = n - 2 - j;
          if (k >= 0) {
-            back.template copy<4>(j, 0, rec + kFacRow * k + 32 * 32);
-            back.template copy<4>(j, 4, rec + kFacRow * k + 32 * 64);
+            back.template copy<4>(j % BD, 0, rec + kFacRow * k + 32 * 32);
+            back.template copy<4>(j % BD, 4, rec + kFacRow * k + 32 * 64);
          }
          cp_async_commit();
       };
@@ -1089,8 +1115,8 @@ __global__ void __launch_bounds__(32) mx_spike_factor_kernel(DeviceState d)
          const int j = n - 2 - k;
          cp_async_wait<BA - 1>();
          float c[16], g[16], v[16];
-         back.read(j, 0, c);
-         back.read(j, 4, g);
+         back.read(j % BD, 0, c);
+         back.read(j % BD, 4, g);
          fetch_back(j + BA);
 #pragma unroll
          for (int m = 0; m < 16; m++) v[m] = 0.f;
@@ -1251,8 +1277,8 @@ __global__ void __launch_bounds__(32) mx_spike_solve_kernel(DeviceState d, int f
    float* ys = d.sp_y + tix(R0, 4, 0, lane);
    auto fetch_rows = [&](int k, int n) {   // V, W and y of row k
       if (k < n) {
-         ring.copy<8>(k, 0, fac + kFacRow * k + 32 * 48);
-         cp_async16_cg(ring.at(k, 8), ys + kFsRow * k);
+         ring.copy<8>(k % kSpikeSolveDepth, 0, fac + kFacRow * k + 32 * 48);
+         cp_async16_cg(ring.at(k % kSpikeSolveDepth, 8), ys + kFsRow * k);
       }
       cp_async_commit();
    };
@@ -1269,8 +1295,8 @@ __global__ void __launch_bounds__(32) mx_spike_solve_kernel(DeviceState d, int f
       auto fetch_back = [&](int j) {
          const int k = n - 2 - j;
          if (k >= 0) {
-            ring.copy<4>(j, 0, fac + kFacRow * k + 32 * 32);
-            cp_async16_cg(ring.at(j, 8), ys + kFsRow * k);
+            ring.copy<4>(j % kSpikeSolveDepth, 0, fac + kFacRow * k + 32 * 32);
+            cp_async16_cg(ring.at(j % kSpikeSolveDepth, 8), ys + kFsRow * k);
          }
          cp_async_commit();
       };
@@ -1280,8 +1306,8 @@ __global__ void __launch_bounds__(32) mx_spike_solve_kernel(DeviceState d, int f
          const int j = n - 2 - k;
          cp_async_wait<AHEAD - 1>();
          float cm[16], yk[4];
-         ring.read(j, 0, cm);
-         ring.read(j, 8, yk);
+         ring.read(j % kSpikeSolveDepth, 0, cm);
+         ring.read(j % kSpikeSolveDepth, 8, yk);
          fetch_back(j + AHEAD);
          mv_sub(cm, yp, yk);
          *reinterpret_cast<float4*>(ys + kFsRow * k) = make_float4(yk[0], yk[1], yk[2], yk[3]);
@@ -1391,29 +1417,29 @@ __global__ void __launch_bounds__(32) mx_spike_solve_kernel(DeviceState d, int f
          bp[c] = zs[8 * pm + c];
       }
       const int* scell = d.row_scell + row0 + s;
-      int sc[kSolveLook];
+      int sc[kSpikeSolveDepth];
 #pragma unroll
-      for (int u = 0; u < kSolveLook; u++) sc[u] = u < n ? scell[u] : 0;
-      for (int k0 = 0; k0 < n; k0 += kSolveLook) {
-         int scn[kSolveLook];
+      for (int u = 0; u < kSpikeSolveDepth; u++) sc[u] = u < n ? scell[u] : 0;
+      for (int k0 = 0; k0 < n; k0 += kSpikeSolveDepth) {
+         int scn[kSpikeSolveDepth];
 #pragma unroll
-         for (int u = 0; u < kSolveLook; u++) scn[u] = k0 + kSolveLook + u < n ? scell[k0 + kSolveLook + u] : 0;
+         for (int u = 0; u < kSpikeSolveDepth; u++) scn[u] = k0 + kSpikeSolveDepth + u < n ? scell[k0 + kSpikeSolveDepth + u] : 0;
 #pragma unroll
-         for (int u = 0; u < kSolveLook; u++) {
+         for (int u = 0; u < kSpikeSolveDepth; u++) {
             const int k = k0 + u;
             if (k >= n) break;
             cp_async_wait<AHEAD - 1>();
             float v[16], w[16], x[4];
-            ring.read(k, 0, v);
-            ring.read(k, 4, w);
-            ring.read(k, 8, x);
+            ring.read(u, 0, v);
+            ring.read(u, 4, w);
+            ring.read(u, 8, x);
             fetch_rows(k + AHEAD, n);
             mv_add(w, bp, x);
             mv_add(v, tn, x);
             st4(d.r32 + 4 * (size_t)sc[u], x);
          }
 #pragma unroll
-         for (int u = 0; u < kSolveLook; u++) sc[u] = scn[u];
+         for (int u = 0; u < kSpikeSolveDepth; u++) sc[u] = scn[u];
       }
       cp_async_wait_all();
    }
