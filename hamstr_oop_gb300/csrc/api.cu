@@ -495,13 +495,15 @@ int hamstr_gpu_create(const hamstr_gpu_params* p, int nCell, int nFace, const in
 namespace {
 // FP32 assembly inside the factorisation (1), or by a kernel of its own (0).  Of
 // its own it costs a pass over the blocks; inside, a row of a chain takes 1.6 us
-// instead of 0.44 us, as its terms are behind two lookups.  A step, own / inside:
-// 512 x 128 0.45 / 0.57 ms, the same mesh 30% split 0.43 / 0.54 ms, 32 meshes of
-// 983,040 cells in all 2.01 / 2.21 ms.  Above 2^24 rows of longer chains the blocks (192
-// bytes a row) are not kept.
+// instead of 0.44 us, as its terms are behind two lookups, until there are chains
+// enough to hide them.  A step, own / inside: 512 x 128 0.45 / 0.57 ms, the same
+// mesh 30% split 0.43 / 0.54 ms, batches with 12,800 chains 2.01 / 2.21 ms, 25,600
+// 3.79 / 3.81, 51,200 7.40 / 6.95, 99,200 14.2 / 13.3.  Meshes whose
+// chains have fewer than 16 rows on average stay with their own (the 30% split).
+// Above 2^24 rows the blocks (192 bytes a row) are not kept.
 int default_mx_fused(const Plan& P)
 {
-   return P.nChain > 0 && P.nRow >= 16ll * P.nChain && P.nRow > (1 << 24) ? 1 : 0;
+   return P.nRow >= 16ll * P.nChain && (P.nChain > (1 << 15) || P.nRow > (1 << 24)) ? 1 : 0;
 }
 
 // How the FP64 line kernels pack open chains before any tuning.

@@ -753,10 +753,10 @@ __device__ __forceinline__ void forward_rows(const RowRing<kSolveVec, DEPTH>& ri
 // that, later the forward sweep's row).  Solutions go straight to r32 (each
 // cell is written once per chain; chains of a wave share no cell).
 // Bound by the chain: with the loads of four rows issued together a row of the
-// longest chain took 480 cycles forward or back, through the ring 230 (512 x 128,
+// longest chain took 650 cycles forward or back, through the ring 280 (512 x 128,
 // 30% split: the four solves of a step 207 -> 103 us; unsplit 170 -> 79 us; 32
-// meshes of 983,040 cells 270 -> 129 us).  Of these 230 about 100 are the chain of
-// operations; with the slots computed a row and not unrolled it was 310.
+// meshes of 983,040 cells 270 -> 129 us).  With the slots
+// computed each row and not unrolled it was 390.
 constexpr int kSolveDepth = 8;
 
 __global__ void __launch_bounds__(128) mx_solve_kernel(DeviceState d, int first, int count)
