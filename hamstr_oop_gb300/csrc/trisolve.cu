@@ -157,11 +157,10 @@ extern "C" int hamstr_gpu_block_tridag4(int nlines, int N, int periodic, const d
 // ------------------------------------------------------------------
 // Allocation-free variant.
 //
-// Some callers cannot allocate device memory on every call: code that runs
-// in a loop beside work on other streams (cudaFree waits for the whole
-// device, so the allocating entry point above stalls everything), and
-// hosts whose device memory is owned by their own pool allocator with a
-// fixed budget.  This variant runs the same kernel with its scratch in a
+// Some callers cannot allocate device memory on every call, or wait for their
+// stream in it: code that runs in a loop beside work on other streams, stream
+// capture, and hosts whose device memory is owned by their own pool allocator
+// with a fixed budget.  This variant runs the same kernel with its scratch in a
 // fixed array that the library image places in device memory when it is
 // loaded: every GPU that loads the library holds these 8 MiB until the
 // process exits, and the call itself allocates nothing.

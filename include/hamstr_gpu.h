@@ -236,7 +236,8 @@ int hamstr_gpu_forces(hamstr_gpu* g, double* out6);
 int hamstr_gpu_autotune(hamstr_gpu* g, int reps, char* report, int report_len);
 
 /* The launch shape itself (no reference counterpart), HAMSTR_SHAPE_N ints:
- *   [0] face kernels' threads per block: 128 or 256
+ *   [0] face kernels' threads per block: 128 or 256 (on small meshes smaller
+ *       blocks, where those load the fullest SM less)
  *   [1] FP64 line kernels' persistent warps per SM: 4 or 8
  *   [2] FP32 line kernels' threads per block: 32, 64 or 128
  *   [3] FP32 blocks assembled inside the factorisation: 0 or 1
@@ -250,10 +251,9 @@ int hamstr_gpu_autotune(hamstr_gpu* g, int reps, char* report, int report_len);
  *       tuned by hamstr_gpu_autotune)
  *   [8] FP64 line kernels: open chains of at most this many rows go 32 to
  *       a warp, one per lane (0: none): 0..64
- *   [9] FP32 line kernels: the loads of several rows issued together (4 in
- *       the solve, 2 in the periodic elimination), where the launch's chains
- *       are all resident at once with the larger register count this takes:
- *       0 or 1 (default 1; not tuned)
+ *   [9] FP32 line kernels: the loads of two rows issued together in the
+ *       periodic chains' last-row elimination, where all chains are resident
+ *       at once: 0 or 1 (default 1; not tuned)
  *  [10] FP32 line kernels: long chains solved by segments (16 rows each,
  *       up to 32, one warp lane per segment, joined by a small cyclic
  *       system on the segment ends) instead of one thread running the whole
@@ -287,12 +287,12 @@ int hamstr_mlp_gemm(const void* A, const void* B, int M, int N, int K, int split
 
 /* The warm-start network (no reference counterpart): 5 -> 256 -> 256 ->
  * 256 -> 4, GELU, BF16 weights and activations with FP32 accumulation,
- * forward and backward on the tensor cores (hamstr_mlp_gemm), Adam on FP32
+ * forward and backward on the tensor cores, Adam on FP32
  * master weights.  Parameters travel as FP32 in the order W1[256][5] b1
  * W2[256][256] b2 W3[256][256] b3 W4[4][256] b4 (hamstr_mlp_nparams()).
  * Device arrays: features [n][5], targets and outputs [n][4], FP32.
  *   _create: batch capacity (rows per pass), seed of the initial weights;
- *   _forward: outputs for n rows (any n, in chunks of the capacity);
+ *   _forward: outputs for n rows (any n, in one launch);
  *   _grad: loss (mean squared error over n <= capacity rows and the 4
  *     outputs) and its gradient, kept for _get_grads;
  *   _train_step: one Adam step (lr; betas 0.9, 0.999) on a minibatch of
@@ -346,16 +346,17 @@ int hamstr_gpu_update_solution(hamstr_gpu* g, const char* qold, const char* qnew
  * periodic = 1 selects the cyclic solver (A_0 couples row 0 to row N-1 and
  * C_{N-1} row N-1 to row 0; needs N >= 2); 0 the open one (A_0, C_{N-1}
  * unused).  stream is a cudaStream_t or NULL.  Scratch of (80 N + 16)
- * doubles per line is allocated and freed inside the call, which
+ * doubles per line comes from a stream-ordered pool of the library's own
+ * (which keeps at most 64 MiB a device between calls); the call
  * synchronises the stream. */
 int hamstr_gpu_block_tridag4(int nlines, int N, int periodic, const double* A, const double* B,
                              const double* C, double* F, void* stream);
 
 /* The same solve without any device allocation (no counterpart in the
  * reference, which has no GPU).  For callers that cannot allocate device
- * memory on every call: loops that run beside work on other streams (the
- * cudaFree of the entry point above waits for the whole device) and hosts
- * whose device memory belongs to their own pool allocator.  Scratch is a
+ * memory on every call or wait for their stream in it: loops that run beside
+ * work on other streams, stream capture, and hosts whose device memory
+ * belongs to their own pool allocator.  Scratch is a
  * fixed 8 MiB array that every GPU loading the library holds until exit;
  * the call needs nlines*(80*N+16) <= 1048576 doubles and returns
  * HAMSTR_GPU_ERR_ARG beyond that.  The first call on a device looks up the
