@@ -396,7 +396,8 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+// every copy of this thread has arrived, committed to a group or not
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // all but the newest N groups of this thread's copies have arrived
 template <int N>
@@ -1269,6 +1270,7 @@ __global__ void __launch_bounds__(32) mx_spike_solve_kernel(DeviceState d, int f
       const int nrow = kRedRow * (P - 1);
       for (int m = 4 * lane; m < nrow; m += 128) cp_async16_cg(red_s + m, red + m);
       if (lane < 24) cp_async16_cg(red_s + kRedLast + 4 * lane, red + kRedLast + 4 * lane);
+      cp_async_commit();   // a group of their own: each lane waits for its copies before the __syncwarp below
    }
    extern __shared__ float4 stage[];
    const RowRing<kSolveVec, kSpikeSolveDepth> ring(stage);
