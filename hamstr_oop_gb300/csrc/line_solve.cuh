@@ -1162,6 +1162,11 @@ __device__ __forceinline__ void team_step(double& w, int h, int k, int j, bool& 
    if (h == 0 && k == S && j == S) w = piv;
 }
 
+// two neighbouring entries of an input block, by doubles: a caller's block may
+// lie on any 8-byte boundary (block_tridag4).  They are loaded a row ahead, so the
+// second load costs nothing measurable.
+__device__ __forceinline__ double2 ld2(const double* __restrict__ p) { return make_double2(p[0], p[1]); }
+
 // Ab, Bb, Cb, stride, N, per, fac, facN and the result as factor_line's
 __device__ __forceinline__ bool factor_line_team(const double* __restrict__ Ab, const double* __restrict__ Bb,
                                                  const double* __restrict__ Cb, size_t stride, int N, bool per,
@@ -1170,7 +1175,7 @@ __device__ __forceinline__ bool factor_line_team(const double* __restrict__ Ab, 
 {
    const int h = lane >> 4, e = lane & 15, k = e >> 2, j = e & 3;
    const double* Wb = h ? Cb : Bb;   // lanes 0-15 hold B', lanes 16-31 the columns of c(i)
-   double2 A = *reinterpret_cast<const double2*>(Ab + 4 * k + 2 * h);   // a(k, 2h) and a(k, 2h+1)
+   double2 A = ld2(Ab + 4 * k + 2 * h);   // a(k, 2h) and a(k, 2h+1)
    double W = Wb[e];
    double P0 = 0.0, P1 = 0.0;        // c'(i-1) entries (2h, j) and (2h+1, j)
    bool bad = false;
@@ -1179,7 +1184,7 @@ __device__ __forceinline__ bool factor_line_team(const double* __restrict__ Ab, 
       double Wn = 0.0;
       if (i + 1 < N) {
          const size_t o = stride * (size_t)(i + 1);
-         An = *reinterpret_cast<const double2*>(Ab + o + 4 * k + 2 * h);
+         An = ld2(Ab + o + 4 * k + 2 * h);
          Wn = Wb[o + e];
       }
       double* rec = fac + (size_t)kFacRec * i;
@@ -1269,14 +1274,14 @@ __device__ __forceinline__ void follow_line_team(const double* __restrict__ Ab, 
    double X[4] = {0.0, 0.0, 0.0, 0.0};   // the previous row's column j of a' (lanes 0-15) or solution
    const int rows = F ? N : N - 1;       // the fill column ends with a(N-2)
    double f = F ? fs[k] : 0.0;
-   double2 A0 = *reinterpret_cast<const double2*>(Ab + 4 * k), A1 = *reinterpret_cast<const double2*>(Ab + 4 * k + 2);
+   double2 A0 = ld2(Ab + 4 * k), A1 = ld2(Ab + 4 * k + 2);
    for (int i = 0; i < rows; i++) {
       const double a[4] = {A0.x, A0.y, A1.x, A1.y};
       double fn = 0.0;
       if (i + 1 < rows) {
          const double* an = Ab + stride * (size_t)(i + 1) + 4 * k;
-         A0 = *reinterpret_cast<const double2*>(an);
-         A1 = *reinterpret_cast<const double2*>(an + 2);
+         A0 = ld2(an);
+         A1 = ld2(an + 2);
          if (F) fn = fs[4 * (i + 1) + k];
       }
       // a(i) = -a(i) a'(i-1), f(i) -= a(i) f(i-1)

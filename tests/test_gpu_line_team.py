@@ -55,3 +55,26 @@ def test_degenerate_pivots(oracle_lib, native_lib, value, periodic):
         with np.errstate(all="ignore"):
             want = oracle_lib.block_tridag4(a[k], b[k], c[k], f[k], periodic)
         assert np.array_equal(got[k], want, equal_nan=True), k
+
+
+@pytest.mark.parametrize("periodic", [False, True])
+@pytest.mark.parametrize("fn", ["block_tridag4", "block_tridag4_noalloc"])
+@pytest.mark.parametrize("odd", ["a", "b", "c", "f", "abcf"])
+def test_operands_on_any_8_byte_boundary(oracle_lib, native_lib, fn, odd, periodic):
+    """An operand may start an odd number of doubles into its storage."""
+    import torch
+    from hamstr_oop_gb300 import native
+    host = dict(zip("abcf", _systems(77, 3, 21)))
+    dev = {}
+    for name, x in host.items():
+        room = torch.empty(x.size + 1, dtype=torch.float64, device="cuda")
+        view = (room[1:] if name in odd else room[:-1]).view(x.shape)
+        view.copy_(torch.from_numpy(x))
+        assert view.data_ptr() % 16 == (8 if name in odd else 0)
+        dev[name] = view
+    getattr(native, fn)(dev["a"], dev["b"], dev["c"], dev["f"], periodic)
+    torch.cuda.synchronize()
+    got = dev["f"].cpu().numpy()
+    for k in range(3):
+        want = oracle_lib.block_tridag4(host["a"][k], host["b"][k], host["c"][k], host["f"][k], periodic)
+        assert np.array_equal(got[k], want), k
