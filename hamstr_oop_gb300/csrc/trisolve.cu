@@ -7,9 +7,12 @@
 // two warps per line, factor_line_team and follow_line_team of
 // line_solve.cuh, so each line's solution is bit-identical to one reference
 // call.  A line is a recurrence over its rows; with the solve (and the periodic
-// fill column) behind the factorisation in a second warp a row takes 4,480
-// cycles open and 5,460 periodic, against 7,150 and 8,000 in one warp, and 52
-// FP64 instructions against 66, so it is the better split at any number of lines.
+// fill column) behind the factorisation in a second warp a row takes 1.95 us
+// open and 2.43 us periodic, against 4.00 and 4.53 in one warp, and 52 FP64
+// instructions against 66, so it is the better split from one line to lines that
+// fill the GPU: one line of 128 rows 512 -> 251 us open, 583 -> 315 periodic, 400
+// lines of 17 rows 70 -> 42 and 81 -> 54, 20,000 lines of 17 rows (FP64 pipe 82%
+// busy either way) 1,434 -> 1,198 us.
 // ##################################################################
 #include <cuda_runtime.h>
 
@@ -125,6 +128,22 @@ cudaError_t scratch_pool(cudaMemPool_t* out)
    return cudaSuccess;
 }
 
+// Scratch the pool does not keep is mapped and unmapped on every call, and
+// cudaMalloc does that faster than a pool does: open lines, pool / cudaMalloc,
+// 200,000 of 17 rows (2.2 GB) 16.3 / 13.1 ms, 9,000 of 33 (192 MB) 1.49 / 1.38,
+// 5,000 (106 MB) 0.86 / 0.85, 4,099 (87 MB, most of it kept) 0.67 / 0.72, 3,200 (68 MB)
+// 0.56 / 0.62.  So the pool serves up to half as much again as it keeps.
+constexpr size_t kPoolServes = kPoolKept + kPoolKept / 2;
+
+cudaError_t scratch_alloc(double** p, size_t bytes, cudaStream_t s, bool* pooled)
+{
+   *pooled = bytes <= kPoolServes;
+   if (!*pooled) return cudaMalloc((void**)p, bytes);
+   cudaMemPool_t pool = nullptr;
+   const cudaError_t e = scratch_pool(&pool);
+   return e != cudaSuccess ? e : cudaMallocFromPoolAsync((void**)p, bytes, pool, s);
+}
+
 }  // namespace
 
 extern "C" int hamstr_gpu_block_tridag4(int nlines, int N, int periodic, const double* A, const double* B,
@@ -134,18 +153,18 @@ extern "C" int hamstr_gpu_block_tridag4(int nlines, int N, int periodic, const d
    if (st || nlines == 0) return st;
    const cudaStream_t s = (cudaStream_t)stream;
    double* scratch = nullptr;
+   bool pooled = false;
    const size_t bytes = (size_t)nlines * ((size_t)kFacRec * N + 16) * sizeof(double);
-   cudaMemPool_t pool = nullptr;
-   cudaError_t e = scratch_pool(&pool);
-   if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void**)&scratch, bytes, pool, s);
+   cudaError_t e = scratch_alloc(&scratch, bytes, s, &pooled);
    if (e != cudaSuccess) {
       cudaGetLastError();
       set_last_error(std::string("block_tridag4 scratch: ") + cudaGetErrorString(e));
       return e == cudaErrorMemoryAllocation ? HAMSTR_GPU_ERR_NOMEM : HAMSTR_GPU_ERR_CUDA;
    }
    st = block_tridag_launch(nlines, N, periodic, A, B, C, F, scratch, s);
-   cudaFreeAsync(scratch, s);
+   if (pooled) cudaFreeAsync(scratch, s);
    e = cudaStreamSynchronize(s);
+   if (!pooled) cudaFree(scratch);
    if (st) return st;
    if (e != cudaSuccess) {
       set_last_error(std::string("block_tridag4: ") + cudaGetErrorString(e));

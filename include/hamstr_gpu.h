@@ -346,9 +346,10 @@ int hamstr_gpu_update_solution(hamstr_gpu* g, const char* qold, const char* qnew
  * periodic = 1 selects the cyclic solver (A_0 couples row 0 to row N-1 and
  * C_{N-1} row N-1 to row 0; needs N >= 2); 0 the open one (A_0, C_{N-1}
  * unused).  stream is a cudaStream_t or NULL.  Scratch of (80 N + 16)
- * doubles per line comes from a stream-ordered pool of the library's own
- * (which keeps at most 64 MiB a device between calls); the call
- * synchronises the stream. */
+ * doubles per line, up to 96 MiB, comes from a stream-ordered pool of the
+ * library's own (which keeps at most 64 MiB a device between calls), more of
+ * it is allocated and freed inside the call; the call synchronises the
+ * stream. */
 int hamstr_gpu_block_tridag4(int nlines, int N, int periodic, const double* A, const double* B,
                              const double* C, double* F, void* stream);
 

@@ -78,3 +78,18 @@ def test_operands_on_any_8_byte_boundary(oracle_lib, native_lib, fn, odd, period
     for k in range(3):
         want = oracle_lib.block_tridag4(host["a"][k], host["b"][k], host["c"][k], host["f"][k], periodic)
         assert np.array_equal(got[k], want), k
+
+
+@pytest.mark.parametrize("periodic", [False, True])
+@pytest.mark.parametrize("nlines", [4700, 4800])
+def test_scratch_from_the_pool_and_beyond_it(native_lib, nlines, periodic):
+    """Calls whose scratch (2,656 doubles a line) is just below and above what
+    the pool serves, 96 MiB, give what smaller calls give on the same lines."""
+    from hamstr_oop_gb300 import native
+    assert (nlines * 2656 * 8 <= 96 << 20) == (nlines == 4700)
+    a, b, c, f = _systems(nlines, 300, 33)
+    want = _solve(native, a, b, c, f, periodic)
+    a, b, c, f = (np.tile(x, (nlines // 300 + 1,) + (1,) * (x.ndim - 1))[:nlines] for x in (a, b, c, f))
+    got = _solve(native, a, b, c, f, periodic)
+    for k in range(0, nlines, 300):
+        assert np.array_equal(got[k:k + 300], want[:min(300, nlines - k)]), k
