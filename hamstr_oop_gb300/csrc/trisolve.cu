@@ -14,7 +14,9 @@
 // lines of 17 rows 70 -> 42 and 81 -> 54, 20,000 lines of 17 rows (FP64 pipe 82%
 // busy either way) 1,434 -> 1,198 us.
 // ##################################################################
+#include <cuda.h>
 #include <cuda_runtime.h>
+#include <cudaTypedefs.h>
 
 #include <mutex>
 #include <string>
@@ -96,9 +98,48 @@ namespace {
 // back to the device when the call's stream is synchronised.  The allocator
 // orders reuse between streams and threads.
 constexpr unsigned long long kPoolKept = 64ull << 20;
+//
+// cudaDeviceReset ends the device's context and the pool with it, so a pool goes
+// by the id of the context it was made in, which is never used again.
 constexpr int kMaxDevices = 64;
 std::mutex g_pool_mutex;
-cudaMemPool_t g_pool[kMaxDevices] = {};
+struct ContextPool {
+   unsigned long long context;
+   cudaMemPool_t pool;
+};
+ContextPool g_pool[kMaxDevices] = {};
+
+template <typename F>
+F driver_entry(const char* name, unsigned version)
+{
+   void* p = nullptr;
+   cudaDriverEntryPointQueryResult q;
+   const bool ok = cudaGetDriverEntryPointByVersion(name, &p, version, cudaEnableDefault, &q) == cudaSuccess &&
+                   q == cudaDriverEntryPointSuccess;
+   return ok ? reinterpret_cast<F>(p) : nullptr;
+}
+
+// the id of the device's primary context, the one the runtime works in
+cudaError_t primary_context_id(int dev, unsigned long long* id)
+{
+   static const auto retain = driver_entry<PFN_cuDevicePrimaryCtxRetain_v7000>("cuDevicePrimaryCtxRetain", 7000);
+   static const auto release = driver_entry<PFN_cuDevicePrimaryCtxRelease_v11000>("cuDevicePrimaryCtxRelease", 11000);
+   static const auto state = driver_entry<PFN_cuDevicePrimaryCtxGetState_v7000>("cuDevicePrimaryCtxGetState", 7000);
+   static const auto ctx_id = driver_entry<PFN_cuCtxGetId_v12000>("cuCtxGetId", 12000);
+   if (!retain || !release || !state || !ctx_id) return cudaErrorNotSupported;
+   unsigned flags = 0;
+   int active = 0;
+   if (state(dev, &flags, &active) != CUDA_SUCCESS) return cudaErrorInitializationError;
+   if (!active) {   // the runtime makes and keeps the next one
+      const cudaError_t e = cudaSetDevice(dev);
+      if (e != cudaSuccess) return e;
+   }
+   CUcontext c = nullptr;
+   if (retain(&c, dev) != CUDA_SUCCESS) return cudaErrorInitializationError;
+   const CUresult r = ctx_id(c, id);
+   release(dev);
+   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInitializationError;
+}
 
 cudaError_t scratch_pool(cudaMemPool_t* out)
 {
@@ -107,7 +148,11 @@ cudaError_t scratch_pool(cudaMemPool_t* out)
    if (e != cudaSuccess) return e;
    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
    std::lock_guard<std::mutex> lock(g_pool_mutex);
-   if (!g_pool[dev]) {
+   ContextPool& have = g_pool[dev];
+   unsigned long long context = 0;
+   e = primary_context_id(dev, &context);
+   if (e != cudaSuccess) return e;
+   if (!have.pool || have.context != context) {
       cudaMemPoolProps props = {};
       props.allocType = cudaMemAllocationTypePinned;
       props.handleTypes = cudaMemHandleTypeNone;
@@ -122,9 +167,9 @@ cudaError_t scratch_pool(cudaMemPool_t* out)
          cudaMemPoolDestroy(p);
          return e;
       }
-      g_pool[dev] = p;
+      have = {context, p};
    }
-   *out = g_pool[dev];
+   *out = have.pool;
    return cudaSuccess;
 }
 

@@ -93,3 +93,73 @@ def test_scratch_from_the_pool_and_beyond_it(native_lib, nlines, periodic):
     got = _solve(native, a, b, c, f, periodic)
     for k in range(0, nlines, 300):
         assert np.array_equal(got[k:k + 300], want[:min(300, nlines - k)]), k
+
+
+def test_threads_and_streams_share_the_scratch_pool(native_lib):
+    """Eight host threads on streams of their own, each with its own systems."""
+    import threading
+    import torch
+    from hamstr_oop_gb300 import native
+    work, bad = [], []
+    for k in range(8):
+        sysk = _systems(40 + k, 30 + k, 20 + 7 * k)
+        work.append((sysk, _solve(native, *sysk, bool(k % 2)), torch.cuda.Stream()))
+
+    def solve(k):
+        (a, b, c, f), want, stream = work[k]
+        with torch.cuda.stream(stream):
+            ta, tb, tc, f0 = (torch.from_numpy(x).cuda() for x in (a, b, c, f))
+            for _ in range(20):
+                tf = f0.clone()
+                native.block_tridag4(ta, tb, tc, tf, bool(k % 2), stream=stream.cuda_stream)
+                if not np.array_equal(tf.cpu().numpy(), want):
+                    bad.append(k)
+    threads = [threading.Thread(target=solve, args=(k,)) for k in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+
+
+AFTER_RESET = r"""
+import ctypes, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+from hamstr_oop_gb300 import native
+lib = native.load()
+rt = ctypes.CDLL("libcudart.so.13")   # the runtime the library is linked with
+
+def solve(a, b, c, f, periodic):
+    dev = []
+    for x in (a, b, c, f):
+        p = ctypes.c_void_p()
+        assert rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(x.nbytes)) == 0
+        assert rt.cudaMemcpy(p, x.ctypes.data_as(ctypes.c_void_p), ctypes.c_size_t(x.nbytes), 1) == 0
+        dev.append(p)
+    assert lib.hamstr_gpu_block_tridag4(f.shape[0], f.shape[1], periodic, *[p.value for p in dev], None) == 0
+    out = np.empty_like(f)
+    assert rt.cudaMemcpy(out.ctypes.data_as(ctypes.c_void_p), dev[3], ctypes.c_size_t(f.nbytes), 2) == 0
+    return out
+
+rng = np.random.default_rng(3)
+a, c = (rng.standard_normal((5, 12, 4, 4)) for _ in range(2))
+b = rng.standard_normal((5, 12, 4, 4)) + 6.0 * np.eye(4)
+f = rng.standard_normal((5, 12, 4))
+first = solve(a, b, c, f, 1)
+for _ in range(2):
+    assert rt.cudaDeviceReset() == 0
+    assert np.array_equal(solve(a, b, c, f, 1), first)
+print("same after a reset")
+"""
+
+
+def test_the_pool_does_not_outlive_its_context():
+    """After cudaDeviceReset, which ends the process's own context, the next
+    call makes a pool in the new one.  In a process of its own."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", AFTER_RESET, root], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same after a reset" in r.stdout, r.stdout + r.stderr
