@@ -235,10 +235,15 @@ constexpr size_t kNoAllocScratchDoubles = size_t(1) << 20;   // 8 MiB
 static __device__ __align__(256) double g_tridag_scratch[kNoAllocScratchDoubles];
 
 std::mutex g_scratch_mutex;
-double* g_scratch_addr[kMaxDevices] = {};
+struct ContextScratch {
+   unsigned long long context;
+   double* addr;
+};
+ContextScratch g_scratch_addr[kMaxDevices] = {};
 
 // Device address of g_tridag_scratch on the current device, looked up once
-// per device (host code only sees a host-side stand-in for the symbol).
+// per context of the device (host code only sees a host-side stand-in for the
+// symbol, and a reset loads the image anew).
 int noalloc_scratch(double** out)
 {
    int dev = 0;
@@ -251,17 +256,24 @@ int noalloc_scratch(double** out)
       set_last_error("block_tridag4_noalloc: device ordinal beyond 63");
       return HAMSTR_GPU_ERR_ARG;
    }
+   unsigned long long context = 0;
+   e = primary_context_id(dev, &context);
+   if (e != cudaSuccess) {
+      set_last_error(std::string("block_tridag4_noalloc: context: ") + cudaGetErrorString(e));
+      return HAMSTR_GPU_ERR_CUDA;
+   }
    std::lock_guard<std::mutex> lock(g_scratch_mutex);
-   if (!g_scratch_addr[dev]) {
+   ContextScratch& have = g_scratch_addr[dev];
+   if (!have.addr || have.context != context) {
       void* p = nullptr;
       e = cudaGetSymbolAddress(&p, g_tridag_scratch);
       if (e != cudaSuccess || !p) {
          set_last_error(std::string("block_tridag4_noalloc: cudaGetSymbolAddress: ") + cudaGetErrorString(e));
          return HAMSTR_GPU_ERR_CUDA;
       }
-      g_scratch_addr[dev] = static_cast<double*>(p);
+      have = {context, static_cast<double*>(p)};
    }
-   *out = g_scratch_addr[dev];
+   *out = have.addr;
    return HAMSTR_GPU_OK;
 }
 

@@ -130,14 +130,14 @@ from hamstr_oop_gb300 import native
 lib = native.load()
 rt = ctypes.CDLL("libcudart.so.13")   # the runtime the library is linked with
 
-def solve(a, b, c, f, periodic):
+def solve(fn, a, b, c, f, periodic):
     dev = []
     for x in (a, b, c, f):
         p = ctypes.c_void_p()
         assert rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(x.nbytes)) == 0
         assert rt.cudaMemcpy(p, x.ctypes.data_as(ctypes.c_void_p), ctypes.c_size_t(x.nbytes), 1) == 0
         dev.append(p)
-    assert lib.hamstr_gpu_block_tridag4(f.shape[0], f.shape[1], periodic, *[p.value for p in dev], None) == 0
+    assert fn(f.shape[0], f.shape[1], periodic, *[p.value for p in dev], None) == 0
     out = np.empty_like(f)
     assert rt.cudaMemcpy(out.ctypes.data_as(ctypes.c_void_p), dev[3], ctypes.c_size_t(f.nbytes), 2) == 0
     return out
@@ -146,17 +146,21 @@ rng = np.random.default_rng(3)
 a, c = (rng.standard_normal((5, 12, 4, 4)) for _ in range(2))
 b = rng.standard_normal((5, 12, 4, 4)) + 6.0 * np.eye(4)
 f = rng.standard_normal((5, 12, 4))
-first = solve(a, b, c, f, 1)
+both = lib.hamstr_gpu_block_tridag4, lib.hamstr_gpu_block_tridag4_noalloc
+first = [solve(fn, a, b, c, f, 1) for fn in both]
+assert np.array_equal(*first)
 for _ in range(2):
     assert rt.cudaDeviceReset() == 0
-    assert np.array_equal(solve(a, b, c, f, 1), first)
+    for fn in both:
+        assert np.array_equal(solve(fn, a, b, c, f, 1), first[0])
 print("same after a reset")
 """
 
 
-def test_the_pool_does_not_outlive_its_context():
+def test_scratch_does_not_outlive_its_context():
     """After cudaDeviceReset, which ends the process's own context, the next
-    call makes a pool in the new one.  In a process of its own."""
+    call makes a pool in the new one, and the allocation-free one looks its
+    scratch up again.  In a process of its own."""
     import os
     import subprocess
     import sys
