@@ -1108,8 +1108,9 @@ __device__ __forceinline__ void solve_line(const double* __restrict__ fac, const
 // flags: a word is kTeamEmpty until the factoring warp has stored it, and again
 // once the follower has read it.  So the recurrence neither waits for its record
 // stores to be performed, as publish_rows would make it, nor spends a barrier on
-// a row (both measured about 490 cycles a row).  kTeamEmpty is a NaN no
-// arithmetic gives; an input block that holds it would make a wait give up.
+// a row (both measured about 490 cycles a row).  kTeamEmpty is a signalling NaN,
+// which no arithmetic gives; the first row's input may hold it, and is taken as the
+// quiet NaN that its first use makes of it (team_input).
 // A row whose pivots' integer reciprocals are undecided (sd::rcp_try) is done
 // again with the operator, so that a row has one such branch instead of four.
 // Cycles per row of a line (one warp each on its sub-partition): factorisation
@@ -1144,6 +1145,13 @@ __device__ __forceinline__ unsigned long long team_word(const unsigned long long
    return v;
 }
 
+// an input value that may reach a word as it is (later rows' went through arithmetic)
+__device__ __forceinline__ double team_input(double v)
+{
+   const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+   return u == kTeamEmpty ? __longlong_as_double((long long)(u | 1ull << 51)) : v;
+}
+
 // one elimination step of factor_line_team: pivot S of the LU of B' (lanes
 // 0-15) with the columns of c (lanes 16-31) substituted along it
 template <int S, bool SOFT>
@@ -1176,7 +1184,7 @@ __device__ __forceinline__ bool factor_line_team(const double* __restrict__ Ab, 
    const int h = lane >> 4, e = lane & 15, k = e >> 2, j = e & 3;
    const double* Wb = h ? Cb : Bb;   // lanes 0-15 hold B', lanes 16-31 the columns of c(i)
    double2 A = ld2(Ab + 4 * k + 2 * h);   // a(k, 2h) and a(k, 2h+1)
-   double W = Wb[e];
+   double W = team_input(Wb[e]);
    double P0 = 0.0, P1 = 0.0;        // c'(i-1) entries (2h, j) and (2h+1, j)
    bool bad = false;
    for (int i = 0; i < N; i++) {
@@ -1287,7 +1295,7 @@ __device__ __forceinline__ void follow_line_team(const double* __restrict__ Ab, 
       // a(i) = -a(i) a'(i-1), f(i) -= a(i) f(i-1)
       double x;
       if (i == 0) {
-         x = h ? f : sel4(a, j);
+         x = h ? f : team_input(sel4(a, j));
       } else {
          x = h ? f : 0.0;
 #pragma unroll

@@ -95,6 +95,23 @@ def test_scratch_from_the_pool_and_beyond_it(native_lib, nlines, periodic):
         assert np.array_equal(got[k:k + 300], want[:min(300, nlines - k)]), k
 
 
+@pytest.mark.parametrize("periodic,n", [(False, 1), (False, 20), (True, 2), (True, 20)])
+@pytest.mark.parametrize("operand", ["a", "b"])
+def test_any_nan_may_stand_in_a_block(oracle_lib, native_lib, operand, periodic, n):
+    """Also the one that marks an empty word of the two warps' ring: the solve
+    ends as for any other NaN, and not by a wait that gives up, which would
+    fill the line with the NaN of all bits set."""
+    from hamstr_oop_gb300 import native
+    a, b, c, f = _systems(13, 3, n)
+    {"a": a, "b": b}[operand].view(np.uint64)[1, 0, 2, 0] = 0xFFF4C3A59B7D6E21
+    got = _solve(native, a, b, c, f, periodic)
+    assert not np.any(got.view(np.uint64) == 0xFFFFFFFFFFFFFFFF)
+    for k in range(3):
+        with np.errstate(all="ignore"):
+            want = oracle_lib.block_tridag4(a[k], b[k], c[k], f[k], periodic)
+        assert np.array_equal(got[k], want, equal_nan=True), k
+
+
 def test_threads_and_streams_share_the_scratch_pool(native_lib):
     """Eight host threads on streams of their own, each with its own systems."""
     import threading
