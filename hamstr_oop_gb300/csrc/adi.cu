@@ -210,13 +210,14 @@ __device__ __forceinline__ void solve_chain(const DeviceState& d, int ich, int l
 
 // chain ich by two warps of a block (line_solve.cuh): its factorisation, and
 // its fill column with its first sweep's solve behind it
+template <bool SD>
 __device__ __forceinline__ bool factor_chain_team(const DeviceState& d, int ich, int lane, TeamShared* ts, bool* ok)
 {
    const int N = d.chain_nrows[ich], row0 = d.chain_row0[ich];
    const bool per = d.chain_periodic[ich] != 0;
    const double* blk = d.blk + 48 * (size_t)row0;
-   return factor_line_team(blk, blk + 16, blk + 32, 48, N, per, d.fac + (size_t)kFacRec * row0,
-                           per ? d.facN + 16 * d.chain_facN[ich] : nullptr, lane, ts, ok);
+   return factor_line_team<SD>(blk, blk + 16, blk + 32, 48, N, per, d.fac + (size_t)kFacRec * row0,
+                               per ? d.facN + 16 * d.chain_facN[ich] : nullptr, lane, ts, ok);
 }
 __device__ __forceinline__ void follow_chain_team(const DeviceState& d, int ich, int lane, TeamShared* ts, bool* ok)
 {
@@ -415,7 +416,7 @@ __global__ void __launch_bounds__(256, 1) adi_factor_kernel(DeviceState d, int n
       if (job == fjob) {
          // factorisation only, its solve follows in warp 1
          if (ich & kPairJob) bad |= factor_pair<SD>(d, ich & ~kPairJob, d.sched_jobs[job + 1], lane, &team.prog);
-         else if (!frozen_chain(d, ich)) bad |= factor_chain_team(d, ich, lane, &team, &ok);
+         else if (!frozen_chain(d, ich)) bad |= factor_chain_team<SD>(d, ich, lane, &team, &ok);
       } else if ((head & kFusedJob) && (ich & kPairJob)) {
          bad |= factor_solve_pair<SD>(d, ich & ~kPairJob, d.sched_jobs[job + 1], lane);
       } else {

@@ -1175,7 +1175,8 @@ __device__ __forceinline__ void team_step(double& w, int h, int k, int j, bool& 
 // second load costs nothing measurable.
 __device__ __forceinline__ double2 ld2(const double* __restrict__ p) { return make_double2(p[0], p[1]); }
 
-// Ab, Bb, Cb, stride, N, per, fac, facN and the result as factor_line's
+// Ab, Bb, Cb, stride, N, per, fac, facN, SD and the result as factor_line's
+template <bool SD = true>
 __device__ __forceinline__ bool factor_line_team(const double* __restrict__ Ab, const double* __restrict__ Bb,
                                                  const double* __restrict__ Cb, size_t stride, int N, bool per,
                                                  double* __restrict__ fac, double* __restrict__ facN, int lane,
@@ -1211,11 +1212,11 @@ __device__ __forceinline__ bool factor_line_team(const double* __restrict__ Ab, 
       }
       const double w0 = w;
       bool rare = false;
-      team_step<0, true>(w, h, k, j, rare);
-      team_step<1, true>(w, h, k, j, rare);
-      team_step<2, true>(w, h, k, j, rare);
-      team_step<3, true>(w, h, k, j, rare);
-      if (__any_sync(kLaneMask, rare)) {
+      team_step<0, SD>(w, h, k, j, rare);
+      team_step<1, SD>(w, h, k, j, rare);
+      team_step<2, SD>(w, h, k, j, rare);
+      team_step<3, SD>(w, h, k, j, rare);
+      if (SD && __any_sync(kLaneMask, rare)) {
          w = w0;
          team_step<0, false>(w, h, k, j, rare);
          team_step<1, false>(w, h, k, j, rare);
@@ -1262,7 +1263,7 @@ __device__ __forceinline__ bool factor_line_team(const double* __restrict__ Ab, 
    __syncwarp();
    const double bN =
       eliminate_last_row(fac, N, ldf<true>(&fac[(size_t)kFacRec * (N - 1) + 32 + e]), lane, &ts->prog);
-   const double w = lu_wavefront<true>(__shfl_sync(kLaneMask, bN, 16 + e), 16 * h, e);
+   const double w = lu_wavefront<SD>(__shfl_sync(kLaneMask, bN, 16 + e), 16 * h, e);
    if (h == 0) facN[e] = w;
    publish_rows(&ts->prog, 2 * N, lane);
    return bad || (h == 0 && k == j && nonfinite(w));
