@@ -305,15 +305,32 @@ __device__ __forceinline__ Weno5Diff<T> weno5_diff(T a, T b, T c, T d, T e)
    return w;
 }
 
-// a smoothness sum without its eps: b1 d d + 0.25 e e.  0.25 e e is formed as
-// 0.25 (e e): they differ only where e e is subnormal, which the eps (1e-15 or
-// 1e-10) added next absorbs
-template <bool SD, bool EXACT = false, typename T>
+// the smoothness sums without their eps: b1 d d + 0.25 e e, the quarter before
+// the product, as the reference forms it
+template <bool SM, bool SC, typename T>
 __device__ __forceinline__ T weno5_smooth(T d, T e)
 {
-   const T s = pm<SD>(pm<SD>(T(13. / 12.), d), d);
-   if (kAsWritten<T, EXACT>) return s + pm<SD>(p2<-2, SD>(e), e);
-   return add2<-2>(pm<SD>(e, e), s);
+   return pm<SM>(pm<SM>(T(13. / 12.), d), d) + pm<SM>(p2<-2, SC>(e), e);
+}
+
+// The three of them where an eps of 1e-15 or more is added next: the quarter goes
+// into the addition, which rounds differently only where e e is subnormal, far
+// below that eps.  But e e overflows earlier, so a sum that is not finite is
+// formed again.  (recon5, 512 x 128 half split: 168 us so, 177 with a scaling each.)
+template <bool SD>
+__device__ __forceinline__ void weno5_smooth3(const Weno5Diff<double>& w, double (&s)[3])
+{
+   const double d[3] = {w.djm1, w.dj, w.djp1}, e[3] = {w.ejm1, w.ej, w.ejp1};
+   unsigned top = 0;
+#pragma unroll
+   for (int k = 0; k < 3; k++) {
+      s[k] = add2<-2>(pm<SD>(e[k], e[k]), pm<SD>(pm<SD>(13. / 12., d[k]), d[k]));
+      top = max(top, (unsigned)__double2hiint(s[k]));
+   }
+   if (top >= 0x7FF00000u) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) s[k] = weno5_smooth<false, false>(d[k], e[k]);
+   }
 }
 
 // WENO5 (reconstruction.cpp:193-239); pow(x, 1) is x.  With SD the
@@ -323,9 +340,9 @@ __device__ __forceinline__ double weno5(double a, double b, double c, double d, 
 {
    const double epsw = 1e-15, b2 = 1. / 6.;
    const Weno5Diff<double> w = weno5_diff<SD>(a, b, c, d, e);
-   const double dis0 = weno5_smooth<SD>(w.djm1, w.ejm1) + epsw;
-   const double dis1 = weno5_smooth<SD>(w.dj, w.ej) + epsw;
-   const double dis2 = weno5_smooth<SD>(w.djp1, w.ejp1) + epsw;
+   double s[3];
+   weno5_smooth3<SD>(w, s);
+   const double dis0 = s[0] + epsw, dis1 = s[1] + epsw, dis2 = s[2] + epsw;
    const double d01 = Dv<double, SD>(dis1).div(dis0);
    const double d02 = Dv<double, SD>(dis2).div(dis0);
    const double ha1 = pc<3, SD>(d01);   // half of a1ba0 = 6 d01: 6 x = 2 (3 x) exactly
@@ -439,9 +456,9 @@ __device__ __forceinline__ Weno5Lin<T> weno5_lin_pre(T a, T b, T c, T d, T e, T 
 {
    Weno5Lin<T> p;
    const Weno5Diff<T> w = weno5_diff<SD>(a, b, c, d, e);
-   p.beta0 = weno5_smooth<kLinSoftMul, EXACT>(w.djm1, w.ejm1) + epsw;
-   p.beta1 = weno5_smooth<kLinSoftMul, EXACT>(w.dj, w.ej) + epsw;
-   p.beta2 = weno5_smooth<kLinSoftMul, EXACT>(w.djp1, w.ejp1) + epsw;
+   p.beta0 = weno5_smooth<kLinSoftMul, SD>(w.djm1, w.ejm1) + epsw;
+   p.beta1 = weno5_smooth<kLinSoftMul, SD>(w.dj, w.ej) + epsw;
+   p.beta2 = weno5_smooth<kLinSoftMul, SD>(w.djp1, w.ejp1) + epsw;
    p.q30 = w.q30;
    p.q31 = w.q31;
    p.q32 = w.q32;
@@ -505,9 +522,9 @@ __device__ __forceinline__ double weno5_with_lin(double a, double b, double c, d
 {
    const double b2 = 1. / 6.;
    const Weno5Diff<double> w = weno5_diff<SD>(a, b, c, d, e);
-   const double s0 = weno5_smooth<SD>(w.djm1, w.ejm1), s1 = weno5_smooth<SD>(w.dj, w.ej),
-                s2 = weno5_smooth<SD>(w.djp1, w.ejp1);
-   const double dis0 = s0 + 1e-15, dis1 = s1 + 1e-15, dis2 = s2 + 1e-15;
+   double s[3];
+   weno5_smooth3<SD>(w, s);
+   const double dis0 = s[0] + 1e-15, dis1 = s[1] + 1e-15, dis2 = s[2] + 1e-15;
    p.q30 = w.q30;
    p.q31 = w.q31;
    p.q32 = w.q32;
@@ -518,9 +535,9 @@ __device__ __forceinline__ double weno5_with_lin(double a, double b, double c, d
    const double w0 = Dv<double, SD>(add2<1>(ha1, 1.0) + a2ba0).div(1.0);
    const double hw1 = ha1 * w0;         // half of w1
    const double w2 = add2<1, -1>(hw1, 1. - w0);
-   p.beta0 = s0 + 1e-10;
-   p.beta1 = s1 + 1e-10;
-   p.beta2 = s2 + 1e-10;
+   p.beta0 = s[0] + 1e-10;
+   p.beta1 = s[1] + 1e-10;
+   p.beta2 = s[2] + 1e-10;
    weno5_lin_fill<double, SD>(p, w.djm1, w.ejm1, w.dj, w.ej, w.djp1, w.ejp1);
    return pm<SD>(b2, add2<1>(pm<SD>(hw1, p.q31), pm<SD>(w0, p.q30)) + pm<SD>(w2, p.q32));
 }
