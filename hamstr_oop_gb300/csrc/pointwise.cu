@@ -11,6 +11,8 @@
 // of a line (WENO: per value and side).  Every expression keeps the
 // reference's operands and association (the unit is compiled with
 // -fmad=false), so each output equals one reference call's bit for bit.
+// (WENO entries above 2^1021 in magnitude are outside of that: there a doubled
+// entry alone overflows in the reference, and here only its sum with others.)
 //
 // These are bound by FP64 issue (15.8 G warp instructions/s), and a hardware
 // division takes 7 of its slots: the divisions, the small constants and, in
@@ -190,9 +192,8 @@ __global__ void __launch_bounds__(kThreads) muscl_deriv_kernel(Lines g, const do
 
 // WENO (reconstruction.cpp:133-160) and, with DERIV, WENO_DERIV
 // (reconstruction.cpp:353-386): entries is .. imax-3; blockIdx.y 0 the left
-// values, 1 the right ones (the same formulas on the entries reversed).  EXACT:
-// eps so small that the weights' derivatives may turn subnormal (recon.cuh)
-template <bool DERIV, bool EXACT>
+// values, 1 the right ones (the same formulas on the entries reversed)
+template <bool DERIV>
 __global__ void __launch_bounds__(kThreads) weno_kernel(Lines g, const double* __restrict__ f,
                                                         const double* __restrict__ dq, double* __restrict__ ql,
                                                         double* __restrict__ qr, int is, double eps)
@@ -208,9 +209,8 @@ __global__ void __launch_bounds__(kThreads) weno_kernel(Lines g, const double* _
       v[k] = f[at + (k - 2) * step];
       if (DERIV) dv[k] = dq[at + (k - 2) * step];
    }
-   out[at] = DERIV ? weno5_lin_apply<double, true, EXACT>(
-                        weno5_lin_pre<double, true, EXACT>(v[0], v[1], v[2], v[3], v[4], eps), dv[0], dv[1], dv[2],
-                        dv[3], dv[4])
+   out[at] = DERIV ? weno5_lin_apply<double, true>(weno5_lin_pre<double, true>(v[0], v[1], v[2], v[3], v[4], eps), dv[0],
+                                                   dv[1], dv[2], dv[3], dv[4])
                    : weno5<true>(v[0], v[1], v[2], v[3], v[4]);
 }
 
@@ -306,7 +306,7 @@ int hamstr_gpu_weno(int nlines, int imax, int nq, const double* f, double* ql, d
    if (nlines == 0 || imax - 2 <= is) return HAMSTR_GPU_OK;
    const Lines g{nlines, imax, nq};
    const dim3 nb(blocks((size_t)nlines * nq * (imax - 2 - is)), 2);
-   weno_kernel<false, false><<<nb, kThreads, 0, (cudaStream_t)stream>>>(g, f, nullptr, ql, qr, is, 1e-15);
+   weno_kernel<false><<<nb, kThreads, 0, (cudaStream_t)stream>>>(g, f, nullptr, ql, qr, is, 1e-15);
    return launched("weno");
 }
 
@@ -322,9 +322,7 @@ int hamstr_gpu_weno_deriv(int nlines, int imax, int nq, const double* f, const d
    if (nlines == 0 || imax - 2 <= is) return HAMSTR_GPU_OK;
    const Lines g{nlines, imax, nq};
    const dim3 nb(blocks((size_t)nlines * nq * (imax - 2 - is)), 2);
-   // every smoothness sum is at least eps, their fourth powers at least 1e-240
-   if (eps >= 1e-60) weno_kernel<true, false><<<nb, kThreads, 0, (cudaStream_t)stream>>>(g, f, dq, ql, qr, is, eps);
-   else weno_kernel<true, true><<<nb, kThreads, 0, (cudaStream_t)stream>>>(g, f, dq, ql, qr, is, eps);
+   weno_kernel<true><<<nb, kThreads, 0, (cudaStream_t)stream>>>(g, f, dq, ql, qr, is, eps);
    return launched("weno_deriv");
 }
 

@@ -273,13 +273,23 @@ __device__ __forceinline__ void muscl_deriv2(T fm1, T f0, T fp1, T fp2, T dm1, T
    }
 }
 
-// Below, 6 x is taken as twice 3 x and the factor 2 moved into the addition that
-// follows, so that it costs nothing.  That is exact where nothing in between is
-// subnormal.  In FP32 the weights' derivatives do reach that range (smoothness
-// sums of 1e-10 to the fourth power), and in FP64 they may where a caller's eps is
-// tiny (EXACT), so there the factors stay as written.
-template <typename T, bool EXACT>
-constexpr bool kAsWritten = EXACT || sizeof(T) == 4;
+// Below, 6 x is three times x, held with a factor 2 to go (a constant of the
+// integer pipes); where it goes into an addition (add2), a product or a dividend
+// on those pipes, the factor costs nothing.  3 x is rounded as 6 x is, for
+// every x: where it is subnormal it is exact.  In FP32 6 x is one multiply.
+template <typename T>
+constexpr int kSix = sizeof(T) == 8 ? 1 : 0;   // 6 x = 2^kSix half6(x)
+template <bool SC, typename T>
+__device__ __forceinline__ T half6(T x)
+{
+   if constexpr (kSix<T> == 1) return pc<3, SC>(x);
+   else return T(6) * x;
+}
+template <bool SC, typename T>
+__device__ __forceinline__ T six(T x)
+{
+   return kSix<T> == 1 ? p2<1, SC>(half6<SC>(x)) : half6<SC>(x);
+}
 
 // the differences d_k, e_k and the candidate stencils of five values
 // (reconstruction.cpp:84-104).  Every factor 2 or 4 goes into the addition it
@@ -345,12 +355,12 @@ __device__ __forceinline__ double weno5(double a, double b, double c, double d, 
    const double dis0 = s[0] + epsw, dis1 = s[1] + epsw, dis2 = s[2] + epsw;
    const double d01 = Dv<double, SD>(dis1).div(dis0);
    const double d02 = Dv<double, SD>(dis2).div(dis0);
-   const double ha1 = pc<3, SD>(d01);   // half of a1ba0 = 6 d01: 6 x = 2 (3 x) exactly
+   const double h1 = half6<SD>(d01);      // a1ba0 = 6 d01
    const double a2ba0 = pc<3, SD>(d02);
-   const double w0 = Dv<double, SD>(add2<1>(ha1, 1.0) + a2ba0).div(1.0);
-   const double hw1 = pm<SD>(ha1, w0);  // half of w1
-   const double w2 = add2<1, -1>(hw1, 1. - w0);
-   return pm<SD>(b2, add2<1>(pm<SD>(hw1, w.q31), pm<SD>(w0, w.q30)) + pm<SD>(w2, w.q32));
+   const double w0 = Dv<double, SD>(add2<1>(h1, 1.0) + a2ba0).div(1.0);
+   const double w1 = pm2<1, SD>(h1, w0);
+   const double w2 = 1. - w0 - w1;
+   return pm<SD>(b2, pm<SD>(w0, w.q30) + pm<SD>(w1, w.q31) + pm<SD>(w2, w.q32));
 }
 
 // WENO_5 linearisation (reconstruction.cpp:358-462); the linear residual
@@ -410,7 +420,7 @@ __device__ __forceinline__ Weno5Lin<T> weno5_lin_get(const T* __restrict__ in, s
 // smoothness sums either 175, without the constants too 187.
 constexpr bool kLinSoftMul = false;
 
-template <typename T, bool SD, bool EXACT = false>
+template <typename T, bool SD>
 __device__ __forceinline__ void weno5_lin_fill(Weno5Lin<T>& p, T djm1, T ejm1, T dj, T ej, T djp1, T ejp1)
 {
    const T b1 = T(13. / 12.), b2 = T(1. / 6.);
@@ -424,34 +434,20 @@ __device__ __forceinline__ void weno5_lin_fill(Weno5Lin<T>& p, T djm1, T ejm1, T
    const Dv<T, SD> r1(p.beta1), r2(p.beta2);
    const T d01 = r1.div(p.beta0);
    const T d02 = r2.div(p.beta0);
-   if constexpr (kAsWritten<T, EXACT>) {
-      const T a1ba0 = T(6.) * d01, a2ba0 = T(3.) * d02;
-      const T w0 = Dv<T, SD>(T(1.0) + a1ba0 + a2ba0).div(T(1.0));
-      const T w1 = a1ba0 * w0;
-      const T w2 = T(1.) - w0 - w1;
-      p.b2w0 = b2 * w0;
-      p.b2w1 = b2 * w1;
-      p.b2w2 = b2 * w2;
-      p.bb12 = p.beta1 * p.beta2;
-      p.dwd = p.bb12 + T(6) * p.beta0 * p.beta2 + T(3) * p.beta0 * p.beta1;
-      p.dwd2 = p.dwd * p.dwd;
-      return;
-   }
-   const T ha1 = pc<3, SD>(d01);   // half of a1ba0 = 6 d01
+   const T h1 = half6<SD>(d01);
    const T a2ba0 = pc<3, SD>(d02);
-   const T w0 = Dv<T, SD>(add2<1>(ha1, T(1.0)) + a2ba0).div(T(1.0));
-   const T hw1 = pm<kLinSoftMul>(ha1, w0);   // half of w1
-   const T w2 = add2<1, -1>(hw1, T(1.) - w0);
+   const T w0 = Dv<T, SD>(add2<kSix<T>>(h1, T(1.0)) + a2ba0).div(T(1.0));
+   const T w1 = pm2<kSix<T>, SD>(h1, w0);
+   const T w2 = T(1.) - w0 - w1;
    p.b2w0 = pm<kLinSoftMul>(b2, w0);
-   p.b2w1 = p2<1, SD>(pm<kLinSoftMul>(b2, hw1));
+   p.b2w1 = pm<kLinSoftMul>(b2, w1);
    p.b2w2 = pm<kLinSoftMul>(b2, w2);
    p.bb12 = pm<kLinSoftMul>(p.beta1, p.beta2);
-   const T b03 = pc<3, SD>(p.beta0);   // 6 beta0 is twice it
-   p.dwd = add2<1>(pm<kLinSoftMul>(b03, p.beta2), p.bb12) + pm<kLinSoftMul>(b03, p.beta1);
+   p.dwd = p.bb12 + pm<kLinSoftMul>(six<SD>(p.beta0), p.beta2) + pm<kLinSoftMul>(pc<3, SD>(p.beta0), p.beta1);
    p.dwd2 = pm<kLinSoftMul>(p.dwd, p.dwd);
 }
 
-template <typename T, bool SD, bool EXACT = false>
+template <typename T, bool SD>
 __device__ __forceinline__ Weno5Lin<T> weno5_lin_pre(T a, T b, T c, T d, T e, T epsw = T(1e-10))
 {
    Weno5Lin<T> p;
@@ -462,11 +458,11 @@ __device__ __forceinline__ Weno5Lin<T> weno5_lin_pre(T a, T b, T c, T d, T e, T 
    p.q30 = w.q30;
    p.q31 = w.q31;
    p.q32 = w.q32;
-   weno5_lin_fill<T, SD, EXACT>(p, w.djm1, w.ejm1, w.dj, w.ej, w.djp1, w.ejp1);
+   weno5_lin_fill<T, SD>(p, w.djm1, w.ejm1, w.dj, w.ej, w.djp1, w.ejp1);
    return p;
 }
 
-template <typename T, bool SD, bool EXACT = false>
+template <typename T, bool SD>
 __device__ __forceinline__ T weno5_lin_apply(const Weno5Lin<T>& p, T a_d, T b_d, T c_d, T d_d, T e_d)
 {
    const T b2 = T(1. / 6.);
@@ -480,31 +476,20 @@ __device__ __forceinline__ T weno5_lin_apply(const Weno5Lin<T>& p, T a_d, T b_d,
    const T beta0 = p.beta0, beta1 = p.beta1, beta2 = p.beta2;
    const T dw0_down = p.dwd;
    const T s12 = pm<kLinSoftMul>(dbeta1, beta2) + pm<kLinSoftMul>(beta1, dbeta2);
-   if constexpr (kAsWritten<T, EXACT>) {
-      const T s6 = T(6) * (dbeta0 * beta2 + beta0 * dbeta2);
-      const T s3 = T(3) * (dbeta0 * beta1 + beta0 * dbeta1);
-      const T up = p.bb12 * (s12 + s6 + s3);
-      const Dv<T, SD> rd(p.dwd2);
-      const T dw0 = rd.div(s12 * dw0_down - up);
-      const T dw1 = rd.div(s6 * dw0_down - Dv<T, SD>(beta1).div(T(6) * up) * beta0);
-      const T dw2 = rd.div(s3 * dw0_down - Dv<T, SD>(beta2).div(T(3) * up) * beta0);
-      return term1 + term2 + term3 + b2 * dw0 * p.q30 + b2 * dw1 * p.q31 + b2 * dw2 * p.q32;
-   }
-   const T h6 = pc<3, SD>(pm<kLinSoftMul>(dbeta0, beta2) + pm<kLinSoftMul>(beta0, dbeta2));
+   const T h6 = half6<SD>(pm<kLinSoftMul>(dbeta0, beta2) + pm<kLinSoftMul>(beta0, dbeta2));
    const T s3 = pc<3, SD>(pm<kLinSoftMul>(dbeta0, beta1) + pm<kLinSoftMul>(beta0, dbeta1));
    const T dw0_up_1 = pm<SD>(s12, dw0_down);
-   const T dw0_up_2 = pm<kLinSoftMul>(p.bb12, add2<1>(h6, s12) + s3);
+   const T dw0_up_2 = pm<kLinSoftMul>(p.bb12, add2<kSix<T>>(h6, s12) + s3);
    const Dv<T, SD> rd(p.dwd2);
    const T dw0 = rd.div(dw0_up_1 - dw0_up_2);
-   const T dw1_up_1 = pm<SD>(h6, dw0_down);   // half of it
-   const T u3 = pc<3, SD>(dw0_up_2);
-   const T dw1_up_2 = pm<kLinSoftMul>(Dv<T, SD>(beta1).div(u3), beta0);   // half of it
-   const T dw1 = rd.div(dw1_up_1 - dw1_up_2);   // half of it
+   const T dw1_up_1 = pm2<kSix<T>, SD>(h6, dw0_down);
+   const T dw1_up_2 = pm<kLinSoftMul>(Dv<T, SD>(beta1).template div2<kSix<T>>(half6<SD>(dw0_up_2)), beta0);
+   const T dw1 = rd.div(dw1_up_1 - dw1_up_2);
    const T dw2_up_1 = pm<SD>(s3, dw0_down);
-   const T dw2_up_2 = pm<kLinSoftMul>(Dv<T, SD>(beta2).div(u3), beta0);
+   const T dw2_up_2 = pm<kLinSoftMul>(Dv<T, SD>(beta2).div(pc<3, SD>(dw0_up_2)), beta0);
    const T dw2 = rd.div(dw2_up_1 - dw2_up_2);
-   const T sum = term1 + term2 + term3 + pm<kLinSoftMul>(pm<kLinSoftMul>(b2, dw0), p.q30);
-   return add2<1>(pm<kLinSoftMul>(pm<kLinSoftMul>(b2, dw1), p.q31), sum) + pm<kLinSoftMul>(pm<kLinSoftMul>(b2, dw2), p.q32);
+   return term1 + term2 + term3 + pm<kLinSoftMul>(pm<kLinSoftMul>(b2, dw0), p.q30) +
+          pm<kLinSoftMul>(pm<kLinSoftMul>(b2, dw1), p.q31) + pm<kLinSoftMul>(pm<kLinSoftMul>(b2, dw2), p.q32);
 }
 
 template <typename T, bool SD>
@@ -530,16 +515,16 @@ __device__ __forceinline__ double weno5_with_lin(double a, double b, double c, d
    p.q32 = w.q32;
    const double d01 = Dv<double, SD>(dis1).div(dis0);
    const double d02 = Dv<double, SD>(dis2).div(dis0);
-   const double ha1 = pc<3, SD>(d01);   // half of a1ba0
+   const double h1 = half6<SD>(d01);
    const double a2ba0 = pc<3, SD>(d02);
-   const double w0 = Dv<double, SD>(add2<1>(ha1, 1.0) + a2ba0).div(1.0);
-   const double hw1 = ha1 * w0;         // half of w1
-   const double w2 = add2<1, -1>(hw1, 1. - w0);
+   const double w0 = Dv<double, SD>(add2<1>(h1, 1.0) + a2ba0).div(1.0);
+   const double w1 = pm2<1, SD>(h1, w0);
+   const double w2 = 1. - w0 - w1;
    p.beta0 = s[0] + 1e-10;
    p.beta1 = s[1] + 1e-10;
    p.beta2 = s[2] + 1e-10;
    weno5_lin_fill<double, SD>(p, w.djm1, w.ejm1, w.dj, w.ej, w.djp1, w.ejp1);
-   return pm<SD>(b2, add2<1>(pm<SD>(hw1, p.q31), pm<SD>(w0, p.q30)) + pm<SD>(w2, p.q32));
+   return pm<SD>(b2, pm<SD>(w0, p.q30) + pm<SD>(w1, p.q31) + pm<SD>(w2, p.q32));
 }
 
 // reconstructed states at the two sides of a face slot, FP64

@@ -173,7 +173,8 @@ __device__ __noinline__ double div_other(double a, double b) { return a / b; }
 inline double div_other(double a, double b) { return a / b; }
 #endif
 
-// a / D.b rounded to nearest even, equal to the `/` operator
+// (2^K a) / D.b rounded to nearest even, equal to the multiply and the `/` operator
+template <int K = 0>
 __host__ __device__ __forceinline__ double div(double a, const Divisor& D)
 {
    const uint64_t A = bits(a);
@@ -181,12 +182,12 @@ __host__ __device__ __forceinline__ double div(double a, const Divisor& D)
    const uint64_t ma = (A & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
    // quotient significand in [1, 2): s = 1 where ma < mb
    const int s = ma < D.mb ? 1 : 0;
-   const int e = ea - D.eb + 1023 - s;
-   if (!D.ok || ea == 0 || ea == 0x7FF || e <= 0 || e >= 0x7FE) {
+   const int e = ea - D.eb + 1023 + K - s;
+   if (!D.ok || ea == 0 || ea >= 0x7FF - K || e <= 0 || e >= 0x7FE) {
       // zero dividends are exact; subnormal, infinite and NaN operands and
       // quotients near or past the normal range go to the operator
       if (D.ok && (A << 1) == 0) return from_bits((A ^ D.sign) & 0x8000000000000000ull);
-      return div_other(a, D.b);
+      return div_other(K == 0 ? a : a * (double)(1 << K), D.b);
    }
    // floor of (ma/mb) 2^63 less an error in [0, 9); 10 + (1 - s) bits are
    // beyond the significand
@@ -249,26 +250,28 @@ __host__ __device__ __forceinline__ double scale2(double x)
    return mul_other(x, kScale);
 }
 
-// a * b rounded to nearest even on the integer pipes, equal to the FP64
-// multiply: for normal operands with a normal product the 53-bit
+// (2^K a) * b rounded to nearest even on the integer pipes, equal to the FP64
+// multiplies (K >= 0: a doubling is exact, and moves the exponent here at no
+// cost): for normal operands with a normal product the 53-bit
 // significands multiply exactly in 128 bits (each shifted to the top of a
 // 64-bit word), the top 53 bits round on the next bit and the OR of the
 // rest; a zero times a zero or a normal number is a signed zero; anything
 // else (subnormal, infinite or NaN operands, a product that overflows or
 // turns subnormal) goes to the multiply.
+template <int K = 0>
 __host__ __device__ __forceinline__ double mul(double a, double b)
 {
    constexpr uint64_t kMant = 0xFFFFFFFFFFFFFull, kHidden = 0x10000000000000ull;
    const uint64_t ua = bits(a), ub = bits(b);
    const uint64_t sign = (ua ^ ub) & 0x8000000000000000ull;
    const int ea = (int)((ua >> 52) & 0x7FF), eb = (int)((ub >> 52) & 0x7FF);
-   const bool na = (unsigned)(ea - 1) < 0x7FEu, nb = (unsigned)(eb - 1) < 0x7FEu;
+   const bool na = (unsigned)(ea - 1) < 0x7FEu - K, nb = (unsigned)(eb - 1) < 0x7FEu;
    if (!na || !nb) {
       const bool za = (ua << 1) == 0, zb = (ub << 1) == 0;
       if ((za && (zb || nb)) || (zb && na)) return from_bits(sign);
-      return mul_other(a, b);
+      return mul_other(K == 0 ? a : a * (double)(1 << K), b);
    }
-   int e = ea + eb - 1023;   // biased exponent of a product in [1, 2)
+   int e = ea + eb - 1023 + K;   // biased exponent of a product in [1, 2)
    const uint64_t A = ((ua & kMant) | kHidden) << 11, B = ((ub & kMant) | kHidden) << 11;
    uint64_t hi = mulhi(A, B), lo = A * B;
    if (hi >> 63) {
@@ -277,7 +280,7 @@ __host__ __device__ __forceinline__ double mul(double a, double b)
       hi = (hi << 1) | (lo >> 63);
       lo <<= 1;
    }
-   if (e < 1) return mul_other(a, b);   // subnormal or zero product
+   if (e < 1) return mul_other(K == 0 ? a : a * (double)(1 << K), b);   // subnormal or zero product
    uint64_t m = hi >> 11;
    const uint64_t g = (hi >> 10) & 1;
    const bool st = ((hi & 0x3FF) | lo) != 0;
@@ -286,7 +289,7 @@ __host__ __device__ __forceinline__ double mul(double a, double b)
       m >>= 1;
       e += 1;
    }
-   if (e > 0x7FE) return mul_other(a, b);   // overflow
+   if (e > 0x7FE) return mul_other(K == 0 ? a : a * (double)(1 << K), b);   // overflow
    return from_bits(sign | ((uint64_t)e << 52) | (m & kMant));
 }
 
@@ -341,6 +344,18 @@ __host__ __device__ __forceinline__ float pm(float a, float b)
    return a * b;
 }
 
+// (2^K a) * b, as pm
+template <int K, bool SOFT>
+__host__ __device__ __forceinline__ double pm2(double a, double b)
+{
+   return SOFT ? sd::mul<K>(a, b) : ((double)(1 << K) * a) * b;
+}
+template <int K, bool SOFT>
+__host__ __device__ __forceinline__ float pm2(float a, float b)
+{
+   return ((float)(1 << K) * a) * b;
+}
+
 // C * x for a small odd C, as pm
 template <int C, bool SOFT>
 __host__ __device__ __forceinline__ double pc(double x)
@@ -356,7 +371,9 @@ __host__ __device__ __forceinline__ float pc(float x)
 // 2^K x + y with one rounding of the sum: the product is exact wherever it
 // neither overflows nor turns subnormal, so this is the reference's multiply
 // and add, in one FP64 instruction instead of one and a scaling on the integer
-// pipes.  S = -1: y - 2^K x.
+// pipes.  For K > 0 it is that for every x up to 2^(1023-K) in magnitude; beyond,
+// the product alone would be infinite and the sum here may not be.  For K < 0 it
+// is that unless 2^K x is subnormal and y not far larger.  S = -1: y - 2^K x.
 template <int K, int S = 1>
 __host__ __device__ __forceinline__ double add2(double x, double y)
 {
@@ -399,12 +416,16 @@ struct Dv {
    T b;
    __device__ __forceinline__ explicit Dv(T b_) : b(b_) {}
    __device__ __forceinline__ T div(T a) const { return a / b; }
+   template <int K>
+   __device__ __forceinline__ T div2(T a) const { return (T(1 << K) * a) / b; }   // (2^K a) / b
 };
 template <>
 struct Dv<double, true> {
    sd::Divisor D;
    __device__ __forceinline__ explicit Dv(double b) : D(sd::divisor(b)) {}
    __device__ __forceinline__ double div(double a) const { return sd::div(a, D); }
+   template <int K>
+   __device__ __forceinline__ double div2(double a) const { return sd::div<K>(a, D); }
 };
 
 }  // namespace hamstr
