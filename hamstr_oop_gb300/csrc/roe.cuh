@@ -44,7 +44,7 @@ __device__ __forceinline__ bool roe_face(double nxd, double nyd, const double (&
    const double gm1 = gam - 1.0;
    const double area = sqrt(nxd * nxd + nyd * nyd);
    const Dv<double, SD> by_area(area);
-   const double half = p2<-1, SD>(area);   // 0.5 x area = x (0.5 area)
+   const double half = p2<-1, SD>(area);   // (0.5 x) area = x (0.5 area) where neither half is subnormal
    const double invArea = by_area.div(1.);
    const double nx = nxd * invArea;
    const double ny = nyd * invArea;
@@ -53,13 +53,13 @@ __device__ __forceinline__ bool roe_face(double nxd, double nyd, const double (&
    const Dv<double, SD> by_rol(rol);
    const double ul = by_rol.div(ql[1]);
    const double vl = by_rol.div(ql[2]);
-   const double pl = gm1 * add2<-1, -1>(rol * (ul * ul + vl * vl), ql[3]);
+   const double pl = gm1 * (ql[3] - p2<-1, SD>(rol) * (ul * ul + vl * vl));
    const double hl = by_rol.div(ql[3] + pl);
    const double ror = qr[0];
    const Dv<double, SD> by_ror(ror);
    const double ur = by_ror.div(qr[1]);
    const double vr = by_ror.div(qr[2]);
-   const double pr = gm1 * add2<-1, -1>(ror * (ur * ur + vr * vr), qr[3]);
+   const double pr = gm1 * (qr[3] - p2<-1, SD>(ror) * (ur * ur + vr * vr));
    const double hr = by_ror.div(qr[3] + pr);
    const double dp = pr - pl;
    const double uconr = ur * nx + vr * ny;
