@@ -39,6 +39,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -660,6 +661,7 @@ struct hamstr_mlp {
    Result* res = nullptr;
    float* host_params = nullptr;   // [kNParams], page-locked: what get_params and get_grads bring (pack_kernel)
    float* dev_params = nullptr;    // its device address
+   std::mutex params_mutex;        // of that buffer: threads may read parameters at the same time
    NetMaps net;
    WgradMaps wg;
 
@@ -960,6 +962,7 @@ static int get_tensors(hamstr_mlp* h, bool grads, float* out)
    const std::vector<View> v = views(h, grads);
    std::copy(v.begin(), v.end(), a.v);
    a.out = h->dev_params;
+   std::lock_guard<std::mutex> lock(h->params_mutex);
    pack_kernel<<<(kNParams + 255) / 256, 256, 0, h->st>>>(a);
    int st = cuda_ok(cudaGetLastError(), "mlp get");
    if (!st) st = cuda_ok(cudaStreamSynchronize(h->st), "mlp get sync");

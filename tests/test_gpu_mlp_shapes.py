@@ -54,3 +54,25 @@ def test_a_batch_below_capacity_trains_the_same(native_lib):
         loss = [net.train_step(fd, td, batch=4864, seed=11, step=k, lr=1e-3) for k in range(2)]
         got.append((loss, net.get_params()))
     assert got[0][0] == got[1][0] and np.array_equal(got[0][1], got[1][1])
+
+
+def test_threads_read_parameters_and_gradients_at_once(native_lib):
+    import threading
+    from hamstr_oop_gb300 import native
+    net = native.Mlp(batch_capacity=256, seed=4)
+    _, _, fd, td = _rows(200, 3)
+    net.grad(fd, td)
+    want = net.get_params(), net.get_grads()
+    bad = []
+
+    def read(k):
+        for _ in range(200):
+            got = net.get_grads() if k % 2 else net.get_params()
+            if not np.array_equal(got, want[k % 2]):
+                bad.append(k)
+    threads = [threading.Thread(target=read, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
