@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(net_threads(EW), EW == 8 ? 2 : 1)
    unsigned char* ring = in + kInBytes;
    __shared__ NetShared<STAGES> s;
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   const int ntiles = (a.n + 127) / 128;
+   const int ntiles = (a.n - 1) / 128 + 1;   // a.n may be the largest int
    const uint32_t full0 = smem_u32(s.full), empty0 = smem_u32(s.empty), acc = smem_u32(&s.acc),
                   input = smem_u32(&s.input);
    if (threadIdx.x == 0) {

@@ -76,3 +76,25 @@ def test_threads_read_parameters_and_gradients_at_once(native_lib):
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_forward_of_the_most_rows(native_lib):
+    """2^31 - 1 rows, 77 GB of inputs and outputs."""
+    import torch
+    from hamstr_oop_gb300 import native
+    n = 2 ** 31 - 1
+    if torch.cuda.mem_get_info()[0] < 100e9:
+        pytest.skip("needs 77 GB of device memory")
+    net = native.Mlp(batch_capacity=256, seed=6)
+    _, _, fd, _ = _rows(1 << 16, 4)
+    feat = torch.empty((n, 5), device="cuda")
+    whole = n // (1 << 16) << 16
+    feat[:whole].view(-1, 1 << 16, 5).copy_(fd.expand(whole >> 16, 1 << 16, 5))
+    feat[whole:].copy_(fd[:n - whole])
+    y, z = net.forward(feat), net.forward(fd)
+    del feat
+    same = all(bool(torch.equal(y[k << 16:(k + 1) << 16], z)) for k in (0, 1, 1000, (whole >> 16) - 1))
+    same = same and bool(torch.equal(y[whole:], z[:n - whole]))
+    del y
+    torch.cuda.empty_cache()
+    assert same
