@@ -111,7 +111,8 @@ struct NetArgs {
    int ld;
    float* G;                      // GELU'(Z): [tile][layer][column][row]
    double* lpart;                 // per 32 rows: loss, db4[4]
-   int* err;
+   int* err;                      // 1 after a wait that gave up
+   int give_up;                   // self-test: the weight tile at which a block's loader gives up (-1: none)
 };
 
 template <int STAGES>
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(net_threads(EW), EW == 8 ? 2 : 1)
             for (int l = 0; l < LAYERS && !*failed; l++)
                for (int st = 0; st < layer_stages(l); st++, it++) {
                   const int slot = it % STAGES, round = it / STAGES;
-                  if (round > 0 && !mbar_wait(empty0 + 8 * slot, (round - 1) & 1, failed)) {
+                  if ((round > 0 && !mbar_wait(empty0 + 8 * slot, (round - 1) & 1, failed)) || it == a.give_up) {
                      *failed = 1;
                      break;
                   }
@@ -391,11 +392,13 @@ __global__ void __launch_bounds__(net_threads(EW), EW == 8 ? 2 : 1)
          // the next tile's input overwrites what the last product has read, and
          // its first product what every warp has read of the accumulator
       }
-      if (!ok && lane == 0) *(volatile int*)a.err = 1;
    }
    __syncwarp();
    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
    __syncthreads();
+   // whichever role gave up: the others may have come to their end, the epilogue
+   // with a product that is not complete
+   if (threadIdx.x == 0 && *failed) *(volatile int*)a.err = 1;
    if (warp == EW + 1)
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)W) : "memory");
 }
@@ -517,6 +520,8 @@ struct UpdateArgs {
    const bf16* dZt[3];
    int ld, B;
    const double* lpart;
+   const int* err;         // the pass's error word: nothing is updated after a wait that gave up
+   int* host_err;
    double* loss;
    int adam;
    float lr, c1, c2;       // c1, c2: bias corrections
@@ -550,6 +555,10 @@ __device__ __forceinline__ float split_sum(const float* __restrict__ part, int s
 __global__ void __launch_bounds__(256) update_kernel(const __grid_constant__ UpdateArgs a)
 {
    const int lane = threadIdx.x & 31;
+   if (*a.err) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) *a.host_err = 1;
+      return;
+   }
    if (blockIdx.x < kWeightBlocks) {
       int i = blockIdx.x * 256 + threadIdx.x;
       if (i < 2 * W * W) {
@@ -659,6 +668,8 @@ struct hamstr_mlp {
    double* lpart;
    Result* host = nullptr;   // and its device address
    Result* res = nullptr;
+   int* err;                 // of the passes before an update, which leaves the parameters as they are then
+   int give_up = -1;         // self-test (hamstr_check_mlp_wait)
    float* host_params = nullptr;   // [kNParams], page-locked: what get_params and get_grads bring (pack_kernel)
    float* dev_params = nullptr;    // its device address
    std::mutex params_mutex;        // of that buffer: threads may read parameters at the same time
@@ -740,6 +751,8 @@ NetArgs net_args(hamstr_mlp* h)
    a.b3 = h->b3.p;
    a.b4 = h->b4.p;
    a.err = &h->res->err;
+   a.give_up = h->give_up;
+   h->give_up = -1;
    return a;
 }
 
@@ -751,6 +764,7 @@ int finish(hamstr_mlp* h, double* loss)
    if (r->err) {
       set_last_error("mlp: a tensor-core pipeline wait timed out");
       h->host->err = 0;
+      cudaMemsetAsync(h->err, 0, sizeof(int), h->st);
       return HAMSTR_GPU_ERR_CUDA;
    }
    if (loss) *loss = r->loss;
@@ -776,6 +790,7 @@ int train(hamstr_mlp* h, const float* feat, const float* targ, long long n_all, 
       a.Ht[l] = h->Ht[l];
       a.dZt[l] = h->dZt[l];
    }
+   a.err = h->err;
    a.ld = h->Bmax;
    a.G = h->G;
    a.lpart = h->lpart;
@@ -790,7 +805,7 @@ int train(hamstr_mlp* h, const float* feat, const float* targ, long long n_all, 
    w.out[1] = h->part3;
    w.out[2] = h->part4;
    w.out[3] = h->part1;
-   w.err = &h->res->err;
+   w.err = h->err;
    wgrad_kernel<<<8 * w.splits, 128, kWgradSmem, h->st>>>(h->wg, w);
    if ((st = cuda_ok(cudaGetLastError(), "mlp weight gradients"))) return st;
    UpdateArgs u = {};
@@ -806,6 +821,8 @@ int train(hamstr_mlp* h, const float* feat, const float* targ, long long n_all, 
    u.ld = h->Bmax;
    u.B = B;
    u.lpart = h->lpart;
+   u.err = h->err;
+   u.host_err = &h->res->err;
    u.loss = &h->res->loss;
    u.adam = adam ? 1 : 0;
    u.lr = lr;
@@ -900,6 +917,7 @@ int hamstr_mlp_create(int Bmax, unsigned long long seed, hamstr_mlp** out)
    A(G, 3 * W * B);
    A(part1, splits * NOP * W); A(part4, splits * NOP * W); A(part2, splits * W * W); A(part3, splits * W * W);
    A(lpart, 5 * (B / 32));
+   A(err, 1);
 #undef A
    if (!st) st = cuda_ok(cudaHostAlloc((void**)&h->host, sizeof(Result), cudaHostAllocMapped), "mlp result");
    if (!st) {
@@ -980,6 +998,13 @@ int hamstr_mlp_get_grads(hamstr_mlp* h, float* out)
 {
    if (!h || !out) return HAMSTR_GPU_ERR_ARG;
    return get_tensors(h, true, out);
+}
+
+int hamstr_check_mlp_wait(hamstr_mlp* h, int tile)
+{
+   if (!h || tile < 0) return HAMSTR_GPU_ERR_ARG;
+   h->give_up = tile;
+   return HAMSTR_GPU_OK;
 }
 
 int hamstr_mlp_forward(hamstr_mlp* h, const float* feat, int n, float* y)

@@ -80,6 +80,7 @@ def load(build_if_missing: bool = False):
         "hamstr_mlp_get_grads": (i, [vp, vp]),
         "hamstr_mlp_forward": (i, [vp, vp, i, vp]),
         "hamstr_mlp_grad": (i, [vp, vp, vp, i, ctypes.POINTER(d)]),
+        "hamstr_check_mlp_wait": (i, [vp, i]),
         "hamstr_mlp_train_step": (i, [vp, vp, vp, ctypes.c_longlong, i, ctypes.c_ulonglong, ctypes.c_ulonglong,
                                       ctypes.c_float, ctypes.POINTER(d)]),
         "hamstr_gpu_autotune": (i, [vp, i, ctypes.c_char_p, i]),

@@ -297,7 +297,10 @@ int hamstr_mlp_gemm(const void* A, const void* B, int M, int N, int K, int split
  *     outputs) and its gradient, kept for _get_grads;
  *   _train_step: one Adam step (lr; betas 0.9, 0.999) on a minibatch of
  *     `batch` rows (a multiple of 128) drawn from n_all rows by a seeded
- *     hash of (seed, step); step counts from 0. */
+ *     hash of (seed, step); step counts from 0.
+ * Waits inside the kernels are bounded; a pass in which one gave up returns
+ * HAMSTR_GPU_ERR_CUDA, and leaves parameters, gradients and Adam's moments as
+ * they were. */
 typedef struct hamstr_mlp hamstr_mlp;
 int hamstr_mlp_nparams(void);
 int hamstr_mlp_create(int batch_capacity, unsigned long long seed, hamstr_mlp** out);
@@ -309,6 +312,12 @@ int hamstr_mlp_forward(hamstr_mlp* h, const float* features, int n, float* outpu
 int hamstr_mlp_grad(hamstr_mlp* h, const float* features, const float* targets, int n, double* loss);
 int hamstr_mlp_train_step(hamstr_mlp* h, const float* features, const float* targets, long long n_all, int batch,
                           unsigned long long seed, unsigned long long step, float lr, double* loss);
+
+/* Self-test hook: in the handle's next pass the weight loader of every block
+ * gives up at its `tile`-th weight tile, as after a wait that ran out.  A block
+ * takes 19 of them for 128 rows of _forward, 37 for 128 rows of _grad and
+ * _train_step. */
+int hamstr_check_mlp_wait(hamstr_mlp* h, int tile);
 
 /* Self-test hook: soft[i] = the integer-pipe division the FP64 kernels use
  * (hamstr_oop_gb300/csrc/softdiv.cuh), hard[i] = the hardware a[i]/b[i],

@@ -98,3 +98,41 @@ def test_forward_of_the_most_rows(native_lib):
     del y
     torch.cuda.empty_cache()
     assert same
+
+
+@pytest.mark.parametrize("tile", [0, 5, 17, 18])
+def test_forward_reports_a_loader_that_gave_up(native_lib, tile):
+    """At the first, a middle and the last weight tile (after which no other
+    role waits any more); the next pass is whole again."""
+    from hamstr_oop_gb300 import native
+    net = native.Mlp(batch_capacity=256, seed=8)
+    _, _, fd, _ = _rows(128, 5)
+    want = net.forward(fd).cpu().numpy()
+    assert native_lib.hamstr_check_mlp_wait(net.h, tile) == 0
+    with pytest.raises(native.HamstrError):
+        net.forward(fd)
+    assert np.array_equal(net.forward(fd).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("tile", [0, 18, 30, 36])
+def test_a_failed_step_changes_nothing(native_lib, tile):
+    """Parameters, gradients and moments: two steps after it are the two steps
+    of a network that never failed."""
+    from hamstr_oop_gb300 import native
+    _, _, fd, td = _rows(1000, 6)
+    got = []
+    for fail in (False, True):
+        net = native.Mlp(batch_capacity=256, seed=9)
+        loss = [net.train_step(fd, td, batch=256, seed=3, step=0, lr=1e-3)]
+        if fail:
+            before = net.get_params(), net.get_grads()
+            for call in (lambda: net.train_step(fd, td, batch=256, seed=3, step=1, lr=1e-3),
+                         lambda: net.grad(fd[:200].contiguous(), td[:200].contiguous())):
+                assert native_lib.hamstr_check_mlp_wait(net.h, tile) == 0
+                with pytest.raises(native.HamstrError):
+                    call()
+            assert np.array_equal(net.get_params(), before[0]) and np.array_equal(net.get_grads(), before[1])
+        loss.append(net.train_step(fd, td, batch=256, seed=3, step=1, lr=1e-3))
+        got.append((loss, net.get_params(), net.get_grads()))
+    assert got[0][0] == got[1][0]
+    assert np.array_equal(got[0][1], got[1][1]) and np.array_equal(got[0][2], got[1][2])
