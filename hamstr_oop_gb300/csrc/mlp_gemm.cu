@@ -170,7 +170,10 @@ int gemm(const GemmArgs& a, cudaStream_t st)
       set_last_error("mlp gemm: need M % 128 == 0, K % 64 == 0, 16-byte aligned operands");
       return HAMSTR_GPU_ERR_ARG;
    }
-   if (!a.C) return HAMSTR_GPU_ERR_ARG;
+   if (!a.C || ((uintptr_t)a.C & 15)) {   // stored by float4
+      set_last_error("mlp gemm: need a 16-byte aligned C");
+      return HAMSTR_GPU_ERR_ARG;
+   }
    switch (a.N) {
       case 16: return launch<16>(a, st);
       case 64: return launch<64>(a, st);

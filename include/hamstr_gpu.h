@@ -278,8 +278,8 @@ int hamstr_gpu_set_shape(hamstr_gpu* g, const int* shape);
 
 /* ---------------- learned warm start (no reference counterpart) --------
  * C[M][N] (+ split * M * N when splits > 1) = A[M][K] * B[N][K]^T with A, B
- * BF16 (K contiguous, 16-byte aligned device arrays) and FP32 accumulation
- * on the tcgen05 tensor cores; M % 128 == 0, K % 64 == 0, N in {16, 64,
+ * BF16 (K contiguous) and C FP32, all 16-byte aligned device arrays, with FP32
+ * accumulation on the tcgen05 tensor cores; M % 128 == 0, K % 64 == 0, N in {16, 64,
  * 128} or a multiple of 256.  K is cut into `splits` ranges whose partial
  * products go to consecutive M*N slabs.  *err (device int) becomes 1 if a
  * wait timed out.  stream: a cudaStream_t or NULL. */

@@ -77,3 +77,11 @@ def test_every_status_code_has_a_message(native_lib):
     assert len(codes) >= 8 and len(set(codes)) == len(codes)
     msgs = [native_lib.hamstr_gpu_strerror(c).decode() for c in codes]
     assert "unknown status" not in msgs and len(set(msgs)) == len(msgs)
+
+
+@pytest.mark.parametrize("which", ["A", "B", "C"])
+def test_gemm_refuses_unaligned_arrays(native_lib, which):
+    """Tiles are loaded and stored 16 bytes at a time; an array off that
+    boundary is refused before anything touches it (no device needed)."""
+    ptr = {k: 0x10000000 + (8 if k == which else 0) for k in "ABC"}
+    assert native_lib.hamstr_mlp_gemm(ptr["A"], ptr["B"], 128, 16, 64, 1, ptr["C"], 0x10000000, None) == -1
