@@ -1308,7 +1308,22 @@ extern "C" int hamstr_gpu_autotune(hamstr_gpu* g, int reps, char* report, int re
    CK(cudaEventCreate(&e0));
    CK(cudaEventCreate(&e1));
    int st = HAMSTR_GPU_OK;
+   // where both block sizes make the same launches (face_threads; of the FP64
+   // kernels none takes the value itself) a candidate of the second half has the
+   // time of its like in the first
+   auto threads_of = [&](int fb) {
+      DeviceState t = d;
+      t.face_block = fb;
+      return face_threads(t);
+   };
+   const size_t half = cands.size() / 2;
+   const bool same = !g->mixed && threads_of(cands.front().fb) == threads_of(cands.back().fb);
    for (Cand& c : cands) {
+      const size_t k = &c - cands.data();
+      if (same && k >= half) {
+         c.ms = cands[k - half].ms;
+         continue;
+      }
       if ((st = g->apply_shape(c.fb, c.wpb, c.mb, c.fused, c.fsoft, c.psoft, c.lanes, wk, c.bundle, ck, c.spike,
                                g->adi_fuse, c.fwpb)))
          break;

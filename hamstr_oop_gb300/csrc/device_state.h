@@ -202,10 +202,12 @@ __device__ __forceinline__ int norm_cell(const DeviceState& d)
 // Threads per block of a launch of one thread per face slot.  The face kernels
 // are bound by each SM's FP64 issue, so a launch lasts as long as its fullest
 // SM: of the tuned block and 64 and 32 threads, the one whose blocks, dealt out
-// evenly, load it least (the larger one where they tie).  164,399 slots: 256
-// threads put 5 blocks on the fullest SM for 4.2 on average, 64 put 17 for 16.9
-// (rhs_face 204 -> 183 us); 8,320 slots: 256 threads use 33 of 152 SMs, 32 all of
-// them (rhs_face 65 -> 38 us).
+// evenly, load it least (the larger one where they tie).  Measured, rhs_face in us
+// with 256, 128, 64, 32 threads | the rule's: 8,320 slots 51, 35, 32, 33 | 33;
+// 33,024 50, 46, 46, 43 | 43; 41,188 78, 66, 62, 61 | 61; 70,831 79, 81, 81, 79 | 79;
+// 131,584 156, 141, 141, 142 | 142; 164,399 193, 176, 175, 175 | 175; 205,440 224, 207,
+// 209, 210 | 210.  (mx_lin_face stages its block's Jacobians in shared memory of a
+// fixed size, so it keeps the block given.)
 inline int face_threads(const DeviceState& d)
 {
    const int nsm = d.nsm > 0 ? d.nsm : 1;

@@ -236,8 +236,10 @@ int hamstr_gpu_forces(hamstr_gpu* g, double* out6);
 int hamstr_gpu_autotune(hamstr_gpu* g, int reps, char* report, int report_len);
 
 /* The launch shape itself (no reference counterpart), HAMSTR_SHAPE_N ints:
- *   [0] face kernels' threads per block: 128 or 256 (on small meshes smaller
- *       blocks, where those load the fullest SM less)
+ *   [0] face kernels' threads per block: 128 or 256.  A launch takes 64 or 32
+ *       instead where those load the fullest SM less, on most meshes, so that
+ *       it then runs the same for both values; only the FP32 form's linear
+ *       face kernel always takes the value given
  *   [1] FP64 line kernels' persistent warps per SM: 4 or 8
  *   [2] FP32 line kernels' threads per block: 32, 64 or 128
  *   [3] FP32 blocks assembled inside the factorisation: 0 or 1
