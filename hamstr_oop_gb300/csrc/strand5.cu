@@ -8,7 +8,7 @@
 // (jacobianRoe.cpp:92-620, frozen eigenvalues, IMODE 1) and the 5x5
 // block-tridiagonal solvers TRISOLVER::blockTridag / blockTridagPeriodic
 // (triSolvers.cpp:443-766).  They are given here batched on device arrays:
-// one thread per face or six lanes per line, every expression with the reference's
+// one thread per face, six lanes or one thread per line, every expression with the reference's
 // operands and association (-fmad=false, IEEE division and square root),
 // so each output equals one reference call's bit for bit.
 // ##################################################################
@@ -212,13 +212,13 @@ __global__ void __launch_bounds__(kThreads) jacobian_roe3d_kernel(int n, const d
 // B', of c(i) and, periodic, of a(i) as it is eliminated, lane 5 the right-hand
 // side.  A row's work is the same instruction on every column, so the block
 // product, the LU and the substitutions of a row are 120 FP64 instructions a
-// warp (215 periodic) for five lines.  One thread a line, as before, spent 587
-// a row for 32 lines: fewer in all, but 4,099 lines were 129 warps on 608 SM
-// sub-partitions, each with 587 instructions of 64 cycles to a row (a
-// sub-partition issues one FP64 instruction per 64 cycles whatever its lanes
-// do), every load on 32 cache lines.  Measured, before -> now: 4,099 lines of 33
-// rows 1,092 -> 313 us open, 2,713 -> 709 periodic; one line 828 -> 233; 60,000
-// lines of 17 rows 2,640 -> 1,750.
+// warp (215 periodic) for five lines.  One thread a line spends 587 a row for 32
+// lines: fewer in all, but 4,099 lines are 129 warps on 608 SM sub-partitions, each
+// with 587 instructions of 64 cycles to a row (a sub-partition issues one FP64
+// instruction per 64 cycles whatever its lanes do), every load on 32 cache lines.
+// Measured, one thread -> six lanes, us a call: 4,099 lines of 33 rows 1,204 -> 273
+// open, 2,823 -> 681 periodic; one line 815 -> 193; 60,000 lines of 17 rows 2,515 ->
+// 1,623.  Where one thread a line is faster: one_thread_a_line below.
 //
 // The LU is unpivoted with reciprocal pivots, each entry's products subtracted
 // in the order of triSolvers.cpp:486-505; the reciprocals are the integer
@@ -465,6 +465,169 @@ __global__ void __launch_bounds__(32) block_tridag5_kernel(int nlines, int N, do
    }
 }
 
+// ---- one thread a line --------------------------------------------------
+// An open line's first row, without a block product, and a short line's last are
+// most of its work here, and 32 lines to a warp instead of five then win as soon as
+// there are lines for every SM.  Longer open lines are faster by six lanes at any
+// number (loads a line apart from lane to lane cost more than the issue slots
+// saved), periodic ones up to a quarter of a million lines.  Measured, six lanes /
+// one thread, us a call:
+//   open, 1 row: 4,099 lines 26 / 27, 9,000 30 / 26, 60,000 81 / 42, 500,000 488 / 175;
+//     2 rows: 45,000 138 / 155, 60,000 176 / 164, 200,000 518 / 466, 1,000,000 2,466 / 2,032;
+//     3 rows: 1,000,000 4,048 / 4,121; 17 rows: 500,000 13,134 / 18,623;
+//   periodic, 2 rows: 90,000 576 / 582, 130,000 817 / 767, 1,000,000 6,064 / 4,601;
+//     3 rows: 130,000 1,357 / 1,360, 200,000 2,065 / 1,971; 5 rows: 200,000 3,726 / 3,686,
+//     300,000 5,570 / 5,020; 17 rows: 200,000 13,667 / 13,858, 300,000 20,477 / 18,945; 33 rows:
+//     200,000 26,924 / 27,485, 300,000 40,350 / 37,642.
+bool one_thread_a_line(int nlines, int N, bool periodic)
+{
+   if (periodic) return nlines >= (N <= 3 ? 130000 : 250000);
+   return N == 1 ? nlines >= 6000 : N == 2 && nlines >= 60000;
+}
+
+// unpivoted LU with reciprocal pivots (triSolvers.cpp:481-506)
+struct LU5 {
+   double b11, b21, b22, b31, b32, b33, b41, b42, b43, b44, b51, b52, b53, b54, b55;
+   double u12, u13, u14, u15, u23, u24, u25, u34, u35, u45;
+};
+
+__device__ __forceinline__ LU5 lu5_factor(const double* b)
+{
+   LU5 u;
+   u.b11 = 1. / b[0];
+   u.u12 = b[1] * u.b11;
+   u.u13 = b[2] * u.b11;
+   u.u14 = b[3] * u.b11;
+   u.u15 = b[4] * u.b11;
+   u.b21 = b[5];
+   u.b22 = 1. / (b[6] - u.b21 * u.u12);
+   u.u23 = (b[7] - u.b21 * u.u13) * u.b22;
+   u.u24 = (b[8] - u.b21 * u.u14) * u.b22;
+   u.u25 = (b[9] - u.b21 * u.u15) * u.b22;
+   u.b31 = b[10];
+   u.b32 = b[11] - u.b31 * u.u12;
+   u.b33 = 1. / (b[12] - u.b31 * u.u13 - u.b32 * u.u23);
+   u.u34 = (b[13] - u.b31 * u.u14 - u.b32 * u.u24) * u.b33;
+   u.u35 = (b[14] - u.b31 * u.u15 - u.b32 * u.u25) * u.b33;
+   u.b41 = b[15];
+   u.b42 = b[16] - u.b41 * u.u12;
+   u.b43 = b[17] - u.b41 * u.u13 - u.b42 * u.u23;
+   u.b44 = 1. / (b[18] - u.b41 * u.u14 - u.b42 * u.u24 - u.b43 * u.u34);
+   u.u45 = (b[19] - u.b41 * u.u15 - u.b42 * u.u25 - u.b43 * u.u35) * u.b44;
+   u.b51 = b[20];
+   u.b52 = b[21] - u.b51 * u.u12;
+   u.b53 = b[22] - u.b51 * u.u13 - u.b52 * u.u23;
+   u.b54 = b[23] - u.b51 * u.u14 - u.b52 * u.u24 - u.b53 * u.u34;
+   u.b55 = 1. / (b[24] - u.b51 * u.u15 - u.b52 * u.u25 - u.b53 * u.u35 - u.b54 * u.u45);
+   return u;
+}
+
+// x[0], x[s], ..., x[4s] <- LU^{-1} x (triSolvers.cpp:508-518)
+__device__ __forceinline__ void lu5_solve(const LU5& u, double* x, int s)
+{
+   const double d1 = x[0] * u.b11;
+   const double d2 = (x[s] - u.b21 * d1) * u.b22;
+   const double d3 = (x[2 * s] - u.b31 * d1 - u.b32 * d2) * u.b33;
+   const double d4 = (x[3 * s] - u.b41 * d1 - u.b42 * d2 - u.b43 * d3) * u.b44;
+   const double d5 = (x[4 * s] - u.b51 * d1 - u.b52 * d2 - u.b53 * d3 - u.b54 * d4) * u.b55;
+   const double x3 = d4 - u.u45 * d5;
+   const double x2 = d3 - u.u34 * x3 - u.u35 * d5;
+   const double x1 = d2 - u.u23 * x2 - u.u24 * x3 - u.u25 * d5;
+   x[4 * s] = d5;
+   x[3 * s] = x3;
+   x[2 * s] = x2;
+   x[s] = x1;
+   x[0] = d1 - u.u12 * x1 - u.u13 * x2 - u.u14 * x3 - u.u15 * d5;
+}
+
+__global__ void __launch_bounds__(kThreads) block_tridag5_thread_kernel(int nlines, int N, int periodic,
+                                                                        double* __restrict__ av,
+                                                                        double* __restrict__ bv,
+                                                                        double* __restrict__ cv,
+                                                                        double* __restrict__ fv)
+{
+   const int line = blockIdx.x * blockDim.x + threadIdx.x;
+   if (line >= nlines) return;
+   const size_t nb = 25 * (size_t)N;
+   double* a = av + line * nb;
+   double* b = bv + line * nb;
+   double* c = cv + line * nb;
+   double* f = fv + line * 5 * (size_t)N;
+   auto A = [&](int i, int k, int j) -> double& { return a[25 * (size_t)i + 5 * k + j]; };
+   auto Bm = [&](int i, int k, int j) -> double& { return b[25 * (size_t)i + 5 * k + j]; };
+   auto C = [&](int i, int k, int j) -> double& { return c[25 * (size_t)i + 5 * k + j]; };
+   auto F = [&](int i, int k) -> double& { return f[5 * (size_t)i + k]; };
+   double t[5][5];
+   for (int i = 0; i < N; i++) {
+      if (i != 0) {
+         for (int k = 0; k < 5; k++)
+            for (int j = 0; j < 5; j++)
+               for (int l = 0; l < 5; l++) Bm(i, k, j) -= A(i, k, l) * C(i - 1, l, j);
+         for (int k = 0; k < 5; k++)
+            for (int j = 0; j < 5; j++) F(i, k) -= A(i, k, j) * F(i - 1, j);
+         if (periodic) {
+            for (int k = 0; k < 5; k++)
+               for (int j = 0; j < 5; j++) t[k][j] = 0;
+            for (int k = 0; k < 5; k++)
+               for (int j = 0; j < 5; j++)
+                  for (int l = 0; l < 5; l++) t[k][j] -= A(i, k, l) * A(i - 1, l, j);
+            for (int k = 0; k < 5; k++)
+               for (int j = 0; j < 5; j++) A(i, k, j) = t[k][j];
+         }
+      }
+      const LU5 u = lu5_factor(&Bm(i, 0, 0));
+      lu5_solve(u, &F(i, 0), 1);
+      if (!periodic) {
+         if (i != N - 1)
+            for (int j = 0; j < 5; j++) lu5_solve(u, &C(i, 0, j), 5);
+      } else if (i != N - 2) {
+         for (int j = 0; j < 5; j++) {
+            lu5_solve(u, &C(i, 0, j), 5);
+            lu5_solve(u, &A(i, 0, j), 5);
+         }
+      } else {
+         for (int k = 0; k < 5; k++)
+            for (int j = 0; j < 5; j++) C(i, j, k) += A(i, j, k);
+         for (int j = 0; j < 5; j++) lu5_solve(u, &C(i, 0, j), 5);
+         for (int k = 0; k < 5; k++)
+            for (int j = 0; j < 5; j++) A(i, k, j) = C(i, k, j);
+      }
+   }
+   if (!periodic) {
+      for (int i = N - 2; i >= 0; i--)
+         for (int k = 0; k < 5; k++)
+            for (int j = 0; j < 5; j++) F(i, k) -= C(i, k, j) * F(i + 1, j);
+      return;
+   }
+   // last-row elimination and solve (triSolvers.cpp:671-749)
+   for (int k = 0; k < 5; k++)
+      for (int j = 0; j < 5; j++) Bm(N - 1, j, k) = (j == k) ? 1.0 : 0.0;
+   for (int i = 0; i < N - 1; i++) {
+      for (int k = 0; k < 5; k++)
+         for (int j = 0; j < 5; j++) t[k][j] = 0;
+      for (int k = 0; k < 5; k++)
+         for (int j = 0; j < 5; j++)
+            for (int l = 0; l < 5; l++) {
+               t[k][j] -= C(N - 1, k, l) * C(i, l, j);
+               Bm(N - 1, k, j) -= C(N - 1, k, l) * A(i, l, j);
+            }
+      for (int k = 0; k < 5; k++)
+         for (int j = 0; j < 5; j++) F(N - 1, k) -= C(N - 1, k, j) * F(i, j);
+      for (int k = 0; k < 5; k++)
+         for (int j = 0; j < 5; j++) C(N - 1, k, j) = t[k][j];
+   }
+   {
+      const LU5 u = lu5_factor(&Bm(N - 1, 0, 0));
+      lu5_solve(u, &F(N - 1, 0), 1);
+   }
+   // back substitution (triSolvers.cpp:751-765)
+   for (int k = 0; k < 5; k++)
+      for (int j = 0; j < 5; j++) F(N - 2, k) -= (C(N - 2, k, j) * F(N - 1, j));
+   for (int i = N - 3; i >= 0; i--)
+      for (int k = 0; k < 5; k++)
+         for (int j = 0; j < 5; j++) F(i, k) -= (C(i, k, j) * F(i + 1, j) + A(i, k, j) * F(N - 1, j));
+}
+
 }  // namespace
 
 extern "C" {
@@ -505,6 +668,10 @@ int hamstr_gpu_block_tridag5(int nlines, int N, int periodic, double* A, double*
       return HAMSTR_GPU_ERR_ARG;
    }
    if (nlines == 0) return HAMSTR_GPU_OK;
+   if (one_thread_a_line(nlines, N, periodic != 0)) {
+      block_tridag5_thread_kernel<<<blocks(nlines), kThreads, 0, (cudaStream_t)stream>>>(nlines, N, periodic, A, B, C, F);
+      return launched("block_tridag5");
+   }
    const unsigned nb = (unsigned)((nlines - 1) / kLinesPerWarp + 1);
    if (periodic) block_tridag5_kernel<true><<<nb, 32, 0, (cudaStream_t)stream>>>(nlines, N, A, B, C, F);
    else block_tridag5_kernel<false><<<nb, 32, 0, (cudaStream_t)stream>>>(nlines, N, A, B, C, F);

@@ -38,3 +38,24 @@ def test_degenerate_pivots(oracle_lib, native_lib, value, periodic):
     a, b, c, f = blocks5(6, 8, 21)
     b[2, 0, 0, 0] = value
     _check(oracle_lib, a, b, c, f, periodic)
+
+
+# the line counts from which a thread takes a whole line (csrc/strand5.cu one_thread_a_line)
+@pytest.mark.parametrize("periodic,n,first", [(False, 1, 6000), (False, 2, 60000), (True, 2, 130000), (True, 3, 130000),
+                                              (True, 4, 250000)])
+def test_many_lines_as_few_lines(native_lib, periodic, n, first):
+    """One more and one fewer line than the rule's count, against the same
+    lines in smaller calls: solution and scratch, bit for bit."""
+    import torch
+    from hamstr_oop_gb300 import native
+    few = 1000
+    host = [torch.from_numpy(x).cuda() for x in blocks5(few, n, 17 * n)]
+    want = [x.clone() for x in host]
+    native.block_tridag5(*want, periodic)
+    for nlines in (first - 1, first, first + 1):
+        got = [x.repeat((nlines // few + 1,) + (1,) * (x.dim() - 1))[:nlines].contiguous() for x in host]
+        native.block_tridag5(*got, periodic)
+        for g, w in zip(got, want):
+            whole = nlines // few * few
+            assert torch.equal(g[:whole].view(-1, few, *w.shape[1:]), w.expand(whole // few, *w.shape))
+            assert torch.equal(g[whole:], w[:nlines - whole])
