@@ -375,7 +375,10 @@ __device__ __forceinline__ bool factor_line_pair(const double* __restrict__ Ab, 
 {
    const int h = lane >> 4, e = lane & 15, k = e >> 2, j = e & 3, hb = 16 * h;
    const int Nmax = max(N, __shfl_xor_sync(kLaneMask, N, 16));
-   double A = 0.0, B = 0.0, C = 0.0, fv = 0.0;
+   // past its end a half has identity blocks, whose pivots' reciprocals stay on the
+   // integer pipes (a zero's would send the whole warp through the division)
+   const double one = k == j ? 1.0 : 0.0;
+   double A = 0.0, B = one, C = 0.0, fv = 0.0;
    if (N > 0) {
       A = Ab[e];
       B = Ab[16 + e];
@@ -386,7 +389,7 @@ __device__ __forceinline__ bool factor_line_pair(const double* __restrict__ Ab, 
    double X[4] = {0.0, 0.0, 0.0, 0.0};   // F: the previous row's solution
    bool bad = false;   // a live row's reciprocal pivot is not finite
    for (int i = 0; i < Nmax; i++) {
-      double An = 0.0, Bn = 0.0, Cn = 0.0, fvn = 0.0;
+      double An = 0.0, Bn = one, Cn = 0.0, fvn = 0.0;
       if (i + 1 < N) {
          const size_t o = stride * (size_t)(i + 1);
          An = Ab[o + e];
@@ -613,7 +616,9 @@ __device__ __forceinline__ bool factor_line_quad(const double* __restrict__ blk,
    bool bad = false;                      // a live row's reciprocal pivot is not finite
    for (int i = 0; i < Nmax; i++) {
       const bool live = i < N;
-      double A[4] = {0.0, 0.0, 0.0, 0.0}, w[4] = {0.0, 0.0, 0.0, 0.0}, C[4] = {0.0, 0.0, 0.0, 0.0};
+      double A[4] = {0.0, 0.0, 0.0, 0.0}, C[4] = {0.0, 0.0, 0.0, 0.0};
+      // (identity blocks past a line's end, as in factor_line_pair)
+      double w[4] = {r == 0 ? 1.0 : 0.0, r == 1 ? 1.0 : 0.0, r == 2 ? 1.0 : 0.0, r == 3 ? 1.0 : 0.0};
       double* rec = fac + (size_t)kFacRec * i;
       if (live) {
          const double* b = blk + stride * (size_t)i;
