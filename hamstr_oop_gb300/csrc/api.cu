@@ -288,6 +288,7 @@ struct hamstr_gpu {
          if (st != HAMSTR_GPU_ERR_NOMEM) return st;
          cudaGetLastError();
          d.mx_fused = 1;
+         d.mx_chunk_chains = mx_chunk ? mx_factor_chunk_capacity(d.mx_block, true) : 0;
       }
       CK(cudaMemsetAsync(d.ff32, 0, 32 * (size_t)d.nSlot * sizeof(float), stream));
       CK(cudaMemsetAsync(d.dq32, 0, 4 * nc * sizeof(float), stream));
@@ -398,7 +399,7 @@ struct hamstr_gpu {
       d.adi_fwpb = adi_fwpb;
       d.mx_block = mx_block;
       mx_chunk = chunk;
-      d.mx_chunk_chains = chunk ? mx_solve_chunk_capacity(mx_block) : 0;
+      d.mx_chunk_chains = chunk ? mx_factor_chunk_capacity(mx_block, mx_fused != 0) : 0;
       invalidate();
       return HAMSTR_GPU_OK;
    }
@@ -725,7 +726,7 @@ int hamstr::create_gpu(const hamstr_gpu_params* p, int nCell, int nFace, const i
       // one warp a block reaches the most SMs (eight steps of 512 x 128 3.59 ms, 3.65
       // with two; with the assembly inside batches are within 1% either way)
       d.mx_block = d.mx_fused ? 64 : 32;
-      d.mx_chunk_chains = mx_solve_chunk_capacity(d.mx_block);
+      d.mx_chunk_chains = mx_factor_chunk_capacity(d.mx_block, d.mx_fused != 0);
       d.sp_on = 1;   // long periodic chains of the FP32 form by segments (2: long open ones too)
       d.face_soft = 1;
       d.piv_soft = 1;   // sd::rcp: shorter latency than the hardware sequence, and off the FP64 pipe

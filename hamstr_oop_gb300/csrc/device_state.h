@@ -252,8 +252,8 @@ void launch_mx_init(const DeviceState& d, cudaStream_t st);
 void launch_mx_assemble(const DeviceState& d, cudaStream_t st);   // no-op when d.mx_fused
 void launch_mx_factor(const DeviceState& d, cudaStream_t st);
 void launch_mx_solve(const DeviceState& d, int first, int count, cudaStream_t st);
-// chains the FP32 solve holds resident at once with `block` threads per block (0 on error)
-int mx_solve_chunk_capacity(int block);
+// chains the FP32 factorisation holds resident at once with `block` threads per block (0 on error)
+int mx_factor_chunk_capacity(int block, bool fused);
 void launch_mx_dq_update(const DeviceState& d, cudaStream_t st);
 // allows the FP32 line kernels their staging shared memory (once per
 // device, before the first launch); nonzero on failure

@@ -1634,14 +1634,16 @@ void launch_mx_solve(const DeviceState& d, int first, int count, cudaStream_t st
    mx_solve_kernel<<<(count + tb - 1) / tb, tb, mx_solve_ring_bytes(tb), st>>>(d, first, count);
 }
 
-int mx_solve_chunk_capacity(int block)
+int mx_factor_chunk_capacity(int block, bool fused)
 {
    int dev = 0, sms = 0, per_sm = 0;
-   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+   if (mx_configure() || cudaGetDevice(&dev) != cudaSuccess) return 0;   // (the query refuses shared memory not allowed yet)
    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mx_solve_kernel, block, mx_solve_ring_bytes(block)) != cudaSuccess)
-      return 0;
-   return sms * per_sm * block;
+   const cudaError_t e = fused ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mx_factor_kernel<true, kElimChunk>,
+                                                                               block, mx_factor_stage_bytes(block))
+                               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mx_factor_kernel<false, kElimChunk>,
+                                                                               block, mx_factor_stage_bytes(block));
+   return e == cudaSuccess ? sms * per_sm * block : 0;
 }
 
 void launch_mx_spike_factor(const DeviceState& d, cudaStream_t st)
