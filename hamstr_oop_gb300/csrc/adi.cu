@@ -224,9 +224,8 @@ __device__ __forceinline__ void follow_chain_team(const DeviceState& d, int ich,
    const int N = d.chain_nrows[ich], row0 = d.chain_row0[ich];
    const bool per = d.chain_periodic[ich] != 0;
    gather_rhs(d, row0, N, lane);
-   follow_line_team<true>(d.blk + 48 * (size_t)row0, 48, d.fac + (size_t)kFacRec * row0,
-                          per ? d.facN + 16 * d.chain_facN[ich] : nullptr, N, per, d.fsc + 4 * (size_t)row0, lane, ts,
-                          ok);
+   follow_line_team(d.blk + 48 * (size_t)row0, 48, d.fac + (size_t)kFacRec * row0,
+                    per ? d.facN + 16 * d.chain_facN[ich] : nullptr, N, per, d.fsc + 4 * (size_t)row0, lane, ts, ok);
    scatter_solution(d, row0, N, lane);
 }
 

@@ -500,8 +500,9 @@ namespace {
 // enough to hide them.  A step, own / inside: 512 x 128 0.45 / 0.57 ms, the same
 // mesh 30% split 0.43 / 0.54 ms, batches with 12,800 chains 2.01 / 2.21 ms, 25,600
 // 3.79 / 3.81, 51,200 7.40 / 6.95, 99,200 14.2 / 13.3.  Meshes whose
-// chains have fewer than 16 rows on average stay with their own (the 30% split).
-// Above 2^24 rows the blocks (192 bytes a row) are not kept.
+// chains have fewer than 16 rows on average stay with their own at any size, as
+// they always have (the 30% split).  The others keep no blocks (192 bytes a row)
+// above 2^24 rows.
 int default_mx_fused(const Plan& P)
 {
    return P.nRow >= 16ll * P.nChain && (P.nChain > (1 << 15) || P.nRow > (1 << 24)) ? 1 : 0;

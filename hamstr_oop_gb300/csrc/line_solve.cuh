@@ -44,11 +44,11 @@ constexpr unsigned kLaneMask = 0xffffffffu;
 // count); the follower waits until the rows it needs are there
 // (wait_rows: the count, then a block-scope fence) before it loads them
 // (ldf).
-// The factoring warp never waits, so every wait ends; the bound (well
-// above the longest legitimate wait, a periodic line's last-row
-// elimination) only guards against a broken schedule: a wait that gives up
-// returns false, the follower waits no more and the caller raises an error
-// word.
+// A warp that publishes so never waits itself, so every wait ends; the bound
+// (well above the longest legitimate wait) only guards against a broken
+// schedule: a wait that gives up returns false, the follower waits no more and
+// the caller raises an error word.  (The two warps of a team, below, also
+// wait for each other; there it says why those waits end.)
 constexpr long kFollowSpin = 1L << 23;
 
 __device__ __forceinline__ void publish_rows(int* prog, int n, int lane)
@@ -1105,8 +1105,11 @@ __device__ __forceinline__ void solve_line(const double* __restrict__ fac, const
 //     the same instructions with the stored LU; then the last row and the
 //     back substitution.
 // Row N-2 of a periodic line adds a(N-2) = -a a'(N-3) to c(N-2), so there the
-// factoring warp waits for the follower's fill column; everywhere else only
-// the follower waits.  Records as factor_line's, bit for bit, except that row
+// factoring warp waits for the follower's fill column, and before it stores an LU
+// row for the ring's slot to be read; everywhere else only the follower waits.
+// These waits end: row i's LU needs the slot of row i - kTeamRing, which the
+// follower empties once it has that row, and the fill of row N-2 needs the LU of
+// rows up to N-3, all stored before the factoring warp waits for it.  Records as factor_line's, bit for bit, except that row
 // N-1's fill column, which nothing reads, is not stored.
 // Measured (384 x 96 block_tridag4, both directions): see trisolve.cu.
 // The LU rows travel through a ring in shared memory whose words are their own
@@ -1274,11 +1277,10 @@ __device__ __forceinline__ bool factor_line_team(const double* __restrict__ Ab, 
    return bad || (h == 0 && k == j && nonfinite(w));
 }
 
-// The second warp of the team: the fill column (periodic) and, with F, the
-// solve of fs (N rows of 4, in place).  A row's a(i) comes from the input
+// The second warp of the team: the fill column (periodic) and the solve of fs
+// (N rows of 4, in place).  A row's a(i) comes from the input
 // blocks, so the fill of row N-2, which the factoring warp waits for, needs
 // nothing of that row's factorisation.
-template <bool F>
 __device__ __forceinline__ void follow_line_team(const double* __restrict__ Ab, size_t stride,
                                                  double* __restrict__ fac, const double* __restrict__ facN, int N,
                                                  bool per, double* __restrict__ fs, int lane,
@@ -1286,17 +1288,16 @@ __device__ __forceinline__ void follow_line_team(const double* __restrict__ Ab, 
 {
    const int h = lane >> 4, e = lane & 15, k = e >> 2, j = e & 3;
    double X[4] = {0.0, 0.0, 0.0, 0.0};   // the previous row's column j of a' (lanes 0-15) or solution
-   const int rows = F ? N : N - 1;       // the fill column ends with a(N-2)
-   double f = F ? fs[k] : 0.0;
+   double f = fs[k];
    double2 A0 = ld2(Ab + 4 * k), A1 = ld2(Ab + 4 * k + 2);
-   for (int i = 0; i < rows; i++) {
+   for (int i = 0; i < N; i++) {
       const double a[4] = {A0.x, A0.y, A1.x, A1.y};
       double fn = 0.0;
-      if (i + 1 < rows) {
+      if (i + 1 < N) {
          const double* an = Ab + stride * (size_t)(i + 1) + 4 * k;
          A0 = ld2(an);
          A1 = ld2(an + 2);
-         if (F) fn = fs[4 * (i + 1) + k];
+         fn = fs[4 * (i + 1) + k];
       }
       // a(i) = -a(i) a'(i-1), f(i) -= a(i) f(i-1)
       double x;
@@ -1311,7 +1312,6 @@ __device__ __forceinline__ void follow_line_team(const double* __restrict__ Ab, 
          __threadfence_block();   // the fill column's records, before the word the factoring warp waits for
          __syncwarp();
          if (h == 0) *(volatile unsigned long long*)&ts->fill[e] = (unsigned long long)__double_as_longlong(x);
-         if (!F) return;
       }
       double* rec = fac + (size_t)kFacRec * i;
       unsigned long long* slot = ts->lu[i % kTeamRing];
@@ -1322,10 +1322,9 @@ __device__ __forceinline__ void follow_line_team(const double* __restrict__ Ab, 
       if (h == 0) *(volatile unsigned long long*)&slot[e] = kTeamEmpty;
       x = lu_solve_lanes(lu, k, x, 16 * h + j, 4, X);
       if (per && h == 0 && i < N - 2) rec[48 + e] = x;
-      if (F && h && j == 0) fs[4 * i + k] = x;
+      if (h && j == 0) fs[4 * i + k] = x;
       f = fn;
    }
-   if (!F) return;
    double xl[4];
 #pragma unroll
    for (int m = 0; m < 4; m++) xl[m] = __shfl_sync(kLaneMask, X[m], 16);

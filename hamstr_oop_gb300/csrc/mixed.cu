@@ -227,6 +227,14 @@ __device__ __forceinline__ void luf_store(float* p, const LUf& u)
    for (int m = 0; m < 16; m += 4) *reinterpret_cast<float4*>(p + m) = make_float4(v[m], v[m + 1], v[m + 2], v[m + 3]);
 }
 
+__device__ __forceinline__ LUf luf_of(const float (&v)[16])
+{
+   LUf u;
+   u.p0 = v[0]; u.u01 = v[1]; u.u02 = v[2]; u.u03 = v[3]; u.l10 = v[4]; u.p1 = v[5]; u.u12 = v[6]; u.u13 = v[7];
+   u.l20 = v[8]; u.l21 = v[9]; u.p2 = v[10]; u.u23 = v[11]; u.l30 = v[12]; u.l31 = v[13]; u.l32 = v[14]; u.p3 = v[15];
+   return u;
+}
+
 __device__ __forceinline__ LUf luf_load(const float* p)
 {
    float v[16];
@@ -235,18 +243,7 @@ __device__ __forceinline__ LUf luf_load(const float* p)
       const float4 a = *reinterpret_cast<const float4*>(p + m);
       v[m] = a.x; v[m + 1] = a.y; v[m + 2] = a.z; v[m + 3] = a.w;
    }
-   LUf u;
-   u.p0 = v[0]; u.u01 = v[1]; u.u02 = v[2]; u.u03 = v[3]; u.l10 = v[4]; u.p1 = v[5]; u.u12 = v[6]; u.u13 = v[7];
-   u.l20 = v[8]; u.l21 = v[9]; u.p2 = v[10]; u.u23 = v[11]; u.l30 = v[12]; u.l31 = v[13]; u.l32 = v[14]; u.p3 = v[15];
-   return u;
-}
-
-__device__ __forceinline__ LUf luf_of(const float (&v)[16])
-{
-   LUf u;
-   u.p0 = v[0]; u.u01 = v[1]; u.u02 = v[2]; u.u03 = v[3]; u.l10 = v[4]; u.p1 = v[5]; u.u12 = v[6]; u.u13 = v[7];
-   u.l20 = v[8]; u.l21 = v[9]; u.p2 = v[10]; u.u23 = v[11]; u.l30 = v[12]; u.l31 = v[13]; u.l32 = v[14]; u.p3 = v[15];
-   return u;
+   return luf_of(v);
 }
 
 // the LU record of a tiled row
@@ -257,16 +254,6 @@ __device__ __forceinline__ void luf_store_t(float* p, const LUf& u)
    st16t(p, v);
 }
 
-__device__ __forceinline__ LUf luf_load_t(const float* p)
-{
-   float v[16];
-   ld16t(p, v);
-   LUf u;
-   u.p0 = v[0]; u.u01 = v[1]; u.u02 = v[2]; u.u03 = v[3]; u.l10 = v[4]; u.p1 = v[5]; u.u12 = v[6]; u.u13 = v[7];
-   u.l20 = v[8]; u.l21 = v[9]; u.p2 = v[10]; u.u23 = v[11]; u.l30 = v[12]; u.l31 = v[13]; u.l32 = v[14]; u.p3 = v[15];
-   return u;
-}
-
 __device__ __forceinline__ void ld16f(const float* p, float (&v)[16])
 {
 #pragma unroll
@@ -274,12 +261,6 @@ __device__ __forceinline__ void ld16f(const float* p, float (&v)[16])
       const float4 a = *reinterpret_cast<const float4*>(p + m);
       v[m] = a.x; v[m + 1] = a.y; v[m + 2] = a.z; v[m + 3] = a.w;
    }
-}
-
-__device__ __forceinline__ void st16f(float* p, const float (&v)[16])
-{
-#pragma unroll
-   for (int m = 0; m < 16; m += 4) *reinterpret_cast<float4*>(p + m) = make_float4(v[m], v[m + 1], v[m + 2], v[m + 3]);
 }
 
 // M <- LU^{-1} M, column by column

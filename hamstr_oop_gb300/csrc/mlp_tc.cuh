@@ -157,13 +157,13 @@ inline PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
    return fn;
 }
 
-// rows x k BF16 matrix (k contiguous, rows ld apart: 0 for k), box of box_rows x 64
-inline bool make_map(CUtensorMap* map, const void* base, int rows, int k, int box_rows, int ld = 0)
+// rows x k BF16 matrix (k contiguous), box of box_rows x 64
+inline bool make_map(CUtensorMap* map, const void* base, int rows, int k, int box_rows)
 {
    auto fn = encode_fn();
    if (!fn) return false;
    cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
-   cuuint64_t strides[1] = {(cuuint64_t)(ld ? ld : k) * 2};
+   cuuint64_t strides[1] = {(cuuint64_t)k * 2};
    cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};   // BK <= k
    cuuint32_t estr[2] = {1, 1};
    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,

@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(64) block_tridag_kernel(int N, int periodic, c
    if (threadIdx.x < 32)
       factor_line_team(A + line * nb, B + line * nb, C + line * nb, 16, N, per, fac, facN, lane, &ts, &ok);
    else
-      follow_line_team<true>(A + line * nb, 16, fac, facN, N, per, F + line * (size_t)N * 4, lane, &ts, &ok);
+      follow_line_team(A + line * nb, 16, fac, facN, N, per, F + line * (size_t)N * 4, lane, &ts, &ok);
    // a wait that gave up (never expected, line_solve.cuh) leaves no plausible solution behind
    if (__syncthreads_or(!ok))
       for (int i = threadIdx.x; i < 4 * N; i += 64) F[line * (size_t)N * 4 + i] = __longlong_as_double(-1);
