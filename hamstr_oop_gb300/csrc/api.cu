@@ -511,11 +511,15 @@ int default_mx_fused(const Plan& P)
 // How the FP64 line kernels pack open chains before any tuning.
 //   lanes    16 (two chains to a warp) is the shorter recurrence by far: a row
 //            takes some 3,700 cycles of a pair's factorisation and 16,800 of a
-//            group of eight's (4 lanes each).  Only where pairs would queue
-//            several deep on every SM sub-partition does the groups' solve pay:
-//            31 conditions in a batch (754 rows of open chains per pair slot,
-//            the longest 128) 4.0 against 5.7 ms, 8 conditions (202) 2.2 against
-//            2.3 the other way, with the factorisation 3.7 against 3.2.
+//            group of eight's (4 lanes each).  Where pairs queue on every SM
+//            sub-partition the groups' fewer instructions a row pay.  A step,
+//            pairs / groups, by the rows per pair slot over the longest chain's:
+//            0.8 (512 x 128 half split) 0.72 / 0.91 ms, 1.2 (two of 512 x 128 30%
+//            split) 1.48 / 1.84, 1.6 (30 of 64 x 16) 0.90 / 0.86, 1.7 (16 of 128 x 32)
+//            1.77 / 1.68, 1.7 (1024 x 128 half split) 1.24 / 1.26, 1.8 (three of 512 x
+//            128 30% split) 2.08 / 2.11, 2.3 (1024 x 256 40% split) 2.56 / 2.17, 2.9
+//            (1024 x 256 half split) 2.36 / 2.01, 4.2 (40 of 128 x 32) 3.34 / 3.18: from
+//            5/3 on.
 //   bundle   chains of up to 8 rows one per lane: the fewest FP64 instructions a
 //            row, but a bundle's rows run one after the other.  Factorisation
 //            and solves of a step, with / without: 33,327 chains 0.40 / 0.69 ms,
@@ -534,7 +538,7 @@ void default_line_packing(const Plan& P, int nsm, int* lanes, int* bundle)
    *bundle = open >= 24 * slots && P.nRow < 16 * (long long)P.nChain ? 8 : 0;
    for (int c = 0; c < P.nChain; c++)
       if (!P.chain_periodic[c] && P.chain_nrows[c] > *bundle) rows += P.chain_nrows[c];
-   *lanes = rows > 3 * 2 * slots * longest ? 4 : 16;
+   *lanes = 3 * rows > 5 * 2 * slots * longest ? 4 : 16;
 }
 
 }  // namespace
