@@ -534,14 +534,14 @@ FP64_WARP_INSTR_PER_S = 15.8e9
 # the per-sweep kernels) give the mean of their launches.
 NCU_PER_LAUNCH = {
     "naca0012_ogrid_512x128_split50_weno5_cfl20_msweep2": {
-        "recon5": {"dram_bytes": 155.0e6, "fp64_inst": 2898203},
-        "rhs_face": {"dram_bytes": 16.8e6, "fp64_inst": 2620380},
-        "adi_assemble": {"dram_bytes": 55.1e6, "fp64_inst": 873663},
-        "adi_factor": {"dram_bytes": 62.7e6, "fp64_inst": 2700985},   # with the first wave's first solve
-        "adi_solve": {"dram_bytes": 20.1e6, "fp64_inst": 300775},
-        "lin_recon5": {"dram_bytes": 209.2e6, "fp64_inst": 2554292},
-        "lin_face": {"dram_bytes": 55.2e6, "fp64_inst": 328832},
-        "lin_cell": {"dram_bytes": 15.6e6, "fp64_inst": 343608},
+        "recon5": {"dram_bytes": 156.7e6, "fp64_inst": 2210264},
+        "rhs_face": {"dram_bytes": 17.5e6, "fp64_inst": 2364235},
+        "adi_assemble": {"dram_bytes": 56.2e6, "fp64_inst": 653608},
+        "adi_factor": {"dram_bytes": 65.4e6, "fp64_inst": 2398875},   # with the first wave's first solve
+        "adi_solve": {"dram_bytes": 20.0e6, "fp64_inst": 300775},
+        "lin_recon5": {"dram_bytes": 211.6e6, "fp64_inst": 2374104},
+        "lin_face": {"dram_bytes": 55.4e6, "fp64_inst": 328832},
+        "lin_cell": {"dram_bytes": 15.7e6, "fp64_inst": 143650},
     },
 }
 

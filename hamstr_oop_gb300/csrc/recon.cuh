@@ -410,9 +410,9 @@ __device__ __forceinline__ Weno5Lin<T> weno5_lin_get(const T* __restrict__ in, s
 // expressions, formed the same way (b1 * 2 is exact).
 // Which multiplies of the linearisation run on the integer pipes with SD (the
 // divisions are there too; results are the same): the candidate stencils'
-// constants, the constant 3 of the weights' derivatives, the products with the
-// weights' common denominator, and in weno5_with_lin the smoothness sums and
-// the final weighting.  A multiply costs there about what it costs on the FP64
+// constants, the constants 3 and 6 of the weights and their derivatives, the
+// second weight, the products with the weights' common denominator, and in
+// weno5_with_lin the smoothness sums and the final weighting.  A multiply costs there about what it costs on the FP64
 // pipe, so the split that fills both wins; the rest (kLinSoftMul) stay on the
 // FP64 pipe.  Measured, 512 x 128 half split, the two lin_recon5 launches of a
 // step: these 315 us, none 366, the candidate and smoothness terms as well 317,
