@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(kThreads) block_tridag5_thread_kernel(int nlin
    double* a = av + line * nb;
    double* b = bv + line * nb;
    double* c = cv + line * nb;
-   double* f = fv + line * 5 * (size_t)N;
+   double* f = fv + (size_t)line * 5 * N;
    auto A = [&](int i, int k, int j) -> double& { return a[25 * (size_t)i + 5 * k + j]; };
    auto Bm = [&](int i, int k, int j) -> double& { return b[25 * (size_t)i + 5 * k + j]; };
    auto C = [&](int i, int k, int j) -> double& { return c[25 * (size_t)i + 5 * k + j]; };

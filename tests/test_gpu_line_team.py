@@ -112,6 +112,26 @@ def test_any_nan_may_stand_in_a_block(oracle_lib, native_lib, operand, periodic,
         assert np.array_equal(got[k], want, equal_nan=True), k
 
 
+def test_a_large_call_gets_what_the_pool_kept(native_lib):
+    """Scratch beyond the pool's share that fits only with what the pool kept
+    from a smaller call, which the driver takes back for it."""
+    import torch
+    from hamstr_oop_gb300 import native
+    need = 9000 * 2656 * 8
+    systems = [torch.from_numpy(np.tile(x, (9000 // 300,) + (1,) * (x.ndim - 1))).cuda() for x in _systems(2, 300, 33)]
+    small = [x[:2900].clone() for x in systems]
+    native.block_tridag4(*small, True)     # 59 MiB of scratch, which the pool keeps
+    torch.cuda.synchronize()
+    free = lambda: torch.cuda.mem_get_info()[0]
+    hog, room = [], need - (24 << 20)
+    while free() - room >= 16 << 20:           # (smaller pieces may take a larger segment)
+        hog.append(torch.empty(min(8 << 30, (free() - room) >> 21 << 21), dtype=torch.uint8, device="cuda"))
+    native.block_tridag4(*systems, True)
+    del hog
+    torch.cuda.empty_cache()
+    assert torch.equal(systems[3][:2900], small[3])
+
+
 def test_threads_and_streams_share_the_scratch_pool(native_lib):
     """Eight host threads on streams of their own, each with its own systems."""
     import threading
